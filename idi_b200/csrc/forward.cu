@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "idiwf_internal.cuh"
+#include "nodes.cuh"
 
 namespace idiwf {
 
@@ -58,7 +59,8 @@ struct SplitRecs {
     double4 *r64;
     float4 *rA;
     float *rC;
-    uint32_t *rmax2;  // per image of the launch: max |r|^2 (float bits, rounded up)
+    uint32_t *rmax2;  // per image of the launch: max |r|^2 (float bits, rounded up); then, for the node
+                      // plan, max |r . e| along each detector axis and max |a| (kMaxImagesPerLaunch each)
 };
 struct DoubleRecs {
     double4 *r64;
@@ -78,7 +80,7 @@ static inline SplitRecs split_recs(void *ws, int64_t nrec) {
     return r;
 }
 static inline size_t split_recs_bytes(int64_t nrec) {
-    return align256(nrec * 32) + align256(nrec * 16) + align256(nrec * 4) + align256(kMaxImagesPerLaunch * 4);
+    return align256(nrec * 32) + align256(nrec * 16) + align256(nrec * 4) + align256(kMaxImagesPerLaunch * 16);
 }
 static inline DoubleRecs double_recs(void *ws, int64_t nrec) {
     char *base = static_cast<char *>(ws) + kWsDataOffset;
@@ -95,13 +97,16 @@ static inline size_t double_recs_bytes(int64_t nrec) {
 // ---------------------------------------------------------------------------
 // prep kernels: caller layout (N,4) f64 [+ amplitudes] -> padded tile records
 // ---------------------------------------------------------------------------
-__global__ void prep_split_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
-                                  const void *__restrict__ amps, int amp_dtype, int w_mode,
-                                  double max_abs, SplitRecs rec, uint32_t *err) {
+__global__ void __launch_bounds__(256)
+    prep_split_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
+                      const void *__restrict__ amps, int amp_dtype, int w_mode, double max_abs, SplitRecs rec,
+                      WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, NodePlan *__restrict__ plan) {
     const int b = blockIdx.y;
     const ImageDesc d = bp.img[b];
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
+    uint32_t *err = &hdr->error;
     uint32_t r2max = 0;  // float bits; non-negative floats order like their bits
+    uint32_t e0max = 0, e1max = 0, amax = 0;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nrec;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = d.rec + j;
@@ -109,6 +114,12 @@ __global__ void prep_split_kernel(const __grid_constant__ BatchParams bp, const 
             const int64_t s = d.src + j;
             const double4 a = reinterpret_cast<const double4 *>(atoms)[s];
             r2max = max(r2max, __float_as_uint(__double2float_ru((a.x * a.x + a.y * a.y) + a.z * a.z)));
+            if (plan) {
+                e0max = max(e0max, __float_as_uint(__double2float_ru(
+                                       fabs(a.x * ng.e[0][0] + a.y * ng.e[0][1] + a.z * ng.e[0][2]))));
+                e1max = max(e1max, __float_as_uint(__double2float_ru(
+                                       fabs(a.x * ng.e[1][0] + a.y * ng.e[1][1] + a.z * ng.e[1][2]))));
+            }
             double psi = a.w * kInvTwoPi;
             psi = psi - rint(psi);
             // the DFMA chain of the kernel starts from this value: the magic
@@ -119,6 +130,7 @@ __global__ void prep_split_kernel(const __grid_constant__ BatchParams bp, const 
             float amp = 1.0f;
             if (amps) amp = amp_dtype == IDIWF_F32 ? static_cast<const float *>(amps)[s]
                                                   : (float)static_cast<const double *>(amps)[s];
+            amax = max(amax, __float_as_uint(fabsf(amp)));
             if (!(fabs(a.x) <= max_abs && fabs(a.y) <= max_abs && fabs(a.z) <= max_abs))
                 record_error(err, kErrRange);
             const double w = w_mode == 1 ? (a.x * a.x + a.y * a.y) + a.z * a.z
@@ -138,6 +150,22 @@ __global__ void prep_split_kernel(const __grid_constant__ BatchParams bp, const 
     // zeroes rmax2 before the launch)
     r2max = __reduce_max_sync(0xffffffffu, r2max);
     if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rec.rmax2[b], r2max);
+    if (!plan) return;
+    e0max = __reduce_max_sync(0xffffffffu, e0max);
+    e1max = __reduce_max_sync(0xffffffffu, e1max);
+    amax = __reduce_max_sync(0xffffffffu, amax);
+    if ((threadIdx.x & 31) == 0) {
+        if (e0max) atomicMax(&rec.rmax2[kMaxImagesPerLaunch + b], e0max);
+        if (e1max) atomicMax(&rec.rmax2[2 * kMaxImagesPerLaunch + b], e1max);
+        if (amax) atomicMax(&rec.rmax2[3 * kMaxImagesPerLaunch + b], amax);
+    }
+    // the block that finishes last plans the launch
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&hdr->ticket, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (s_last) plan_nodes(bp, g, ng, rec.rmax2, hdr, plan);
 }
 
 __global__ void prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
@@ -215,11 +243,13 @@ __device__ __forceinline__ void finish_pixel(const GeomParams &g, int p, double 
 // final per-pixel step.  partials: [ksplit][n_images][npix] double2.
 template <bool NF, bool SCALE>
 __global__ void fwd_finish_kernel(const GeomParams g, const double2 *__restrict__ partials, int ksplit,
-                                  int n_images, void *__restrict__ out, int out_kind) {
+                                  int n_images, void *__restrict__ out, int out_kind,
+                                  const NodePlan *__restrict__ plan) {
     const int npix = g.nx * g.ny;
     const int64_t total = (int64_t)n_images * npix;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
          t += (int64_t)gridDim.x * blockDim.x) {
+        if (plan && plan->img[t / npix].path == kPathNodes) continue;
         double re = 0.0, im = 0.0;
         for (int c = 0; c < ksplit; ++c) {
             const double2 v = partials[(int64_t)c * total + t];
@@ -597,7 +627,8 @@ template <int PPT, bool NF, bool SCALE, bool SECOND, bool CHUNKED, int PATH>
 __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) : 1))
     fwd_split_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, SplitRecs rec,
                      void *__restrict__ out, int out_kind, WsHeader *__restrict__ hdr,
-                     uint64_t *__restrict__ cta_ns, double2 *__restrict__ partials) {
+                     uint64_t *__restrict__ cta_ns, double2 *__restrict__ partials,
+                     const NodePlan *__restrict__ plan) {
     static_assert(PPT % 2 == 0, "pixels are processed in f32x2 pairs");
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar[2];
@@ -607,7 +638,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
     const int tid = threadIdx.x;
     bool mine = false;
     for (int i = tid; i < bp.n_images; i += blockDim.x) {
-        const int path = split_path(g, rec.rmax2[i], bp.groups != 0, false);
+        const int path = plan ? plan->img[i].path : split_path(g, rec.rmax2[i], bp.groups != 0, false);
         s_path[i] = (uint8_t)path;
         mine |= path == PATH;
         if (PATH == kPathPixel && path == kPathReject && blockIdx.x == 0) record_error(&hdr->error, kErrGeometry);
@@ -672,6 +703,280 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
         return;
     }
     if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+}
+
+// ---------------------------------------------------------------------------
+// band-limited evaluation: node sums, weights, interpolation
+// ---------------------------------------------------------------------------
+// Sine and cosine of pi x, |x| <= 0.52: least-maximum polynomials in x^2, fitted for
+// this range (residuals 5.6e-9 and 4e-10; 2.8e-8 rms in FP32), two values at a time.
+// On the FMA pipe they cost 5.5 instructions a pair, about what the MUFU pair and
+// its argument scaling hold the issue port for, at a fifth of the MUFU's error.
+__device__ __forceinline__ void sincospi2(float2 x, float2 &sn, float2 &cs) {
+    const float2 z = __fmul2_rn(x, x);
+    float2 p = __ffma2_rn(f2(0.07687149941921234f, 0.07687149941921234f), z, f2(-0.5978690981864929f, -0.5978690981864929f));
+    float2 q = __ffma2_rn(f2(-0.024310700595378876f, -0.024310700595378876f), z, f2(0.23489117622375488f, 0.23489117622375488f));
+    p = __ffma2_rn(p, z, f2(2.5500025749206543f, 2.5500025749206543f));
+    q = __ffma2_rn(q, z, f2(-1.3352038860321045f, -1.3352038860321045f));
+    p = __ffma2_rn(p, z, f2(-5.167705059051514f, -5.167705059051514f));
+    q = __ffma2_rn(q, z, f2(4.058708667755127f, 4.058708667755127f));
+    p = __ffma2_rn(p, z, f2(3.141592502593994f, 3.141592502593994f));
+    q = __ffma2_rn(q, z, f2(-4.934802055358887f, -4.934802055358887f));
+    sn = __fmul2_rn(p, x);
+    cs = __ffma2_rn(q, z, f2(1.0f, 1.0f));
+}
+
+// Node sums of the images [img0, img1) on kPathNodes, as the split kernel's
+// per-pixel path (FP64 phase per pair, second-order near field) at the nodes'
+// fractional pixel positions.
+//
+// Work is tiles of kNodeTile nodes x blocks of 64 emitters; the CTAs that fit (four
+// 128-thread CTAs per SM) each take an equal, contiguous share of it, so the shares
+// end together and a CTA sets up a tile's geometry once or twice in all.  The FP32
+// sums of 16 emitters are added to fixed-point totals (64-bit integers, the image's
+// power of two as the unit's inverse, below 2^-59 of the largest possible sum), which
+// go to the node accumulators by atomics: integer sums do not depend on how
+// the work was cut, so results stay the same from run to run and from batch to batch.
+//
+// A node sum stands for many pixels, so it is formed more exactly than the direct
+// kernels' pixels: polynomial sine and cosine, and short FP32 partials.
+constexpr int kNodeFold = 16;
+template <bool NF, bool SCALE, bool SECOND>
+__global__ void __launch_bounds__(kNodeThreads, 4)
+    node_sum_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, SplitRecs rec,
+                    const NodePlan *__restrict__ plan, unsigned long long *__restrict__ acc, int64_t entries,
+                    WsHeader *__restrict__ hdr, uint64_t *__restrict__ cta_ns, int img0, int img1) {
+    constexpr int PPT = kNodePPT, PH = PPT / 2;
+    constexpr uint32_t kStage = kNodeTE * kSplitRecBytes;
+    __shared__ __align__(128) unsigned char smem[2 * kStage];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int s_abort;
+    __shared__ long long s_w0[kMaxImagesPerLaunch];
+    const int tid = threadIdx.x;
+    const int64_t wbeg = plan->img[img0].w0, wend = img1 < bp.n_images ? plan->img[img1].w0 : plan->total;
+    if (wend == wbeg) return;
+    const uint64_t t_start = globaltimer_ns();
+    const int nimg = img1 - img0;
+    for (int i = tid; i < nimg; i += kNodeThreads) s_w0[i] = plan->img[img0 + i].w0;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        s_abort = 0;
+        mbar_fence_init();
+        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+    }
+    __syncthreads();
+    int64_t pos = wbeg + (wend - wbeg) * blockIdx.x / gridDim.x;
+    const int64_t end = wbeg + (wend - wbeg) * (blockIdx.x + 1) / gridDim.x;
+    uint32_t issued = 0, consumed = 0;
+    while (pos < end) {
+        int lo = 0, hi = nimg;  // last image with w0 <= pos (those without work share the next one's w0)
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_w0[mid] <= pos) lo = mid;
+            else hi = mid;
+        }
+        const int img = img0 + lo;
+        const NodeImage ni = plan->img[img];
+        const ImageDesc d = bp.img[img];
+        const int tile = (int)((pos - ni.w0) / ni.nblk), b0 = (int)((pos - ni.w0) % ni.nblk);
+        const int b1 = (int)min((int64_t)ni.nblk, b0 + (end - pos));
+        pos += b1 - b0;
+        const int nodes = ni.n0 * ni.n1;
+        const int len = (b1 - b0) * kNodeBlock, nt = (len + kNodeTE - 1) / kNodeTE;
+        auto issue = [&](int t) {
+            const uint32_t slot = issued & 1;
+            unsigned char *st = smem + slot * kStage;
+            const int cnt = min(kNodeTE, len - t * kNodeTE);  // a multiple of kNodeBlock
+            const int64_t r0 = d.rec + (int64_t)b0 * kNodeBlock + (int64_t)t * kNodeTE;
+            mbar_arrive_expect_tx(&bar[slot], cnt * kSplitRecBytes);
+            bulk_g2s(st, rec.r64 + r0, cnt * 32, &bar[slot]);
+            bulk_g2s(st + kNodeTE * 32, rec.rA + r0, cnt * 16, &bar[slot]);
+            bulk_g2s(st + kNodeTE * 48, rec.rC + r0, cnt * 4, &bar[slot]);
+            ++issued;
+        };
+        if (tid == 0)
+            for (int t = 0; t < 2 && t < nt; ++t) issue(t);
+
+        const int m0 = tile * kNodeTile + tid * PPT;
+        double nqx[PPT], nqy[PPT], nqz[PPT];
+        float2 cx[PH], cy[PH], cz[PH], hh[PH], iD[PH], iD2[PH];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            const int m = min(m0 + i, nodes - 1);
+            const int a = m / ni.n1, b = m - a * ni.n1;
+            const PixelDir q = pixel_dir(g, node_index(ni.n0, a, g.nx), node_index(ni.n1, b, g.ny));
+            nqx[i] = q.nqx;
+            nqy[i] = q.nqy;
+            nqz[i] = q.nqz;
+            // -h in half turns, pairs with the negated w
+            const float fx = (float)q.ux, fy = (float)q.uy, fz = (float)q.uz, fh = (float)(-g.kp * q.invD);
+            const float fi = (float)q.invD, fi2 = (float)(q.invD * q.invD);
+            if (i & 1) {
+                cx[i / 2].y = fx; cy[i / 2].y = fy; cz[i / 2].y = fz; hh[i / 2].y = fh; iD[i / 2].y = fi; iD2[i / 2].y = fi2;
+            } else {
+                cx[i / 2].x = fx; cy[i / 2].x = fy; cz[i / 2].x = fz; hh[i / 2].x = fh; iD[i / 2].x = fi; iD2[i / 2].x = fi2;
+            }
+        }
+        long long sre[PPT], sim[PPT];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) sre[i] = sim[i] = 0;
+
+        for (int t = 0; t < nt; ++t) {
+            const uint32_t slot = consumed & 1;
+            if (!mbar_wait_bounded(&bar[slot], (consumed >> 1) & 1)) {
+                record_error(&hdr->error, kErrTimeout);
+                s_abort = 1;
+            }
+            const unsigned char *st = smem + slot * kStage;
+            const double4 *s64 = reinterpret_cast<const double4 *>(st);
+            const float4 *sA = reinterpret_cast<const float4 *>(st + kNodeTE * 32);
+            const float *sC = reinterpret_cast<const float *>(st + kNodeTE * 48);
+            const int cnt = min(kNodeTE, len - t * kNodeTE);
+            for (int jb = 0; jb < cnt; jb += kNodeFold) {
+                float2 are[PH], aim[PH];
+#pragma unroll
+                for (int q = 0; q < PH; ++q) are[q] = aim[q] = f2(0.f, 0.f);
+#pragma unroll 4
+                for (int j = jb; j < jb + kNodeFold; ++j) {
+                    const double4 r = s64[j];
+                    const float4 A = sA[j];
+                    const float a1 = sC[j];
+                    const float2 a2 = f2(a1, a1);
+#pragma unroll
+                    for (int q = 0; q < PH; ++q) {
+                        uint32_t w[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int i = 2 * q + e;
+                            double tt = __fma_rn(nqx[i], r.x, r.w);
+                            tt = __fma_rn(nqy[i], r.y, tt);
+                            tt = __fma_rn(nqz[i], r.z, tt);
+                            w[e] = (uint32_t)__double2loint(tt);
+                        }
+                        // x = u - 1.5 in half turns from bits 30..8, plus the 8 bits below
+                        // (the last 2^-24 takes back the record's half-step rounding offset)
+                        const float2 u = f2(__uint_as_float(((w[0] >> 8) & 0x007FFFFFu) | 0x3F800000u),
+                                            __uint_as_float(((w[1] >> 8) & 0x007FFFFFu) | 0x3F800000u));
+                        const float2 v = f2(__uint_as_float((w[0] & 0xFFu) | 0x3F800000u),
+                                            __uint_as_float((w[1] & 0xFFu) | 0x3F800000u));
+                        constexpr float kLow = 0x1p-8f - 0x1p-24f;
+                        float2 x = __ffma2_rn(v, f2(kLow, kLow), __fadd2_rn(u, f2(-1.50390625f, -1.50390625f)));
+                        float2 amp = a2;
+                        if (NF) {
+                            float2 s = __fmul2_rn(cx[q], f2(A.x, A.x));
+                            s = __ffma2_rn(cy[q], f2(A.y, A.y), s);
+                            s = __ffma2_rn(cz[q], f2(A.z, A.z), s);
+                            const float2 w2 = __ffma2_rn(s, s, f2(A.w, A.w));  // s^2 - |r|^2
+                            x = __ffma2_rn(hh[q], w2, x);                      // h (|r|^2 - s^2)
+                            if (SCALE) amp = __fmul2_rn(a2, __ffma2_rn(s, iD2[q], iD[q]));
+                        } else if (SECOND) {
+                            x = __ffma2_rn(hh[q], f2(A.w, A.w), x);  // (-h)(-(x^2+y^2))
+                        }
+                        amp.x = __uint_as_float(__float_as_uint(amp.x) ^ (w[0] & 0x80000000u));
+                        amp.y = __uint_as_float(__float_as_uint(amp.y) ^ (w[1] & 0x80000000u));
+                        float2 sn, cs;
+                        sincospi2(x, sn, cs);
+                        are[q] = __ffma2_rn(amp, cs, are[q]);
+                        aim[q] = __ffma2_rn(amp, sn, aim[q]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < PH; ++q) {
+                    sre[2 * q] += __float2ll_rn(are[q].x * ni.scale);
+                    sre[2 * q + 1] += __float2ll_rn(are[q].y * ni.scale);
+                    sim[2 * q] += __float2ll_rn(aim[q].x * ni.scale);
+                    sim[2 * q + 1] += __float2ll_rn(aim[q].y * ni.scale);
+                }
+            }
+            ++consumed;
+            __syncthreads();
+            if (s_abort) {
+                // wait (bounded) for copies still in flight into this CTA's shared memory
+                if (tid == 0)
+                    while (consumed < issued) {
+                        mbar_wait_bounded(&bar[consumed & 1], (consumed >> 1) & 1);
+                        ++consumed;
+                    }
+                return;
+            }
+            if (tid == 0 && t + 2 < nt) issue(t + 2);
+        }
+        unsigned long long *dst = acc + (int64_t)(img - img0) * entries * 2;
+#pragma unroll
+        for (int i = 0; i < PPT; ++i)
+            if (m0 + i < nodes) {
+                atomicAdd(dst + 2 * (m0 + i), (unsigned long long)sre[i]);
+                atomicAdd(dst + 2 * (m0 + i) + 1, (unsigned long long)sim[i]);
+            }
+    }
+    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+}
+
+// Buffers of one group of images: node sums (fixed point, then FP64), interpolation
+// weights of both axes, and the intermediate W[j][a] = sum_b L_y[j][b] V[a][b]
+// (pixel columns x nodes along x).
+struct NodeBuffers {
+    double2 *v;         // [image of the group][entries]
+    int64_t entries;
+    double *lx, *ly;    // [image of the group][nx or ny][n0 or n1]
+    double2 *w;         // [image of the group][ny][n0]
+    int64_t lx_stride, ly_stride, w_stride;
+};
+
+// Node sums from fixed point to FP64, in place, and the interpolation weights.
+__global__ void __launch_bounds__(256) node_weights_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
+                                                           NodeBuffers nb, int img0) {
+    const NodeImage ni = plan->img[img0 + blockIdx.y];
+    if (ni.path != kPathNodes) return;
+    const int nodes = ni.n0 * ni.n1;
+    const double unit = 1.0 / (double)ni.scale;
+    double2 *v = nb.v + blockIdx.y * nb.entries;
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < nodes; m += gridDim.x * blockDim.x) {
+        const longlong2 x = reinterpret_cast<const longlong2 *>(v)[m];
+        v[m] = make_double2((double)x.x * unit, (double)x.y * unit);
+    }
+    const int lane = threadIdx.x & 31;
+    double *lx = nb.lx + blockIdx.y * nb.lx_stride, *ly = nb.ly + blockIdx.y * nb.ly_stride;
+    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nx + g.ny; row += gridDim.x * 8) {
+        if (row < g.nx) node_weights_row(lx, ni.n0, g.nx, row, lane);
+        else node_weights_row(ly, ni.n1, g.ny, row - g.nx, lane);
+    }
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 4) node_interp_y_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
+                                                                     NodeBuffers nb, int img0) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int img = img0 + blockIdx.y;
+    const NodeImage ni = plan->img[img];
+    if (ni.path != kPathNodes) return;
+    const double *L = nb.ly + blockIdx.y * nb.ly_stride;
+    const double2 *V = nb.v + blockIdx.y * nb.entries;
+    double2 *W = nb.w + blockIdx.y * nb.w_stride;
+    const int tm = (g.ny + kGemmM - 1) / kGemmM, tn = (ni.n0 + kGemmN - 1) / kGemmN;
+    for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
+        interp_tile(*reinterpret_cast<GemmSmem *>(smem), L, V, g.ny, ni.n0, ni.n1, t % tm * kGemmM, t / tm * kGemmN,
+                    [&](int j, int a, double re, double im) { W[(size_t)j * ni.n0 + a] = make_double2(re, im); });
+}
+
+template <bool NF, bool SCALE>
+__global__ void __launch_bounds__(kGemmThreads, 4) node_interp_x_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
+                                                                     NodeBuffers nb, int img0, void *__restrict__ out,
+                                                                     int out_kind) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int img = img0 + blockIdx.y;
+    const NodeImage ni = plan->img[img];
+    if (ni.path != kPathNodes) return;
+    const double *L = nb.lx + blockIdx.y * nb.lx_stride;
+    const double2 *W = nb.w + blockIdx.y * nb.w_stride;
+    const int64_t obase = (int64_t)img * g.nx * g.ny;
+    const int tm = (g.nx + kGemmM - 1) / kGemmM, tn = (g.ny + kGemmN - 1) / kGemmN;
+    for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
+        interp_tile(*reinterpret_cast<GemmSmem *>(smem), L, W, g.nx, g.ny, ni.n0, t % tm * kGemmM, t / tm * kGemmN,
+                    [&](int i, int j, double re, double im) {
+                        const int p = i * g.ny + j;
+                        finish_pixel<NF, SCALE>(g, p, re, im, out, out_kind, obase + p);
+                    });
 }
 
 // ---------------------------------------------------------------------------
@@ -891,6 +1196,37 @@ GeomParams make_geom(const idiwf_geom *g) {
     return p;
 }
 
+NodeGeom make_node_geom(const GeomParams &g) {
+    NodeGeom n;
+    std::memset(&n, 0, sizeof(n));
+    const double *M = g.rot;
+    const double c[3][3] = {{M[0], M[3], M[6]}, {M[1], M[4], M[7]}, {M[2], M[5], M[8]}};
+    const auto dot = [](const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
+    const int size[2] = {g.nx, g.ny};
+    const double off[2] = {g.offx, g.offy};
+    double len[2], far[2];  // length of a unit step along each axis; largest |pixel coordinate|
+    for (int a = 0; a < 2; ++a) {
+        len[a] = std::sqrt(dot(c[a], c[a]));
+        for (int i = 0; i < 3; ++i) n.e[a][i] = len[a] > 0 ? c[a][i] / len[a] : 0.0;
+        far[a] = std::max(std::fabs((0.0 - size[a] * 0.5) * g.pixelsize + off[a]),
+                          std::fabs((size[a] - 1 - size[a] * 0.5) * g.pixelsize + off[a]));
+    }
+    if (!(g.dmin > 0) || !std::isfinite(g.dmin)) return n;
+    n.ok = 1;
+    n.inv_d = 1.0 / g.dmin;
+    for (int a = 0; a < 2; ++a) {
+        const double half = 0.5 * (size[a] - 1) * std::fabs(g.pixelsize) * len[a];
+        n.phi[a] = g.k * half / g.dmin;
+        n.t[a] = half / g.dmin;
+        // |d . e| over the detector, over a lower bound of |d|
+        const double de = far[a] * len[a] + far[1 - a] * std::fabs(dot(c[1 - a], n.e[a])) +
+                          std::fabs(g.detz * dot(c[2], n.e[a]));
+        n.s[a] = std::min(1.0, de / g.dmin);
+        if (!(n.t[a] <= kNodeMaxT)) n.ok = 0;
+    }
+    return n;
+}
+
 static idiwf_status validate_geom(const idiwf_geom *g) {
     if (!g) return set_error(IDIWF_ERR_INVALID_ARGUMENT, "geom is NULL");
     if (g->nx <= 0 || g->ny <= 0)
@@ -1009,10 +1345,61 @@ static size_t partials_bytes(const idiwf_geom *g, const idiwf_batch *b, int kspl
     return align256((size_t)ksplit * std::min(b->n_images, kMaxImagesPerLaunch) * g->nx * g->ny * 16);
 }
 
+// Whether a call may take nodes at all: split precision without
+// pixel_groups = -1, and an image with pairs enough.
+static bool nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
+    if (precision != IDIWF_SPLIT || !s.groups) return false;
+    int64_t nmax = 0;
+    for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
+    return (double)nmax * g->nx * g->ny >= kNodeMinPairs && make_node_geom(make_geom(g)).ok;
+}
+
+// Node part of the workspace: the plan, and buffers for groups of images that
+// together stay within kNodeGroupBytes.
+constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
+struct NodeLayout {
+    size_t v, lx, ly, w, total;  // offsets from the node region's start (the plan)
+    int group;
+    NodeBuffers at(char *base, const idiwf_geom *g) const {
+        NodeBuffers nb;
+        nb.v = reinterpret_cast<double2 *>(base + v);
+        nb.entries = node_entries((int64_t)g->nx * g->ny);
+        nb.lx = reinterpret_cast<double *>(base + lx);
+        nb.ly = reinterpret_cast<double *>(base + ly);
+        nb.w = reinterpret_cast<double2 *>(base + w);
+        nb.lx_stride = (int64_t)g->nx * node_cap(g->nx);
+        nb.ly_stride = (int64_t)g->ny * node_cap(g->ny);
+        nb.w_stride = (int64_t)g->ny * node_cap(g->nx);
+        return nb;
+    }
+};
+static NodeLayout node_layout(const idiwf_geom *g, int n_images) {
+    NodeLayout L;
+    const int imgs = std::min(n_images, kMaxImagesPerLaunch);
+    const size_t v = (size_t)node_entries((int64_t)g->nx * g->ny) * 16, lx = (size_t)g->nx * node_cap(g->nx) * 8,
+                 ly = (size_t)g->ny * node_cap(g->ny) * 8, w = (size_t)g->ny * node_cap(g->nx) * 16;
+    L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / (v + lx + ly + w)));
+    size_t o = align256(sizeof(NodePlan));
+    L.v = o;
+    o += align256(L.group * v);
+    L.lx = o;
+    o += align256(L.group * lx);
+    L.ly = o;
+    o += align256(L.group * ly);
+    L.w = o;
+    L.total = o + align256(L.group * w);
+    return L;
+}
+
+static size_t node_region_offset(const idiwf_geom *g, const idiwf_batch *b, int64_t nrec, int ksplit) {
+    return kWsDataOffset + split_recs_bytes(nrec) + partials_bytes(g, b, ksplit);
+}
+
 static size_t forward_ws_bytes(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
     const int64_t nrec = std::max<int64_t>(total_records(b, s.te), 1);
     if (precision != IDIWF_SPLIT) return kWsDataOffset + double_recs_bytes(nrec);
-    return kWsDataOffset + split_recs_bytes(nrec) + partials_bytes(g, b, choose_ksplit(g, b));
+    return node_region_offset(g, b, nrec, choose_ksplit(g, b)) +
+           (nodes_possible(g, b, precision, s) ? node_layout(g, b->n_images).total : 0);
 }
 
 // Dynamic shared memory of a forward kernel: two stages of emitter records,
@@ -1104,6 +1491,38 @@ static int resident_ctas(void *fn, int threads, size_t smem) {
     return occ;
 }
 
+// Node sums and interpolation of the images on kPathNodes (each kernel returns at
+// once where there is none).
+static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, const BatchParams &bp,
+                                 const SplitRecs &rec, const NodePlan *plan, const NodeLayout &nl, char *node_base,
+                                 WsHeader *hdr, uint64_t *cta_ns, void *out, int out_kind, cudaStream_t stream) {
+    const bool nf = geom->flags & IDIWF_NF, sc = geom->flags & IDIWF_SCALE, so = geom->flags & IDIWF_SECONDORDER;
+    NodeBuffers nb = nl.at(node_base, geom);
+    void *fs = nf ? (sc ? (void *)node_sum_kernel<true, true, false> : (void *)node_sum_kernel<true, false, false>)
+                  : (so ? (void *)node_sum_kernel<false, false, true> : (void *)node_sum_kernel<false, false, false>);
+    void *fx = nf ? (void *)node_interp_x_kernel<true, false>
+                  : (sc ? (void *)node_interp_x_kernel<false, true> : (void *)node_interp_x_kernel<false, false>);
+    idiwf_status st = ensure_smem((void *)node_interp_y_kernel, sizeof(GemmSmem));
+    if (st == IDIWF_OK) st = ensure_smem(fx, sizeof(GemmSmem));
+    if (st != IDIWF_OK) return st;
+    const int grid = std::min(sm_count() * resident_ctas(fs, kNodeThreads, 0), kMaxCtas);
+    const int ty = (g.ny + kGemmM - 1) / kGemmM * ((node_cap(g.nx) + kGemmN - 1) / kGemmN);
+    const int tx = (g.nx + kGemmM - 1) / kGemmM * ((g.ny + kGemmN - 1) / kGemmN);
+    for (int i0 = 0; i0 < bp.n_images; i0 += nl.group) {
+        int i1 = std::min(i0 + nl.group, bp.n_images);
+        const int n = i1 - i0;
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(nb.v, 0, (size_t)n * nb.entries * 16, stream));
+        void *as[] = {(void *)&bp, (void *)&g, (void *)&rec, &plan, &nb.v, &nb.entries, &hdr, &cta_ns, &i0, &i1};
+        IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), as, 0, stream));
+        node_weights_kernel<<<dim3((g.nx + g.ny + 15) / 16, n), 256, 0, stream>>>(g, plan, nb, i0);
+        node_interp_y_kernel<<<dim3(std::min(ty, 64), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
+        IDIWF_CUDA_CHECK(cudaGetLastError());
+        void *ax[] = {(void *)&g, &plan, &nb, &i0, &out, &out_kind};
+        IDIWF_CUDA_CHECK(cudaLaunchKernel(fx, dim3(std::min(tx, 4096), n), dim3(kGemmThreads), ax, sizeof(GemmSmem), stream));
+    }
+    return IDIWF_OK;
+}
+
 // Launch the forward for images [i0, i1) of the batch (records of the whole
 // batch are laid out by `rec_base`).
 static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, int precision,
@@ -1121,6 +1540,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
     if (precision != IDIWF_SPLIT) ksplit = 1;
     bp.ksplit = ksplit;
     bp.groups = precision == IDIWF_SPLIT && s.groups && geom->ny % kRun == 0;
+    bp.nodes = nodes_possible(geom, b, precision, s);
     bp.total_units = bp.n_images * bp.tiles_per_image * ksplit;
     int max_tiles = 0;
     std::vector<int> ord(bp.n_images);
@@ -1144,23 +1564,33 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                       (size_t)i0 * npix * (out_kind == IDIWF_OUT_C128 ? 16 : (out_kind == IDIWF_OUT_I32 ? 4 : 8));
 
     // prep
-    if (precision == IDIWF_SPLIT)
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
-    if (max_tiles > 0) {
-        dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), bp.n_images);
+    const NodeLayout nl = bp.nodes ? node_layout(geom, b->n_images) : NodeLayout{};
+    char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, nrec, ksplit) : 0);
+    NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
+    const NodeGeom ng = make_node_geom(g);
+    // work counters and the prep kernel's ticket (words 3 to 5; the error word, the
+    // CTA count and the pair count carry over from launch to launch of a call)
+    IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter, 0, sizeof(uint32_t), stream));
+    if (precision == IDIWF_SPLIT) {
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter2, 0, 3 * sizeof(uint32_t), stream));
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * 4 * kMaxImagesPerLaunch,
+                                         stream));
+    }
+    if (max_tiles > 0 || plan) {  // (the prep kernel also writes the plan)
+        dim3 pgrid((unsigned)std::max<int64_t>(std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), 1),
+                   bp.n_images);
         if (precision == IDIWF_SPLIT) {
             const int w_mode = (geom->flags & IDIWF_NF) ? 1 : ((geom->flags & IDIWF_SECONDORDER) ? 2 : 0);
             // emitter coordinates must keep |q.r| inside the magic binade
             const double max_abs = kMaxTurns / (3.0 * 2.0 * geom->k * kInvTwoPi);
             prep_split_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
-                                                         max_abs, split_recs(ws, nrec), &hdr->error);
+                                                         max_abs, split_recs(ws, nrec), hdr, g, ng, plan);
         } else {
             prep_double_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype,
                                                           double_recs(ws, nrec));
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter, 0, sizeof(uint32_t), stream));
 
     auto grid_for = [&](void *fn, size_t smem, int &grid) -> idiwf_status {
         idiwf_status st = ensure_smem(fn, smem);
@@ -1174,11 +1604,10 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
         double2 *partials = ksplit > 1 ? reinterpret_cast<double2 *>(static_cast<char *>(ws) + kWsDataOffset +
                                                                      split_recs_bytes(nrec))
                                        : nullptr;
-        void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns, &partials};
+        void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns, &partials, &plan};
         // the pixel-run kernel, the per-pixel kernel for the images beyond the
         // runs' bound, and in the near field the exact kernel (each returns at
         // once when it has no image)
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter2, 0, 2 * sizeof(uint32_t), stream));  // + work_counter3
         for (const int path : {kPathRuns, kPathPixel, kPathExact}) {
             if (path == kPathRuns && !bp.groups) continue;
             if (path == kPathExact && !(geom->flags & IDIWF_NF)) continue;
@@ -1195,15 +1624,16 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
             const bool nf = geom->flags & IDIWF_NF, sc = geom->flags & IDIWF_SCALE;
             if (nf)
                 fwd_finish_kernel<true, false><<<blocks, 256, 0, stream>>>(g, partials, ksplit, bp.n_images,
-                                                                           out_chunk, out_kind);
+                                                                           out_chunk, out_kind, plan);
             else if (sc)
                 fwd_finish_kernel<false, true><<<blocks, 256, 0, stream>>>(g, partials, ksplit, bp.n_images,
-                                                                           out_chunk, out_kind);
+                                                                           out_chunk, out_kind, plan);
             else
                 fwd_finish_kernel<false, false><<<blocks, 256, 0, stream>>>(g, partials, ksplit, bp.n_images,
-                                                                            out_chunk, out_kind);
+                                                                            out_chunk, out_kind, plan);
             IDIWF_CUDA_CHECK(cudaGetLastError());
         }
+        if (plan) return launch_nodes(geom, g, bp, rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     } else {
         DoubleRecs rec = double_recs(ws, nrec);
         void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns};
@@ -1233,6 +1663,7 @@ static idiwf_status forward_impl(const idiwf_geom *geom, const idiwf_batch *b, i
     // reset the work counter and the error word: errors reported by
     // idiwf_workspace_error() are those of the most recent call
     IDIWF_CUDA_CHECK(cudaMemsetAsync(ws, 0, 2 * sizeof(uint32_t), stream));
+    IDIWF_CUDA_CHECK(cudaMemsetAsync(&static_cast<WsHeader *>(ws)->pairs, 0, sizeof(unsigned long long), stream));
     const int ksplit = precision == IDIWF_SPLIT ? choose_ksplit(geom, b) : 1;
     for (int i0 = 0; i0 < b->n_images; i0 += kMaxImagesPerLaunch) {
         const int i1 = std::min(b->n_images, i0 + kMaxImagesPerLaunch);
@@ -1478,11 +1909,12 @@ extern "C" idiwf_status idiwf_forward_noalloc(const idiwf_geom *geom, const idiw
         const double max_abs = kMaxTurns / (3.0 * 2.0 * geom->k * kInvTwoPi);
         dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), bp.n_images);
         prep_split_kernel<<<pgrid, 256, 0, stream>>>(bp, batch->atoms, batch->amplitudes, batch->amp_dtype, w_mode,
-                                                     max_abs, rec, &hdr->error);
+                                                     max_abs, rec, hdr, g, NodeGeom{}, nullptr);
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
     double2 *no_partials = nullptr;  // bp.ksplit == 0: the kernels write the outputs themselves
-    void *args[] = {&bp, (void *)&g, &rec, &out, &out_kind, &hdr, &cta_ns, &no_partials};
+    NodePlan *no_plan = nullptr;         // every image takes its direct path
+    void *args[] = {&bp, (void *)&g, &rec, &out, &out_kind, &hdr, &cta_ns, &no_partials, &no_plan};
     // the pixel-run, per-pixel and (near field) exact kernels, each returning
     // at once without images; the persistent grid is clamped to the CTAs that
     // fit at once, as in idiwf_forward

@@ -42,8 +42,10 @@ struct WsHeader {
     uint32_t work_counter2; // second work queue (split forward: per-pixel kernel; time path: full sorts)
     uint32_t work_counter3; // third work queue (split forward: exact near-field kernel; time path:
                             // warm-started sorts given up)
-    uint32_t pad32;
-    uint64_t pad[29];
+    uint32_t ticket;        // finished blocks of the split forward's prep kernel
+    uint32_t pad32[2];
+    unsigned long long pairs;  // emitter-pixel (or emitter-node) pairs the split forward evaluates
+    uint64_t pad[27];
 };
 static_assert(sizeof(WsHeader) == 256, "workspace header is 256 bytes");
 constexpr int kMaxCtas = 4096;                       // per-CTA timing slots
@@ -137,6 +139,7 @@ struct BatchParams {
     int32_t total_units;      // n_images * tiles_per_image * ksplit
     int32_t ksplit;           // emitter chunks per (image, pixel tile); 0 or 1 = none
     int32_t groups;           // split forward: phase per pixel run + FP32 offsets where bounded
+    int32_t nodes;            // split forward: band-limited evaluation where it pays
     ImageDesc img[kMaxImagesPerLaunch];
     uint16_t order[kMaxImagesPerLaunch];  // images by descending emitter count
 };

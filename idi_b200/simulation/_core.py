@@ -310,6 +310,15 @@ def cta_times(device=None, role="main") -> np.ndarray:
     return np.frombuffer(buf, dtype=np.uint64, count=n.value).copy()
 
 
+def evaluated_pairs(device=None, role="main") -> int:
+    """Emitter-pixel pairs (emitter-node pairs for images evaluated on nodes) that the
+    last split-precision forward on ``device`` formed (synchronises; 0 where it had no
+    image large enough for nodes, which is then emitters x pixels)."""
+    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    ws = WORKSPACES.get(256, dev, role)
+    return int(ws[32:40].cpu().numpy().view(np.uint64)[0])
+
+
 def backward_workspace_error(device=None):
     """Raise if the last adjoint call recorded a device-side error (synchronises)."""
     workspace_error(device, "backward")

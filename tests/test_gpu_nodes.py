@@ -1,0 +1,117 @@
+"""Band-limited evaluation (nodes and interpolation) of the split forward: against
+the cancellation-free FP64 oracle at the edges of its tiles and of its dispatch."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+import oracle  # noqa: E402
+from helpers import K64, atoms, rng, sphere  # noqa: E402
+from idi_b200 import _native as nat  # noqa: E402
+from idi_b200.simulation import _core  # noqa: E402
+
+# 2-norm of the field error over that of the field.  Per pair, in radians (rms): the FP32
+# angle in half turns 5e-8, the polynomials 3e-8 each, FP32 directions and near-field
+# term 5e-8; FP32 sums over 16 emitters 8.5e-8; interpolation below 1e-8.  In quadrature
+# 1.2e-7; the bound leaves a factor 2 for the pixels' uneven weights.
+FIELD_2NORM = 2.4e-7
+
+
+def _err(E, ref):
+    return np.linalg.norm(E - ref) / np.linalg.norm(ref)
+
+
+def _forward(at, off, geom, amps=None, out=nat.OUT_C128, config=None):
+    t = torch.from_numpy(np.ascontiguousarray(at)).cuda()
+    a = None if amps is None else torch.from_numpy(np.ascontiguousarray(amps)).cuda()
+    E = _core.forward(t, off, geom, nat.SPLIT, out, amplitudes=a, config=config).cpu().numpy()
+    _core.workspace_error()
+    return E, _core.evaluated_pairs()
+
+
+@pytest.mark.parametrize("ndet,n,r,tilt", [
+    ([64, 64], 2048, 0.01, (0, 0)),        # the smallest images that take nodes; whole tiles
+    ([65, 131], 1029, 0.008, (0.1, -0.05)),  # one past a tile in both directions, ragged emitters
+    ([300, 77], 517, 0.012, (0, 0.2)),
+    ([1000, 24], 400, 0.006, (0, 0)),      # a strip: few nodes across
+])
+@pytest.mark.parametrize("settings", ["", "nf", "nf scale", "scale", "secondorder"])
+def test_forward_nodes_vs_oracle(ndet, n, r, tilt, settings):
+    g = rng(ndet[0] + n)
+    at = atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n))
+    amp = g.uniform(0.5, 1.5, n)
+    flags, _, _ = _core.parse_settings(settings)
+    off = (300.0, -200.0)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, tilt, off, flags)
+    oflags = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(oracle.geometry(ndet, 75.0, 1e5, K64, tilt, off), oflags, at, amp)
+    for dt in (np.float32, np.float64):
+        E, pairs = _forward(at, [0, n], geom, amp.astype(dt))
+        assert 0 < pairs < n * ndet[0] * ndet[1] / 4
+        # float32 amplitudes are the kernel's own precision: compare with theirs
+        assert _err(E[0], ref) < FIELD_2NORM + 4e-8, (dt, _err(E[0], ref))
+
+
+def test_mixed_batch_is_the_same_image_by_image():
+    """Images on nodes, direct ones, empty ones in one batch: each the same, bit for bit, as
+    alone (the fixed-point sums do not depend on how the work is cut), in fields and intensities."""
+    g = rng(4)
+    spec = [(3000, 0.01), (0, 0.01), (500, 0.4), (2500, 0.02), (700, 0.01), (20001, 0.004)]
+    imgs = [atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n)) for n, r in spec]
+    off = np.concatenate([[0], np.cumsum([n for n, _ in spec])])
+    geom = _core.make_geom([96, 101], 75.0, 1e5, K64, flags=nat.NF)
+    for out in (nat.OUT_C128, nat.OUT_I32):
+        E, pairs = _forward(np.concatenate(imgs), off, geom, out=out)
+        assert pairs < off[-1] * 96 * 101
+        for b, a in enumerate(imgs):
+            if len(a) == 0:
+                assert np.all(E[b] == 0)
+            elif spec[b] != (500, 0.4):  # (a small direct image alone is split over emitters)
+                assert np.array_equal(E[b], _forward(a, [0, len(a)], geom, out=out)[0][0]), b
+
+
+def test_more_images_than_a_group_of_node_buffers():
+    """Images beyond one group's buffers (512 MB) go through the same buffers again."""
+    g = rng(5)
+    n, nimg = 400, 60
+    pos = sphere(g, n, 0.01)
+    imgs = [atoms(pos, g.uniform(0, 2 * np.pi, n)) for _ in range(nimg)]
+    geom = _core.make_geom([600, 700], 75.0, 1e5, K64)
+    E, pairs = _forward(np.concatenate(imgs), np.arange(nimg + 1) * n, geom, out=nat.OUT_C64)
+    assert pairs < nimg * n * 600 * 700 / 4
+    for b in (0, 31, 59):
+        ref = oracle.wavefield(oracle.geometry([600, 700], 75.0, 1e5, K64), 0, imgs[b])
+        assert _err(E[b], ref) < FIELD_2NORM + 4e-8, b  # (complex64 output)
+
+
+def test_dispatch_limits():
+    """What leaves the node path: an amplitude without a fixed-point sum, a detector too
+    wide for its distance, too few pairs, pixel_groups = -1; the results are the direct kernels'."""
+    g = rng(6)
+    n = 3000
+    at = atoms(sphere(g, n, 0.01), g.uniform(0, 2 * np.pi, n))
+    geom = _core.make_geom([72, 64], 75.0, 1e5, K64, flags=nat.NF)
+    full = n * 72 * 64
+    E, pairs = _forward(at, [0, n], geom, np.ones(n))
+    assert 0 < pairs < full / 4
+    D, pairs = _forward(at, [0, n], geom, np.ones(n), config={"pixel_groups": -1})
+    assert _err(E[0], D[0]) < 1e-6  # the direct kernels' 2.7e-7 and this path's
+    amp = np.ones(n, np.float32)
+    amp[7] = np.inf
+    X, pairs = _forward(at, [0, n], geom, amp)
+    assert pairs == full and not np.isfinite(X).any()
+    # huge and tiny amplitudes scale through
+    for s in (1e30, 1e-30):
+        X, pairs = _forward(at, [0, n], geom, np.full(n, s, np.float32))
+        assert pairs < full / 4 and _err(X[0] / s, E[0]) < 1e-6
+    Z, _ = _forward(at, [0, n], geom, np.zeros(n))
+    assert np.all(Z == 0)
+    wide = _core.make_geom([72, 64], 75.0 * 30, 1e5, K64, flags=nat.NF)  # half-extent 0.8 of the distance
+    at2 = atoms(sphere(g, n, 0.0005), g.uniform(0, 2 * np.pi, n))
+    W, pairs = _forward(at2, [0, n], wide)
+    assert pairs in (0, full)
+    ref = oracle.wavefield(oracle.geometry([72, 64], 75.0 * 30, 1e5, K64), oracle.NF | oracle.ACCURATE, at2)
+    assert _err(W[0], ref) < 1e-6
