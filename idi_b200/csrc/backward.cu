@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "idiwf_internal.cuh"
+#include "nodes.cuh"
 
 namespace idiwf {
 
@@ -78,7 +79,35 @@ struct BwdLayout {
     int npix_pad;          // pixels rounded up to the chunk size
     int n_chunks, chunk_px;
     int64_t nrec;          // emitter records (images padded to the emitter block)
-    size_t off_p64, off_pf, off_pg, off_pd, off_rb64, off_rbf, off_px, off_rmax, off_erec64, off_erecf, off_part, total;
+    size_t off_p64, off_pf, off_pg, off_pd, off_rb64, off_rbf, off_px, off_rmax, off_erec64, off_erecf, off_part;
+    // node part (nodes: some image may take it): the plan, and per group of images the
+    // interpolation weights, the half-contracted pixel weights and the node records
+    int nodes, group;
+    size_t off_plan, off_lx, off_ly, off_t, off_n64, off_nf;
+    size_t lx_bytes, ly_bytes, t_bytes;  // per image of a group
+    int64_t entries;                     // node records per image
+    size_t total;
+};
+
+// Node sums of the adjoint: emitters per block, nodes per stage, largest chunk of nodes
+// whose sums stay in FP32.
+constexpr int kAdjEmitters = 4;
+constexpr int kAdjBlock = kNodeThreads * kAdjEmitters;
+constexpr int kAdjTile = 64;
+constexpr int kAdjChunk = 512;
+constexpr size_t kAdjGroupBytes = (size_t)512 << 20;
+
+struct AdjImage {
+    int32_t path, n0, n1;
+    int32_t cpx, nchunks;  // nodes per chunk (a multiple of kAdjTile), chunks
+    int32_t nblocks;       // emitter blocks of kAdjBlock
+    int32_t unit0;         // work units (blocks x chunks) of the images before it
+    int32_t pad;
+};
+struct AdjPlan {
+    int32_t total_units, n_direct, n_nodes, pad;
+    AdjImage img[kMaxImagesPerLaunch];
+    uint32_t counter[kMaxImagesPerLaunch];  // work queue of the group that starts at this image
 };
 
 // Pixels per work unit: 2048, 1024 or 512, whichever gives the shortest
@@ -113,7 +142,7 @@ static int bwd_chunk_px(const idiwf_geom *g, const idiwf_batch *b) {
 }
 
 static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
-    BwdLayout L;
+    BwdLayout L{};
     const int64_t npix = (int64_t)g->nx * g->ny;
     const int eb = kBwdThreads * kBwdMaxPE;
     L.chunk_px = bwd_chunk_px(g, b);
@@ -133,10 +162,27 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     L.off_rb64 = o; o += align256((size_t)L.npix_pad / kRun * 32);
     L.off_rbf = o; o += align256((size_t)L.npix_pad / kRun * 32);
     L.off_px = o;  o += align256((size_t)L.npix_pad * 16);
-    L.off_rmax = o; o += align256((size_t)kMaxImagesPerLaunch * 4);
+    L.off_rmax = o; o += align256((size_t)kMaxImagesPerLaunch * 4 * 3);
     L.off_erec64 = o; o += align256((size_t)L.nrec * 32);
     L.off_erecf = o;  o += align256((size_t)L.nrec * 16);
     L.off_part = o;   o += align256((size_t)L.n_chunks * L.nrec * kBwdNAcc * 4);
+    int64_t nmax = 0;
+    for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
+    L.nodes = (double)nmax * (double)npix >= kNodeMinPairs && make_node_geom(make_geom(g)).ok;
+    if (L.nodes) {
+        L.entries = node_entries(npix);
+        L.lx_bytes = (size_t)g->nx * node_cap(g->nx) * 8;
+        L.ly_bytes = (size_t)g->ny * node_cap(g->ny) * 8;
+        L.t_bytes = (size_t)g->ny * node_cap(g->nx) * 16;
+        const size_t per = L.lx_bytes + L.ly_bytes + L.t_bytes + (size_t)L.entries * 80;
+        L.group = (int)std::max<size_t>(1, std::min<size_t>(b->n_images, kAdjGroupBytes / per));
+        L.off_plan = o; o += align256(sizeof(AdjPlan));
+        L.off_lx = o;   o += align256(L.group * L.lx_bytes);
+        L.off_ly = o;   o += align256(L.group * L.ly_bytes);
+        L.off_t = o;    o += align256(L.group * L.t_bytes);
+        L.off_n64 = o;  o += align256((size_t)L.group * L.entries * 32);
+        L.off_nf = o;   o += align256((size_t)L.group * L.entries * 48);
+    }
     L.total = o;
     return L;
 }
@@ -174,7 +220,9 @@ __device__ __forceinline__ double nf_constant_turns(const GeomParams &g, double 
 // ---- pixel prep: geometry (image independent) ------------------------------
 __global__ void bwd_pixel_geom_kernel(const GeomParams g, int npix, int npix_pad, int runs,
                                       double4 *__restrict__ p64, float4 *__restrict__ pf, float4 *__restrict__ pd,
-                                      double4 *__restrict__ rb64, float4 *__restrict__ rbf, float4 *__restrict__ px) {
+                                      double4 *__restrict__ rb64, float4 *__restrict__ rbf, float4 *__restrict__ px,
+                                      const AdjPlan *__restrict__ plan) {
+    if (plan && plan->n_direct == 0) return;  // every image runs over nodes
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix_pad; p += gridDim.x * blockDim.x) {
         const int pc = min(p, npix - 1);
         const int ix = pc / g.ny, iy = pc - ix * g.ny;
@@ -223,15 +271,17 @@ __global__ void bwd_pixel_geom_kernel(const GeomParams g, int npix, int npix_pad
 // ---- pixel prep: G'_p = 2 g_p conj(E_p) exp(2 pi i C'_p) per image --------
 // C'_p is the near-field constant phase k (|d| - d_z) that the per-pair
 // phase leaves out; folding it into G keeps the per-pair FP64 chain at three
-// DFMA.
-template <bool NF>
+// DFMA.  Images on nodes keep G' in FP64, as (re, im) for the contraction, with the far
+// field's 1/|d| (SCALE) folded in as well.
+template <bool NF, bool SCALE>
 __global__ void bwd_pixel_g_kernel(const GeomParams g, const double2 *__restrict__ field,
                                    const double *__restrict__ gI, int npix, int npix_pad, int n_images,
-                                   float4 *__restrict__ pg) {
+                                   float4 *__restrict__ pg, const AdjPlan *__restrict__ plan) {
     const int64_t total = (int64_t)npix_pad * n_images;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int b = (int)(t / npix_pad);
         const int p = (int)(t - (int64_t)b * npix_pad);
+        const bool nodes = plan && plan->img[b].path == kPathNodes;
         float gr = 0.f, gi = 0.f;
         if (p < npix) {
             const double2 e = field[(int64_t)b * npix + p];
@@ -247,6 +297,16 @@ __global__ void bwd_pixel_g_kernel(const GeomParams g, const double2 *__restrict
                 i = r * sn + i * cs;
                 r = r2;
             }
+            if (nodes) {
+                if (!NF && SCALE) {
+                    const int ix = p / g.ny, iy = p - ix * g.ny;
+                    const double invD = pixel_dir(g, ix, iy).invD;
+                    r *= invD;
+                    i *= invD;
+                }
+                reinterpret_cast<double2 *>(pg)[t] = make_double2(r, i);
+                continue;
+            }
             gr = (float)r;
             gi = (float)i;
         }
@@ -254,11 +314,57 @@ __global__ void bwd_pixel_g_kernel(const GeomParams g, const double2 *__restrict
     }
 }
 
+// Plan of one call, by one block: every image's path, and for those on nodes their grid and
+// chunks.  The chunks make about 2400 units of a single image, as far as the partial-sum
+// buffer (max_chunks) reaches.
+__device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, const NodeGeom &ng, const uint32_t *ext,
+                                    int nodes, int max_chunks, AdjPlan *plan) {
+    __shared__ int s_units[kMaxImagesPerLaunch];
+    __threadfence();
+    int direct = 0;
+    for (int i = threadIdx.x; i < bp.n_images; i += blockDim.x) {
+        const uint32_t r2 = __ldcg(ext + i);
+        const int n = bp.img[i].n;
+        AdjImage ai;
+        ai.path = split_path(g, r2, bp.runs != 0, true);
+        ai.n0 = ai.n1 = ai.cpx = ai.nchunks = ai.nblocks = ai.unit0 = ai.pad = 0;
+        if (nodes && (ai.path == kPathRuns || ai.path == kPathPixel) &&
+            node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
+                      ai.n0, ai.n1) &&
+            nodes_pay(n, g.nx, g.ny, ai.n0, ai.n1, 1.05e12, 7.5e11)) {
+            ai.path = kPathNodes;
+            const int m = ai.n0 * ai.n1;
+            ai.nblocks = (n + kAdjBlock - 1) / kAdjBlock;
+            const int want = max(1, min((m + kAdjTile - 1) / kAdjTile, (2400 + ai.nblocks - 1) / ai.nblocks));
+            const int cpx = max(min((m + want - 1) / want, kAdjChunk), (m + max_chunks - 1) / max_chunks);
+            ai.cpx = (cpx + kAdjTile - 1) / kAdjTile * kAdjTile;
+            ai.nchunks = (m + ai.cpx - 1) / ai.cpx;
+        }
+        direct += n > 0 && ai.path != kPathNodes && ai.path != kPathReject;
+        s_units[i] = ai.nblocks * ai.nchunks;
+        plan->img[i] = ai;
+        plan->counter[i] = 0;
+    }
+    direct = __syncthreads_count(direct > 0);
+    if (threadIdx.x == 0) {
+        int u = 0;
+        for (int i = 0; i < bp.n_images; ++i) {
+            plan->img[i].unit0 = u;
+            u += s_units[i];
+        }
+        plan->total_units = u;
+        plan->n_direct = direct;
+    }
+}
+
 // ---- emitter prep: records padded per image to the emitter block ------------
-__global__ void bwd_emitter_prep_kernel(const __grid_constant__ BwdParams bp, const double *__restrict__ atoms,
-                                        double4 *__restrict__ e64, float4 *__restrict__ ef, int w_mode,
-                                        uint32_t *__restrict__ rmax2) {
+__global__ void __launch_bounds__(256)
+    bwd_emitter_prep_kernel(const __grid_constant__ BwdParams bp, const double *__restrict__ atoms,
+                            double4 *__restrict__ e64, float4 *__restrict__ ef, int w_mode,
+                            uint32_t *__restrict__ rmax2, const GeomParams g, const NodeGeom ng, int nodes,
+                            int max_chunks, AdjPlan *__restrict__ plan, WsHeader *__restrict__ hdr) {
     const int b = blockIdx.y;
+    uint32_t e0max = 0, e1max = 0;
     const BwdImage d = bp.img[b];
     const int64_t nrec = (int64_t)d.nblocks * bp.eb;
     uint32_t r2max = 0;  // float bits; non-negative floats order like their bits
@@ -267,6 +373,12 @@ __global__ void bwd_emitter_prep_kernel(const __grid_constant__ BwdParams bp, co
         if (j < d.n) {
             const double4 a = reinterpret_cast<const double4 *>(atoms)[d.src + j];
             r2max = max(r2max, __float_as_uint(__double2float_ru((a.x * a.x + a.y * a.y) + a.z * a.z)));
+            if (plan) {
+                e0max = max(e0max, __float_as_uint(__double2float_ru(
+                                       fabs(a.x * ng.e[0][0] + a.y * ng.e[0][1] + a.z * ng.e[0][2]))));
+                e1max = max(e1max, __float_as_uint(__double2float_ru(
+                                       fabs(a.x * ng.e[1][0] + a.y * ng.e[1][1] + a.z * ng.e[1][2]))));
+            }
             double psi = a.w * kInvTwoPi;
             psi = psi - rint(psi);
             // magic binade + 1/2 turn (angle = 2pi (u - 1.5)) + 2^-24 turn rounding bias
@@ -283,6 +395,20 @@ __global__ void bwd_emitter_prep_kernel(const __grid_constant__ BwdParams bp, co
     // |r|_max of the image for the pixel-run bound (zeroed by the caller)
     r2max = __reduce_max_sync(0xffffffffu, r2max);
     if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rmax2[b], r2max);
+    if (!plan) return;
+    e0max = __reduce_max_sync(0xffffffffu, e0max);
+    e1max = __reduce_max_sync(0xffffffffu, e1max);
+    if ((threadIdx.x & 31) == 0) {
+        if (e0max) atomicMax(&rmax2[kMaxImagesPerLaunch + b], e0max);
+        if (e1max) atomicMax(&rmax2[2 * kMaxImagesPerLaunch + b], e1max);
+    }
+    // the block that finishes last plans the call
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&hdr->ticket, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (s_last) plan_adjoint(bp, g, ng, rmax2, nodes, max_chunks, plan);
 }
 
 __device__ __forceinline__ float2 g2(float a, float b) { return make_float2(a, b); }
@@ -597,7 +723,7 @@ template <bool NF, bool SCALE, bool SECOND, int PE, bool EXACTK>
 __global__ void __launch_bounds__(kBwdThreads) bwd_split_kernel(const __grid_constant__ BwdParams bp,
                                                                 const BwdRecs R, float *__restrict__ part,
                                                                 int64_t nrec, WsHeader *__restrict__ hdr,
-                                                                GeomParams g) {
+                                                                GeomParams g, const AdjPlan *__restrict__ plan) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int s_unit, s_abort, s_img, s_ib;
@@ -605,7 +731,7 @@ __global__ void __launch_bounds__(kBwdThreads) bwd_split_kernel(const __grid_con
     const int tid = threadIdx.x;
     bool mine = false;
     for (int i = tid; i < bp.n_images; i += blockDim.x) {
-        const int path = split_path(g, R.rmax2[i], bp.runs != 0, true);
+        const int path = plan ? plan->img[i].path : split_path(g, R.rmax2[i], bp.runs != 0, true);
         s_path[i] = (uint8_t)path;
         // run base carries the near-field term: 1.5 k r^2 run_span / D <= kNfbPhaseTol (squared)
         const double r2 = (double)__uint_as_float(R.rmax2[i]);
@@ -688,6 +814,242 @@ __global__ void __launch_bounds__(kBwdThreads) bwd_split_kernel(const __grid_con
         }
 }
 
+// ---------------------------------------------------------------------------
+// adjoint over nodes
+// ---------------------------------------------------------------------------
+struct AdjBuffers {
+    double *lx, *ly;    // [image of the group][nx or ny][n0 or n1]
+    double2 *t;         // [image of the group][ny][n0]: pixel weights contracted along x
+    double4 *n64;       // [image of the group][entries] {-q' (turns), 0}
+    float4 *nf;         // [image of the group][entries][3] {d_hat, -h in half turns} {q, kappa} {G, 1/|d|, 1/|d|^2}
+    int64_t lx_stride, ly_stride, t_stride, entries;
+};
+
+__global__ void __launch_bounds__(256) adj_weights_kernel(const GeomParams g, const AdjPlan *__restrict__ plan,
+                                                          AdjBuffers nb, int img0) {
+    const AdjImage ai = plan->img[img0 + blockIdx.y];
+    if (ai.path != kPathNodes) return;
+    const int lane = threadIdx.x & 31;
+    double *lx = nb.lx + blockIdx.y * nb.lx_stride, *ly = nb.ly + blockIdx.y * nb.ly_stride;
+    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nx + g.ny; row += gridDim.x * 8) {
+        if (row < g.nx) node_weights_row(lx, ai.n0, g.nx, row, lane);
+        else node_weights_row(ly, ai.n1, g.ny, row - g.nx, lane);
+    }
+}
+
+// T[j][a] = sum_i L_x[i][a] G[i][j]
+__global__ void __launch_bounds__(kGemmThreads, 4) adj_contract_x_kernel(const GeomParams g,
+                                                                         const AdjPlan *__restrict__ plan, AdjBuffers nb,
+                                                                         const double2 *__restrict__ pg, int npix_pad,
+                                                                         int img0) {
+    __shared__ __align__(16) GemmTSmem sm;
+    const int img = img0 + blockIdx.y;
+    const AdjImage ai = plan->img[img];
+    if (ai.path != kPathNodes) return;
+    const double *L = nb.lx + blockIdx.y * nb.lx_stride;
+    const double2 *G = pg + (int64_t)img * npix_pad;
+    double2 *T = nb.t + blockIdx.y * nb.t_stride;
+    const int tm = (ai.n0 + kGemmTM - 1) / kGemmTM, tn = (g.ny + kGemmTN - 1) / kGemmTN;
+    for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
+        contract_tile(sm, L, G, ai.n0, g.ny, g.nx, t % tm * kGemmTM, t / tm * kGemmTN,
+                      [&](int a, int j, double re, double im) { T[(size_t)j * ai.n0 + a] = make_double2(re, im); });
+}
+
+// Node weights sum_j L_y[j][b] T[j][a], and the node records: geometry at the node's
+// fractional pixel position with its weight.
+__global__ void __launch_bounds__(kGemmThreads, 4) adj_contract_y_kernel(const GeomParams g,
+                                                                         const AdjPlan *__restrict__ plan,
+                                                                         AdjBuffers nb, int img0) {
+    __shared__ __align__(16) GemmTSmem sm;
+    const AdjImage ai = plan->img[img0 + blockIdx.y];
+    if (ai.path != kPathNodes) return;
+    const double *L = nb.ly + blockIdx.y * nb.ly_stride;
+    const double2 *T = nb.t + blockIdx.y * nb.t_stride;
+    double4 *n64 = nb.n64 + blockIdx.y * nb.entries;
+    float4 *nf = nb.nf + blockIdx.y * nb.entries * 3;
+    const int tm = (ai.n1 + kGemmTM - 1) / kGemmTM, tn = (ai.n0 + kGemmTN - 1) / kGemmTN;
+    for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
+        contract_tile(sm, L, T, ai.n1, ai.n0, g.ny, t % tm * kGemmTM, t / tm * kGemmTN,
+                      [&](int b, int a, double re, double im) {
+                          const int m = a * ai.n1 + b;
+                          const PixelDir q = pixel_dir(g, node_index(ai.n0, a, g.nx), node_index(ai.n1, b, g.ny));
+                          n64[m] = make_double4(q.nqx, q.nqy, q.nqz, 0.0);
+                          nf[3 * m] = make_float4((float)q.ux, (float)q.uy, (float)q.uz, (float)(-g.kp * q.invD));
+                          nf[3 * m + 1] = make_float4((float)(-kTwoPi * q.nqx), (float)(-kTwoPi * q.nqy),
+                                                      (float)(-kTwoPi * q.nqz), (float)(g.k * q.invD));
+                          nf[3 * m + 2] = make_float4((float)re, (float)im, (float)q.invD, (float)(q.invD * q.invD));
+                      });
+}
+
+// The adjoint sum over nodes: as bwd_unit's per-pair path (FP64 turns, second-order near
+// field, the six sums), with the forward node kernel's angles and polynomials.  A unit is
+// a block of 512 emitters (four per thread, in registers) x a chunk of nodes, staged 64 at
+// a time; its FP32 sums go to the same partial-sum buffer as the direct kernels'.
+template <bool NF, bool SCALE, bool SECOND>
+__global__ void __launch_bounds__(kNodeThreads, 4)
+    adj_node_kernel(const __grid_constant__ BwdParams bp, const AdjPlan *__restrict__ plan_c, AdjBuffers nb,
+                    const double4 *__restrict__ e64, const float4 *__restrict__ ef, float *__restrict__ part,
+                    int64_t nrec, WsHeader *__restrict__ hdr, AdjPlan *__restrict__ plan, int img0, int img1) {
+    constexpr int PE = kAdjEmitters, PH = PE / 2;
+    constexpr uint32_t kStage = kAdjTile * 80;
+    __shared__ __align__(128) unsigned char smem[2 * kStage];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int s_unit, s_abort;
+    __shared__ int s_u0[kMaxImagesPerLaunch];
+    const int tid = threadIdx.x;
+    const int ubeg = plan_c->img[img0].unit0, uend = img1 < bp.n_images ? plan_c->img[img1].unit0 : plan_c->total_units;
+    if (ubeg == uend) return;
+    const int nimg = img1 - img0;
+    for (int i = tid; i < nimg; i += kNodeThreads) s_u0[i] = plan_c->img[img0 + i].unit0;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        s_abort = 0;
+        mbar_fence_init();
+        s_unit = ubeg + (int)atomicAdd(&plan->counter[img0], 1u);
+    }
+    uint32_t issued = 0, consumed = 0;
+    for (;;) {
+        __syncthreads();
+        const int unit = s_unit;
+        if (unit >= uend) break;
+        int lo = 0, hi = nimg;  // last image with unit0 <= unit (those without units share the next one's)
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_u0[mid] <= unit) lo = mid;
+            else hi = mid;
+        }
+        const AdjImage ai = plan_c->img[img0 + lo];
+        const BwdImage d = bp.img[img0 + lo];
+        const int ib = (unit - ai.unit0) / ai.nchunks, chunk = (unit - ai.unit0) % ai.nchunks;
+        const int nodes = ai.n0 * ai.n1;
+        const int p0 = chunk * ai.cpx, len = min(ai.cpx, nodes - p0), nt = (len + kAdjTile - 1) / kAdjTile;
+        const double4 *n64 = nb.n64 + lo * nb.entries + p0;
+        const float4 *nf = nb.nf + (lo * nb.entries + p0) * 3;
+        auto issue = [&](int t) {
+            const uint32_t slot = issued & 1;
+            unsigned char *st = smem + slot * kStage;
+            const int cnt = min(kAdjTile, len - t * kAdjTile);
+            mbar_arrive_expect_tx(&bar[slot], cnt * 80);
+            bulk_g2s(st, n64 + t * kAdjTile, cnt * 32, &bar[slot]);
+            bulk_g2s(st + kAdjTile * 32, nf + t * kAdjTile * 3, cnt * 48, &bar[slot]);
+            ++issued;
+        };
+        int next = 0;
+        if (tid == 0) {
+            for (int t = 0; t < 2 && t < nt; ++t) issue(t);
+            next = ubeg + (int)atomicAdd(&plan->counter[img0], 1u);
+        }
+        // emitters tid, tid + 128, ... of the block; records beyond the image's own are
+        // read from its padding, or clamped to its last, and not stored
+        const int j0 = ib * kAdjBlock + tid;
+        double ex[PE], ey[PE], ez[PE], ep[PE];
+        float2 fx[PH], fy[PH], fz[PH], fw[PH];
+#pragma unroll
+        for (int e = 0; e < PE; ++e) {
+            const int64_t r = d.rec + min(j0 + e * kNodeThreads, d.n - 1);
+            const double4 a = e64[r];
+            ex[e] = a.x;
+            ey[e] = a.y;
+            ez[e] = a.z;
+            // the records carry +1/2 + 2^-24 turn; the half-turn angles want +1/4 + 2^-25
+            ep[e] = a.w - (0.25 + 0x1p-25);
+            const float4 f = ef[r];
+            if (e & 1) { fx[e / 2].y = f.x; fy[e / 2].y = f.y; fz[e / 2].y = f.z; fw[e / 2].y = f.w; }
+            else       { fx[e / 2].x = f.x; fy[e / 2].x = f.y; fz[e / 2].x = f.z; fw[e / 2].x = f.w; }
+        }
+        float2 ac[kBwdNAcc][PH];
+#pragma unroll
+        for (int a = 0; a < kBwdNAcc; ++a)
+#pragma unroll
+            for (int q = 0; q < PH; ++q) ac[a][q] = g2(0.f, 0.f);
+        for (int t = 0; t < nt; ++t) {
+            const uint32_t slot = consumed & 1;
+            if (!mbar_wait_bounded(&bar[slot], (consumed >> 1) & 1)) {
+                record_error(&hdr->error, kErrTimeout);
+                s_abort = 1;
+            }
+            const unsigned char *st = smem + slot * kStage;
+            const double4 *s64 = reinterpret_cast<const double4 *>(st);
+            const float4 *sf = reinterpret_cast<const float4 *>(st + kAdjTile * 32);
+            const int cnt = min(kAdjTile, len - t * kAdjTile);
+#pragma unroll 2
+            for (int j = 0; j < cnt; ++j) {
+                const double4 P = s64[j];
+                const float4 F0 = sf[3 * j], F1 = sf[3 * j + 1], F2 = sf[3 * j + 2];
+#pragma unroll
+                for (int q = 0; q < PH; ++q) {
+                    uint32_t w[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int i = 2 * q + e;
+                        double tt = __fma_rn(P.x, ex[i], ep[i]);
+                        tt = __fma_rn(P.y, ey[i], tt);
+                        tt = __fma_rn(P.z, ez[i], tt);
+                        w[e] = (uint32_t)__double2loint(tt);
+                    }
+                    float2 x = half_turns2(w[0], w[1]);
+                    float2 s = g2(0.f, 0.f);
+                    if (NF) {
+                        s = __fmul2_rn(g2(F0.x, F0.x), fx[q]);
+                        s = __ffma2_rn(g2(F0.y, F0.y), fy[q], s);
+                        s = __ffma2_rn(g2(F0.z, F0.z), fz[q], s);
+                        x = __ffma2_rn(g2(F0.w, F0.w), __ffma2_rn(s, s, fw[q]), x);  // h (|r|^2 - s^2)
+                    } else if (SECOND) {
+                        x = __ffma2_rn(g2(F0.w, F0.w), fw[q], x);
+                    }
+                    float2 sn, cs;
+                    sincospi2(x, sn, cs);
+                    sn = g2(flip_sign(sn.x, w[0]), flip_sign(sn.y, w[1]));
+                    cs = g2(flip_sign(cs.x, w[0]), flip_sign(cs.y, w[1]));
+                    // z = G' e^{i phi'}
+                    float2 zi = __ffma2_rn(g2(F2.y, F2.y), cs, __fmul2_rn(g2(F2.x, F2.x), sn));
+                    if (NF && SCALE) {
+                        const float2 wt = __ffma2_rn(s, g2(F2.w, F2.w), g2(F2.z, F2.z));
+                        const float2 zr = __ffma2_rn(g2(-F2.y, -F2.y), sn, __fmul2_rn(g2(F2.x, F2.x), cs));
+                        zi = __fmul2_rn(zi, wt);
+                        ac[0][q] = __ffma2_rn(zr, wt, ac[0][q]);
+                        // Re z grad w, grad w = d_hat / |d|^2
+                        const float2 c = __fmul2_rn(zr, g2(F2.w, F2.w));
+                        ac[2][q] = __ffma2_rn(c, g2(F0.x, F0.x), ac[2][q]);
+                        ac[3][q] = __ffma2_rn(c, g2(F0.y, F0.y), ac[3][q]);
+                        ac[4][q] = __ffma2_rn(c, g2(F0.z, F0.z), ac[4][q]);
+                    } else {
+                        ac[0][q] = __ffma2_rn(g2(F2.x, F2.x), cs, ac[0][q]);
+                        ac[0][q] = __ffma2_rn(g2(-F2.y, -F2.y), sn, ac[0][q]);
+                    }
+                    ac[1][q] = __fadd2_rn(ac[1][q], zi);
+                    ac[2][q] = __ffma2_rn(zi, g2(F1.x, F1.x), ac[2][q]);
+                    ac[3][q] = __ffma2_rn(zi, g2(F1.y, F1.y), ac[3][q]);
+                    ac[4][q] = __ffma2_rn(zi, g2(F1.z, F1.z), ac[4][q]);
+                    if (NF || SECOND) ac[5][q] = __ffma2_rn(zi, g2(F1.w, F1.w), ac[5][q]);
+                }
+            }
+            ++consumed;
+            __syncthreads();
+            if (s_abort) {
+                // wait (bounded) for copies still in flight into this CTA's shared memory
+                if (tid == 0)
+                    while (consumed < issued) {
+                        mbar_wait_bounded(&bar[consumed & 1], (consumed >> 1) & 1);
+                        ++consumed;
+                    }
+                return;
+            }
+            if (tid == 0 && t + 2 < nt) issue(t + 2);
+        }
+        float *dst = part + ((size_t)chunk * nrec + d.rec) * kBwdNAcc;
+#pragma unroll
+        for (int e = 0; e < PE; ++e) {
+            const int j = j0 + e * kNodeThreads;
+            if (j < d.n)
+#pragma unroll
+                for (int a = 0; a < kBwdNAcc; ++a) dst[(size_t)j * kBwdNAcc + a] = (e & 1) ? ac[a][e / 2].y : ac[a][e / 2].x;
+        }
+        if (tid == 0) s_unit = next;
+    }
+}
+
 // ---- chunk reduction + final gradients -------------------------------------
 // Per image path as in the adjoint kernels: the exact path's correction
 // acc[5] multiplies all of r, the paraxial one (x, y, 0); images outside the
@@ -699,7 +1061,8 @@ __global__ void __launch_bounds__(256) bwd_reduce_kernel(const __grid_constant__
                                                          const void *__restrict__ amps, int amp_dtype,
                                                          double *__restrict__ grad_atoms,
                                                          double *__restrict__ grad_amp, const GeomParams g,
-                                                         const uint32_t *__restrict__ rmax2) {
+                                                         const uint32_t *__restrict__ rmax2,
+                                                         const AdjPlan *__restrict__ plan) {
     // 32 emitters per block (one per lane); the 8 warps take every 8th chunk,
     // so the partial sums of a chunk are read as 32 consecutive records; the
     // 8 warp sums are added in warp order (a fixed order: the result does not
@@ -707,7 +1070,8 @@ __global__ void __launch_bounds__(256) bwd_reduce_kernel(const __grid_constant__
     __shared__ double red[8][32][kBwdNAcc + 1];
     const int b = blockIdx.y;
     const BwdImage d = bp.img[b];
-    const int path = split_path(g, rmax2[b], bp.runs != 0, true);
+    const int path = plan ? plan->img[b].path : split_path(g, rmax2[b], bp.runs != 0, true);
+    const int n_chunks = path == kPathNodes ? plan->img[b].nchunks : bp.n_chunks;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < d.n; j0 += (int64_t)gridDim.x * 32) {
         const int64_t j = j0 + lane;
@@ -716,7 +1080,7 @@ __global__ void __launch_bounds__(256) bwd_reduce_kernel(const __grid_constant__
         for (int a = 0; a < kBwdNAcc; ++a) acc[a] = 0.0;
         if (j < d.n && path != kPathReject) {
             const int64_t r = d.rec + j;
-            for (int c = w; c < bp.n_chunks; c += 8) {
+            for (int c = w; c < n_chunks; c += 8) {
                 const float *src = part + ((size_t)c * nrec + r) * kBwdNAcc;
 #pragma unroll
                 for (int a = 0; a < kBwdNAcc; ++a) acc[a] += (double)src[a];
@@ -859,35 +1223,40 @@ extern "C" idiwf_status idiwf_backward(const idiwf_geom *geom, const idiwf_batch
     for (int i = 0; i < batch->n_images; ++i) bp.unit_img[i] = ord[i];
     bp.total_units = total_blocks * L.n_chunks;
 
+    // work counters, the prep kernel's ticket and the error word
+    IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, 6 * sizeof(uint32_t), stream));
+    AdjPlan *plan = L.nodes ? reinterpret_cast<AdjPlan *>(ws + L.off_plan) : nullptr;
+    const int nodes = L.nodes && !(cfg && cfg->pixel_groups < 0);
     const int pthreads = 256;
+    {
+        const int w_mode = nf ? 1 : (so ? 2 : 0);
+        dim3 grid((unsigned)std::max(1, (max_blocks * eb + 255) / 256), batch->n_images);
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(rmax2, 0, sizeof(uint32_t) * 3 * kMaxImagesPerLaunch, stream));
+        bwd_emitter_prep_kernel<<<grid, 256, 0, stream>>>(bp, batch->atoms, e64, ef, w_mode, rmax2, g,
+                                                          make_node_geom(g), nodes, L.n_chunks, plan, hdr);
+        IDIWF_CUDA_CHECK(cudaGetLastError());
+    }
     bwd_pixel_geom_kernel<<<(L.npix_pad + pthreads - 1) / pthreads, pthreads, 0, stream>>>(
-        g, npix, L.npix_pad, bp.runs, p64, pf, pd, rb64, rbf, px);
+        g, npix, L.npix_pad, bp.runs, p64, pf, pd, rb64, rbf, px, plan);
     IDIWF_CUDA_CHECK(cudaGetLastError());
     {
         const int64_t tot = (int64_t)L.npix_pad * batch->n_images;
         const int blocks = (int)std::min<int64_t>((tot + pthreads - 1) / pthreads, 65535);
+        const double2 *f = static_cast<const double2 *>(field);
         if (nf)
-            bwd_pixel_g_kernel<true><<<blocks, pthreads, 0, stream>>>(g, static_cast<const double2 *>(field),
-                                                                      grad_intensity, npix, L.npix_pad,
-                                                                      batch->n_images, pg);
+            bwd_pixel_g_kernel<true, false><<<blocks, pthreads, 0, stream>>>(g, f, grad_intensity, npix, L.npix_pad,
+                                                                             batch->n_images, pg, plan);
+        else if (sc)
+            bwd_pixel_g_kernel<false, true><<<blocks, pthreads, 0, stream>>>(g, f, grad_intensity, npix, L.npix_pad,
+                                                                             batch->n_images, pg, plan);
         else
-            bwd_pixel_g_kernel<false><<<blocks, pthreads, 0, stream>>>(g, static_cast<const double2 *>(field),
-                                                                       grad_intensity, npix, L.npix_pad,
-                                                                       batch->n_images, pg);
+            bwd_pixel_g_kernel<false, false><<<blocks, pthreads, 0, stream>>>(g, f, grad_intensity, npix, L.npix_pad,
+                                                                              batch->n_images, pg, plan);
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
-    {
-        const int w_mode = nf ? 1 : (so ? 2 : 0);
-        dim3 grid((unsigned)std::max(1, (max_blocks * eb + 255) / 256), batch->n_images);
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(rmax2, 0, sizeof(uint32_t) * batch->n_images, stream));
-        bwd_emitter_prep_kernel<<<grid, 256, 0, stream>>>(bp, batch->atoms, e64, ef, w_mode, rmax2);
-        IDIWF_CUDA_CHECK(cudaGetLastError());
-    }
-    // work counters (paraxial and exact kernels) and the error word
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, 5 * sizeof(uint32_t), stream));
     int64_t nrec = L.nrec;
     BwdRecs R{e64, ef, p64, pf, pg, pd, rb64, rbf, px, rmax2};
-    void *args[] = {&bp, &R, &part, &nrec, &hdr, (void *)&g};
+    void *args[] = {&bp, &R, &part, &nrec, &hdr, (void *)&g, &plan};
     const size_t smem = 2 * (size_t)kStageMax;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -904,16 +1273,47 @@ extern "C" idiwf_status idiwf_backward(const idiwf_geom *geom, const idiwf_batch
         const int grid = (int)std::min<int64_t>(bp.total_units, (int64_t)sms * std::max(occ, 1));
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(kBwdThreads), args, smem, stream));
     }
+    if (nodes) {
+        AdjBuffers nb;
+        nb.lx = reinterpret_cast<double *>(ws + L.off_lx);
+        nb.ly = reinterpret_cast<double *>(ws + L.off_ly);
+        nb.t = reinterpret_cast<double2 *>(ws + L.off_t);
+        nb.n64 = reinterpret_cast<double4 *>(ws + L.off_n64);
+        nb.nf = reinterpret_cast<float4 *>(ws + L.off_nf);
+        nb.lx_stride = (int64_t)(L.lx_bytes / 8);
+        nb.ly_stride = (int64_t)(L.ly_bytes / 8);
+        nb.t_stride = (int64_t)(L.t_bytes / 16);
+        nb.entries = L.entries;
+        void *fn = nf ? (sc ? (void *)adj_node_kernel<true, true, false> : (void *)adj_node_kernel<true, false, false>)
+                      : (so ? (void *)adj_node_kernel<false, false, true> : (void *)adj_node_kernel<false, false, false>);
+        int occ = 1;
+        IDIWF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kNodeThreads, 0));
+        const int grid = sms * std::max(occ, 1);
+        const int tx = (node_cap(g.nx) + kGemmTM - 1) / kGemmTM * ((g.ny + kGemmTN - 1) / kGemmTN);
+        const int ty = (node_cap(g.ny) + kGemmTM - 1) / kGemmTM * ((node_cap(g.nx) + kGemmTN - 1) / kGemmTN);
+        const double2 *pg2 = reinterpret_cast<const double2 *>(pg);
+        for (int i0 = 0; i0 < bp.n_images; i0 += L.group) {
+            int i1 = std::min(i0 + L.group, bp.n_images);
+            const int n = i1 - i0;
+            adj_weights_kernel<<<dim3((g.nx + g.ny + 15) / 16, n), 256, 0, stream>>>(g, plan, nb, i0);
+            adj_contract_x_kernel<<<dim3(std::min(tx, 1024), n), kGemmThreads, 0, stream>>>(g, plan, nb, pg2,
+                                                                                           L.npix_pad, i0);
+            adj_contract_y_kernel<<<dim3(std::min(ty, 256), n), kGemmThreads, 0, stream>>>(g, plan, nb, i0);
+            IDIWF_CUDA_CHECK(cudaGetLastError());
+            void *an[] = {&bp, &plan, &nb, &e64, &ef, &part, &nrec, &hdr, &plan, &i0, &i1};
+            IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(kNodeThreads), an, 0, stream));
+        }
+    }
     {
         int64_t max_n = 1;
         for (int i = 0; i < batch->n_images; ++i) max_n = std::max<int64_t>(max_n, bp.img[i].n);
         dim3 rgrid((unsigned)std::min<int64_t>((max_n + 31) / 32, 65535), batch->n_images);
         if (nf || so)
             bwd_reduce_kernel<true><<<rgrid, 256, 0, stream>>>(bp, part, nrec, batch->atoms, batch->amplitudes,
-                                                                batch->amp_dtype, grad_atoms, grad_amp, g, rmax2);
+                                                                batch->amp_dtype, grad_atoms, grad_amp, g, rmax2, plan);
         else
             bwd_reduce_kernel<false><<<rgrid, 256, 0, stream>>>(bp, part, nrec, batch->atoms, batch->amplitudes,
-                                                                 batch->amp_dtype, grad_atoms, grad_amp, g, rmax2);
+                                                                 batch->amp_dtype, grad_atoms, grad_amp, g, rmax2, plan);
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
     return IDIWF_OK;

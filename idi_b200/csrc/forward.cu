@@ -708,24 +708,6 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
 // ---------------------------------------------------------------------------
 // band-limited evaluation: node sums, weights, interpolation
 // ---------------------------------------------------------------------------
-// Sine and cosine of pi x, |x| <= 0.52: least-maximum polynomials in x^2, fitted for
-// this range (residuals 5.6e-9 and 4e-10; 2.8e-8 rms in FP32), two values at a time.
-// On the FMA pipe they cost 5.5 instructions a pair, about what the MUFU pair and
-// its argument scaling hold the issue port for, at a fifth of the MUFU's error.
-__device__ __forceinline__ void sincospi2(float2 x, float2 &sn, float2 &cs) {
-    const float2 z = __fmul2_rn(x, x);
-    float2 p = __ffma2_rn(f2(0.07687149941921234f, 0.07687149941921234f), z, f2(-0.5978690981864929f, -0.5978690981864929f));
-    float2 q = __ffma2_rn(f2(-0.024310700595378876f, -0.024310700595378876f), z, f2(0.23489117622375488f, 0.23489117622375488f));
-    p = __ffma2_rn(p, z, f2(2.5500025749206543f, 2.5500025749206543f));
-    q = __ffma2_rn(q, z, f2(-1.3352038860321045f, -1.3352038860321045f));
-    p = __ffma2_rn(p, z, f2(-5.167705059051514f, -5.167705059051514f));
-    q = __ffma2_rn(q, z, f2(4.058708667755127f, 4.058708667755127f));
-    p = __ffma2_rn(p, z, f2(3.141592502593994f, 3.141592502593994f));
-    q = __ffma2_rn(q, z, f2(-4.934802055358887f, -4.934802055358887f));
-    sn = __fmul2_rn(p, x);
-    cs = __ffma2_rn(q, z, f2(1.0f, 1.0f));
-}
-
 // Node sums of the images [img0, img1) on kPathNodes, as the split kernel's
 // per-pixel path (FP64 phase per pair, second-order near field) at the nodes'
 // fractional pixel positions.
@@ -854,14 +836,7 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
                             tt = __fma_rn(nqz[i], r.z, tt);
                             w[e] = (uint32_t)__double2loint(tt);
                         }
-                        // x = u - 1.5 in half turns from bits 30..8, plus the 8 bits below
-                        // (the last 2^-24 takes back the record's half-step rounding offset)
-                        const float2 u = f2(__uint_as_float(((w[0] >> 8) & 0x007FFFFFu) | 0x3F800000u),
-                                            __uint_as_float(((w[1] >> 8) & 0x007FFFFFu) | 0x3F800000u));
-                        const float2 v = f2(__uint_as_float((w[0] & 0xFFu) | 0x3F800000u),
-                                            __uint_as_float((w[1] & 0xFFu) | 0x3F800000u));
-                        constexpr float kLow = 0x1p-8f - 0x1p-24f;
-                        float2 x = __ffma2_rn(v, f2(kLow, kLow), __fadd2_rn(u, f2(-1.50390625f, -1.50390625f)));
+                        float2 x = half_turns2(w[0], w[1]);
                         float2 amp = a2;
                         if (NF) {
                             float2 s = __fmul2_rn(cx[q], f2(A.x, A.x));
@@ -873,8 +848,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
                         } else if (SECOND) {
                             x = __ffma2_rn(hh[q], f2(A.w, A.w), x);  // (-h)(-(x^2+y^2))
                         }
-                        amp.x = __uint_as_float(__float_as_uint(amp.x) ^ (w[0] & 0x80000000u));
-                        amp.y = __uint_as_float(__float_as_uint(amp.y) ^ (w[1] & 0x80000000u));
+                        amp.x = flip_sign(amp.x, w[0]);
+                        amp.y = flip_sign(amp.y, w[1]);
                         float2 sn, cs;
                         sincospi2(x, sn, cs);
                         are[q] = __ffma2_rn(amp, cs, are[q]);

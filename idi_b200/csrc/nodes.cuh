@@ -131,15 +131,14 @@ constexpr double kNodeMinPairs = 8e6;
 
 // Whether an image of n emitters goes through its n0 x n1 grid: the grid fits
 // the buffers, and the pairs saved outweigh the interpolation.  The rates are
-// the kernels' measured ones (pixel runs, per-pixel pairs and node pairs per
-// second; FP64 multiply-adds per second of the interpolation); the choice depends on
+// the kernels' measured ones: direct pairs and node pairs per second, FP64
+// multiply-adds per second of the interpolation.  The choice depends on
 // the image and the geometry alone, as split_path's does.
-__device__ __forceinline__ bool nodes_pay(int n, int nx, int ny, int path, int n0, int n1) {
+__device__ __forceinline__ bool nodes_pay(int n, int nx, int ny, int n0, int n1, double direct_rate, double node_rate) {
     const double npix = (double)nx * ny, m = (double)n0 * n1, pairs = (double)n * npix;
     if (n0 > node_cap(nx) || n1 > node_cap(ny) || m > 0.25 * npix + 4096.0 || pairs < kNodeMinPairs) return false;
-    const double direct = pairs * (path == kPathRuns ? 1.0 / 1.8e12 : 1.0 / 1.5e12);
     const double mads = 2.0 * n0 * (npix + (double)n1 * ny);
-    return n * m * (1.0 / 1.2e12) + (mads + 100.0 * npix) * (1.0 / 1.2e13) < direct;
+    return n * m / node_rate + (mads + 100.0 * npix) * (1.0 / 1.2e13) < pairs / direct_rate;
 }
 
 // Plan of one launch, by one block: every image's path, grid, fixed-point scale and
@@ -164,7 +163,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
             amax < 0x7f800000u &&  // (an infinite or NaN amplitude has no fixed-point sum)
             node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
                       ni.n0, ni.n1) &&
-            nodes_pay(n, g.nx, g.ny, ni.path, ni.n0, ni.n1)) {
+            nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, ni.path == kPathRuns ? 1.8e12 : 1.5e12, 1.0e12)) {
             ni.path = kPathNodes;
             const int m = ni.n0 * ni.n1;
             ni.ntiles = (m + kNodeTile - 1) / kNodeTile;
@@ -189,6 +188,39 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         }
         plan->total = w;
     }
+}
+
+// Sine and cosine of pi x, |x| <= 0.52: least-maximum polynomials in x^2, fitted for
+// this range (residuals 5.6e-9 and 4e-10; 2.8e-8 rms in FP32), two values at a time.
+// On the FMA pipe they cost 5.5 instructions a pair, about what the MUFU pair and
+// its argument scaling hold the issue port for, at a fifth of the MUFU's error.
+__device__ __forceinline__ void sincospi2(float2 x, float2 &sn, float2 &cs) {
+    const float2 z = __fmul2_rn(x, x);
+    float2 p = __ffma2_rn(make_float2(0.07687149941921234f, 0.07687149941921234f), z, make_float2(-0.5978690981864929f, -0.5978690981864929f));
+    float2 q = __ffma2_rn(make_float2(-0.024310700595378876f, -0.024310700595378876f), z, make_float2(0.23489117622375488f, 0.23489117622375488f));
+    p = __ffma2_rn(p, z, make_float2(2.5500025749206543f, 2.5500025749206543f));
+    q = __ffma2_rn(q, z, make_float2(-1.3352038860321045f, -1.3352038860321045f));
+    p = __ffma2_rn(p, z, make_float2(-5.167705059051514f, -5.167705059051514f));
+    q = __ffma2_rn(q, z, make_float2(4.058708667755127f, 4.058708667755127f));
+    p = __ffma2_rn(p, z, make_float2(3.141592502593994f, 3.141592502593994f));
+    q = __ffma2_rn(q, z, make_float2(-4.934802055358887f, -4.934802055358887f));
+    sn = __fmul2_rn(p, x);
+    cs = __ffma2_rn(q, z, make_float2(1.0f, 1.0f));
+}
+
+// Half-turn angles of a pair of phases from the low words of their FP64 turns (the
+// magic binade, +1/4 + 2^-25 turn): bit 31 is the half turn's sign, x = u - 1.5 in half
+// turns comes from bits 30..8, plus the 8 bits below (the last 2^-24 takes back the
+// half-step rounding offset).
+__device__ __forceinline__ float2 half_turns2(uint32_t w0, uint32_t w1) {
+    constexpr float kLow = 0x1p-8f - 0x1p-24f;
+    const float2 u = make_float2(__uint_as_float(((w0 >> 8) & 0x007FFFFFu) | 0x3F800000u),
+                                 __uint_as_float(((w1 >> 8) & 0x007FFFFFu) | 0x3F800000u));
+    const float2 v = make_float2(__uint_as_float((w0 & 0xFFu) | 0x3F800000u), __uint_as_float((w1 & 0xFFu) | 0x3F800000u));
+    return __ffma2_rn(v, make_float2(kLow, kLow), __fadd2_rn(u, make_float2(-1.50390625f, -1.50390625f)));
+}
+__device__ __forceinline__ float flip_sign(float x, uint32_t w) {
+    return __uint_as_float(__float_as_uint(x) ^ (w & 0x80000000u));
 }
 
 // ---------------------------------------------------------------------------
@@ -295,7 +327,91 @@ __device__ __forceinline__ void interp_tile(GemmSmem &sm, const double *__restri
     __syncthreads();
 }
 
-#endif  // __CUDACC__
+// ---------------------------------------------------------------------------
+// the transpose: Y[m][n] = sum_k A[k][m] X[k][n], A real (K x M), X complex (K x N),
+// both FP64 with m and n contiguous
+// ---------------------------------------------------------------------------
+// The contraction runs over pixels and the result is small (nodes x pixel columns, then
+// nodes x nodes), so tiles are small too, 32 x 16 complex, and the four warps of a CTA
+// share each K block of 16 (one k step each); their sums are added in warp order.
+constexpr int kGemmTM = 32, kGemmTN = 16;
+constexpr int kGemmTLd = 36;
+union GemmTSmem {
+    struct {
+        double a[2][kGemmK * kGemmTLd];
+        double b[2][kGemmK * kGemmTLd];
+    };
+    double2 y[4][kGemmTM * (kGemmTN + 1)];
+};
 
+template <class Store>
+__device__ __forceinline__ void contract_tile(GemmTSmem &sm, const double *__restrict__ A, const double2 *__restrict__ X,
+                                              int M, int N, int K, int i0, int j0, const Store &store) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double acc[4][4][2];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    const int nk = (K + kGemmK - 1) / kGemmK;
+    auto issue = [&](int kb) {
+        const int s = kb & 1, k0 = kb * kGemmK;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {  // 16 rows x 32 doubles; M is even
+            const int c = tid + q * kGemmThreads, k = c >> 4, m = (c & 15) * 2;
+            const bool ok = k0 + k < K && i0 + m < M;
+            cp_async16(&sm.a[s][k * kGemmTLd + m], A + (ok ? (size_t)(k0 + k) * M + i0 + m : 0), ok);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {  // 16 rows x 16 complex
+            const int c = tid + q * kGemmThreads, k = c >> 4, n = c & 15;
+            const bool ok = k0 + k < K && j0 + n < N;
+            cp_async16(&sm.b[s][k * kGemmTLd + 2 * n], X + (ok ? (size_t)(k0 + k) * N + j0 + n : 0), ok);
+        }
+        cp_async_commit();
+    };
+    issue(0);
+    for (int kb = 0; kb < nk; ++kb) {
+        if (kb + 1 < nk) {
+            issue(kb + 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        const double *sa = sm.a[kb & 1] + (warp * 4 + (lane & 3)) * kGemmTLd + (lane >> 2);
+        const double *sb = sm.b[kb & 1] + (warp * 4 + (lane & 3)) * kGemmTLd + (lane >> 2);
+        double fa[4], fb[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) fa[t] = sa[t * 8];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) fb[t] = sb[t * 8];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) dmma884(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            sm.y[warp][(a * 8 + (lane >> 2)) * (kGemmTN + 1) + b * 4 + (lane & 3)] =
+                make_double2(acc[a][b][0], acc[a][b][1]);
+    __syncthreads();
+    for (int c = tid; c < kGemmTM * kGemmTN; c += kGemmThreads) {
+        const int m = c % kGemmTM, n = c / kGemmTM, at = m * (kGemmTN + 1) + n;
+        double2 v = sm.y[0][at];
+#pragma unroll
+        for (int w = 1; w < 4; ++w) {
+            v.x += sm.y[w][at].x;
+            v.y += sm.y[w][at].y;
+        }
+        if (i0 + m < M && j0 + n < N) store(i0 + m, j0 + n, v.x, v.y);
+    }
+    __syncthreads();
+}
+
+#endif  // __CUDACC__
 
 }  // namespace idiwf

@@ -115,3 +115,116 @@ def test_dispatch_limits():
     assert pairs in (0, full)
     ref = oracle.wavefield(oracle.geometry([72, 64], 75.0 * 30, 1e5, K64), oracle.NF | oracle.ACCURATE, at2)
     assert _err(W[0], ref) < 1e-6
+
+
+# 2-norm of the gradients' errors.  The adjoint pairs carry the forward's 1.2e-7, their FP32
+# sums over at most 512 nodes 2.4e-8 sqrt(512 / 2) = 3.8e-7, and G = 4 (I - T) conj(E) about
+# three times the field's relative error; 7e-7 in quadrature, times 4 for what cancels in
+# the gradients of a sum of random signs.
+ADJOINT_2NORM = 3e-6
+
+
+def _exact_nf(ndet, tilt, off, scale, at, amp, target=None):
+    """Near-field E, or with a target the gradients (position, phase, amplitude) of
+    sum (|E|^2 - target)^2, in FP64 from the path difference without cancellation (the
+    oracle's adjoint follows the reference's |d - r| - d_z, about 5e-7 rad a pair)."""
+    M = _core.rotation(tilt[0], tilt[1], 0.0)
+    x = (np.arange(ndet[0]) - ndet[0] / 2) * 75.0 + off[0]
+    y = (np.arange(ndet[1]) - ndet[1] / 2) * 75.0 + off[1]
+    d = np.stack([*(a.ravel() for a in np.meshgrid(x, y, indexing="ij")), np.full(x.size * y.size, 1e5)], 1) @ M.T
+    r, psi = at[:, :3], at[:, 3]
+    E = np.empty(len(d), complex)
+    gp, gpsi, ga = np.zeros_like(r), np.zeros(len(r)), np.zeros(len(r))
+    for grad in (False, True):
+        if grad and target is None:
+            break
+        for s in range(0, len(d), 512):
+            dd = d[s:s + 512]
+            D = np.sqrt((dd ** 2).sum(1))[:, None]
+            num = (r * r).sum(1)[None] - 2 * dd @ r.T
+            L = np.sqrt(D * D + num)
+            c = (dd[:, :2] ** 2).sum(1)[:, None] / (D + dd[:, 2:])
+            ph = K64 * (num / (L + D) + r[:, 2][None] + c) + psi[None]
+            w = 1 / L if scale else np.ones_like(L)
+            e = np.exp(1j * ph)
+            if not grad:
+                E[s:s + 512] = (w * e) @ amp
+                continue
+            G = (4 * (np.abs(E[s:s + 512]) ** 2 - target.ravel()[s:s + 512]) * E[s:s + 512].conj())[:, None]
+            z = G * e
+            ga += (w * z.real).sum(0)
+            dphi = -amp * w * z.imag
+            gpsi += dphi.sum(0)
+            diff = dd[:, None, :] - r[None]
+            gp += np.einsum("pj,pjk->jk", -K64 * dphi / L, diff)
+            gp[:, 2] += K64 * dphi.sum(0)
+            if scale:
+                gp += np.einsum("pj,pjk->jk", amp * z.real * w ** 3, diff)
+    return E.reshape(ndet) if target is None else (gp, gpsi, ga)
+
+
+@pytest.mark.parametrize("ndet,n,r,tilt", [
+    ([64, 64], 2048, 0.01, (0, 0)),
+    ([65, 131], 1029, 0.008, (0.1, -0.05)),
+    ([300, 77], 517, 0.012, (0, 0.2)),
+])
+@pytest.mark.parametrize("settings", ["", "nf", "nf scale", "scale", "secondorder"])
+def test_adjoint_nodes_vs_oracle(ndet, n, r, tilt, settings):
+    """The adjoint over nodes, in a batch with a direct and an empty image, against the oracle."""
+    g = rng(ndet[0] + n)
+    pos, ph, amp = sphere(g, n, r), g.uniform(0, 2 * np.pi, n), g.uniform(0.5, 1.5, n)
+    small = 70
+    pos2, ph2 = sphere(g, small, 0.3), g.uniform(0, 2 * np.pi, small)
+    flags, _, _ = _core.parse_settings(settings)
+    off = (300.0, -200.0)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, tilt, off, flags)
+    og = oracle.geometry(ndet, 75.0, 1e5, K64, tilt, off)
+    of = oracle.flags_from_settings(settings)
+    at = np.concatenate([atoms(pos, ph), atoms(pos2, ph2)])
+    a = np.concatenate([amp, np.ones(small)])
+    offs = [0, n, n, n + small]
+    t_at, t_a = torch.from_numpy(at).cuda(), torch.from_numpy(a).cuda()
+    E = _core.forward(t_at, offs, geom, nat.SPLIT, nat.OUT_C128, amplitudes=t_a)
+    moved = atoms(pos + g.normal(0, 5e-5, pos.shape), ph)
+    near = "nf" in settings
+    field = _exact_nf(ndet, tilt, off, "scale" in settings, moved, amp) if near else oracle.wavefield(og, of, moved, amp)
+    target = np.abs(field) ** 2
+    gI = 2 * (E.real ** 2 + E.imag ** 2 - torch.from_numpy(target).cuda()[None])
+    res = []
+    for cfg in (None, {"pixel_groups": -1}):
+        ga, gamp = _core.backward(t_at, offs, geom, E, gI.contiguous(), amplitudes=t_a, config=cfg)
+        _core.backward_workspace_error()
+        res.append((ga.cpu().numpy(), gamp.cpu().numpy()))
+    (ga, gamp), (da, damp) = res
+    assert not np.array_equal(ga[:n], da[:n])  # the node path was taken
+    if near:
+        gpos_o, gpsi_o, gamp_o = _exact_nf(ndet, tilt, off, "scale" in settings, at[:n], amp, target)
+    else:
+        E_o = oracle.wavefield(og, of, at[:n], amp)
+        _, gpos_o, gpsi_o, gamp_o = oracle.adjoint(og, of, at[:n], amp, E_o, target)
+    assert _err(ga[:n, :3], gpos_o) < ADJOINT_2NORM, _err(ga[:n, :3], gpos_o)
+    assert _err(ga[:n, 3], gpsi_o) < ADJOINT_2NORM, _err(ga[:n, 3], gpsi_o)
+    assert _err(gamp[:n], gamp_o) < ADJOINT_2NORM, _err(gamp[:n], gamp_o)
+    assert _err(ga[n:], da[n:]) < 1e-5 and _err(gamp[n:], damp[n:]) < 1e-5  # the direct image: runs against pairs
+
+
+def test_adjoint_nodes_groups_and_large_counts():
+    """Images of a batch give the gradients they give alone, more of them than a group's buffers
+    hold, and chunks grow where an image has many emitter blocks."""
+    g = rng(12)
+    counts = [300, 40000] + [300] * 30
+    imgs = [atoms(sphere(g, c, 0.01), g.uniform(0, 2 * np.pi, c)) for c in counts]
+    at = torch.from_numpy(np.concatenate(imgs)).cuda()
+    offs = np.concatenate([[0], np.cumsum(counts)])
+    geom = _core.make_geom([600, 700], 75.0, 1e5, K64, flags=nat.NF)
+    E = _core.forward(at, offs, geom, nat.SPLIT, nat.OUT_C128)
+    gI = (E.real ** 2 + E.imag ** 2).contiguous()
+    ga, gamp = _core.backward(at, offs, geom, E, gI)
+    for b in (0, 1, 31):
+        lo, hi = offs[b], offs[b + 1]
+        one, one_amp = _core.backward(at[lo:hi].contiguous(), [0, hi - lo], geom, E[b:b + 1].contiguous(),
+                                      gI[b:b + 1].contiguous())
+        assert torch.equal(ga[lo:hi], one) and torch.equal(gamp[lo:hi], one_amp), b
+        da, _ = _core.backward(at[lo:hi].contiguous(), [0, hi - lo], geom, E[b:b + 1].contiguous(),
+                               gI[b:b + 1].contiguous(), config={"pixel_groups": -1})
+        assert _err(one.cpu().numpy(), da.cpu().numpy()) < 1e-5, b
