@@ -330,7 +330,7 @@ __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, co
         ai.n0 = ai.n1 = ai.cpx = ai.nchunks = ai.nblocks = ai.unit0 = ai.pad = 0;
         if (nodes && (ai.path == kPathRuns || ai.path == kPathPixel) &&
             node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
-                      ai.n0, ai.n1) &&
+                      false, ai.n0, ai.n1) &&
             nodes_pay(n, g.nx, g.ny, ai.n0, ai.n1, 1.05e12, 7.5e11)) {
             ai.path = kPathNodes;
             const int m = ai.n0 * ai.n1;

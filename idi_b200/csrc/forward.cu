@@ -105,21 +105,13 @@ __global__ void __launch_bounds__(256)
     const ImageDesc d = bp.img[b];
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
     uint32_t *err = &hdr->error;
-    uint32_t r2max = 0;  // float bits; non-negative floats order like their bits
-    uint32_t e0max = 0, e1max = 0, amax = 0;
+    NodeExtents ex;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nrec;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = d.rec + j;
         if (j < d.n) {
             const int64_t s = d.src + j;
             const double4 a = reinterpret_cast<const double4 *>(atoms)[s];
-            r2max = max(r2max, __float_as_uint(__double2float_ru((a.x * a.x + a.y * a.y) + a.z * a.z)));
-            if (plan) {
-                e0max = max(e0max, __float_as_uint(__double2float_ru(
-                                       fabs(a.x * ng.e[0][0] + a.y * ng.e[0][1] + a.z * ng.e[0][2]))));
-                e1max = max(e1max, __float_as_uint(__double2float_ru(
-                                       fabs(a.x * ng.e[1][0] + a.y * ng.e[1][1] + a.z * ng.e[1][2]))));
-            }
             double psi = a.w * kInvTwoPi;
             psi = psi - rint(psi);
             // the DFMA chain of the kernel starts from this value: the magic
@@ -130,7 +122,7 @@ __global__ void __launch_bounds__(256)
             float amp = 1.0f;
             if (amps) amp = amp_dtype == IDIWF_F32 ? static_cast<const float *>(amps)[s]
                                                   : (float)static_cast<const double *>(amps)[s];
-            amax = max(amax, __float_as_uint(fabsf(amp)));
+            ex.add(ng, a, amp);
             if (!(fabs(a.x) <= max_abs && fabs(a.y) <= max_abs && fabs(a.z) <= max_abs))
                 record_error(err, kErrRange);
             const double w = w_mode == 1 ? (a.x * a.x + a.y * a.y) + a.z * a.z
@@ -146,48 +138,45 @@ __global__ void __launch_bounds__(256)
             rec.rC[r] = 0.0f;
         }
     }
-    // |r|_max of the image for the split kernel's pixel-run bound (the caller
-    // zeroes rmax2 before the launch)
-    r2max = __reduce_max_sync(0xffffffffu, r2max);
-    if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rec.rmax2[b], r2max);
-    if (!plan) return;
-    e0max = __reduce_max_sync(0xffffffffu, e0max);
-    e1max = __reduce_max_sync(0xffffffffu, e1max);
-    amax = __reduce_max_sync(0xffffffffu, amax);
-    if ((threadIdx.x & 31) == 0) {
-        if (e0max) atomicMax(&rec.rmax2[kMaxImagesPerLaunch + b], e0max);
-        if (e1max) atomicMax(&rec.rmax2[2 * kMaxImagesPerLaunch + b], e1max);
-        if (amax) atomicMax(&rec.rmax2[3 * kMaxImagesPerLaunch + b], amax);
+    // the image's extents, for the pixel-run bound and the node plan (the caller zeroes
+    // them before the launch); the block that finishes last plans the launch
+    if (!plan) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, ex.r2);
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(&rec.rmax2[b], m);
+        return;
     }
-    // the block that finishes last plans the launch
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&hdr->ticket, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (s_last) plan_nodes(bp, g, ng, rec.rmax2, hdr, plan);
+    ex.raise(rec.rmax2, b);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, rec.rmax2, false, hdr, plan);
 }
 
-__global__ void prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
-                                   const void *__restrict__ amps, int amp_dtype, DoubleRecs rec) {
+__global__ void __launch_bounds__(256)
+    prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
+                       const void *__restrict__ amps, int amp_dtype, DoubleRecs rec, WsHeader *__restrict__ hdr,
+                       const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext, NodePlan *__restrict__ plan) {
     const int b = blockIdx.y;
     const ImageDesc d = bp.img[b];
+    NodeExtents ex;
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nrec;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = d.rec + j;
         if (j < d.n) {
             const int64_t s = d.src + j;
-            rec.r64[r] = reinterpret_cast<const double4 *>(atoms)[s];
+            const double4 a = reinterpret_cast<const double4 *>(atoms)[s];
+            rec.r64[r] = a;
             double amp = 1.0;
             if (amps) amp = amp_dtype == IDIWF_F32 ? (double)static_cast<const float *>(amps)[s]
                                                   : static_cast<const double *>(amps)[s];
             rec.ra[r] = amp;
+            if (plan) ex.add(ng, a, __double2float_ru(fabs(amp)));
         } else {
             rec.r64[r] = make_double4(0, 0, 0, 0);
             rec.ra[r] = 0.0;
         }
     }
+    if (!plan) return;
+    ex.raise(ext, b);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, true, hdr, plan);
 }
 
 // ---------------------------------------------------------------------------
@@ -888,6 +877,156 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
     if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
 }
 
+// Node sums in FP64 (IDIWF_DOUBLE in the far field, and in the near field with
+// IDIWF_ACCURATE): the direct FP64 kernel's phases at the nodes' positions, without the
+// near field's pixel constant; the plain near field keeps the direct kernel, whose
+// |d - r| - d_z rounding is no smooth function of the pixel.  Shares, blocks and
+// fixed-point totals as in node_sum_kernel; a block's 64 emitters are added in FP64.
+// Four images of 2,000 emitters on 256^2 pixels (76^2 nodes): whole call 0.31 ms against
+// 2.87 ms, error against extended references 2.7e-15 against 1e-14 (sums without Kahan
+// steps, but a twelfth of the pairs and exact totals).
+template <bool ACC, bool SCALE, bool SECOND>
+__global__ void __launch_bounds__(kNodeThreads)
+    node_sum64_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, DoubleRecs rec,
+                      const NodePlan *__restrict__ plan, unsigned long long *__restrict__ acc, int64_t entries,
+                      WsHeader *__restrict__ hdr, uint64_t *__restrict__ cta_ns, int img0, int img1) {
+    constexpr int PPT = kNodePPT64;
+    constexpr uint32_t kStage = kNodeBlock * kDoubleRecBytes;
+    __shared__ __align__(128) unsigned char smem[2 * kStage];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int s_abort;
+    __shared__ long long s_w0[kMaxImagesPerLaunch];
+    const int tid = threadIdx.x;
+    const int64_t wbeg = plan->img[img0].w0, wend = img1 < bp.n_images ? plan->img[img1].w0 : plan->total;
+    if (wend == wbeg) return;
+    const uint64_t t_start = globaltimer_ns();
+    const int nimg = img1 - img0;
+    for (int i = tid; i < nimg; i += kNodeThreads) s_w0[i] = plan->img[img0 + i].w0;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        s_abort = 0;
+        mbar_fence_init();
+        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+    }
+    __syncthreads();
+    int64_t pos = wbeg + (wend - wbeg) * blockIdx.x / gridDim.x;
+    const int64_t end = wbeg + (wend - wbeg) * (blockIdx.x + 1) / gridDim.x;
+    uint32_t issued = 0, consumed = 0;
+    while (pos < end) {
+        int lo = 0, hi = nimg;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_w0[mid] <= pos) lo = mid;
+            else hi = mid;
+        }
+        const int img = img0 + lo;
+        const NodeImage ni = plan->img[img];
+        const ImageDesc d = bp.img[img];
+        const int tile = (int)((pos - ni.w0) / ni.nblk), b0 = (int)((pos - ni.w0) % ni.nblk);
+        const int nt = (int)min((int64_t)ni.nblk, b0 + (end - pos)) - b0;
+        pos += nt;
+        const int nodes = ni.n0 * ni.n1;
+        // a block of 64 emitters per stage, as many as the image's records hold
+        const int nrec = d.ntiles * bp.te;
+        auto count = [&](int t) { return min(kNodeBlock, nrec - (b0 + t) * kNodeBlock); };
+        auto issue = [&](int t) {
+            const uint32_t slot = issued & 1;
+            unsigned char *st = smem + slot * kStage;
+            const int cnt = count(t);  // a multiple of 16
+            const int64_t r0 = d.rec + (int64_t)(b0 + t) * kNodeBlock;
+            mbar_arrive_expect_tx(&bar[slot], cnt * kDoubleRecBytes);
+            bulk_g2s(st, rec.r64 + r0, cnt * 32, &bar[slot]);
+            bulk_g2s(st + kNodeBlock * 32, rec.ra + r0, cnt * 8, &bar[slot]);
+            ++issued;
+        };
+        if (tid == 0)
+            for (int t = 0; t < 2 && t < nt; ++t) issue(t);
+
+        const int m0 = tile * kNodeTile64 + tid;
+        double px[PPT], py[PPT], pz[PPT], D[PPT], qx[PPT], qy[PPT], qz[PPT], c2[PPT];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            const int m = min(m0 + i * kNodeThreads, nodes - 1);
+            const int a = m / ni.n1, b = m - a * ni.n1;
+            const double fa = node_index(ni.n0, a, g.nx), fb = node_index(ni.n1, b, g.ny);
+            pixel_cpu_at(g, fa, fb, px[i], py[i], pz[i]);
+            const PixelDir q = pixel_dir(g, fa, fb);
+            D[i] = sqrt(px[i] * px[i] + py[i] * py[i] + pz[i] * pz[i]);
+            qx[i] = g.k * q.ux;
+            qy[i] = g.k * q.uy;
+            qz[i] = -kTwoPi * q.nqz;
+            c2[i] = 0.5 * g.k * q.invD;
+        }
+        long long sre[PPT], sim[PPT];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) sre[i] = sim[i] = 0;
+        for (int t = 0; t < nt; ++t) {
+            const uint32_t slot = consumed & 1;
+            if (!mbar_wait_bounded(&bar[slot], (consumed >> 1) & 1)) {
+                record_error(&hdr->error, kErrTimeout);
+                s_abort = 1;
+            }
+            const unsigned char *st = smem + slot * kStage;
+            const double4 *s64 = reinterpret_cast<const double4 *>(st);
+            const double *sa = reinterpret_cast<const double *>(st + kNodeBlock * 32);
+            const int cnt = min(count(t), d.n - (b0 + t) * kNodeBlock);
+            double re[PPT], im[PPT];
+#pragma unroll
+            for (int i = 0; i < PPT; ++i) re[i] = im[i] = 0.0;
+            for (int j = 0; j < cnt; ++j) {
+                const double4 r = s64[j];
+                const double aj = sa[j];
+#pragma unroll
+                for (int i = 0; i < PPT; ++i) {
+                    double phase, w = aj;
+                    if (ACC) {
+                        const double a = px[i] - r.x, b = py[i] - r.y, c = pz[i] - r.z;
+                        const double dist = sqrt(fma(c, c, fma(a, a, b * b)));
+                        const double rr = fma(r.z, r.z, fma(r.x, r.x, r.y * r.y));
+                        const double dr = fma(pz[i], r.z, fma(px[i], r.x, py[i] * r.y));
+                        phase = fma(g.k, (rr - 2.0 * dr) / (dist + D[i]) + r.z, r.w);
+                        if (SCALE) w = aj / dist;
+                    } else {
+                        phase = r.w - fma(r.z, qz[i], fma(r.x, qx[i], r.y * qy[i]));
+                        if (SECOND) phase = fma(c2[i], fma(r.x, r.x, r.y * r.y), phase);
+                    }
+                    double sn, cs;
+                    sincos(phase, &sn, &cs);
+                    re[i] = fma(w, cs, re[i]);
+                    im[i] = fma(w, sn, im[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < PPT; ++i) {
+                sre[i] += __double2ll_rn(re[i] * (double)ni.scale);
+                sim[i] += __double2ll_rn(im[i] * (double)ni.scale);
+            }
+            ++consumed;
+            __syncthreads();
+            if (s_abort) {
+                if (tid == 0)
+                    while (consumed < issued) {
+                        mbar_wait_bounded(&bar[consumed & 1], (consumed >> 1) & 1);
+                        ++consumed;
+                    }
+                return;
+            }
+            if (tid == 0 && t + 2 < nt) issue(t + 2);
+        }
+        unsigned long long *dst = acc + (int64_t)(img - img0) * entries * 2;
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            const int m = m0 + i * kNodeThreads;
+            if (m < nodes) {
+                atomicAdd(dst + 2 * m, (unsigned long long)sre[i]);
+                atomicAdd(dst + 2 * m + 1, (unsigned long long)sim[i]);
+            }
+        }
+    }
+    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+}
+
 // Buffers of one group of images: node sums (fixed point, then FP64), interpolation
 // weights of both axes, and the intermediate W[j][a] = sum_b L_y[j][b] V[a][b]
 // (pixel columns x nodes along x).
@@ -962,12 +1101,20 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
                                                          const GeomParams g, DoubleRecs rec,
                                                          void *__restrict__ out, int out_kind,
                                                          WsHeader *__restrict__ hdr,
-                                                         uint64_t *__restrict__ cta_ns) {
+                                                         uint64_t *__restrict__ cta_ns,
+                                                         const NodePlan *__restrict__ plan) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int s_unit, s_abort;
+    __shared__ uint8_t s_skip[kMaxImagesPerLaunch];  // images evaluated on nodes
 
     const int tid = threadIdx.x;
+    bool mine = false;
+    for (int i = tid; i < bp.n_images; i += blockDim.x) {
+        s_skip[i] = plan && plan->img[i].path == kPathNodes;
+        mine |= !s_skip[i];
+    }
+    if (!__syncthreads_or(mine)) return;
     const int TE = bp.te;
     const uint32_t stage_bytes = (uint32_t)TE * kDoubleRecBytes;
     const uint64_t t_start = globaltimer_ns();
@@ -986,7 +1133,12 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
 
     for (;;) {
         __syncthreads();
-        if (tid == 0) s_unit = (int)atomicAdd(&hdr->work_counter, 1u);
+        if (tid == 0) {
+            int u;
+            do u = (int)atomicAdd(&hdr->work_counter, 1u);
+            while (u < bp.total_units && s_skip[bp.order[u / bp.tiles_per_image]]);
+            s_unit = u;
+        }
         __syncthreads();
         const int unit = s_unit;
         if (unit >= bp.total_units) break;
@@ -1320,20 +1472,22 @@ static size_t partials_bytes(const idiwf_geom *g, const idiwf_batch *b, int kspl
     return align256((size_t)ksplit * std::min(b->n_images, kMaxImagesPerLaunch) * g->nx * g->ny * 16);
 }
 
-// Whether a call may take nodes at all: split precision without
-// pixel_groups = -1, and an image with pairs enough.
+// Whether a call may take nodes at all: not with pixel_groups = -1, not in FP64's plain
+// near field (its rounding is the reference's, and no smooth function of the pixel),
+// and only with an image of pairs enough.
 static bool nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
-    if (precision != IDIWF_SPLIT || !s.groups) return false;
+    const bool split = precision == IDIWF_SPLIT;
+    if (!s.groups || (!split && (g->flags & IDIWF_NF) && !(g->flags & IDIWF_ACCURATE))) return false;
     int64_t nmax = 0;
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
-    return (double)nmax * g->nx * g->ny >= kNodeMinPairs && make_node_geom(make_geom(g)).ok;
+    return (double)nmax * g->nx * g->ny >= (split ? kNodeMinPairs : kNodeMinPairs64) && make_node_geom(make_geom(g)).ok;
 }
 
 // Node part of the workspace: the plan, and buffers for groups of images that
 // together stay within kNodeGroupBytes.
 constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
 struct NodeLayout {
-    size_t v, lx, ly, w, total;  // offsets from the node region's start (the plan)
+    size_t ext, v, lx, ly, w, total;  // offsets from the node region's start (the plan)
     int group;
     NodeBuffers at(char *base, const idiwf_geom *g) const {
         NodeBuffers nb;
@@ -1355,6 +1509,8 @@ static NodeLayout node_layout(const idiwf_geom *g, int n_images) {
                  ly = (size_t)g->ny * node_cap(g->ny) * 8, w = (size_t)g->ny * node_cap(g->nx) * 16;
     L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / (v + lx + ly + w)));
     size_t o = align256(sizeof(NodePlan));
+    L.ext = o;  // the FP64 prep kernel's extents
+    o += align256(kMaxImagesPerLaunch * 16);
     L.v = o;
     o += align256(L.group * v);
     L.lx = o;
@@ -1366,14 +1522,14 @@ static NodeLayout node_layout(const idiwf_geom *g, int n_images) {
     return L;
 }
 
-static size_t node_region_offset(const idiwf_geom *g, const idiwf_batch *b, int64_t nrec, int ksplit) {
+static size_t node_region_offset(const idiwf_geom *g, const idiwf_batch *b, int precision, int64_t nrec, int ksplit) {
+    if (precision != IDIWF_SPLIT) return kWsDataOffset + double_recs_bytes(nrec);
     return kWsDataOffset + split_recs_bytes(nrec) + partials_bytes(g, b, ksplit);
 }
 
 static size_t forward_ws_bytes(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
     const int64_t nrec = std::max<int64_t>(total_records(b, s.te), 1);
-    if (precision != IDIWF_SPLIT) return kWsDataOffset + double_recs_bytes(nrec);
-    return node_region_offset(g, b, nrec, choose_ksplit(g, b)) +
+    return node_region_offset(g, b, precision, nrec, choose_ksplit(g, b)) +
            (nodes_possible(g, b, precision, s) ? node_layout(g, b->n_images).total : 0);
 }
 
@@ -1469,12 +1625,15 @@ static int resident_ctas(void *fn, int threads, size_t smem) {
 // Node sums and interpolation of the images on kPathNodes (each kernel returns at
 // once where there is none).
 static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, const BatchParams &bp,
-                                 const SplitRecs &rec, const NodePlan *plan, const NodeLayout &nl, char *node_base,
-                                 WsHeader *hdr, uint64_t *cta_ns, void *out, int out_kind, cudaStream_t stream) {
+                                 const SplitRecs *split, const DoubleRecs *dbl, const NodePlan *plan,
+                                 const NodeLayout &nl, char *node_base, WsHeader *hdr, uint64_t *cta_ns, void *out, int out_kind, cudaStream_t stream) {
     const bool nf = geom->flags & IDIWF_NF, sc = geom->flags & IDIWF_SCALE, so = geom->flags & IDIWF_SECONDORDER;
     NodeBuffers nb = nl.at(node_base, geom);
     void *fs = nf ? (sc ? (void *)node_sum_kernel<true, true, false> : (void *)node_sum_kernel<true, false, false>)
                   : (so ? (void *)node_sum_kernel<false, false, true> : (void *)node_sum_kernel<false, false, false>);
+    if (dbl)
+        fs = nf ? (sc ? (void *)node_sum64_kernel<true, true, false> : (void *)node_sum64_kernel<true, false, false>)
+                : (so ? (void *)node_sum64_kernel<false, false, true> : (void *)node_sum64_kernel<false, false, false>);
     void *fx = nf ? (void *)node_interp_x_kernel<true, false>
                   : (sc ? (void *)node_interp_x_kernel<false, true> : (void *)node_interp_x_kernel<false, false>);
     idiwf_status st = ensure_smem((void *)node_interp_y_kernel, sizeof(GemmSmem));
@@ -1487,7 +1646,7 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
         int i1 = std::min(i0 + nl.group, bp.n_images);
         const int n = i1 - i0;
         IDIWF_CUDA_CHECK(cudaMemsetAsync(nb.v, 0, (size_t)n * nb.entries * 16, stream));
-        void *as[] = {(void *)&bp, (void *)&g, (void *)&rec, &plan, &nb.v, &nb.entries, &hdr, &cta_ns, &i0, &i1};
+        void *as[] = {(void *)&bp, (void *)&g, dbl ? (void *)dbl : (void *)split, &plan, &nb.v, &nb.entries, &hdr, &cta_ns, &i0, &i1};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), as, 0, stream));
         node_weights_kernel<<<dim3((g.nx + g.ny + 15) / 16, n), 256, 0, stream>>>(g, plan, nb, i0);
         node_interp_y_kernel<<<dim3(std::min(ty, 64), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
@@ -1540,7 +1699,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
 
     // prep
     const NodeLayout nl = bp.nodes ? node_layout(geom, b->n_images) : NodeLayout{};
-    char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, nrec, ksplit) : 0);
+    char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, precision, nrec, ksplit) : 0);
     NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
     const NodeGeom ng = make_node_geom(g);
     // work counters and the prep kernel's ticket (words 3 to 5; the error word, the
@@ -1561,8 +1720,13 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
             prep_split_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                          max_abs, split_recs(ws, nrec), hdr, g, ng, plan);
         } else {
+            uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
+            if (plan) {
+                IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), stream));
+                IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, kMaxImagesPerLaunch * 16, stream));
+            }
             prep_double_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype,
-                                                          double_recs(ws, nrec));
+                                                          double_recs(ws, nrec), hdr, g, ng, ext, plan);
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
@@ -1608,16 +1772,17 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                                                                             out_chunk, out_kind, plan);
             IDIWF_CUDA_CHECK(cudaGetLastError());
         }
-        if (plan) return launch_nodes(geom, g, bp, rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
+        if (plan) return launch_nodes(geom, g, bp, &rec, nullptr, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     } else {
         DoubleRecs rec = double_recs(ws, nrec);
-        void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns};
+        void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns, &plan};
         void *fn = kernel_for(precision, s.ppt, geom->flags, false);
         const size_t smem = fwd_smem(precision, s, kPathPixel);
         int grid = 0;
         idiwf_status st = grid_for(fn, smem, grid);
         if (st != IDIWF_OK) return st;
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(s.threads), args, smem, stream));
+        if (plan) return launch_nodes(geom, g, bp, nullptr, &rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     }
     return IDIWF_OK;
 }

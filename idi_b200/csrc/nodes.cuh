@@ -24,6 +24,9 @@
 // distance, used up to kNodeMaxT.  tests/test_nodes_math.py holds the rule to
 // 1e-8 over random geometries, emitters at the largest distance from the
 // origin (an image's other emitters, and the pixels inside, are far below).
+//
+// The FP64 kernel's images take a finer grid, 5 + 9.6 Phi^(1/3) + 30 t, which holds the
+// interpolation to about 2e-15 per emitter, below the rounding of the phases (k r 1e-16).
 #pragma once
 
 #include "idiwf_internal.cuh"
@@ -37,6 +40,8 @@ constexpr int kNodeThreads = 128;    // node kernel: threads per CTA, nodes per 
 constexpr int kNodePPT = 4;
 constexpr int kNodeTile = kNodeThreads * kNodePPT;
 constexpr int kNodeTE = 128;
+constexpr int kNodePPT64 = 2;        // FP64: nodes per thread
+constexpr int kNodeTile64 = kNodeThreads * kNodePPT64;
 constexpr int kNodeBlock = 64;       // emitters per work item and tile
 // Largest near-field or second-order phase (radians) that the node kernel's sine
 // and cosine polynomials take on top of the half turn (they hold to 1.04 half turns).
@@ -74,9 +79,9 @@ NodeGeom make_node_geom(const GeomParams &g);
 #if defined(__CUDACC__)
 
 // Nodes along one axis (even, for the 16-byte copies of weight rows) for a phase
-// half-range phi.
-__device__ __forceinline__ int node_count(double phi, double t) {
-    const double n = phi + 3.7 + 6.33 * cbrt(phi) + 14.0 * t;
+// half-range phi; fine: the FP64 kernel's.
+__device__ __forceinline__ int node_count(double phi, double t, bool fine) {
+    const double n = fine ? phi + 5.0 + 9.6 * cbrt(phi) + 30.0 * t : phi + 3.7 + 6.33 * cbrt(phi) + 14.0 * t;
     return n < (double)(2 * kNodeMax) ? ((int)ceil(n) + 1) / 2 * 2 : 2 * kNodeMax;
 }
 
@@ -86,15 +91,15 @@ __device__ __forceinline__ int node_count(double phi, double t) {
 // and by no more than k/|d| |r|; the near-field and second-order terms add up
 // to 2 |r|/|d| of that.
 __device__ __forceinline__ bool node_grid(const GeomParams &g, const NodeGeom &ng, uint32_t r2bits, uint32_t xbits,
-                                          uint32_t ybits, int &n0, int &n1) {
+                                          uint32_t ybits, bool fine, int &n0, int &n1) {
     const double r = sqrt((double)__uint_as_float(r2bits));
     if (!ng.ok || !(r * ng.inv_d <= 0.25)) return false;  // (a NaN fails too)
-    if ((g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) && !(0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra)) return false;
+    if (!fine && (g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) && !(0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra)) return false;
     const double f = 1.0 + 2.0 * r * ng.inv_d;
     const double ex = fmin(r, (double)__uint_as_float(xbits) + ng.s[0] * r);
     const double ey = fmin(r, (double)__uint_as_float(ybits) + ng.s[1] * r);
-    n0 = node_count(ng.phi[0] * ex * f, ng.t[0]);
-    n1 = node_count(ng.phi[1] * ey * f, ng.t[1]);
+    n0 = node_count(ng.phi[0] * ex * f, ng.t[0], fine);
+    n1 = node_count(ng.phi[1] * ey * f, ng.t[1], fine);
     return n0 <= kNodeMax && n1 <= kNodeMax;
 }
 
@@ -126,26 +131,58 @@ __device__ __forceinline__ void node_weights_row(double *__restrict__ L, int n, 
 }
 
 // Fewest pairs of an image for which nodes are considered: below it the three
-// further kernels cost more than the direct sum.
-constexpr double kNodeMinPairs = 8e6;
+// further kernels cost more than the direct sum (split precision, FP64).
+constexpr double kNodeMinPairs = 8e6, kNodeMinPairs64 = 2e6;
 
 // Whether an image of n emitters goes through its n0 x n1 grid: the grid fits
 // the buffers, and the pairs saved outweigh the interpolation.  The rates are
 // the kernels' measured ones: direct pairs and node pairs per second, FP64
 // multiply-adds per second of the interpolation.  The choice depends on
 // the image and the geometry alone, as split_path's does.
-__device__ __forceinline__ bool nodes_pay(int n, int nx, int ny, int n0, int n1, double direct_rate, double node_rate) {
+__device__ __forceinline__ bool nodes_pay(int n, int nx, int ny, int n0, int n1, double direct_rate, double node_rate,
+                                          double min_pairs = kNodeMinPairs) {
     const double npix = (double)nx * ny, m = (double)n0 * n1, pairs = (double)n * npix;
-    if (n0 > node_cap(nx) || n1 > node_cap(ny) || m > 0.25 * npix + 4096.0 || pairs < kNodeMinPairs) return false;
+    if (n0 > node_cap(nx) || n1 > node_cap(ny) || m > 0.25 * npix + 4096.0 || pairs < min_pairs) return false;
     const double mads = 2.0 * n0 * (npix + (double)n1 * ny);
     return n * m / node_rate + (mads + 100.0 * npix) * (1.0 / 1.2e13) < pairs / direct_rate;
 }
 
+// Largest extents of an emitter for the plan: |r|^2, |r . e| along both detector axes, |a|
+// (float bits, rounded up), raised per warp into ext (kMaxImagesPerLaunch of each).
+struct NodeExtents {
+    uint32_t r2 = 0, e0 = 0, e1 = 0, a = 0;
+    __device__ __forceinline__ void add(const NodeGeom &ng, const double4 &p, float amp) {
+        r2 = max(r2, __float_as_uint(__double2float_ru((p.x * p.x + p.y * p.y) + p.z * p.z)));
+        e0 = max(e0, __float_as_uint(__double2float_ru(fabs(p.x * ng.e[0][0] + p.y * ng.e[0][1] + p.z * ng.e[0][2]))));
+        e1 = max(e1, __float_as_uint(__double2float_ru(fabs(p.x * ng.e[1][0] + p.y * ng.e[1][1] + p.z * ng.e[1][2]))));
+        a = max(a, __float_as_uint(fabsf(amp)));
+    }
+    __device__ __forceinline__ void raise(uint32_t *ext, int b) const {
+        const uint32_t v[4] = {r2, e0, e1, a};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, v[k]);
+            if ((threadIdx.x & 31) == 0 && m) atomicMax(ext + k * kMaxImagesPerLaunch + b, m);
+        }
+    }
+};
+// True in every thread of the grid's last block to get here (a ticket in the header);
+// what the other blocks raised is then visible.
+__device__ __forceinline__ bool last_block(WsHeader *hdr) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&hdr->ticket, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    return s_last != 0;
+}
+
 // Plan of one launch, by one block: every image's path, grid, fixed-point scale and
-// share of the work.  ext: per image max |r|^2, then max |r . e| along the two axes,
+// share of the work.  fine: the FP64 kernel's images (their direct path counts as
+// kPathPixel).  ext: per image max |r|^2, then max |r . e| along the two axes,
 // then max |a| (float bits), kMaxImagesPerLaunch each.
 __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, const NodeGeom &ng,
-                                  const uint32_t *ext, WsHeader *hdr, NodePlan *plan) {
+                                  const uint32_t *ext, bool fine, WsHeader *hdr, NodePlan *plan) {
     __shared__ long long s_work[kMaxImagesPerLaunch];
     __threadfence();
     const int npix = g.nx * g.ny;
@@ -154,19 +191,23 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         const uint32_t r2 = __ldcg(ext + i), amax = __ldcg(ext + 3 * kMaxImagesPerLaunch + i);
         const int n = bp.img[i].n;
         NodeImage ni;
-        ni.path = split_path(g, r2, bp.groups != 0, false);
+        ni.path = fine ? kPathPixel : split_path(g, r2, bp.groups != 0, false);
         ni.w0 = 0;
         ni.n0 = ni.n1 = ni.ntiles = ni.nblk = 0;
         ni.scale = 1.0f;
         unsigned long long pr = (unsigned long long)n * npix;
         if (bp.nodes && (ni.path == kPathRuns || ni.path == kPathPixel) &&
-            amax < 0x7f800000u &&  // (an infinite or NaN amplitude has no fixed-point sum)
+            // (amplitudes whose fixed-point unit would leave FP32's exponents, infinite or NaN
+            // ones take the direct kernels)
+            (amax == 0u || (amax >= __float_as_uint(0x1p-40f) && amax <= __float_as_uint(0x1p100f))) &&
             node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
-                      ni.n0, ni.n1) &&
-            nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, ni.path == kPathRuns ? 1.8e12 : 1.5e12, 1.0e12)) {
+                      fine, ni.n0, ni.n1) &&
+            (fine ? nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, 1.6e11, 1.3e11, kNodeMinPairs64)
+                  : nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, ni.path == kPathRuns ? 1.8e12 : 1.5e12, 1.0e12))) {
             ni.path = kPathNodes;
             const int m = ni.n0 * ni.n1;
-            ni.ntiles = (m + kNodeTile - 1) / kNodeTile;
+            const int tile = fine ? kNodeTile64 : kNodeTile;
+            ni.ntiles = (m + tile - 1) / tile;
             ni.nblk = (n + kNodeBlock - 1) / kNodeBlock;
             pr = (unsigned long long)n * m;
             // |sum| <= n max |a| [times the largest 1/|d - r| <= 4/(3 D)] < 2^e

@@ -131,12 +131,15 @@ size_t idiwf_forward_workspace_size(const idiwf_geom *geom, const idiwf_batch *b
  * IDIWF_ERR_UNSUPPORTED in the workspace (idiwf_workspace_error); the FP64
  * kernel (IDIWF_DOUBLE) has no such limit.
  *
- * IDIWF_SPLIT evaluates an image whose field the detector oversamples (an
- * object of a few nanometres on ordinary pixels) at the points of a
- * Chebyshev grid over the detector and interpolates, where that is the
- * cheaper way; the interpolation error is below 1e-8 per emitter.  The choice
- * depends on the image and the geometry alone.  idiwf_config's pixel_groups =
- * -1 keeps the direct sum for every image.
+ * An image whose field the detector oversamples (an object of a few
+ * nanometres on ordinary pixels) is evaluated at the points of a Chebyshev
+ * grid over the detector and interpolated, where that is the cheaper way;
+ * the interpolation error is below 1e-8 per emitter with IDIWF_SPLIT, and
+ * about 2e-15 with IDIWF_DOUBLE (there in the far field and, with
+ * IDIWF_ACCURATE, in the near field; the plain near field follows the
+ * reference's rounding of |d - r| - d_z pixel by pixel).  The choice depends
+ * on the image and the geometry alone.  idiwf_config's pixel_groups = -1
+ * keeps the direct sum for every image.
  */
 idiwf_status idiwf_forward(const idiwf_geom *geom, const idiwf_batch *batch, int32_t precision,
                            int32_t out_kind, void *out, void *workspace, size_t workspace_bytes,

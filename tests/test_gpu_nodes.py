@@ -103,10 +103,11 @@ def test_dispatch_limits():
     amp[7] = np.inf
     X, pairs = _forward(at, [0, n], geom, amp)
     assert pairs == full and not np.isfinite(X).any()
-    # huge and tiny amplitudes scale through
-    for s in (1e30, 1e-30):
+    # large and small amplitudes scale through; beyond FP32's exponents for the sums' unit
+    # (2^-40, 2^100) the direct kernels take them
+    for s, nodes in ((1e30, True), (1e-12, True), (1e-30, False), (1e35, False)):
         X, pairs = _forward(at, [0, n], geom, np.full(n, s, np.float32))
-        assert pairs < full / 4 and _err(X[0] / s, E[0]) < 1e-6
+        assert (pairs < full / 4) == nodes and _err(X[0] / s, E[0]) < 1e-6, s
     Z, _ = _forward(at, [0, n], geom, np.zeros(n))
     assert np.all(Z == 0)
     wide = _core.make_geom([72, 64], 75.0 * 30, 1e5, K64, flags=nat.NF)  # half-extent 0.8 of the distance
@@ -115,6 +116,38 @@ def test_dispatch_limits():
     assert pairs in (0, full)
     ref = oracle.wavefield(oracle.geometry([72, 64], 75.0 * 30, 1e5, K64), oracle.NF | oracle.ACCURATE, at2)
     assert _err(W[0], ref) < 1e-6
+
+
+@pytest.mark.parametrize("ndet,n,r,tilt", [
+    ([64, 64], 600, 0.01, (0, 0)),
+    ([65, 131], 1029, 0.008, (0.1, -0.05)),
+    ([300, 77], 517, 0.012, (0, 0.2)),
+])
+@pytest.mark.parametrize("settings", ["double", "double scale", "double secondorder", "nf accurate", "nf scale accurate"])
+def test_fp64_nodes_vs_oracle(ndet, n, r, tilt, settings):
+    """FP64 on nodes (far field, and the near field without cancellation) against the oracle; the
+    plain near field keeps the direct kernel."""
+    g = rng(ndet[1] + n)
+    at = atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n))
+    amp = g.uniform(0.5, 1.5, n)
+    flags, prec, _ = _core.parse_settings(settings)
+    assert prec == nat.DOUBLE
+    t, a = torch.from_numpy(at).cuda(), torch.from_numpy(amp).cuda()
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, tilt, flags=flags)
+    E = _core.forward(t, [0, n], geom, nat.DOUBLE, nat.OUT_C128, amplitudes=a).cpu().numpy()[0]
+    _core.workspace_error()
+    assert 0 < _core.evaluated_pairs() < n * ndet[0] * ndet[1] / 2
+    of = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(oracle.geometry(ndet, 75.0, 1e5, K64, tilt), of, at, amp)
+    if "nf" in settings:
+        # k (|d| - d_z), up to 1e7 rad, rounds differently in the two: compare what it cancels from
+        E, ref = np.abs(E), np.abs(ref)
+    # phases of up to 70 rad formed in about five roundings of 2^-53 of that, on both sides
+    # (1e-14 each); FP64 sums and interpolation a few 1e-16; the grid 2e-15 per emitter
+    assert _err(E, ref) < 3e-14, _err(E, ref)
+    one = _core.make_geom(ndet, 75.0, 1e5, K64, tilt, flags=nat.NF)
+    _core.forward(t, [0, n], one, nat.DOUBLE, nat.OUT_C128, amplitudes=a)
+    assert _core.evaluated_pairs() == 0
 
 
 # 2-norm of the gradients' errors.  The adjoint pairs carry the forward's 1.2e-7, their FP32

@@ -90,3 +90,33 @@ def test_sine_and_cosine_polynomials():
     # chain whose last two steps weigh most
     assert np.abs(sn - np.sin(np.pi * x.astype(np.float64))).max() < 2e-7
     assert np.abs(cs - np.cos(np.pi * x.astype(np.float64))).max() < 2e-7
+
+
+@pytest.mark.parametrize("t", [0.02, 0.2, 0.6])
+@pytest.mark.parametrize("phi", [0.1, 4.0, 30.0, 120.0])
+def test_fine_grid_interpolation_error(t, phi):
+    """The FP64 kernel's grid, along one axis in extended precision: within 5e-15."""
+    ld = np.longdouble
+    g = rng(int(100 * t) + int(phi))
+    D, k, N = ld(1e5), ld(32000), 61
+    half = ld(t) * D
+    r_max = ld(phi) * D / (k * half)
+    n = int(np.ceil(phi + 5.0 + 9.6 * np.cbrt(phi) + 30.0 * t))
+    n = (n + 1) // 2 * 2
+    pi = ld(np.pi) + ld(1.2246467991473532e-16)
+    th = (2 * np.arange(n) + 1).astype(ld) * pi / (2 * n)
+    x = (2 * np.arange(N) - (N - 1)).astype(ld) / (N - 1)
+    d = x[:, None] - np.cos(th)
+    c = np.where(np.arange(n) % 2, -1, 1) * np.sin(th) / np.where(np.abs(d) < 1e-30, ld(1e-30), d)
+    L = c / c.sum(1, keepdims=True)
+    for trial in range(9):
+        r = g.normal(size=3) * [(1, 1, 1), (1, 0.01, 0.01), (0.01, 0.01, 1)][trial % 3]
+        r = (r / np.linalg.norm(r)).astype(ld) * r_max
+        u0, v0 = (ld(0), ld(0)) if trial < 6 else (ld(0.2) * D, ld(0.1) * D)
+
+        def parts(u):
+            p = np.stack([u + u0, np.full_like(u, v0), np.full_like(u, D)], -1)
+            ph = k * (r[2] - (p * r).sum(1) / np.sqrt((p * p).sum(1)))
+            return np.stack([np.cos(ph), np.sin(ph)])
+
+        assert np.abs(parts(half * x) - parts(half * np.cos(th)) @ L.T).max() < 5e-15
