@@ -162,7 +162,7 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     L.off_rb64 = o; o += align256((size_t)L.npix_pad / kRun * 32);
     L.off_rbf = o; o += align256((size_t)L.npix_pad / kRun * 32);
     L.off_px = o;  o += align256((size_t)L.npix_pad * 16);
-    L.off_rmax = o; o += align256((size_t)kMaxImagesPerLaunch * 4 * 3);
+    L.off_rmax = o; o += align256((size_t)kMaxImagesPerLaunch * 4 * kNodeExt);
     L.off_erec64 = o; o += align256((size_t)L.nrec * 32);
     L.off_erecf = o;  o += align256((size_t)L.nrec * 16);
     L.off_part = o;   o += align256((size_t)L.n_chunks * L.nrec * kBwdNAcc * 4);
@@ -328,10 +328,26 @@ __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, co
         AdjImage ai;
         ai.path = split_path(g, r2, bp.runs != 0, true);
         ai.n0 = ai.n1 = ai.cpx = ai.nchunks = ai.nblocks = ai.unit0 = ai.pad = 0;
-        if (nodes && (ai.path == kPathRuns || ai.path == kPathPixel) &&
-            node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
-                      false, ai.n0, ai.n1) &&
-            nodes_pay(n, g.nx, g.ny, ai.n0, ai.n1, 1.05e12, 7.5e11)) {
+        const double r = sqrt((double)__uint_as_float(r2)), pairs = (double)n * g.nx * g.ny;
+        bool use = false;
+        if (nodes && n > 0 && (ai.path == kPathRuns || ai.path == kPathPixel) && pairs >= kNodeMinPairs &&
+            node_reach(g, ng, r, false)) {
+            double e[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                e[k] = fmax((double)key_float(__ldcg(ext + (2 + k) * kMaxImagesPerLaunch + i)),
+                            (double)key_float(__ldcg(ext + (5 + k) * kMaxImagesPerLaunch + i)));
+            NodeImage t;
+            t.ncell = 1;
+            t.pix = 0;
+            node_grid(ng, r, r, e[0], e[1], false, t.n0, t.n1);
+            t.g0 = ai.n0 = t.n0;
+            t.g1 = ai.n1 = t.n1;
+            use = t.n0 <= node_cap(g.nx) && t.n1 <= node_cap(g.ny) &&
+                  (double)t.n0 * t.n1 <= (double)node_entries((int64_t)g.nx * g.ny) &&
+                  node_cost(n, g.nx, g.ny, t, 6.5e11) < pairs / 1.05e12;
+        }
+        if (use) {
             ai.path = kPathNodes;
             const int m = ai.n0 * ai.n1;
             ai.nblocks = (n + kAdjBlock - 1) / kAdjBlock;
@@ -364,7 +380,7 @@ __global__ void __launch_bounds__(256)
                             uint32_t *__restrict__ rmax2, const GeomParams g, const NodeGeom ng, int nodes,
                             int max_chunks, AdjPlan *__restrict__ plan, WsHeader *__restrict__ hdr) {
     const int b = blockIdx.y;
-    uint32_t e0max = 0, e1max = 0;
+    NodeExtents ex;
     const BwdImage d = bp.img[b];
     const int64_t nrec = (int64_t)d.nblocks * bp.eb;
     uint32_t r2max = 0;  // float bits; non-negative floats order like their bits
@@ -373,12 +389,7 @@ __global__ void __launch_bounds__(256)
         if (j < d.n) {
             const double4 a = reinterpret_cast<const double4 *>(atoms)[d.src + j];
             r2max = max(r2max, __float_as_uint(__double2float_ru((a.x * a.x + a.y * a.y) + a.z * a.z)));
-            if (plan) {
-                e0max = max(e0max, __float_as_uint(__double2float_ru(
-                                       fabs(a.x * ng.e[0][0] + a.y * ng.e[0][1] + a.z * ng.e[0][2]))));
-                e1max = max(e1max, __float_as_uint(__double2float_ru(
-                                       fabs(a.x * ng.e[1][0] + a.y * ng.e[1][1] + a.z * ng.e[1][2]))));
-            }
+            if (plan) ex.add(ng, a, 0.0f);
             double psi = a.w * kInvTwoPi;
             psi = psi - rint(psi);
             // magic binade + 1/2 turn (angle = 2pi (u - 1.5)) + 2^-24 turn rounding bias
@@ -392,23 +403,15 @@ __global__ void __launch_bounds__(256)
             ef[r] = make_float4(0, 0, 0, 0);
         }
     }
-    // |r|_max of the image for the pixel-run bound (zeroed by the caller)
-    r2max = __reduce_max_sync(0xffffffffu, r2max);
-    if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rmax2[b], r2max);
-    if (!plan) return;
-    e0max = __reduce_max_sync(0xffffffffu, e0max);
-    e1max = __reduce_max_sync(0xffffffffu, e1max);
-    if ((threadIdx.x & 31) == 0) {
-        if (e0max) atomicMax(&rmax2[kMaxImagesPerLaunch + b], e0max);
-        if (e1max) atomicMax(&rmax2[2 * kMaxImagesPerLaunch + b], e1max);
-    }
+    // the image's extents, for the pixel-run bound and the node plan (zeroed by the caller);
     // the block that finishes last plans the call
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&hdr->ticket, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (s_last) plan_adjoint(bp, g, ng, rmax2, nodes, max_chunks, plan);
+    if (!plan) {
+        r2max = __reduce_max_sync(0xffffffffu, r2max);
+        if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rmax2[b], r2max);
+        return;
+    }
+    ex.raise(rmax2, b);
+    if (last_block(hdr)) plan_adjoint(bp, g, ng, rmax2, nodes, max_chunks, plan);
 }
 
 __device__ __forceinline__ float2 g2(float a, float b) { return make_float2(a, b); }
@@ -832,8 +835,8 @@ __global__ void __launch_bounds__(256) adj_weights_kernel(const GeomParams g, co
     const int lane = threadIdx.x & 31;
     double *lx = nb.lx + blockIdx.y * nb.lx_stride, *ly = nb.ly + blockIdx.y * nb.ly_stride;
     for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nx + g.ny; row += gridDim.x * 8) {
-        if (row < g.nx) node_weights_row(lx, ai.n0, g.nx, row, lane);
-        else node_weights_row(ly, ai.n1, g.ny, row - g.nx, lane);
+        if (row < g.nx) node_weights_row(lx, ai.n0, pixel_x(g.nx, row), row, lane);
+        else node_weights_row(ly, ai.n1, pixel_x(g.ny, row - g.nx), row - g.nx, lane);
     }
 }
 
@@ -1231,7 +1234,7 @@ extern "C" idiwf_status idiwf_backward(const idiwf_geom *geom, const idiwf_batch
     {
         const int w_mode = nf ? 1 : (so ? 2 : 0);
         dim3 grid((unsigned)std::max(1, (max_blocks * eb + 255) / 256), batch->n_images);
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(rmax2, 0, sizeof(uint32_t) * 3 * kMaxImagesPerLaunch, stream));
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(rmax2, 0, sizeof(uint32_t) * kNodeExt * kMaxImagesPerLaunch, stream));
         bwd_emitter_prep_kernel<<<grid, 256, 0, stream>>>(bp, batch->atoms, e64, ef, w_mode, rmax2, g,
                                                           make_node_geom(g), nodes, L.n_chunks, plan, hdr);
         IDIWF_CUDA_CHECK(cudaGetLastError());

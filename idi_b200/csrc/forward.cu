@@ -59,8 +59,7 @@ struct SplitRecs {
     double4 *r64;
     float4 *rA;
     float *rC;
-    uint32_t *rmax2;  // per image of the launch: max |r|^2 (float bits, rounded up); then, for the node
-                      // plan, max |r . e| along each detector axis and max |a| (kMaxImagesPerLaunch each)
+    uint32_t *rmax2;  // per image of the launch: max |r|^2 (float bits, rounded up), where there is no node plan
 };
 struct DoubleRecs {
     double4 *r64;
@@ -80,7 +79,7 @@ static inline SplitRecs split_recs(void *ws, int64_t nrec) {
     return r;
 }
 static inline size_t split_recs_bytes(int64_t nrec) {
-    return align256(nrec * 32) + align256(nrec * 16) + align256(nrec * 4) + align256(kMaxImagesPerLaunch * 16);
+    return align256(nrec * 32) + align256(nrec * 16) + align256(nrec * 4) + align256(kMaxImagesPerLaunch * 4);
 }
 static inline DoubleRecs double_recs(void *ws, int64_t nrec) {
     char *base = static_cast<char *>(ws) + kWsDataOffset;
@@ -97,62 +96,221 @@ static inline size_t double_recs_bytes(int64_t nrec) {
 // ---------------------------------------------------------------------------
 // prep kernels: caller layout (N,4) f64 [+ amplitudes] -> padded tile records
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float load_amp(const void *__restrict__ amps, int amp_dtype, int64_t s) {
+    if (!amps) return 1.0f;
+    return amp_dtype == IDIWF_F32 ? static_cast<const float *>(amps)[s]
+                                  : (float)static_cast<const double *>(amps)[s];
+}
+// Record r of emitter a, its FP64 part relative to `centre`.
+__device__ __forceinline__ void split_record(const SplitRecs &rec, int64_t r, const double4 &a, float amp, int w_mode,
+                                             double max_abs, uint32_t *err, double cx, double cy, double cz) {
+    double psi = a.w * kInvTwoPi;
+    psi = psi - rint(psi);
+    // the DFMA chain of the kernel starts from this value: the magic
+    // binade, +1/4 turn (bit 31 of the fixed-point phase then marks
+    // the half turn centred on pi) and +2^-25 turn (rounds instead of
+    // truncating to the 23 angle bits the kernel keeps)
+    psi = (kTurnMagic + 0.25 + 0x1p-25) + psi;
+    if (!(fabs(a.x) <= max_abs && fabs(a.y) <= max_abs && fabs(a.z) <= max_abs)) record_error(err, kErrRange);
+    const double w = w_mode == 1 ? (a.x * a.x + a.y * a.y) + a.z * a.z : (w_mode == 2 ? a.x * a.x + a.y * a.y : 0.0);
+    // w is stored negated: the kernel forms s^2 - w and subtracts h times it
+    rec.r64[r] = make_double4(a.x - cx, a.y - cy, a.z - cz, psi);
+    rec.rA[r] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)(-w));
+    rec.rC[r] = amp;
+}
+__device__ __forceinline__ void empty_record(const SplitRecs &rec, int64_t r) {
+    rec.r64[r] = make_double4(0, 0, 0, 0);
+    rec.rA[r] = make_float4(0, 0, 0, 0);
+    rec.rC[r] = 0.0f;
+}
+
+// Sort of the emitters by cell (images cut into cells): counts per block of kCellSort
+// emitters, their prefix over the blocks, the first record block (64 emitters) of every
+// cell, and the cells' totals.
+struct CellSort {
+    int *counts;   // [block][kCellMax]; an image's blocks start at (its first emitter / kCellSort) + image
+    int *first;    // [image][kCellMax + 1] in blocks of kNodeBlock records
+    int *total;    // [image][kCellMax]
+};
+__device__ __forceinline__ int64_t sort_block0(const BatchParams &bp, int img) {
+    return (bp.img[img].src - bp.img[0].src) / kCellSort + img;
+}
+
+// Extents of every image and the plan.
+__global__ void __launch_bounds__(256)
+    node_extents_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
+                        const void *__restrict__ amps, int amp_dtype, uint32_t *__restrict__ ext,
+                        WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, NodeCaps caps,
+                        NodePlan *__restrict__ plan) {
+    const int b = blockIdx.y;
+    const ImageDesc d = bp.img[b];
+    NodeExtents ex;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < d.n; j += (int64_t)gridDim.x * blockDim.x)
+        ex.add(ng, reinterpret_cast<const double4 *>(atoms)[d.src + j], load_amp(amps, amp_dtype, d.src + j));
+    ex.raise(ext, b);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, caps, hdr, plan);
+}
+
+// Emitters per cell of every sort block; an image's last block turns the counts into
+// offsets and lays the cells out, each on whole blocks of 64 records.
+__global__ void __launch_bounds__(256)
+    cell_count_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms, const NodeGeom ng,
+                      NodePlan *__restrict__ plan, CellSort cs) {
+    __shared__ int s_cnt[kCellMax], s_part[8];
+    __shared__ int s_last;
+    const int img = blockIdx.y, tid = threadIdx.x;
+    const NodeImage &pi = plan->img[img];
+    if (pi.path != kPathNodes || pi.ncell == 1) return;
+    const NodeImage ni = pi;
+    const ImageDesc d = bp.img[img];
+    const int nb = (d.n + kCellSort - 1) / kCellSort;
+    int *counts = cs.counts + sort_block0(bp, img) * kCellMax;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        for (int c = tid; c < ni.ncell; c += 256) s_cnt[c] = 0;
+        __syncthreads();
+        for (int j = b * kCellSort + tid; j < min((b + 1) * kCellSort, d.n); j += 256)
+            atomicAdd(&s_cnt[cell_of(ng, ni, reinterpret_cast<const double4 *>(atoms)[d.src + j])], 1);
+        __syncthreads();
+        for (int c = tid; c < ni.ncell; c += 256) counts[(int64_t)b * kCellMax + c] = s_cnt[c];
+        __syncthreads();
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&plan->img[img].ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int blocks0 = 0;
+    for (int c0 = 0; c0 < ni.ncell; c0 += 256) {
+        const int c = c0 + tid;
+        int sum = 0;
+        if (c < ni.ncell) {
+            // 16 loads in flight at a time: the chain is the additions, not the memory
+            for (int b0 = 0; b0 < nb; b0 += 16) {
+                int v[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    v[k] = b0 + k < nb ? __ldcg(counts + (int64_t)(b0 + k) * kCellMax + c) : 0;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    if (b0 + k < nb) counts[(int64_t)(b0 + k) * kCellMax + c] = sum;
+                    sum += v[k];
+                }
+            }
+            cs.total[img * kCellMax + c] = sum;
+        }
+        // exclusive scan of the cells' record blocks over the 256 threads
+        const int nblk = (sum + kNodeBlock - 1) / kNodeBlock;
+        int x = nblk;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((tid & 31) >= o) x += y;
+        }
+        if ((tid & 31) == 31) s_part[tid >> 5] = x;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 8; ++w) {
+            before += w < (tid >> 5) ? s_part[w] : 0;
+            all += s_part[w];
+        }
+        if (c < ni.ncell) cs.first[img * (kCellMax + 1) + c] = blocks0 + before + x - nblk;
+        blocks0 += all;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        cs.first[img * (kCellMax + 1) + ni.ncell] = blocks0;
+        plan->img[img].nblk = blocks0;
+    }
+}
+
+// Records.  MAKE_PLAN: the launch has no cells, and where there is a plan it is made here
+// (extents on the way, by the block that finishes last); else the plan is given, and
+// images cut into cells are written in cell order (stable: the order of an emitter's
+// records, and with it the rounding of the sums, does not depend on timing).
+template <bool MAKE_PLAN>
 __global__ void __launch_bounds__(256)
     prep_split_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                       const void *__restrict__ amps, int amp_dtype, int w_mode, double max_abs, SplitRecs rec,
-                      WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, NodePlan *__restrict__ plan) {
-    const int b = blockIdx.y;
+                      WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext,
+                      NodeCaps caps, NodePlan *__restrict__ plan, CellSort cs) {
+    const int b = blockIdx.y, tid = threadIdx.x;
     const ImageDesc d = bp.img[b];
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
     uint32_t *err = &hdr->error;
     NodeExtents ex;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nrec;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = d.rec + j;
-        if (j < d.n) {
-            const int64_t s = d.src + j;
-            const double4 a = reinterpret_cast<const double4 *>(atoms)[s];
-            double psi = a.w * kInvTwoPi;
-            psi = psi - rint(psi);
-            // the DFMA chain of the kernel starts from this value: the magic
-            // binade, +1/4 turn (bit 31 of the fixed-point phase then marks
-            // the half turn centred on pi) and +2^-25 turn (rounds instead of
-            // truncating to the 23 angle bits the kernel keeps)
-            psi = (kTurnMagic + 0.25 + 0x1p-25) + psi;
-            float amp = 1.0f;
-            if (amps) amp = amp_dtype == IDIWF_F32 ? static_cast<const float *>(amps)[s]
-                                                  : (float)static_cast<const double *>(amps)[s];
-            ex.add(ng, a, amp);
-            if (!(fabs(a.x) <= max_abs && fabs(a.y) <= max_abs && fabs(a.z) <= max_abs))
-                record_error(err, kErrRange);
-            const double w = w_mode == 1 ? (a.x * a.x + a.y * a.y) + a.z * a.z
-                                         : (w_mode == 2 ? a.x * a.x + a.y * a.y : 0.0);
-            // w is stored negated: the kernel forms s^2 - w and subtracts h times it
-            const float fx = (float)a.x, fy = (float)a.y, fz = (float)a.z, fw = (float)(-w);
-            rec.r64[r] = make_double4(a.x, a.y, a.z, psi);
-            rec.rA[r] = make_float4(fx, fy, fz, fw);
-            rec.rC[r] = amp;
-        } else {
-            rec.r64[r] = make_double4(0, 0, 0, 0);
-            rec.rA[r] = make_float4(0, 0, 0, 0);
-            rec.rC[r] = 0.0f;
+    if (!MAKE_PLAN && plan->img[b].path == kPathNodes && plan->img[b].ncell > 1) {
+        __shared__ int s_at[kCellMax];
+        const NodeImage ni = plan->img[b];
+        const int nb = (d.n + kCellSort - 1) / kCellSort;
+        const int *counts = cs.counts + sort_block0(bp, b) * kCellMax;
+        const int *first = cs.first + b * (kCellMax + 1);
+        for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
+            for (int c = tid; c < ni.ncell; c += 256)
+                s_at[c] = first[c] * kNodeBlock + counts[(int64_t)blk * kCellMax + c];
+            __syncthreads();
+            for (int j0 = blk * kCellSort; j0 < min((blk + 1) * kCellSort, d.n); j0 += 256) {
+                const int j = j0 + tid;
+                const bool in = j < d.n;
+                double4 a = make_double4(0, 0, 0, 0);
+                int c = -1;
+                if (in) {
+                    a = reinterpret_cast<const double4 *>(atoms)[d.src + j];
+                    c = cell_of(ng, ni, a);
+                }
+                // rank among the block's earlier emitters of the cell, warp after warp
+                const uint32_t same = __match_any_sync(0xffffffffu, c);
+                const int lane = tid & 31, rank = __popc(same & ((1u << lane) - 1u));
+                int at = 0;
+                for (int w = 0; w < 8; ++w) {
+                    if ((tid >> 5) == w && in) at = s_at[c] + rank;
+                    __syncwarp();
+                    if ((tid >> 5) == w && in && rank == 0) s_at[c] += __popc(same);
+                    __syncthreads();
+                }
+                if (in) {
+                    double ctr[3];
+                    cell_centre(ng, ni, c, ctr);
+                    split_record(rec, d.rec + at, a, load_amp(amps, amp_dtype, d.src + j), w_mode, max_abs, err, ctr[0],
+                                 ctr[1], ctr[2]);
+                }
+            }
+            __syncthreads();
         }
-    }
-    // the image's extents, for the pixel-run bound and the node plan (the caller zeroes
-    // them before the launch); the block that finishes last plans the launch
-    if (!plan) {
-        const uint32_t m = __reduce_max_sync(0xffffffffu, ex.r2);
-        if ((threadIdx.x & 31) == 0 && m) atomicMax(&rec.rmax2[b], m);
+        // the rest of every cell's last record block
+        for (int c = blockIdx.x; c < ni.ncell; c += gridDim.x) {
+            const int end = first[c + 1] * kNodeBlock, at = first[c] * kNodeBlock + cs.total[b * kCellMax + c] + tid;
+            if (at < end) empty_record(rec, d.rec + at);
+        }
         return;
     }
-    ex.raise(rec.rmax2, b);
-    if (last_block(hdr)) plan_nodes(bp, g, ng, rec.rmax2, false, hdr, plan);
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + tid; j < nrec; j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = d.rec + j;
+        if (j < d.n) {
+            const double4 a = reinterpret_cast<const double4 *>(atoms)[d.src + j];
+            const float amp = load_amp(amps, amp_dtype, d.src + j);
+            if (MAKE_PLAN) ex.add(ng, a, amp);
+            split_record(rec, r, a, amp, w_mode, max_abs, err, 0.0, 0.0, 0.0);
+        } else {
+            empty_record(rec, r);
+        }
+    }
+    if (!MAKE_PLAN) return;
+    // without a plan: |r|_max for the pixel-run bound (the caller zeroes it before the launch)
+    if (!plan) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, ex.v[0]);
+        if ((tid & 31) == 0 && m) atomicMax(&rec.rmax2[b], m);
+        return;
+    }
+    ex.raise(ext, b);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, caps, hdr, plan);
 }
 
 __global__ void __launch_bounds__(256)
     prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                        const void *__restrict__ amps, int amp_dtype, DoubleRecs rec, WsHeader *__restrict__ hdr,
-                       const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext, NodePlan *__restrict__ plan) {
+                       const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext, NodeCaps caps,
+                       NodePlan *__restrict__ plan) {
     const int b = blockIdx.y;
     const ImageDesc d = bp.img[b];
     NodeExtents ex;
@@ -176,7 +334,7 @@ __global__ void __launch_bounds__(256)
     }
     if (!plan) return;
     ex.raise(ext, b);
-    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, true, hdr, plan);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, true, caps, hdr, plan);
 }
 
 // ---------------------------------------------------------------------------
@@ -204,10 +362,9 @@ __device__ __forceinline__ void store_pixel(void *out, int out_kind, int64_t idx
 // near-field constant phase k (|d| - d_z) (left out of the per-pair sum,
 // applied here in FP64 for field outputs), then the store.
 template <bool NF, bool SCALE>
-__device__ __forceinline__ void finish_pixel(const GeomParams &g, int p, double re, double im, void *out,
-                                             int out_kind, int64_t idx) {
+__device__ __forceinline__ void finish_pixel_at(const GeomParams &g, int ix, int iy, double re, double im, void *out,
+                                                int out_kind, int64_t idx) {
     if ((!NF && SCALE) || (NF && out_kind <= IDIWF_OUT_C64)) {
-        const int ix = p / g.ny, iy = p - ix * g.ny;
         double dx, dy, dz;
         pixel_cpu(g, ix, iy, dx, dy, dz);
         const double rho2 = dx * dx + dy * dy;
@@ -226,6 +383,12 @@ __device__ __forceinline__ void finish_pixel(const GeomParams &g, int p, double 
         }
     }
     store_pixel(out, out_kind, idx, re, im);
+}
+template <bool NF, bool SCALE>
+__device__ __forceinline__ void finish_pixel(const GeomParams &g, int p, double re, double im, void *out,
+                                             int out_kind, int64_t idx) {
+    const int ix = p / g.ny;
+    finish_pixel_at<NF, SCALE>(g, ix, p - ix * g.ny, re, im, out, out_kind, idx);
 }
 
 // Sum of the emitter-chunk partials of every pixel, in chunk order, then the
@@ -701,34 +864,81 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
 // per-pixel path (FP64 phase per pair, second-order near field) at the nodes'
 // fractional pixel positions.
 //
-// Work is tiles of kNodeTile nodes x blocks of 64 emitters; the CTAs that fit (four
-// 128-thread CTAs per SM) each take an equal, contiguous share of it, so the shares
-// end together and a CTA sets up a tile's geometry once or twice in all.  The FP32
+// Work is tiles of kNodeTile nodes x blocks of 64 emitters (of each cell in turn); the CTAs
+// that fit (six 128-thread CTAs per SM) each take an equal, contiguous share of it, so
+// the shares end together and a CTA sets up a tile's geometry once or twice per cell.  The FP32
 // sums of 16 emitters are added to fixed-point totals (64-bit integers, the image's
-// power of two as the unit's inverse, below 2^-59 of the largest possible sum), which
+// power of two as the unit's inverse, below 2^-58 of the largest possible sum), which
 // go to the node accumulators by atomics: integer sums do not depend on how
 // the work was cut, so results stay the same from run to run and from batch to batch.
 //
 // A node sum stands for many pixels, so it is formed more exactly than the direct
 // kernels' pixels: polynomial sine and cosine, and short FP32 partials.
+
+// Buffers of one group of images: sums on the target grid and of the cells (fixed point),
+// interpolation weights of both axes, from the target grid to the pixels and from the
+// cells' grid to the target's, the cells' sums interpolated along y, and the intermediate
+// W[j][a] = sum_b L_y[j][b] V[a][b] (pixel columns x nodes along x).
+struct NodeBuffers {
+    double2 *v, *f, *y;  // [image of the group][entries]
+    NodeCaps caps;
+    double *lx, *ly;     // [image of the group][nx or ny][n0 or n1]
+    double *sx, *sy;     // [image of the group][n0 or n1][g0 or g1]
+    double2 *w;          // [image of the group][ny][n0]
+    int64_t lx_stride, ly_stride, w_stride, sx_stride, sy_stride;
+};
+
+// Work of the images [img0, img0 + nimg), prefixed in s_w0 (nimg + 1 entries), by one block of
+// kNodeThreads threads.
+__device__ __forceinline__ void image_work(const NodePlan *__restrict__ plan, int img0, int nimg, long long *s_w0) {
+    __shared__ long long s_sum[kNodeThreads / 32];
+    const int tid = threadIdx.x;
+    long long base = 0;
+    for (int i0 = 0; i0 < nimg; i0 += kNodeThreads) {
+        const int i = i0 + tid;
+        long long w = 0;
+        if (i < nimg) {
+            const NodeImage &ni = plan->img[img0 + i];
+            w = (long long)ni.ntiles * ni.nblk;
+        }
+        long long x = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((tid & 31) >= o) x += y;
+        }
+        if ((tid & 31) == 31) s_sum[tid >> 5] = x;
+        __syncthreads();
+        long long before = base;
+        for (int k = 0; k < kNodeThreads / 32; ++k) {
+            before += k < (tid >> 5) ? s_sum[k] : 0;
+            base += s_sum[k];
+        }
+        if (i < nimg) s_w0[i] = before + x - w;
+        __syncthreads();
+    }
+    if (tid == 0) s_w0[nimg] = base;
+    __syncthreads();
+}
+
 constexpr int kNodeFold = 16;
 template <bool NF, bool SCALE, bool SECOND>
-__global__ void __launch_bounds__(kNodeThreads, 4)
+__global__ void __launch_bounds__(kNodeThreads, 6)
     node_sum_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, SplitRecs rec,
-                    const NodePlan *__restrict__ plan, unsigned long long *__restrict__ acc, int64_t entries,
+                    const NodePlan *__restrict__ plan, NodeBuffers nb, const int *__restrict__ first,
                     WsHeader *__restrict__ hdr, uint64_t *__restrict__ cta_ns, int img0, int img1) {
     constexpr int PPT = kNodePPT, PH = PPT / 2;
     constexpr uint32_t kStage = kNodeTE * kSplitRecBytes;
     __shared__ __align__(128) unsigned char smem[2 * kStage];
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int s_abort;
-    __shared__ long long s_w0[kMaxImagesPerLaunch];
+    __shared__ long long s_w0[kMaxImagesPerLaunch + 1];
     const int tid = threadIdx.x;
-    const int64_t wbeg = plan->img[img0].w0, wend = img1 < bp.n_images ? plan->img[img1].w0 : plan->total;
-    if (wend == wbeg) return;
     const uint64_t t_start = globaltimer_ns();
     const int nimg = img1 - img0;
-    for (int i = tid; i < nimg; i += kNodeThreads) s_w0[i] = plan->img[img0 + i].w0;
+    image_work(plan, img0, nimg, s_w0);
+    const int64_t wend = s_w0[nimg];
+    if (wend == 0) return;
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -737,23 +947,51 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
         if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
     }
     __syncthreads();
-    int64_t pos = wbeg + (wend - wbeg) * blockIdx.x / gridDim.x;
-    const int64_t end = wbeg + (wend - wbeg) * (blockIdx.x + 1) / gridDim.x;
+    int64_t pos = wend * blockIdx.x / gridDim.x;
+    const int64_t end = wend * (blockIdx.x + 1) / gridDim.x;
     uint32_t issued = 0, consumed = 0;
+    int img = -1, seg = 0;
+    NodeImage ni;
     while (pos < end) {
-        int lo = 0, hi = nimg;  // last image with w0 <= pos (those without work share the next one's w0)
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_w0[mid] <= pos) lo = mid;
-            else hi = mid;
+        if (img < 0 || pos >= s_w0[img - img0 + 1]) {
+            int lo = 0, hi = nimg;  // last image with w0 <= pos (those without work share the next one's w0)
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (s_w0[mid] <= pos) lo = mid;
+                else hi = mid;
+            }
+            img = img0 + lo;
+            ni = plan->img[img];
+            seg = -1;
         }
-        const int img = img0 + lo;
-        const NodeImage ni = plan->img[img];
         const ImageDesc d = bp.img[img];
-        const int tile = (int)((pos - ni.w0) / ni.nblk), b0 = (int)((pos - ni.w0) % ni.nblk);
-        const int b1 = (int)min((int64_t)ni.nblk, b0 + (end - pos));
+        const int64_t rel = pos - s_w0[img - img0];
+        // the cell: blocks [f0, f1) of the image's records
+        int f0 = 0, f1 = ni.nblk;
+        if (ni.ncell > 1) {
+            const int *fs = first + img * (kCellMax + 1);
+            const int at = (int)(rel / ni.ntiles);  // record block of the position
+            if (seg < 0 || fs[seg + 1] > at) {
+                int lo = 0, hi = ni.ncell;
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (fs[mid] <= at) lo = mid;
+                    else hi = mid;
+                }
+                seg = lo;
+            } else {
+                while (fs[seg + 1] <= at) ++seg;
+            }
+            f0 = fs[seg];
+            f1 = fs[seg + 1];
+        } else {
+            seg = 0;
+        }
+        const int tile = (int)((rel - (int64_t)f0 * ni.ntiles) / (f1 - f0));
+        const int b0 = f0 + (int)((rel - (int64_t)f0 * ni.ntiles) % (f1 - f0));
+        const int b1 = (int)min((int64_t)f1, b0 + (end - pos));
         pos += b1 - b0;
-        const int nodes = ni.n0 * ni.n1;
+        const int nodes = ni.g0 * ni.g1;
         const int len = (b1 - b0) * kNodeBlock, nt = (len + kNodeTE - 1) / kNodeTE;
         auto issue = [&](int t) {
             const uint32_t slot = issued & 1;
@@ -775,8 +1013,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
 #pragma unroll
         for (int i = 0; i < PPT; ++i) {
             const int m = min(m0 + i, nodes - 1);
-            const int a = m / ni.n1, b = m - a * ni.n1;
-            const PixelDir q = pixel_dir(g, node_index(ni.n0, a, g.nx), node_index(ni.n1, b, g.ny));
+            const int a = m / ni.g1, b = m - a * ni.g1;
+            const PixelDir q = pixel_dir(g, node_index(ni.g0, a, g.nx), node_index(ni.g1, b, g.ny));
             nqx[i] = q.nqx;
             nqy[i] = q.nqy;
             nqz[i] = q.nqz;
@@ -803,12 +1041,13 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
             const double4 *s64 = reinterpret_cast<const double4 *>(st);
             const float4 *sA = reinterpret_cast<const float4 *>(st + kNodeTE * 32);
             const float *sC = reinterpret_cast<const float *>(st + kNodeTE * 48);
-            const int cnt = min(kNodeTE, len - t * kNodeTE);
+            // (a warp whose nodes all lie past the grid's end has nothing to add)
+            const int cnt = tile * kNodeTile + (tid & ~31) * PPT < nodes ? min(kNodeTE, len - t * kNodeTE) : 0;
             for (int jb = 0; jb < cnt; jb += kNodeFold) {
                 float2 are[PH], aim[PH];
 #pragma unroll
                 for (int q = 0; q < PH; ++q) are[q] = aim[q] = f2(0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 8
                 for (int j = jb; j < jb + kNodeFold; ++j) {
                     const double4 r = s64[j];
                     const float4 A = sA[j];
@@ -866,7 +1105,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
             }
             if (tid == 0 && t + 2 < nt) issue(t + 2);
         }
-        unsigned long long *dst = acc + (int64_t)(img - img0) * entries * 2;
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(
+            ni.ncell > 1 ? nb.f + (img - img0) * nb.caps.f + (int64_t)seg * nodes : nb.v + (img - img0) * nb.caps.v);
 #pragma unroll
         for (int i = 0; i < PPT; ++i)
             if (m0 + i < nodes) {
@@ -888,20 +1128,20 @@ __global__ void __launch_bounds__(kNodeThreads, 4)
 template <bool ACC, bool SCALE, bool SECOND>
 __global__ void __launch_bounds__(kNodeThreads)
     node_sum64_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, DoubleRecs rec,
-                      const NodePlan *__restrict__ plan, unsigned long long *__restrict__ acc, int64_t entries,
+                      const NodePlan *__restrict__ plan, NodeBuffers nb, const int *__restrict__ first,
                       WsHeader *__restrict__ hdr, uint64_t *__restrict__ cta_ns, int img0, int img1) {
     constexpr int PPT = kNodePPT64;
     constexpr uint32_t kStage = kNodeBlock * kDoubleRecBytes;
     __shared__ __align__(128) unsigned char smem[2 * kStage];
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int s_abort;
-    __shared__ long long s_w0[kMaxImagesPerLaunch];
+    __shared__ long long s_w0[kMaxImagesPerLaunch + 1];
     const int tid = threadIdx.x;
-    const int64_t wbeg = plan->img[img0].w0, wend = img1 < bp.n_images ? plan->img[img1].w0 : plan->total;
-    if (wend == wbeg) return;
     const uint64_t t_start = globaltimer_ns();
     const int nimg = img1 - img0;
-    for (int i = tid; i < nimg; i += kNodeThreads) s_w0[i] = plan->img[img0 + i].w0;
+    image_work(plan, img0, nimg, s_w0);
+    const int64_t wend = s_w0[nimg];
+    if (wend == 0) return;
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -910,8 +1150,8 @@ __global__ void __launch_bounds__(kNodeThreads)
         if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
     }
     __syncthreads();
-    int64_t pos = wbeg + (wend - wbeg) * blockIdx.x / gridDim.x;
-    const int64_t end = wbeg + (wend - wbeg) * (blockIdx.x + 1) / gridDim.x;
+    int64_t pos = wend * blockIdx.x / gridDim.x;
+    const int64_t end = wend * (blockIdx.x + 1) / gridDim.x;
     uint32_t issued = 0, consumed = 0;
     while (pos < end) {
         int lo = 0, hi = nimg;
@@ -923,7 +1163,8 @@ __global__ void __launch_bounds__(kNodeThreads)
         const int img = img0 + lo;
         const NodeImage ni = plan->img[img];
         const ImageDesc d = bp.img[img];
-        const int tile = (int)((pos - ni.w0) / ni.nblk), b0 = (int)((pos - ni.w0) % ni.nblk);
+        const int64_t rel = pos - s_w0[lo];
+        const int tile = (int)(rel / ni.nblk), b0 = (int)(rel % ni.nblk);
         const int nt = (int)min((int64_t)ni.nblk, b0 + (end - pos)) - b0;
         pos += nt;
         const int nodes = ni.n0 * ni.n1;
@@ -1014,7 +1255,7 @@ __global__ void __launch_bounds__(kNodeThreads)
             }
             if (tid == 0 && t + 2 < nt) issue(t + 2);
         }
-        unsigned long long *dst = acc + (int64_t)(img - img0) * entries * 2;
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(nb.v + (img - img0) * nb.caps.v);
 #pragma unroll
         for (int i = 0; i < PPT; ++i) {
             const int m = m0 + i * kNodeThreads;
@@ -1027,50 +1268,226 @@ __global__ void __launch_bounds__(kNodeThreads)
     if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
 }
 
-// Buffers of one group of images: node sums (fixed point, then FP64), interpolation
-// weights of both axes, and the intermediate W[j][a] = sum_b L_y[j][b] V[a][b]
-// (pixel columns x nodes along x).
-struct NodeBuffers {
-    double2 *v;         // [image of the group][entries]
-    int64_t entries;
-    double *lx, *ly;    // [image of the group][nx or ny][n0 or n1]
-    double2 *w;         // [image of the group][ny][n0]
-    int64_t lx_stride, ly_stride, w_stride;
-};
+// Zeroes the sums that the group's images use.
+__global__ void __launch_bounds__(256) node_zero_kernel(const NodePlan *__restrict__ plan, NodeBuffers nb, int img0) {
+    const NodeImage &ni = plan->img[img0 + blockIdx.y];
+    if (ni.path != kPathNodes) return;
+    const int64_t nv = (int64_t)ni.n0 * ni.n1, nf = ni.ncell > 1 ? (int64_t)ni.ncell * ni.g0 * ni.g1 : 0;
+    double2 *v = nb.v + blockIdx.y * nb.caps.v, *f = nb.f + blockIdx.y * nb.caps.f;
+    for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv + nf; i += gridDim.x * blockDim.x)
+        (i < nv ? v[i] : f[i - nv]) = make_double2(0.0, 0.0);
+}
 
-// Node sums from fixed point to FP64, in place, and the interpolation weights.
+// The interpolation weights.
 __global__ void __launch_bounds__(256) node_weights_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
                                                            NodeBuffers nb, int img0) {
     const NodeImage ni = plan->img[img0 + blockIdx.y];
     if (ni.path != kPathNodes) return;
-    const int nodes = ni.n0 * ni.n1;
-    const double unit = 1.0 / (double)ni.scale;
-    double2 *v = nb.v + blockIdx.y * nb.entries;
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < nodes; m += gridDim.x * blockDim.x) {
-        const longlong2 x = reinterpret_cast<const longlong2 *>(v)[m];
-        v[m] = make_double2((double)x.x * unit, (double)x.y * unit);
-    }
     const int lane = threadIdx.x & 31;
     double *lx = nb.lx + blockIdx.y * nb.lx_stride, *ly = nb.ly + blockIdx.y * nb.ly_stride;
-    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nx + g.ny; row += gridDim.x * 8) {
-        if (row < g.nx) node_weights_row(lx, ni.n0, g.nx, row, lane);
-        else node_weights_row(ly, ni.n1, g.ny, row - g.nx, lane);
+    double *sx = nb.sx + blockIdx.y * nb.sx_stride, *sy = nb.sy + blockIdx.y * nb.sy_stride;
+    const int fine = ni.pix ? 0 : g.nx + g.ny, rows = fine + (ni.ncell > 1 ? ni.n0 + ni.n1 : 0);
+    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8) {
+        if (row < fine) {
+            if (row < g.nx) node_weights_row(lx, ni.n0, pixel_x(g.nx, row), row, lane);
+            else node_weights_row(ly, ni.n1, pixel_x(g.ny, row - g.nx), row - g.nx, lane);
+        } else {
+            const int i = row - fine;
+            if (i < ni.n0) node_weights_row(sx, ni.g0, ni.pix ? pixel_x(g.nx, i) : node_x(ni.n0, i), i, lane);
+            else node_weights_row(sy, ni.g1, ni.pix ? pixel_x(g.ny, i - ni.n0) : node_x(ni.n1, i - ni.n0), i - ni.n0, lane);
+        }
+    }
+}
+
+// Cells, along y: Y[cell][B][a] = sum_b S_y[B][b] F[cell][a][b].
+__global__ void __launch_bounds__(kGemmThreads, 4) cell_interp_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
+                                                                      NodeBuffers nb, int img0) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const NodeImage ni = plan->img[img0 + blockIdx.y];
+    if (ni.path != kPathNodes || ni.ncell == 1) return;
+    const double unit = 1.0 / (double)ni.scale;
+    const double *S = nb.sy + blockIdx.y * nb.sy_stride;
+    const int tm = (ni.n1 + kGemmM - 1) / kGemmM, tn = (ni.g0 + kGemmN - 1) / kGemmN;
+    for (int t = blockIdx.x; t < tm * tn * ni.ncell; t += gridDim.x) {
+        const int cell = t / (tm * tn), u = t - cell * (tm * tn);
+        double2 *Y = nb.y + blockIdx.y * nb.caps.y + (int64_t)cell * ni.n1 * ni.g0;
+        interp_tile<true>(*reinterpret_cast<GemmSmem *>(smem), S,
+                          nb.f + blockIdx.y * nb.caps.f + (int64_t)cell * ni.g0 * ni.g1, ni.n1, ni.g0, ni.g1,
+                          u % tm * kGemmM, u / tm * kGemmN, unit,
+                          [&](int B, int a, double re, double im) { Y[(size_t)B * ni.g0 + a] = make_double2(re, im); });
+    }
+}
+
+// Cells, along x, and their sum: V[A][B] += exp(i theta_cell(A, B)) sum_a S_x[A][a] Y[cell][B][a],
+// theta = the phase of the cell's centre at the target point.  A CTA takes an equal,
+// contiguous share of (image, target tile, cell), 32 x 32 targets each; the cells' tiles
+// are FP64 products (mma.m8n8k4, K in blocks of 16 by cp.async), turned by the
+// phase (FP64 turns, polynomial sine and cosine) and added in registers; a tile's total goes
+// to the fixed-point sums by atomics.
+constexpr int kExpTile = 32;
+struct ExpandSmem {
+    double a[2][kExpTile * kGemmLd];
+    double2 b[2][kExpTile * kGemmLd];
+    double nq[3][kExpTile * (kExpTile + 1)];  // turns per length at the targets
+};
+__global__ void __launch_bounds__(kGemmThreads, 4) cell_expand_kernel(const GeomParams g, const NodeGeom ng,
+                                                                      const NodePlan *__restrict__ plan, NodeBuffers nb,
+                                                                      int img0, int img1) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    ExpandSmem &sm = *reinterpret_cast<ExpandSmem *>(smem);
+    __shared__ long long s_w0[kMaxImagesPerLaunch + 1];
+    const int tid = threadIdx.x, lane = tid & 31, wr = (tid >> 5) >> 1, wc = (tid >> 5) & 1;
+    const int nimg = img1 - img0;
+    if (tid == 0) {
+        long long w = 0;
+        for (int i = 0; i < nimg; ++i) {
+            s_w0[i] = w;
+            const NodeImage &ni = plan->img[img0 + i];
+            if (ni.path == kPathNodes && ni.ncell > 1)
+                w += (long long)((ni.n0 + kExpTile - 1) / kExpTile) * ((ni.n1 + kExpTile - 1) / kExpTile) * ni.ncell;
+        }
+        s_w0[nimg] = w;
+    }
+    __syncthreads();
+    const int64_t wend = s_w0[nimg];
+    int64_t pos = wend * blockIdx.x / gridDim.x;
+    const int64_t end = wend * (blockIdx.x + 1) / gridDim.x;
+    while (pos < end) {
+        int lo = 0, hi = nimg;  // last image with w0 <= pos
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_w0[mid] <= pos) lo = mid;
+            else hi = mid;
+        }
+        const NodeImage ni = plan->img[img0 + lo];
+        const int64_t rel = pos - s_w0[lo];
+        const int tile = (int)(rel / ni.ncell), c0 = (int)(rel % ni.ncell);
+        const int c1 = (int)min((int64_t)ni.ncell, c0 + (end - pos));
+        pos += c1 - c0;
+        const int t0 = (ni.n0 + kExpTile - 1) / kExpTile, A0 = tile % t0 * kExpTile, B0 = tile / t0 * kExpTile;
+        const double *S = nb.sx + lo * nb.sx_stride;
+        const double2 *Y = nb.y + lo * nb.caps.y;
+        const int K = ni.g0, nk = (K + kGemmK - 1) / kGemmK;
+        __syncthreads();
+        for (int i = tid; i < kExpTile * kExpTile; i += kGemmThreads) {
+            const int A = min(A0 + i / kExpTile, ni.n0 - 1), B = min(B0 + i % kExpTile, ni.n1 - 1);
+            const PixelDir q = pixel_dir(g, ni.pix ? (double)A : node_index(ni.n0, A, g.nx),
+                                         ni.pix ? (double)B : node_index(ni.n1, B, g.ny));
+            const int at = i / kExpTile * (kExpTile + 1) + i % kExpTile;
+            sm.nq[0][at] = q.nqx;
+            sm.nq[1][at] = q.nqy;
+            sm.nq[2][at] = q.nqz;
+        }
+        double tot[2][4][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) tot[a][b][0] = tot[a][b][1] = 0.0;
+        const int steps = (c1 - c0) * nk;
+        auto issue = [&](int st) {
+            const int s = st & 1, cell = c0 + st / nk, k0 = st % nk * kGemmK;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {  // 32 rows x 16 doubles
+                const int c = tid + q * kGemmThreads, r = c >> 3, k = (c & 7) * 2;
+                const bool ok = A0 + r < ni.n0 && k0 + k < K;
+                cp_async16(&sm.a[s][r * kGemmLd + k], S + (ok ? (size_t)(A0 + r) * K + k0 + k : 0), ok);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // 32 rows x 16 complex
+                const int c = tid + q * kGemmThreads, r = c >> 4, k = c & 15;
+                const bool ok = B0 + r < ni.n1 && k0 + k < K;
+                cp_async16(&sm.b[s][r * kGemmLd + k], Y + (ok ? ((size_t)cell * ni.n1 + B0 + r) * K + k0 + k : 0), ok);
+            }
+            cp_async_commit();
+        };
+        issue(0);
+        int st = 0;
+        for (int cell = c0; cell < c1; ++cell) {
+            double acc[2][4][2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+            for (int kb = 0; kb < nk; ++kb, ++st) {
+                if (st + 1 < steps) {
+                    issue(st + 1);
+                    cp_async_wait<1>();
+                } else {
+                    cp_async_wait<0>();
+                }
+                __syncthreads();
+                const double *sa = sm.a[st & 1] + (wr * 16 + (lane >> 2)) * kGemmLd + (lane & 3);
+                const double *sb = reinterpret_cast<const double *>(sm.b[st & 1] + (wc * 16 + (lane >> 3)) * kGemmLd +
+                                                                    (lane & 3)) + ((lane >> 2) & 1);
+#pragma unroll
+                for (int k = 0; k < kGemmK; k += 4) {
+                    double fa[2], fb[4];
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) fa[t] = sa[t * 8 * kGemmLd + k];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) fb[t] = sb[(t * 4 * kGemmLd + k) * 2];
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) dmma884(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+                }
+                __syncthreads();
+            }
+            double ctr[3];
+            cell_centre(ng, ni, cell, ctr);
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; b += 2) {
+                    uint32_t w[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int at = (wr * 16 + a * 8 + (lane >> 2)) * (kExpTile + 1) + wc * 16 + (b + e) * 4 + (lane & 3);
+                        double t = __fma_rn(sm.nq[0][at], ctr[0], kTurnMagic + 0.25 + 0x1p-25);
+                        t = __fma_rn(sm.nq[1][at], ctr[1], t);
+                        t = __fma_rn(sm.nq[2][at], ctr[2], t);
+                        w[e] = (uint32_t)__double2loint(t);
+                    }
+                    float2 sn, cs;
+                    sincospi2(half_turns2(w[0], w[1]), sn, cs);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const double c = flip_sign(e ? cs.y : cs.x, w[e]), s = flip_sign(e ? sn.y : sn.x, w[e]);
+                        const double re = acc[a][b + e][0], im = acc[a][b + e][1];
+                        tot[a][b + e][0] += c * re - s * im;
+                        tot[a][b + e][1] += c * im + s * re;
+                    }
+                }
+        }
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(nb.v + lo * nb.caps.v);
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int A = A0 + wr * 16 + a * 8 + (lane >> 2), B = B0 + wc * 16 + b * 4 + (lane & 3);
+                if (A < ni.n0 && B < ni.n1) {
+                    unsigned long long *o = dst + 2 * ((int64_t)A * ni.n1 + B);
+                    atomicAdd(o, (unsigned long long)__double2ll_rn(tot[a][b][0] * (double)ni.scale));
+                    atomicAdd(o + 1, (unsigned long long)__double2ll_rn(tot[a][b][1] * (double)ni.scale));
+                }
+            }
     }
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 4) node_interp_y_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
                                                                      NodeBuffers nb, int img0) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int img = img0 + blockIdx.y;
-    const NodeImage ni = plan->img[img];
-    if (ni.path != kPathNodes) return;
+    const NodeImage ni = plan->img[img0 + blockIdx.y];
+    if (ni.path != kPathNodes || ni.pix) return;
+    const double unit = 1.0 / (double)ni.scale;
     const double *L = nb.ly + blockIdx.y * nb.ly_stride;
-    const double2 *V = nb.v + blockIdx.y * nb.entries;
+    const double2 *V = nb.v + blockIdx.y * nb.caps.v;
     double2 *W = nb.w + blockIdx.y * nb.w_stride;
     const int tm = (g.ny + kGemmM - 1) / kGemmM, tn = (ni.n0 + kGemmN - 1) / kGemmN;
     for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
-        interp_tile(*reinterpret_cast<GemmSmem *>(smem), L, V, g.ny, ni.n0, ni.n1, t % tm * kGemmM, t / tm * kGemmN,
-                    [&](int j, int a, double re, double im) { W[(size_t)j * ni.n0 + a] = make_double2(re, im); });
+        interp_tile<true>(*reinterpret_cast<GemmSmem *>(smem), L, V, g.ny, ni.n0, ni.n1, t % tm * kGemmM,
+                          t / tm * kGemmN, unit,
+                          [&](int j, int a, double re, double im) { W[(size_t)j * ni.n0 + a] = make_double2(re, im); });
 }
 
 template <bool NF, bool SCALE>
@@ -1081,16 +1498,22 @@ __global__ void __launch_bounds__(kGemmThreads, 4) node_interp_x_kernel(const Ge
     const int img = img0 + blockIdx.y;
     const NodeImage ni = plan->img[img];
     if (ni.path != kPathNodes) return;
+    const int64_t obase = (int64_t)img * g.nx * g.ny;
+    if (ni.pix) {  // the sums are the pixels'
+        const double unit = 1.0 / (double)ni.scale;
+        const longlong2 *V = reinterpret_cast<const longlong2 *>(nb.v + blockIdx.y * nb.caps.v);
+        for (int p = blockIdx.x * kGemmThreads + threadIdx.x; p < g.nx * g.ny; p += gridDim.x * kGemmThreads)
+            finish_pixel<NF, SCALE>(g, p, (double)V[p].x * unit, (double)V[p].y * unit, out, out_kind, obase + p);
+        return;
+    }
     const double *L = nb.lx + blockIdx.y * nb.lx_stride;
     const double2 *W = nb.w + blockIdx.y * nb.w_stride;
-    const int64_t obase = (int64_t)img * g.nx * g.ny;
     const int tm = (g.nx + kGemmM - 1) / kGemmM, tn = (g.ny + kGemmN - 1) / kGemmN;
     for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
-        interp_tile(*reinterpret_cast<GemmSmem *>(smem), L, W, g.nx, g.ny, ni.n0, t % tm * kGemmM, t / tm * kGemmN,
-                    [&](int i, int j, double re, double im) {
-                        const int p = i * g.ny + j;
-                        finish_pixel<NF, SCALE>(g, p, re, im, out, out_kind, obase + p);
-                    });
+        interp_tile<false>(*reinterpret_cast<GemmSmem *>(smem), L, W, g.nx, g.ny, ni.n0, t % tm * kGemmM, t / tm * kGemmN,
+                           1.0, [&](int i, int j, double re, double im) {
+                               finish_pixel_at<NF, SCALE>(g, i, j, re, im, out, out_kind, obase + i * g.ny + j);
+                           });
 }
 
 // ---------------------------------------------------------------------------
@@ -1338,6 +1761,10 @@ NodeGeom make_node_geom(const GeomParams &g) {
         far[a] = std::max(std::fabs((0.0 - size[a] * 0.5) * g.pixelsize + off[a]),
                           std::fabs((size[a] - 1 - size[a] * 0.5) * g.pixelsize + off[a]));
     }
+    n.e[2][0] = n.e[0][1] * n.e[1][2] - n.e[0][2] * n.e[1][1];
+    n.e[2][1] = n.e[0][2] * n.e[1][0] - n.e[0][0] * n.e[1][2];
+    n.e[2][2] = n.e[0][0] * n.e[1][1] - n.e[0][1] * n.e[1][0];
+    n.ortho = std::fabs(dot(n.e[0], n.e[1])) <= 1e-12;
     if (!(g.dmin > 0) || !std::isfinite(g.dmin)) return n;
     n.ok = 1;
     n.inv_d = 1.0 / g.dmin;
@@ -1441,15 +1868,6 @@ static idiwf_status resolve_shape(const idiwf_geom *g, const idiwf_batch *b, int
     return IDIWF_OK;
 }
 
-static int64_t total_records(const idiwf_batch *b, int te) {
-    int64_t t = 0;
-    for (int i = 0; i < b->n_images; ++i) {
-        const int64_t n = b->offsets[i + 1] - b->offsets[i];
-        t += (n + te - 1) / te * te;
-    }
-    return t;
-}
-
 // Emitter chunks per (image, pixel tile) for the split kernel: 1 when the
 // batch has pixel tiles for at least 3/4 of one wave of CTA slots (two per
 // SM), else about two waves' worth of units.  Depends only on the problem and
@@ -1472,53 +1890,99 @@ static size_t partials_bytes(const idiwf_geom *g, const idiwf_batch *b, int kspl
     return align256((size_t)ksplit * std::min(b->n_images, kMaxImagesPerLaunch) * g->nx * g->ny * 16);
 }
 
-// Whether a call may take nodes at all: not with pixel_groups = -1, not in FP64's plain
-// near field (its rounding is the reference's, and no smooth function of the pixel),
-// and only with an image of pairs enough.
-static bool nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
+// Whether a call may take nodes at all (1), and cells (2): not with pixel_groups = -1, not
+// in FP64's plain near field (its rounding is the reference's, and no smooth function of
+// the pixel), and only with an image of pairs (emitters) enough.
+static int nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
     const bool split = precision == IDIWF_SPLIT;
-    if (!s.groups || (!split && (g->flags & IDIWF_NF) && !(g->flags & IDIWF_ACCURATE))) return false;
+    if (!s.groups || (!split && (g->flags & IDIWF_NF) && !(g->flags & IDIWF_ACCURATE))) return 0;
     int64_t nmax = 0;
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
-    return (double)nmax * g->nx * g->ny >= (split ? kNodeMinPairs : kNodeMinPairs64) && make_node_geom(make_geom(g)).ok;
+    if ((double)nmax * g->nx * g->ny < (split ? kNodeMinPairs : kNodeMinPairs64)) return 0;
+    const NodeGeom ng = make_node_geom(make_geom(g));
+    if (!ng.ok) return 0;
+    return split && nmax >= kCellMinEmitters && ng.ortho ? 2 : 1;
 }
 
-// Node part of the workspace: the plan, and buffers for groups of images that
-// together stay within kNodeGroupBytes.
+// Records of an image: whole emitter tiles, and for images that may be cut into cells
+// up to 63 empty ones per cell.
+static int64_t image_records(int64_t n, int te, int nodes) {
+    const int64_t r = (n + te - 1) / te * te;
+    if (nodes < 2 || n < kCellMinEmitters) return r;
+    return r + (std::min<int64_t>(kCellMax, n / 64) * kNodeBlock + te - 1) / te * te;
+}
+static int64_t total_records(const idiwf_batch *b, int te, int nodes) {
+    int64_t t = 0;
+    for (int i = 0; i < b->n_images; ++i) t += image_records(b->offsets[i + 1] - b->offsets[i], te, nodes);
+    return t;
+}
+
+// Node part of the workspace: the plan, the emitters' sort, and buffers for groups of
+// images that together stay within kNodeGroupBytes.
 constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
 struct NodeLayout {
-    size_t ext, v, lx, ly, w, total;  // offsets from the node region's start (the plan)
+    size_t ext, counts, first, tot, v, f, y, lx, ly, sx, sy, w, total;  // offsets from the region's start (the plan)
     int group;
+    NodeCaps caps;
     NodeBuffers at(char *base, const idiwf_geom *g) const {
         NodeBuffers nb;
         nb.v = reinterpret_cast<double2 *>(base + v);
-        nb.entries = node_entries((int64_t)g->nx * g->ny);
+        nb.f = reinterpret_cast<double2 *>(base + f);
+        nb.y = reinterpret_cast<double2 *>(base + y);
+        nb.caps = caps;
         nb.lx = reinterpret_cast<double *>(base + lx);
         nb.ly = reinterpret_cast<double *>(base + ly);
+        nb.sx = reinterpret_cast<double *>(base + sx);
+        nb.sy = reinterpret_cast<double *>(base + sy);
         nb.w = reinterpret_cast<double2 *>(base + w);
         nb.lx_stride = (int64_t)g->nx * node_cap(g->nx);
         nb.ly_stride = (int64_t)g->ny * node_cap(g->ny);
+        nb.sx_stride = (int64_t)std::max(g->nx, node_cap(g->nx)) * kCellNodes;
+        nb.sy_stride = (int64_t)std::max(g->ny, node_cap(g->ny)) * kCellNodes;
         nb.w_stride = (int64_t)g->ny * node_cap(g->nx);
         return nb;
     }
+    CellSort sort(char *base) const {
+        return CellSort{reinterpret_cast<int *>(base + counts), reinterpret_cast<int *>(base + first),
+                        reinterpret_cast<int *>(base + tot)};
+    }
 };
-static NodeLayout node_layout(const idiwf_geom *g, int n_images) {
+static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int nodes) {
     NodeLayout L;
-    const int imgs = std::min(n_images, kMaxImagesPerLaunch);
-    const size_t v = (size_t)node_entries((int64_t)g->nx * g->ny) * 16, lx = (size_t)g->nx * node_cap(g->nx) * 8,
-                 ly = (size_t)g->ny * node_cap(g->ny) * 8, w = (size_t)g->ny * node_cap(g->nx) * 16;
-    L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / (v + lx + ly + w)));
+    const bool cells = nodes > 1;
+    const int imgs = std::min(b->n_images, kMaxImagesPerLaunch);
+    int64_t nmax = 0, nlaunch = 0;  // largest image, largest number of emitters of a launch
+    for (int i = 0; i < b->n_images; ++i) {
+        nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
+        if (i % kMaxImagesPerLaunch == 0)
+            nlaunch = std::max(nlaunch, b->offsets[std::min(i + kMaxImagesPerLaunch, b->n_images)] - b->offsets[i]);
+    }
+    L.caps = node_caps((int64_t)g->nx * g->ny, nmax, cells);
+    const size_t v = (size_t)L.caps.v * 16, f = (size_t)L.caps.f * 16, y = (size_t)L.caps.y * 16,
+                 lx = (size_t)g->nx * node_cap(g->nx) * 8, ly = (size_t)g->ny * node_cap(g->ny) * 8,
+                 sx = cells ? (size_t)std::max(g->nx, node_cap(g->nx)) * kCellNodes * 8 : 0,
+                 sy = cells ? (size_t)std::max(g->ny, node_cap(g->ny)) * kCellNodes * 8 : 0,
+                 w = (size_t)g->ny * node_cap(g->nx) * 16;
+    L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / (v + f + y + lx + ly + sx + sy + w)));
     size_t o = align256(sizeof(NodePlan));
-    L.ext = o;  // the FP64 prep kernel's extents
-    o += align256(kMaxImagesPerLaunch * 16);
-    L.v = o;
-    o += align256(L.group * v);
-    L.lx = o;
-    o += align256(L.group * lx);
-    L.ly = o;
-    o += align256(L.group * ly);
-    L.w = o;
-    L.total = o + align256(L.group * w);
+    const auto take = [&](size_t bytes) {
+        const size_t at = o;
+        o += align256(bytes);
+        return at;
+    };
+    L.ext = take((size_t)kMaxImagesPerLaunch * 4 * kNodeExt);
+    L.counts = take(cells ? (size_t)(nlaunch / kCellSort + imgs + 1) * kCellMax * 4 : 0);
+    L.first = take(cells ? (size_t)imgs * (kCellMax + 1) * 4 : 0);
+    L.tot = take(cells ? (size_t)imgs * kCellMax * 4 : 0);
+    L.v = take(L.group * v);
+    L.f = take(L.group * f);
+    L.y = take(L.group * y);
+    L.lx = take(L.group * lx);
+    L.ly = take(L.group * ly);
+    L.sx = take(L.group * sx);
+    L.sy = take(L.group * sy);
+    L.w = take(L.group * w);
+    L.total = o;
     return L;
 }
 
@@ -1528,9 +1992,10 @@ static size_t node_region_offset(const idiwf_geom *g, const idiwf_batch *b, int 
 }
 
 static size_t forward_ws_bytes(const idiwf_geom *g, const idiwf_batch *b, int precision, const LaunchShape &s) {
-    const int64_t nrec = std::max<int64_t>(total_records(b, s.te), 1);
+    const int nodes = nodes_possible(g, b, precision, s);
+    const int64_t nrec = std::max<int64_t>(total_records(b, s.te, nodes), 1);
     return node_region_offset(g, b, precision, nrec, choose_ksplit(g, b)) +
-           (nodes_possible(g, b, precision, s) ? node_layout(g, b->n_images).total : 0);
+           (nodes ? node_layout(g, b, nodes).total : 0);
 }
 
 // Dynamic shared memory of a forward kernel: two stages of emitter records,
@@ -1624,11 +2089,13 @@ static int resident_ctas(void *fn, int threads, size_t smem) {
 
 // Node sums and interpolation of the images on kPathNodes (each kernel returns at
 // once where there is none).
-static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, const BatchParams &bp,
+static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, const NodeGeom &ng, const BatchParams &bp,
                                  const SplitRecs *split, const DoubleRecs *dbl, const NodePlan *plan,
                                  const NodeLayout &nl, char *node_base, WsHeader *hdr, uint64_t *cta_ns, void *out, int out_kind, cudaStream_t stream) {
     const bool nf = geom->flags & IDIWF_NF, sc = geom->flags & IDIWF_SCALE, so = geom->flags & IDIWF_SECONDORDER;
-    NodeBuffers nb = nl.at(node_base, geom);
+    const NodeBuffers nb = nl.at(node_base, geom);
+    const int *first = nl.sort(node_base).first;
+    const bool cells = bp.nodes > 1;
     void *fs = nf ? (sc ? (void *)node_sum_kernel<true, true, false> : (void *)node_sum_kernel<true, false, false>)
                   : (so ? (void *)node_sum_kernel<false, false, true> : (void *)node_sum_kernel<false, false, false>);
     if (dbl)
@@ -1638,20 +2105,29 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
                   : (sc ? (void *)node_interp_x_kernel<false, true> : (void *)node_interp_x_kernel<false, false>);
     idiwf_status st = ensure_smem((void *)node_interp_y_kernel, sizeof(GemmSmem));
     if (st == IDIWF_OK) st = ensure_smem(fx, sizeof(GemmSmem));
+    if (st == IDIWF_OK) st = ensure_smem((void *)cell_interp_kernel, sizeof(GemmSmem));
+    if (st == IDIWF_OK) st = ensure_smem((void *)cell_expand_kernel, sizeof(ExpandSmem));
     if (st != IDIWF_OK) return st;
     const int grid = std::min(sm_count() * resident_ctas(fs, kNodeThreads, 0), kMaxCtas);
+    const int egrid = sm_count() * resident_ctas((void *)cell_expand_kernel, kGemmThreads, sizeof(ExpandSmem));
     const int ty = (g.ny + kGemmM - 1) / kGemmM * ((node_cap(g.nx) + kGemmN - 1) / kGemmN);
     const int tx = (g.nx + kGemmM - 1) / kGemmM * ((g.ny + kGemmN - 1) / kGemmN);
     for (int i0 = 0; i0 < bp.n_images; i0 += nl.group) {
         int i1 = std::min(i0 + nl.group, bp.n_images);
         const int n = i1 - i0;
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(nb.v, 0, (size_t)n * nb.entries * 16, stream));
-        void *as[] = {(void *)&bp, (void *)&g, dbl ? (void *)dbl : (void *)split, &plan, &nb.v, &nb.entries, &hdr, &cta_ns, &i0, &i1};
+        // (about two blocks per SM over the group's images)
+        const int per = std::max(1, (2 * sm_count() + n - 1) / n);
+        node_zero_kernel<<<dim3(per, n), 256, 0, stream>>>(plan, nb, i0);
+        void *as[] = {(void *)&bp, (void *)&g, dbl ? (void *)dbl : (void *)split, &plan, (void *)&nb, &first, &hdr, &cta_ns, &i0, &i1};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), as, 0, stream));
         node_weights_kernel<<<dim3((g.nx + g.ny + 15) / 16, n), 256, 0, stream>>>(g, plan, nb, i0);
+        if (cells) {
+            cell_interp_kernel<<<dim3(4 * per, n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
+            cell_expand_kernel<<<egrid, kGemmThreads, sizeof(ExpandSmem), stream>>>(g, ng, plan, nb, i0, i1);
+        }
         node_interp_y_kernel<<<dim3(std::min(ty, 64), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
         IDIWF_CUDA_CHECK(cudaGetLastError());
-        void *ax[] = {(void *)&g, &plan, &nb, &i0, &out, &out_kind};
+        void *ax[] = {(void *)&g, &plan, (void *)&nb, &i0, &out, &out_kind};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fx, dim3(std::min(tx, 4096), n), dim3(kGemmThreads), ax, sizeof(GemmSmem), stream));
     }
     return IDIWF_OK;
@@ -1698,7 +2174,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                       (size_t)i0 * npix * (out_kind == IDIWF_OUT_C128 ? 16 : (out_kind == IDIWF_OUT_I32 ? 4 : 8));
 
     // prep
-    const NodeLayout nl = bp.nodes ? node_layout(geom, b->n_images) : NodeLayout{};
+    const NodeLayout nl = bp.nodes ? node_layout(geom, b, bp.nodes) : NodeLayout{};
     char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, precision, nrec, ksplit) : 0);
     NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
     const NodeGeom ng = make_node_geom(g);
@@ -1707,9 +2183,13 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
     IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter, 0, sizeof(uint32_t), stream));
     if (precision == IDIWF_SPLIT) {
         IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter2, 0, 3 * sizeof(uint32_t), stream));
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * 4 * kMaxImagesPerLaunch,
-                                         stream));
+        if (!plan)
+            IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
+    } else if (plan) {
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), stream));
     }
+    uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
+    if (plan) IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, (size_t)kMaxImagesPerLaunch * 4 * kNodeExt, stream));
     if (max_tiles > 0 || plan) {  // (the prep kernel also writes the plan)
         dim3 pgrid((unsigned)std::max<int64_t>(std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), 1),
                    bp.n_images);
@@ -1717,16 +2197,26 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
             const int w_mode = (geom->flags & IDIWF_NF) ? 1 : ((geom->flags & IDIWF_SECONDORDER) ? 2 : 0);
             // emitter coordinates must keep |q.r| inside the magic binade
             const double max_abs = kMaxTurns / (3.0 * 2.0 * geom->k * kInvTwoPi);
-            prep_split_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
-                                                         max_abs, split_recs(ws, nrec), hdr, g, ng, plan);
-        } else {
-            uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
-            if (plan) {
-                IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), stream));
-                IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, kMaxImagesPerLaunch * 16, stream));
+            const CellSort cs = nl.sort(node_base);
+            if (bp.nodes > 1) {
+                // extents and plan, the emitters' sort by cell, then the records
+                int nbig = 0;
+                for (int i = 0; i < bp.n_images; ++i) nbig = std::max(nbig, bp.img[i].n);
+                node_extents_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, ext, hdr, g,
+                                                               ng, nl.caps, plan);
+                cell_count_kernel<<<dim3((nbig + kCellSort - 1) / kCellSort, bp.n_images), 256, 0, stream>>>(
+                    bp, b->atoms, ng, plan, cs);
+                prep_split_kernel<false><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
+                                                                    max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
+                                                                    nl.caps, plan, cs);
+            } else {
+                prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
+                                                                   max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
+                                                                   nl.caps, plan, cs);
             }
+        } else {
             prep_double_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype,
-                                                          double_recs(ws, nrec), hdr, g, ng, ext, plan);
+                                                          double_recs(ws, nrec), hdr, g, ng, ext, nl.caps, plan);
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
@@ -1772,7 +2262,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                                                                             out_chunk, out_kind, plan);
             IDIWF_CUDA_CHECK(cudaGetLastError());
         }
-        if (plan) return launch_nodes(geom, g, bp, &rec, nullptr, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
+        if (plan) return launch_nodes(geom, g, ng, bp, &rec, nullptr, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     } else {
         DoubleRecs rec = double_recs(ws, nrec);
         void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns, &plan};
@@ -1782,7 +2272,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
         idiwf_status st = grid_for(fn, smem, grid);
         if (st != IDIWF_OK) return st;
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(s.threads), args, smem, stream));
-        if (plan) return launch_nodes(geom, g, bp, nullptr, &rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
+        if (plan) return launch_nodes(geom, g, ng, bp, nullptr, &rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     }
     return IDIWF_OK;
 }
@@ -1795,10 +2285,9 @@ static idiwf_status forward_impl(const idiwf_geom *geom, const idiwf_batch *b, i
         return set_error(IDIWF_ERR_WORKSPACE, "workspace smaller than idiwf_forward_workspace_size()");
     if (reinterpret_cast<uintptr_t>(ws) & 255) return set_error(IDIWF_ERR_WORKSPACE, "workspace must be 256-byte aligned");
     std::vector<int64_t> rec_base(b->n_images + 1, 0);
-    for (int i = 0; i < b->n_images; ++i) {
-        const int64_t n = b->offsets[i + 1] - b->offsets[i];
-        rec_base[i + 1] = rec_base[i] + (n + s.te - 1) / s.te * s.te;
-    }
+    const int nodes = nodes_possible(geom, b, precision, s);
+    for (int i = 0; i < b->n_images; ++i)
+        rec_base[i + 1] = rec_base[i] + image_records(b->offsets[i + 1] - b->offsets[i], s.te, nodes);
     const int64_t nrec = std::max<int64_t>(rec_base[b->n_images], 1);
     // reset the work counter and the error word: errors reported by
     // idiwf_workspace_error() are those of the most recent call
@@ -2048,8 +2537,9 @@ extern "C" idiwf_status idiwf_forward_noalloc(const idiwf_geom *geom, const idiw
         const int w_mode = (geom->flags & IDIWF_NF) ? 1 : ((geom->flags & IDIWF_SECONDORDER) ? 2 : 0);
         const double max_abs = kMaxTurns / (3.0 * 2.0 * geom->k * kInvTwoPi);
         dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), bp.n_images);
-        prep_split_kernel<<<pgrid, 256, 0, stream>>>(bp, batch->atoms, batch->amplitudes, batch->amp_dtype, w_mode,
-                                                     max_abs, rec, hdr, g, NodeGeom{}, nullptr);
+        prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, batch->atoms, batch->amplitudes, batch->amp_dtype, w_mode,
+                                                           max_abs, rec, hdr, g, NodeGeom{}, nullptr, NodeCaps{},
+                                                           nullptr, CellSort{});
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
     double2 *no_partials = nullptr;  // bp.ksplit == 0: the kernels write the outputs themselves

@@ -8,9 +8,9 @@
 // points of a tensor Chebyshev grid (first kind) laid over the whole
 // detector, and the pixels follow by polynomial interpolation, two real
 // contractions in FP64: E = L_x V L_y^T.  Measured on a B200, whole calls: two
-// images of 50,000 emitters on 1024^2 pixels (64^2 nodes) 0.69 ms against 57.9 ms by
-// the direct kernels; eight of 2,000 on 256^2 0.26 against 0.80 ms; field error
-// against FP64 9e-8 against 2.1e-7.  The adjoint runs the transpose: the
+// images of 50,000 emitters on 1024^2 pixels (66^2 nodes) 0.69 ms against 57.9 ms by
+// the direct kernels, 0.39 ms with the emitters cut into cells (below); eight of 2,000 on
+// 256^2 0.25 against 0.80 ms; field error against FP64 1.0e-7 against 2.1e-7.  The adjoint runs the transpose: the
 // pixel weights are contracted onto the nodes, and the adjoint sum runs over
 // nodes in place of pixels.
 //
@@ -37,7 +37,7 @@ constexpr int kPathNodes = 4;        // split_path() continued: nodes and interp
 constexpr int kNodeMax = 1024;       // nodes per axis
 constexpr double kNodeMaxT = 0.6;
 constexpr int kNodeThreads = 128;    // node kernel: threads per CTA, nodes per thread, emitters per stage
-constexpr int kNodePPT = 4;
+constexpr int kNodePPT = 2;
 constexpr int kNodeTile = kNodeThreads * kNodePPT;
 constexpr int kNodeTE = 128;
 constexpr int kNodePPT64 = 2;        // FP64: nodes per thread
@@ -47,32 +47,70 @@ constexpr int kNodeBlock = 64;       // emitters per work item and tile
 // and cosine polynomials take on top of the half turn (they hold to 1.04 half turns).
 constexpr double kNodeMaxExtra = 0.06;
 
+// Cells: a large or dense object is cut into boxes along the detector axes and the beam.
+// A box's field, with the phase of its centre taken out, has the box's band limit, so its
+// emitters are summed on a grid of far fewer nodes; the boxes' fields are then
+// interpolated to the target grid (the image's nodes, or the pixels themselves) and added
+// up with the phases of their centres.  The plan weighs the cells' sums, which shrink
+// with the cell, against the interpolation, which grows with their number.  Measured, with
+// cells against without (whole calls): 24 images of 1,000 to 100,000 emitters on 512^2
+// pixels 3.1 against 11.7 ms; 300,000 emitters in a micrometre on 128^2 pixels, which
+// undersample it, 1.20 against 3.30 ms (direct).
+constexpr int kCellMax = 512;        // cells per image
+constexpr int kCellNodes = 64;       // nodes per axis of a cell's grid
+constexpr int kCellMinEmitters = 4096;  // images below this are not cut
+constexpr int kCellSort = 1024;      // emitters per block of the sort
+
 // Node geometry of a detector (host side, make_node_geom): Phi per unit of
 // emitter extent, curvature ratios, and the largest |d_hat . e| along each axis.
 struct NodeGeom {
-    double e[2][3];  // unit vectors of the detector axes
+    double e[3][3];  // unit vectors of the detector axes and their normal
     double phi[2], t[2], s[2];
     double inv_d;
-    int32_t ok;
+    int32_t ok, ortho;  // ortho: the axes are orthonormal (cells need it)
 };
 
 struct NodeImage {
     int64_t w0;         // work (tiles x blocks of kNodeBlock emitters) of the images before it
     int32_t path;       // split path of the image
-    int32_t n0, n1;     // nodes along x and y
-    int32_t ntiles, nblk;
+    int32_t n0, n1;     // target grid: nodes along x and y, or (pix) the pixels
+    int32_t pix;
+    int32_t ntiles, nblk;  // node tiles of a sum (of each cell), blocks of emitters (in all)
     float scale;        // power of two: the node sums are kept as fixed point, value x scale
+    int32_t ncell;      // 1: the sum goes straight to the target grid
+    int32_t c[3];       // cells along the detector axes and the normal
+    int32_t g0, g1;     // nodes of a cell's grid
+    uint32_t ticket;    // finished blocks of the sort's count kernel
+    double lo[3], size[3], inv[3];  // cells: origin, edges, 1/edges
 };
 struct NodePlan {
     int64_t total;      // work of all images
     int64_t pad;
     NodeImage img[kMaxImagesPerLaunch];
 };
+// What the buffers of an image hold: sums on the target grid, sums of the cells, and the
+// cells' sums interpolated along one axis.
+struct NodeCaps {
+    int64_t v, f, y;
+};
 
 // Node sums of an image (16 bytes each), and the node limits along each axis that
 // the weight and intermediate arrays hold.
 __host__ __device__ inline int64_t node_entries(int64_t npix) { return npix / 4 + 4096; }
 __host__ __device__ inline int node_cap(int n) { return (n / 2 + 64 < kNodeMax ? n / 2 + 64 : kNodeMax) / 2 * 2; }
+
+__host__ __device__ inline NodeCaps node_caps(int64_t npix, int64_t nmax, bool cells) {
+    NodeCaps c;
+    c.v = node_entries(npix);
+    c.f = c.y = 0;
+    if (cells) {
+        const int64_t n = nmax / 64 < kCellMax ? nmax / 64 : kCellMax;
+        if (npix <= (1 << 18) && c.v < npix) c.v = npix;  // the pixels as the target
+        c.f = n * 2304 < (1 << 19) ? n * 2304 : (1 << 19);
+        c.y = n * 16384 < 3 * (1 << 20) ? n * 16384 : 3 * (1 << 20);
+    }
+    return c;
+}
 
 NodeGeom make_node_geom(const GeomParams &g);
 
@@ -85,22 +123,20 @@ __device__ __forceinline__ int node_count(double phi, double t, bool fine) {
     return n < (double)(2 * kNodeMax) ? ((int)ceil(n) + 1) / 2 * 2 : 2 * kNodeMax;
 }
 
-// Nodes of an image from its largest |r|^2 and largest |r . e| along the two
-// detector axes (float bits, rounded up); false when no grid within the limits
-// exists.  Along e the phase changes by at most k/|d| (|r . e| + |d_hat . e| |r|),
-// and by no more than k/|d| |r|; the near-field and second-order terms add up
-// to 2 |r|/|d| of that.
-__device__ __forceinline__ bool node_grid(const GeomParams &g, const NodeGeom &ng, uint32_t r2bits, uint32_t xbits,
-                                          uint32_t ybits, bool fine, int &n0, int &n1) {
-    const double r = sqrt((double)__uint_as_float(r2bits));
-    if (!ng.ok || !(r * ng.inv_d <= 0.25)) return false;  // (a NaN fails too)
-    if (!fine && (g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) && !(0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra)) return false;
-    const double f = 1.0 + 2.0 * r * ng.inv_d;
-    const double ex = fmin(r, (double)__uint_as_float(xbits) + ng.s[0] * r);
-    const double ey = fmin(r, (double)__uint_as_float(ybits) + ng.s[1] * r);
-    n0 = node_count(ng.phi[0] * ex * f, ng.t[0], fine);
-    n1 = node_count(ng.phi[1] * ey * f, ng.t[1], fine);
-    return n0 <= kNodeMax && n1 <= kNodeMax;
+// Whether an object reaching r from the origin may take nodes at all (a NaN may not).
+__device__ __forceinline__ bool node_reach(const GeomParams &g, const NodeGeom &ng, double r, bool fine) {
+    if (!ng.ok || !(r * ng.inv_d <= 0.25)) return false;
+    return fine || !(g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) || 0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra;
+}
+// Nodes along both axes for emitters within rho of a centre, |rho . e| <= ex, ey along the
+// axes, of an object reaching r from the origin.  Along e the phase changes by at most
+// k/|d| (|rho . e| + |d_hat . e| |rho|), and by no more than k/|d| |rho|; the
+// near-field and second-order terms, of the whole r, add up to 2 (|r|/|d|) k |r|/|d|.
+__device__ __forceinline__ void node_grid(const NodeGeom &ng, double r, double rho, double ex, double ey, bool fine,
+                                          int &n0, int &n1) {
+    const double more = 2.0 * r * r * ng.inv_d;
+    n0 = node_count(ng.phi[0] * (fmin(rho, ex + ng.s[0] * rho) + more), ng.t[0], fine);
+    n1 = node_count(ng.phi[1] * (fmin(rho, ey + ng.s[1] * rho) + more), ng.t[1], fine);
 }
 
 // Node m of n on [-1, 1], its barycentric weight, and the (fractional) pixel
@@ -112,10 +148,12 @@ __device__ __forceinline__ double node_w(int n, int m) {
 }
 __device__ __forceinline__ double node_index(int n, int m, int N) { return 0.5 * (N - 1) * (1.0 + node_x(n, m)); }
 
-// Interpolation weights of one axis, row i: L[i][m], m < n, by the barycentric
+// Pixel i of N on [-1, 1].
+__device__ __forceinline__ double pixel_x(int N, int i) { return N > 1 ? (2 * i - (N - 1)) / (double)(N - 1) : 0.0; }
+
+// Interpolation weights of one axis at x, row i: L[i][m], m < n, by the barycentric
 // formula (Berrut and Trefethen, SIAM Review 46(3), 2004), one warp per row.
-__device__ __forceinline__ void node_weights_row(double *__restrict__ L, int n, int N, int i, int lane) {
-    const double x = N > 1 ? (2 * i - (N - 1)) / (double)(N - 1) : 0.0;
+__device__ __forceinline__ void node_weights_row(double *__restrict__ L, int n, double x, int i, int lane) {
     double sum = 0.0;
     for (int m = lane; m < n; m += 32) {
         double d = x - node_x(n, m);
@@ -134,36 +172,44 @@ __device__ __forceinline__ void node_weights_row(double *__restrict__ L, int n, 
 // further kernels cost more than the direct sum (split precision, FP64).
 constexpr double kNodeMinPairs = 8e6, kNodeMinPairs64 = 2e6;
 
-// Whether an image of n emitters goes through its n0 x n1 grid: the grid fits
-// the buffers, and the pairs saved outweigh the interpolation.  The rates are
-// the kernels' measured ones: direct pairs and node pairs per second, FP64
-// multiply-adds per second of the interpolation.  The choice depends on
-// the image and the geometry alone, as split_path's does.
-__device__ __forceinline__ bool nodes_pay(int n, int nx, int ny, int n0, int n1, double direct_rate, double node_rate,
-                                          double min_pairs = kNodeMinPairs) {
-    const double npix = (double)nx * ny, m = (double)n0 * n1, pairs = (double)n * npix;
-    if (n0 > node_cap(nx) || n1 > node_cap(ny) || m > 0.25 * npix + 4096.0 || pairs < min_pairs) return false;
-    const double mads = 2.0 * n0 * (npix + (double)n1 * ny);
-    return n * m / node_rate + (mads + 100.0 * npix) * (1.0 / 1.2e13) < pairs / direct_rate;
+// Floats as unsigned integers in their order (0 lies below them all).
+__device__ __forceinline__ uint32_t float_key(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float key_float(uint32_t k) {
+    return __uint_as_float(k & 0x80000000u ? k & 0x7fffffffu : ~k);
 }
 
-// Largest extents of an emitter for the plan: |r|^2, |r . e| along both detector axes, |a|
-// (float bits, rounded up), raised per warp into ext (kMaxImagesPerLaunch of each).
+// Largest extents of an emitter for the plan: |r|^2 and |a| (float bits, rounded up), and
+// r . e and -r . e along the three axes (keys, rounded up), raised per warp into ext
+// (kMaxImagesPerLaunch of each).
+constexpr int kNodeExt = 8;
 struct NodeExtents {
-    uint32_t r2 = 0, e0 = 0, e1 = 0, a = 0;
+    uint32_t v[kNodeExt] = {0, 0, 0, 0, 0, 0, 0, 0};
     __device__ __forceinline__ void add(const NodeGeom &ng, const double4 &p, float amp) {
-        r2 = max(r2, __float_as_uint(__double2float_ru((p.x * p.x + p.y * p.y) + p.z * p.z)));
-        e0 = max(e0, __float_as_uint(__double2float_ru(fabs(p.x * ng.e[0][0] + p.y * ng.e[0][1] + p.z * ng.e[0][2]))));
-        e1 = max(e1, __float_as_uint(__double2float_ru(fabs(p.x * ng.e[1][0] + p.y * ng.e[1][1] + p.z * ng.e[1][2]))));
-        a = max(a, __float_as_uint(fabsf(amp)));
-    }
-    __device__ __forceinline__ void raise(uint32_t *ext, int b) const {
-        const uint32_t v[4] = {r2, e0, e1, a};
+        v[0] = max(v[0], __float_as_uint(__double2float_ru((p.x * p.x + p.y * p.y) + p.z * p.z)));
+        v[1] = max(v[1], __float_as_uint(fabsf(amp)));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t m = __reduce_max_sync(0xffffffffu, v[k]);
-            if ((threadIdx.x & 31) == 0 && m) atomicMax(ext + k * kMaxImagesPerLaunch + b, m);
+        for (int k = 0; k < 3; ++k) {
+            const double x = p.x * ng.e[k][0] + p.y * ng.e[k][1] + p.z * ng.e[k][2];
+            v[2 + k] = max(v[2 + k], float_key(__double2float_ru(x)));
+            v[5 + k] = max(v[5 + k], float_key(__double2float_ru(-x)));
         }
+    }
+    // (one atomic per block and extent: a warp's own would queue up on the image's words)
+    __device__ __forceinline__ void raise(uint32_t *ext, int b) const {
+        __shared__ uint32_t s_max[kNodeExt];
+        if (threadIdx.x < kNodeExt) s_max[threadIdx.x] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kNodeExt; ++k) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, v[k]);
+            if ((threadIdx.x & 31) == 0 && m) atomicMax(&s_max[k], m);
+        }
+        __syncthreads();
+        if (threadIdx.x < kNodeExt && s_max[threadIdx.x])
+            atomicMax(ext + threadIdx.x * kMaxImagesPerLaunch + b, s_max[threadIdx.x]);
     }
 };
 // True in every thread of the grid's last block to get here (a ticket in the header);
@@ -177,49 +223,150 @@ __device__ __forceinline__ bool last_block(WsHeader *hdr) {
     return s_last != 0;
 }
 
-// Plan of one launch, by one block: every image's path, grid, fixed-point scale and
-// share of the work.  fine: the FP64 kernel's images (their direct path counts as
-// kPathPixel).  ext: per image max |r|^2, then max |r . e| along the two axes,
-// then max |a| (float bits), kMaxImagesPerLaunch each.
+// Seconds of an image's evaluation on nodes: the sums, the cells' interpolation to the
+// target grid and their phases, and the last interpolation to the pixels; rates
+// as measured (node pairs per second; FP64 multiply-adds per second).
+__device__ __forceinline__ double node_cost(double n, int nx, int ny, const NodeImage &ni, double pair_rate) {
+    const double npix = (double)nx * ny, m = (double)((ni.g0 * ni.g1 + 127) / 128) * 128.0;
+    double t = (n + 32.0 * ni.ncell) * m / pair_rate;
+    if (ni.ncell > 1) {
+        const double t0 = (ni.n0 + 31) / 32 * 32.0, t1 = (ni.n1 + 31) / 32 * 32.0;
+        t += ni.ncell * (2.0 * ((ni.n1 + 63) / 64 * 64.0) * ((ni.g0 + 31) / 32 * 32.0) * ni.g1 * (1.0 / 0.9e13) +
+                         t0 * t1 * (2.0 * ni.g0 * (1.0 / 0.9e13) + 1.6e-12));
+    }
+    if (!ni.pix) t += 2.0 * ni.n0 * (npix + (double)ni.n1 * ny) * (1.0 / 1.2e13);
+    return t + 100.0 * npix * (1.0 / 1.2e13);
+}
+
+// Plan of one launch, by one block: every image's path, grids, fixed-point scale and
+// share of the work; one warp per image, whose lanes try the ways to cut it.  The choice
+// depends on the image and the geometry alone, as split_path's does.  fine: the FP64
+// kernel's images (their direct path counts as kPathPixel).
 __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, const NodeGeom &ng,
-                                  const uint32_t *ext, bool fine, WsHeader *hdr, NodePlan *plan) {
+                                  const uint32_t *ext, bool fine, NodeCaps caps, WsHeader *hdr, NodePlan *plan) {
     __shared__ long long s_work[kMaxImagesPerLaunch];
     __threadfence();
-    const int npix = g.nx * g.ny;
-    unsigned long long pairs = 0;
-    for (int i = threadIdx.x; i < bp.n_images; i += blockDim.x) {
-        const uint32_t r2 = __ldcg(ext + i), amax = __ldcg(ext + 3 * kMaxImagesPerLaunch + i);
+    const int npix = g.nx * g.ny, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < bp.n_images; i += blockDim.x >> 5) {
+        uint32_t x[kNodeExt];
+#pragma unroll
+        for (int k = 0; k < kNodeExt; ++k) x[k] = __ldcg(ext + k * kMaxImagesPerLaunch + i);
         const int n = bp.img[i].n;
+        const uint32_t amax = x[1];
         NodeImage ni;
-        ni.path = fine ? kPathPixel : split_path(g, r2, bp.groups != 0, false);
+        ni.path = fine ? kPathPixel : split_path(g, x[0], bp.groups != 0, false);
         ni.w0 = 0;
-        ni.n0 = ni.n1 = ni.ntiles = ni.nblk = 0;
+        ni.n0 = ni.n1 = ni.g0 = ni.g1 = ni.pix = ni.ntiles = ni.nblk = 0;
         ni.scale = 1.0f;
+        ni.ncell = ni.c[0] = ni.c[1] = ni.c[2] = 1;
+        ni.ticket = 0;
+        const double r = sqrt((double)__uint_as_float(x[0]));
+        const double pairs = (double)n * npix;
+        const int direct = ni.path;
         unsigned long long pr = (unsigned long long)n * npix;
-        if (bp.nodes && (ni.path == kPathRuns || ni.path == kPathPixel) &&
-            // (amplitudes whose fixed-point unit would leave FP32's exponents, infinite or NaN
-            // ones take the direct kernels)
-            (amax == 0u || (amax >= __float_as_uint(0x1p-40f) && amax <= __float_as_uint(0x1p100f))) &&
-            node_grid(g, ng, r2, __ldcg(ext + kMaxImagesPerLaunch + i), __ldcg(ext + 2 * kMaxImagesPerLaunch + i),
-                      fine, ni.n0, ni.n1) &&
-            (fine ? nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, 1.6e11, 1.3e11, kNodeMinPairs64)
-                  : nodes_pay(n, g.nx, g.ny, ni.n0, ni.n1, ni.path == kPathRuns ? 1.8e12 : 1.5e12, 1.0e12))) {
-            ni.path = kPathNodes;
-            const int m = ni.n0 * ni.n1;
-            const int tile = fine ? kNodeTile64 : kNodeTile;
-            ni.ntiles = (m + tile - 1) / tile;
-            ni.nblk = (n + kNodeBlock - 1) / kNodeBlock;
-            pr = (unsigned long long)n * m;
-            // |sum| <= n max |a| [times the largest 1/|d - r| <= 4/(3 D)] < 2^e
-            double bound = (double)n * (double)__uint_as_float(amax);
-            if ((g.flags & IDIWF_NF) && (g.flags & IDIWF_SCALE)) bound *= 1.4 * ng.inv_d;
-            if (bound > 0.0) ni.scale = (float)scalbn(1.0, min(max(60 - (ilogb(bound) + 1), -120), 120));
+        long long work = 0;
+        // (amplitudes whose fixed-point unit would leave FP32's exponents, infinite or NaN
+        // ones take the direct kernels)
+        if (bp.nodes && n > 0 && (direct == kPathRuns || direct == kPathPixel) &&
+            pairs >= (fine ? kNodeMinPairs64 : kNodeMinPairs) && node_reach(g, ng, r, fine) &&
+            (amax == 0u || (amax >= __float_as_uint(0x1p-40f) && amax <= __float_as_uint(0x1p100f)))) {
+            double lo[3], w[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = -(double)key_float(x[5 + k]);
+                w[k] = fmax((double)key_float(x[2 + k]) - lo[k], 1e-12 * r);
+            }
+            // the uncut object, about the origin
+            NodeImage best = ni;
+            node_grid(ng, r, r, fmax(lo[0] + w[0], -lo[0]), fmax(lo[1] + w[1], -lo[1]), fine, best.n0, best.n1);
+            best.g0 = best.n0;
+            best.g1 = best.n1;
+            const bool whole = best.n0 <= node_cap(g.nx) && best.n1 <= node_cap(g.ny) &&
+                               (double)best.n0 * best.n1 <= (double)node_entries(npix);
+            const double rate = fine ? 1.3e11 : 1.0e12;
+            double cost = pairs / (fine ? 1.6e11 : (direct == kPathRuns ? 1.8e12 : 1.5e12));
+            bool use = false;
+            if (whole) {
+                const double c = node_cost(n, g.nx, g.ny, best, rate);
+                use = c < cost;
+                cost = fmin(c, cost);
+            }
+            if (bp.nodes > 1 && n >= kCellMinEmitters) {
+                // lanes 0..15: to the image's nodes, 16..31: to the pixels; edges of 1/2 .. 1/36
+                NodeImage cut = best;
+                cut.pix = lane >> 4;
+                if (cut.pix) {
+                    cut.n0 = g.nx;
+                    cut.n1 = g.ny;
+                }
+                const int ci = lane & 15, parts = ci < 6 ? ci + 2 : (ci < 10 ? 2 * ci - 4 : 4 * ci - 24);
+                const double edge = fmax(w[0], w[1]) / parts;
+                cut.c[0] = (int)fmin(ceil(w[0] / edge - 1e-9), 1e6);
+                cut.c[1] = (int)fmin(ceil(w[1] / edge - 1e-9), 1e6);
+                cut.c[2] = (int)fmin(ceil(w[2] * fmax(ng.s[0], ng.s[1]) / edge), 1e6);
+                cut.c[0] = max(cut.c[0], 1);
+                cut.c[1] = max(cut.c[1], 1);
+                cut.c[2] = max(cut.c[2], 1);
+                const double nc = (double)cut.c[0] * cut.c[1] * cut.c[2];
+                double c = 1e30;
+                if (nc > 1.0 && nc <= kCellMax && nc * 64.0 <= n && (cut.pix ? (double)npix <= (double)caps.v : whole)) {
+                    cut.ncell = (int)nc;
+                    double h[3];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        cut.lo[k] = lo[k];
+                        cut.size[k] = w[k] / cut.c[k];
+                        cut.inv[k] = cut.c[k] / w[k];
+                        h[k] = 0.5 * cut.size[k] * (1.0 + 1e-9);
+                    }
+                    node_grid(ng, r, sqrt(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]), h[0], h[1], fine, cut.g0, cut.g1);
+                    if (cut.g0 <= kCellNodes && cut.g1 <= kCellNodes && nc * cut.g0 * cut.g1 <= (double)caps.f &&
+                        nc * cut.n1 * cut.g0 <= (double)caps.y)
+                        c = node_cost(n, g.nx, g.ny, cut, rate);
+                }
+                double least = c;
+#pragma unroll
+                for (int o = 16; o; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
+                const int who = __ffs(__ballot_sync(0xffffffffu, c == least)) - 1;
+                if (least < 0.95 * cost) {
+                    use = true;
+                    // the winner's choice, to every lane
+                    best.pix = who >> 4;
+                    best.n0 = __shfl_sync(0xffffffffu, cut.n0, who);
+                    best.n1 = __shfl_sync(0xffffffffu, cut.n1, who);
+                    best.g0 = __shfl_sync(0xffffffffu, cut.g0, who);
+                    best.g1 = __shfl_sync(0xffffffffu, cut.g1, who);
+                    best.ncell = __shfl_sync(0xffffffffu, cut.ncell, who);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        best.c[k] = __shfl_sync(0xffffffffu, cut.c[k], who);
+                        best.lo[k] = lo[k];
+                        best.size[k] = w[k] / best.c[k];
+                        best.inv[k] = best.c[k] / w[k];
+                    }
+                }
+            }
+            if (use) {
+                ni = best;
+                ni.path = kPathNodes;
+                const int m = ni.g0 * ni.g1, tile = fine ? kNodeTile64 : kNodeTile;
+                ni.ntiles = (m + tile - 1) / tile;
+                ni.nblk = (n + kNodeBlock - 1) / kNodeBlock;  // (the sort replaces it where there are cells)
+                pr = (unsigned long long)n * m;
+                work = (long long)ni.ntiles * ni.nblk;
+                // |sum| <= n max |a| [times the largest 1/|d - r| <= 4/(3 D)] < 2^e; three bits to
+                // spare for the interpolated cells' partial sums
+                double bound = (double)n * (double)__uint_as_float(amax);
+                if ((g.flags & IDIWF_NF) && (g.flags & IDIWF_SCALE)) bound *= 1.4 * ng.inv_d;
+                if (bound > 0.0) ni.scale = (float)scalbn(1.0, min(max(59 - (ilogb(bound) + 1), -120), 120));
+            }
         }
-        pairs += pr;
-        s_work[i] = (long long)ni.ntiles * ni.nblk;
-        plan->img[i] = ni;
+        if (lane == 0) {
+            atomicAdd(&hdr->pairs, pr);
+            s_work[i] = work;
+            plan->img[i] = ni;
+        }
     }
-    atomicAdd(&hdr->pairs, pairs);
     __syncthreads();
     if (threadIdx.x == 0) {
         long long w = 0;
@@ -229,6 +376,31 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         }
         plan->total = w;
     }
+}
+
+// Cell of an emitter, and a cell's centre; written with explicit roundings so that every
+// kernel places an emitter alike.
+__device__ __forceinline__ int cell_of(const NodeGeom &ng, const NodeImage &ni, const double4 &p) {
+    int id = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double x = __fma_rn(p.z, ng.e[k][2], __fma_rn(p.y, ng.e[k][1], __dmul_rn(p.x, ng.e[k][0])));
+        const int c = min(max((int)floor(__dmul_rn(__dsub_rn(x, ni.lo[k]), ni.inv[k])), 0), ni.c[k] - 1);
+        id = id * ni.c[k] + c;
+    }
+    return id;
+}
+__device__ __forceinline__ void cell_centre(const NodeGeom &ng, const NodeImage &ni, int id, double r[3]) {
+    int c[3];
+    c[2] = id % ni.c[2];
+    c[1] = id / ni.c[2] % ni.c[1];
+    c[0] = id / (ni.c[2] * ni.c[1]);
+    double x[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[k] = __fma_rn(c[k] + 0.5, ni.size[k], ni.lo[k]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        r[a] = __fma_rn(x[2], ng.e[2][a], __fma_rn(x[1], ng.e[1][a], __dmul_rn(x[0], ng.e[0][a])));
 }
 
 // Sine and cosine of pi x, |x| <= 0.52: least-maximum polynomials in x^2, fitted for
@@ -299,10 +471,11 @@ union GemmSmem {
     double2 y[kGemmM * (kGemmN + 1)];  // the finished tile, for stores along rows
 };
 
-// One tile at (i0, j0); `store(i, j, re, im)` receives every element inside M x N.
-template <class Store>
+// One tile at (i0, j0); `store(i, j, re, im)` receives every element inside M x N.  FIXED: X
+// holds fixed-point sums (two 64-bit integers, value / unit).
+template <bool FIXED, class Store>
 __device__ __forceinline__ void interp_tile(GemmSmem &sm, const double *__restrict__ L, const double2 *__restrict__ X,
-                                            int M, int N, int K, int i0, int j0, const Store &store) {
+                                            int M, int N, int K, int i0, int j0, double unit, const Store &store) {
     const int tid = threadIdx.x, lane = tid & 31, wr = (tid >> 5) >> 1, wc = (tid >> 5) & 1;
     double acc[4][4][2];
 #pragma unroll
@@ -322,7 +495,13 @@ __device__ __forceinline__ void interp_tile(GemmSmem &sm, const double *__restri
         for (int q = 0; q < kGemmN * kGemmK / kGemmThreads; ++q) {
             const int c = tid + q * kGemmThreads, r = c / kGemmK, k = c % kGemmK;
             const bool ok = j0 + r < N && k0 + k < K;
-            cp_async16(&sm.b[s][r * kGemmLd + k], X + (ok ? (size_t)(j0 + r) * K + k0 + k : 0), ok);
+            if (FIXED) {
+                longlong2 v = make_longlong2(0, 0);
+                if (ok) v = reinterpret_cast<const longlong2 *>(X)[(size_t)(j0 + r) * K + k0 + k];
+                sm.b[s][r * kGemmLd + k] = make_double2((double)v.x * unit, (double)v.y * unit);
+            } else {
+                cp_async16(&sm.b[s][r * kGemmLd + k], X + (ok ? (size_t)(j0 + r) * K + k0 + k : 0), ok);
+            }
         }
         cp_async_commit();
     };

@@ -261,3 +261,43 @@ def test_adjoint_nodes_groups_and_large_counts():
         da, _ = _core.backward(at[lo:hi].contiguous(), [0, hi - lo], geom, E[b:b + 1].contiguous(),
                                gI[b:b + 1].contiguous(), config={"pixel_groups": -1})
         assert _err(one.cpu().numpy(), da.cpu().numpy()) < 1e-5, b
+
+
+@pytest.mark.parametrize("ndet,n,r,flat", [
+    ([64, 80], 100000, 0.15, 1.0),    # wider than the detector's sampling: cells straight to the pixels
+    ([200, 333], 9001, 0.03, 1.0),    # to the image's nodes; ragged in every direction
+    ([300, 500], 60000, 0.02, 0.01),  # a thin sheet (one layer of cells)
+    ([128, 128], 70000, 0.08, 0.3),
+])
+@pytest.mark.parametrize("settings", ["", "nf", "nf scale"])
+def test_forward_cells_vs_oracle(ndet, n, r, flat, settings):
+    """Objects cut into cells, tilted and off the origin, beside images that are not cut."""
+    g = rng(n)
+    pos = sphere(g, n, r) * [1, 1, flat] + [0.01, -0.02, 0.005]
+    at = atoms(pos, g.uniform(0, 2 * np.pi, n))
+    small = atoms(sphere(g, 900, 0.006), g.uniform(0, 2 * np.pi, 900))
+    amp = g.uniform(0.5, 1.5, n + 900).astype(np.float32)
+    flags, _, _ = _core.parse_settings(settings)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, (0.1, -0.2), flags=flags)
+    E, pairs = _forward(np.concatenate([small, at]), [0, 900, 900 + n], geom, amp)
+    assert pairs < (n + 900) * ndet[0] * ndet[1] / 2
+    og = oracle.geometry(ndet, 75.0, 1e5, K64, (0.1, -0.2))
+    of = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(og, of, at, amp[900:].astype(np.float64))
+    assert _err(E[1], ref) < FIELD_2NORM, _err(E[1], ref)
+    alone, _ = _forward(at, [0, n], geom, amp[900:])
+    assert np.array_equal(alone[0], E[1])
+
+
+def test_cells_degenerate_objects():
+    """All emitters at one point, on a line, and one far from the rest."""
+    g = rng(77)
+    n = 6000
+    geom = _core.make_geom([96, 96], 75.0, 1e5, K64, flags=nat.NF)
+    og = oracle.geometry([96, 96], 75.0, 1e5, K64)
+    for pos in (np.zeros((n, 3)) + [0.003, 0.001, -0.002],
+                np.stack([g.uniform(-0.1, 0.1, n), np.zeros(n), np.zeros(n)], 1),
+                np.concatenate([sphere(g, n - 1, 0.005), [[0.09, -0.08, 0.02]]])):
+        at = atoms(pos, g.uniform(0, 2 * np.pi, n))
+        E, _ = _forward(at, [0, n], geom)
+        assert _err(E[0], oracle.wavefield(og, oracle.NF | oracle.ACCURATE, at)) < FIELD_2NORM
