@@ -85,6 +85,7 @@ EXPORTED = (
     "idiwf_fft_autocorr_1d",
     "idiwf_tune",
     "idiwf_workspace_error",
+    "idiwf_error_collect",
     "idiwf_microbench",
     "idiwf_last_error_string",
     "idiwf_version",
@@ -252,6 +253,8 @@ def load():
     L.idiwf_tune.restype = st
     L.idiwf_workspace_error.argtypes = [vp, vp]
     L.idiwf_workspace_error.restype = st
+    L.idiwf_error_collect.argtypes = [vp, vp, ctypes.c_int32, vp]
+    L.idiwf_error_collect.restype = st
     L.idiwf_microbench.argtypes = [ctypes.c_int32, vp, vp, P(ctypes.c_double)]
     L.idiwf_microbench.restype = st
     L.idiwf_last_error_string.argtypes = []

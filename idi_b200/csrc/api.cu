@@ -100,6 +100,21 @@ extern "C" const char *idiwf_last_error_string(void) { return g_last_error.c_str
 
 extern "C" int32_t idiwf_version(void) { return (1 << 16) | 1; }
 
+namespace idiwf {
+__global__ void error_or_kernel(WsHeader *__restrict__ acc, const WsHeader *__restrict__ hdr) { acc->error |= hdr->error; }
+}  // namespace idiwf
+
+extern "C" idiwf_status idiwf_error_collect(void *acc, const void *workspace, int32_t first, cudaStream_t stream) {
+    if (!acc || !workspace) return set_error(IDIWF_ERR_INVALID_ARGUMENT, "acc or workspace is NULL");
+    if (first) {
+        IDIWF_CUDA_CHECK(cudaMemcpyAsync(acc, workspace, sizeof(WsHeader), cudaMemcpyDeviceToDevice, stream));
+        return IDIWF_OK;
+    }
+    error_or_kernel<<<1, 1, 0, stream>>>(static_cast<WsHeader *>(acc), static_cast<const WsHeader *>(workspace));
+    IDIWF_CUDA_CHECK(cudaGetLastError());
+    return IDIWF_OK;
+}
+
 extern "C" idiwf_status idiwf_workspace_error(const void *workspace, cudaStream_t stream) {
     if (!workspace) return set_error(IDIWF_ERR_INVALID_ARGUMENT, "workspace is NULL");
     WsHeader h;

@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <tuple>
@@ -2178,16 +2179,16 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
     char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, precision, nrec, ksplit) : 0);
     NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
     const NodeGeom ng = make_node_geom(g);
-    // work counters and the prep kernel's ticket (words 3 to 5; the error word, the
-    // CTA count and the pair count carry over from launch to launch of a call)
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter, 0, sizeof(uint32_t), stream));
-    if (precision == IDIWF_SPLIT) {
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter2, 0, 3 * sizeof(uint32_t), stream));
-        if (!plan)
-            IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
-    } else if (plan) {
-        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), stream));
+    // the header's counters and ticket; its error word and pair count add up over a
+    // call's launches, so only the first launch clears all of it
+    if (i0 == 0) {
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, offsetof(WsHeader, pad), stream));
+    } else {
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter, 0, sizeof(uint32_t), stream));
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(&hdr->work_counter2, 0, 3 * sizeof(uint32_t), stream));  // to the ticket
     }
+    if (precision == IDIWF_SPLIT && !plan)
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
     uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
     if (plan) IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, (size_t)kMaxImagesPerLaunch * 4 * kNodeExt, stream));
     if (max_tiles > 0 || plan) {  // (the prep kernel also writes the plan)
@@ -2289,10 +2290,6 @@ static idiwf_status forward_impl(const idiwf_geom *geom, const idiwf_batch *b, i
     for (int i = 0; i < b->n_images; ++i)
         rec_base[i + 1] = rec_base[i] + image_records(b->offsets[i + 1] - b->offsets[i], s.te, nodes);
     const int64_t nrec = std::max<int64_t>(rec_base[b->n_images], 1);
-    // reset the work counter and the error word: errors reported by
-    // idiwf_workspace_error() are those of the most recent call
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(ws, 0, 2 * sizeof(uint32_t), stream));
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(&static_cast<WsHeader *>(ws)->pairs, 0, sizeof(unsigned long long), stream));
     const int ksplit = precision == IDIWF_SPLIT ? choose_ksplit(geom, b) : 1;
     for (int i0 = 0; i0 < b->n_images; i0 += kMaxImagesPerLaunch) {
         const int i1 = std::min(b->n_images, i0 + kMaxImagesPerLaunch);

@@ -217,23 +217,27 @@ class ErrorWord:
     The library records device-side errors (emitters out of the split range, a
     near-field image outside the split kernels' range, a bounded wait that ran
     out) in the workspace header, and every call clears them.  Calls given an
-    ``ErrorWord`` OR their word into this 256-byte device buffer (laid out like
-    a workspace header) on their stream, without synchronising; :meth:`check`
-    reads it once (synchronises) and raises with the library's message."""
+    ``ErrorWord`` keep their words in this 256-byte device buffer (laid out like
+    a workspace header) on their stream, without synchronising: a copy of the
+    header for the first call (most have one), the others' words OR-ed in;
+    :meth:`check` reads it once (synchronises) and raises with the library's
+    message."""
 
     def __init__(self, device):
         self.device = torch.device(device)
-        self.buf = torch.zeros(256, dtype=torch.uint8, device=self.device)
-        self._word = self.buf[4:8].view(torch.int32)
+        self.buf = torch.empty(256, dtype=torch.uint8, device=self.device)
+        self._first = True
 
     def collect(self, workspace: torch.Tensor):
-        self._word.bitwise_or_(workspace[4:8].view(torch.int32))
+        nat.check(nat.load().idiwf_error_collect(self.buf.data_ptr(), workspace.data_ptr(), int(self._first),
+                                                 _stream(self.device)))
+        self._first = False
 
     def check(self):
-        lib = nat.load()
-        st = lib.idiwf_workspace_error(ctypes.c_void_p(self.buf.data_ptr()), _stream(self.device))
-        self._word.zero_()
-        nat.check(st)
+        if self._first:
+            return  # no call since the last check
+        self._first = True
+        nat.check(nat.load().idiwf_workspace_error(self.buf.data_ptr(), _stream(self.device)))
 
 
 def forward(

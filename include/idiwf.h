@@ -569,6 +569,12 @@ idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *batch, int32_
  * were outside the split-precision phase range. */
 idiwf_status idiwf_workspace_error(const void *workspace, cudaStream_t stream);
 
+/* Keeps the error word of the call that last used `workspace` in `acc` (256
+ * bytes of DEVICE memory, laid out like a workspace header), stream-ordered:
+ * first != 0 copies the header, first == 0 ORs the word into the one already
+ * there.  idiwf_workspace_error(acc, stream) then reports all of them. */
+idiwf_status idiwf_error_collect(void *acc, const void *workspace, int32_t first, cudaStream_t stream);
+
 /*
  * Pipe-throughput microbenchmark used to measure the roofline denominators:
  * kind 0 = MUFU sin+cos (ops/s), 1 = FP64 FMA (flop/s counted as 2 per FMA),
