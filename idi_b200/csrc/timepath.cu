@@ -7,63 +7,95 @@
 //   x_0 = a_0,  x_m = a_m + exp(-(t_m - t_{m-1})/tau) x_{m-1}
 //   I_p = sum_{m<n-1} -tau/2 |x_m|^2 expm1(-2 (t_{m+1}-t_m)/tau) + tau/2 |x_{n-1}|^2
 //
-// One CTA (512 threads) handles one pixel at a time; CTAs take chunks of
-// consecutive pixels from an atomic queue and walk each chunk in serpentine
-// order (row by row, every other row backwards), so consecutive pixels of a
-// CTA are detector neighbours.  Arrival times are computed in FP64 with the
-// exact rounding sequence of the reference (np.inner as
+// One CTA handles one pixel at a time, with 32 to 512 threads by the emitter
+// count, so that up to 16 pixels share an SM; CTAs take equal shares of consecutive
+// pixels and walk them in serpentine order (row by row, every other row backwards),
+// so consecutive pixels of a CTA are detector neighbours.  Arrival times are
+// computed in FP64 with the exact rounding sequence of the reference (np.inner as
 // fma(q2,z,fma(q1,y,q0*x)), IEEE division by c), so the keys -- and therefore
 // the sorted order -- are bit for bit those of the reference.
 //
 // Sorting.  Between neighbouring pixels the keys move by far less than their
 // spacing (the arrival-time spread of the emission times dominates the
 // geometric term), so the previous pixel's order is almost the new one.  The
-// kernel keeps the order in shared memory as position-ordered arrays of keys
-// (FP64) and 16-bit emitter indices, recomputes the keys in that order, and
-// repairs it with insertion sorts over windows of 40 positions, alternating
-// between two window grids offset by 20 until every window boundary is in
-// order (an exact check: each window is sorted, so the whole array is sorted
-// exactly when every boundary pair is).  After a bounded number of window
-// passes -- and for a CTA's first pixel -- the exact full sort runs: 8192
-// buckets by a monotone FP64 map of the key (so bucket order is key order),
-// insertion sort inside each bucket by (key, emitter index), and an on-chip
-// LSD radix sort (8 passes of 8 bits, per-warp ranking with __match_any_sync)
-// if a bucket overflows.  Every path sorts by (key, emitter index), so the
-// order does not depend on which one ran.
+// kernel keeps the order in shared memory as position-ordered 16-bit emitter
+// indices and the keys in a table by emitter, and repairs the order while it scans
+// it: short windows around the starts of the threads' runs, then every thread
+// streams its run through a sorted buffer of four entries (scan_run), with an exact
+// check.  Where that is not enough, insertion sorts over windows of one run each,
+// alternating between two window grids offset by half a run until every window
+// boundary is in order (each window is sorted, so the whole array is sorted exactly
+// when every boundary pair is).  After a bounded number of window passes -- and for
+// a CTA's first pixel -- the exact full sort runs: 16 buckets per thread by a
+// monotone FP64 map of the key (so bucket order is key order), insertion sort inside
+// each bucket by (key, emitter index), and an on-chip LSD radix sort (8 passes of 8
+// bits, per-warp ranking with __match_any_sync) if a bucket overflows.  Every path
+// sorts by (key, emitter index), so the order does not depend on which one ran.
 //
-// The decaying scan is one pass: each thread keeps its run of 40 positions as
+// The decaying scan is one pass: each thread keeps its run of up to 40 positions as
 // an affine map x -> D x + B plus three sums from which the run's share of the
 // interval integral follows once the block scan delivers the entering x.
+//
+// What bounds it.  20,000 emitters, 256 x 256 pixels (one CTA per SM), cycles per
+// pixel: key pass 12k (40 bytes per emitter from L2 at 64 B per cycle and SM), run
+// starts 4k, streaming scan 43k, run ends and block scan 6k.  The scan gathers one
+// 32-byte row per emitter, every lane from another line, and an SM issues one line
+// request to L2 in about two cycles, which is those 43k (measured by taking parts
+// out: without sine, cosine and expm1 43k, without the gather 26k).  15.3 ms, against
+// 18.2 ms when the order was repaired by a window pass of its own (18k cycles) ahead
+// of the scan.  Phases kept in shared memory beside the keys, where they fit (up to
+// 11,000 emitters), measured no faster: below 10,000 emitters it is FP64 and issue at
+// 16 warps per SM.
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "idiwf_internal.cuh"
 
 namespace idiwf {
 
-constexpr int kTimeThreads = 512;
+constexpr int kTimeThreads = 512;  // most threads of a CTA (time_kernel), all of them (time_kernel_large)
 constexpr int kTimeWarps = kTimeThreads / 32;
-constexpr int kTimeIPT = 40;                                 // items per thread
+constexpr int kTimeIPT = 40;                                 // most positions per thread
 constexpr int kTimeMaxN = kTimeThreads * kTimeIPT;           // 20480
-constexpr int kCoarse = 1024;                                 // coarse bins of the bucket map
-// Slots of the position-ordered index array: one pad slot after every 80
-// positions, so that the 40-position runs of a warp's threads start in
-// different banks when every thread walks its own run.
-constexpr int kSlotGroup = 2 * kTimeIPT;
-constexpr int kTimeSlots = kTimeMaxN + kTimeMaxN / kSlotGroup;
-__device__ __forceinline__ int slot(int m) { return m + m / kSlotGroup; }
-constexpr size_t kTimeSmem = (size_t)kTimeMaxN * 8           // key table (by emitter index)
-                             + (size_t)kTimeSlots * 2        // emitter index per sorted position
-                             + (size_t)kTimeWarps * 256 * 4  // per-warp digit counters
-                             + 256 * 4 + 1024                // digit bases + scan scratch
-                             + (kCoarse + 4) * 4;            // first fine bucket per coarse bin
-static_assert(kTimeSmem + 256 <= 232448, "time kernel shared memory above the per-block limit");
+constexpr int kCoarse = 1024;                                // coarse bins of the large kernel's bucket map
+
+// Shape of one on-chip pixel: `threads` threads of `ipt` positions each (even,
+// threads * ipt >= n).  The position-ordered index array has two pad slots after
+// every two runs, so that the runs of a warp's threads start in different banks
+// when every thread walks its own run, and a pair of positions (even, odd) stays
+// one 32-bit word.
+struct TimeShape {
+    int threads, ipt;
+    uint32_t inv_group;  // ceil(2^32 / (2 ipt)): m / (2 ipt) = umulhi(m, inv_group) for m < 2^15
+    int smem;            // dynamic shared memory, bytes
+};
+__device__ __forceinline__ int slot(const TimeShape &sh, int m) { return m + 2 * (int)__umulhi((uint32_t)m, sh.inv_group); }
+// Shared memory: key table by emitter, order slots, per-warp digit counters (the
+// bucket counters, 16 per thread of 16 bits, share them), digit bases or coarse
+// bins (2 per thread), and 8 doubles of scratch per warp.
+static TimeShape time_shape(int threads, int n) {
+    TimeShape s;
+    s.threads = threads;
+    s.ipt = 2 * std::max(1, (n + 2 * threads - 1) / (2 * threads));
+    s.inv_group = (uint32_t)((((uint64_t)1 << 32) + 2 * s.ipt - 1) / (uint64_t)(2 * s.ipt));
+    s.smem = threads * s.ipt * 8 + (threads * s.ipt + threads) * 2 + (threads / 32) * 1024 +
+             std::max(256, 2 * threads + 4) * 4 + (threads / 32) * 64;
+    return s;
+}
+// Shared memory of one SM and what each resident CTA takes beside its dynamic part.
+constexpr int kSmShared = 228 * 1024, kCtaShared = 1024 + 256;
+// The largest shape's (every launch sets this limit, whatever its own size, so that
+// calls from several threads do not lower it under one another).
+constexpr int kTimeSmemMax = kTimeMaxN * 8 + (kTimeMaxN + kTimeThreads) * 2 + kTimeWarps * 1024 +
+                             (2 * kTimeThreads + 4) * 4 + kTimeWarps * 64;
+static_assert(kTimeSmemMax + kCtaShared <= kSmShared, "time kernel shared memory above the per-block limit");
 // Window passes tried on the previous pixel's order before the full sort.
 constexpr int kWarmPasses = 8;
 // Failed warm starts in a row after which a CTA stops trying them.
 constexpr int kWarmMaxFails = 3;
-// Key of the padding positions n..kTimeMaxN-1 in a full sort: the positive NaN
+// Key of the padding positions from n on in a radix sort: the positive NaN
 // with the largest payload, whose order-preserving image is the largest of all
 // 64-bit patterns, so the radix sort leaves the padding behind every real key
 // (NaN keys included) and positions below n always hold real emitters.
@@ -116,6 +148,9 @@ __device__ __forceinline__ double div_rn(double a, double c, double ic) {
     const double r = __fma_rn(-c, q0, a);
     return __fma_rn(r, ic, q0);
 }
+
+// div_rn's range [2^-960, 2^1000] on the high word of |q0|: from kDivLow, kDivSpan wide.
+constexpr uint32_t kDivLow = (1023u - 960u) << 20, kDivSpan = 1960u << 20;
 
 // MK: divide by c with div_rn (the on-chip kernel) or the library division (the
 // large-count kernel, whose 64 registers the inlined correction would spill);
@@ -175,14 +210,14 @@ __device__ __forceinline__ void path_only(double dx, double dy, double dz, doubl
 // instructions of the polynomials).
 __constant__ double kInvFact[11] = {1.0,       1.0,        1.0 / 2,     1.0 / 6,      1.0 / 24,      1.0 / 120,
                                     1.0 / 720, 1.0 / 5040, 1.0 / 40320, 1.0 / 362880, 1.0 / 3628800};
-__device__ __forceinline__ double expm1_neg(double x) {
-    if (!(x <= 0.0625)) return expm1(-x);
+__device__ __forceinline__ double expm1_near(double x) {
     const double t = -x;
     double q = kInvFact[10];
 #pragma unroll
     for (int k = 9; k >= 1; --k) q = __fma_rn(q, t, kInvFact[k]);
     return t * q;  // t (1 + t/2! + ... + t^9/10!)
 }
+__device__ __forceinline__ double expm1_neg(double x) { return x <= 0.0625 ? expm1_near(x) : expm1(-x); }
 
 // sin and cos of x (FP64), for the time path's amplitudes.  Cody-Waite
 // reduction (W. J. Cody and W. Waite, Software Manual for the Elementary
@@ -202,12 +237,10 @@ __constant__ double kSinC[8] = {1.0 / 355687428096000.0, -1.0 / 1307674368000.0,
 __constant__ double kCosC[9] = {1.0 / 6402373705728000.0, -1.0 / 20922789888000.0, 1.0 / 87178291200.0,
                                 -1.0 / 479001600.0,       1.0 / 3628800.0,         -1.0 / 40320.0,
                                 1.0 / 720.0,              -1.0 / 24.0,             0.5};
-__device__ __forceinline__ void sincos_cw(double x, double &sn, double &cs) {
-    if (!(fabs(x) <= 0x1p30)) {
-        sincos(x, &sn, &cs);
-        return;
-    }
-    const double nd = rint(x * kCW[0]);
+__device__ __forceinline__ void sincos_near(double x, double &sn, double &cs) {
+    // rint by the 1.5 2^52 addition, whose sum holds n in its low bits (|n| < 2^31)
+    const double big = __fma_rn(x, kCW[0], 0x1.8p52);
+    const double nd = big - 0x1.8p52;
     double a = __fma_rn(-nd, kCW[1], x);
     a = __fma_rn(-nd, kCW[2], a);
     const double a2 = a * a;
@@ -219,29 +252,58 @@ __device__ __forceinline__ void sincos_cw(double x, double &sn, double &cs) {
 #pragma unroll
     for (int i = 1; i < 9; ++i) pc = __fma_rn(pc, a2, kCosC[i]);
     const double co = __fma_rn(-a2, pc, 1.0);
-    const int q = (int)(((long long)nd) & 3);
+    const int q = __double2loint(big) & 3;
     sn = (q & 1) ? co : s;
     cs = (q & 1) ? s : co;
     if (q == 1 || q == 2) cs = -cs;
     if (q >= 2) sn = -sn;
 }
 
-// CW: sine and cosine by sincos_cw (the on-chip kernel) or the library (the
-// 64-register large-count kernel).
-template <bool NF, bool SCALE, bool CW = true>
+// Amplitude by the library's sine and cosine (the 64-register large-count kernel;
+// the on-chip one evaluates positions in pairs below).
+template <bool NF, bool SCALE>
 __device__ __forceinline__ void amplitude(double k, double s, double psi, double dist, double &re, double &im) {
     double th;
     if (!NF) th = -__dsub_rn(__dmul_rn(s, k), psi);  // time.py:94 exp(-1j*(s*k-phases))
     else th = __dadd_rn(__dmul_rn(s, k), psi);       // simtime.cu:71 phase = s*k + w
     double sn, cs;
-    if (CW) sincos_cw(th, sn, cs);
-    else sincos(th, &sn, &cs);
+    sincos(th, &sn, &cs);
     if (SCALE) {
         cs = __ddiv_rn(cs, dist);
         sn = __ddiv_rn(sn, dist);
     }
     re = cs;
     im = sn;
+}
+
+// Phase of one emitter (and its distance), the argument of amplitude().
+template <bool NF>
+__device__ __forceinline__ void phase_of(double k, double dx, double dy, double dz, double dn, double q0, double q1,
+                                         double q2, const double4 &a, double &th, double &dist) {
+    double s;
+    path_only<NF>(dx, dy, dz, dn, q0, q1, q2, a, s, dist);
+    th = NF ? __dadd_rn(__dmul_rn(s, k), a.w) : -__dsub_rn(__dmul_rn(s, k), a.w);
+}
+
+// sincos_cw of two arguments and expm1_neg of two gaps, with one range check for
+// both so that the four (two) polynomials run side by side.
+__device__ __forceinline__ void sincos_pair(double x0, double x1, double &s0, double &c0, double &s1, double &c1) {
+    if (!(fabs(x0) <= 0x1p30 && fabs(x1) <= 0x1p30)) {
+        sincos(x0, &s0, &c0);
+        sincos(x1, &s1, &c1);
+        return;
+    }
+    sincos_near(x0, s0, c0);
+    sincos_near(x1, s1, c1);
+}
+__device__ __forceinline__ void expm1_neg_pair(double x0, double x1, double &e0, double &e1) {
+    if (!(x0 <= 0.0625 && x1 <= 0.0625)) {
+        e0 = expm1_neg(x0);
+        e1 = expm1_neg(x1);
+        return;
+    }
+    e0 = expm1_near(x0);
+    e1 = expm1_near(x1);
 }
 
 // Block-wide min / max of the keys; result broadcast through smem (2 doubles).
@@ -260,7 +322,7 @@ __device__ __forceinline__ void block_minmax(double &lo, double &hi, double *sm)
     __syncthreads();
     lo = sm[0];
     hi = sm[1];
-    for (int w = 1; w < kTimeWarps; ++w) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) {
         lo = fmin(lo, sm[2 * w]);
         hi = fmax(hi, sm[2 * w + 1]);
     }
@@ -273,24 +335,24 @@ __device__ __forceinline__ void block_minmax(double &lo, double &hi, double *sm)
 // The map has two levels so that buckets hold about the same number of keys
 // whatever the keys' distribution (arrival times are near-Gaussian, and a
 // linear map crowds the middle buckets, whose insertion sort then holds the
-// whole CTA at the next barrier): u = (t - kmin) kCoarse / (kmax - kmin) picks
+// whole CTA at the next barrier): u = (t - kmin) (coarse bins) / (kmax - kmin) picks
 // coarse bin c = floor(u); coarse bin c owns the fine buckets [B_c, B_c+1),
-// B_c = c + floor(P_c (kBuckets - kCoarse) / n) with P_c the keys below bin c
+// B_c = c + floor(P_c (buckets - coarse bins) / n) with P_c the keys below bin c
 // (at least one bucket per coarse bin), and the key goes to fine bucket
 // B_c + floor((u - c) (B_c+1 - B_c)), clamped into the bin's range.  Every step
 // is monotone in t.  Returns false (perm undefined) when a bucket holds more
-// than kMaxBucket keys; the caller then runs the radix sort.  cnt: kBuckets/2
-// words of packed 16-bit counters; coarse: kCoarse + 1 words.
-constexpr int kBuckets = 8192;
+// than kMaxBucket keys; the caller then runs the radix sort.  16 buckets and 2
+// coarse bins per thread; cnt: 8 words of packed 16-bit counters per thread.
 constexpr int kMaxBucket = 128;
-constexpr int kBucketsPerThread = kBuckets / kTimeThreads;  // 16
-constexpr int kCoarsePerThread = kCoarse / kTimeThreads;    // 2
+constexpr int kBucketsPerThread = 16;
+constexpr int kCoarsePerThread = 2;
 
-__device__ __forceinline__ int coarse_of(double u) { return min(max(__double2int_rz(u), 0), kCoarse - 1); }
+__device__ __forceinline__ int coarse_of(double u, int ncoarse) { return min(max(__double2int_rz(u), 0), ncoarse - 1); }
 
-__device__ __forceinline__ uint32_t fine_bucket(double t, double kmin, double scale, const uint32_t *coarse) {
+__device__ __forceinline__ uint32_t fine_bucket(double t, double kmin, double scale, const uint32_t *coarse,
+                                                int ncoarse) {
     const double u = __dmul_rn(__dsub_rn(t, kmin), scale);
-    const int c = coarse_of(u);
+    const int c = coarse_of(u, ncoarse);
     const uint32_t b0 = coarse[c], nb = coarse[c + 1] - b0;
     const int f = __double2int_rz(__dmul_rn(__dsub_rn(u, (double)c), (double)nb));
     return b0 + (uint32_t)min(max(f, 0), (int)nb - 1);
@@ -302,20 +364,21 @@ __device__ __forceinline__ uint32_t cnt_get(const uint32_t *cnt, uint32_t b) {
 
 __device__ bool bucket_sort(const double *keytab, uint16_t *perm, uint32_t *cnt, uint32_t *coarse, int n,
                             double kmin, double kmax, double *scratch, int *s_flag) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
+    const int nbuckets = kBucketsPerThread * T, ncoarse = kCoarsePerThread * T;
     if (!(kmax > kmin)) {
         // all keys equal (or one key): stable order is emitter order
-        for (int m = tid; m < n; m += kTimeThreads) perm[m] = (uint16_t)m;
+        for (int m = tid; m < n; m += T) perm[m] = (uint16_t)m;
         __syncthreads();
         return true;
     }
-    const double scale = (double)kCoarse / (kmax - kmin);
-    for (int w = tid; w < kBuckets / 2; w += kTimeThreads) cnt[w] = 0u;
-    for (int c = tid; c <= kCoarse; c += kTimeThreads) coarse[c] = 0u;
+    const double scale = (double)ncoarse / (kmax - kmin);
+    for (int w = tid; w < nbuckets / 2; w += T) cnt[w] = 0u;
+    for (int c = tid; c <= ncoarse; c += T) coarse[c] = 0u;
     if (tid == 0) *s_flag = 0;
     __syncthreads();
-    for (int j = tid; j < n; j += kTimeThreads)
-        atomicAdd(&coarse[coarse_of(__dmul_rn(__dsub_rn(keytab[j], kmin), scale))], 1u);
+    for (int j = tid; j < n; j += T)
+        atomicAdd(&coarse[coarse_of(__dmul_rn(__dsub_rn(keytab[j], kmin), scale), ncoarse)], 1u);
     __syncthreads();
     uint32_t *wsum = reinterpret_cast<uint32_t *>(scratch);  // 16 words
     {
@@ -340,10 +403,10 @@ __device__ bool bucket_sort(const double *keytab, uint16_t *perm, uint32_t *cnt,
 #pragma unroll
         for (int i = 0; i < kCoarsePerThread; ++i) {
             const int c = tid * kCoarsePerThread + i;
-            coarse[c] = (uint32_t)c + (uint32_t)(((uint64_t)pre * (kBuckets - kCoarse)) / (uint64_t)n);
+            coarse[c] = (uint32_t)c + (uint32_t)(((uint64_t)pre * (nbuckets - ncoarse)) / (uint64_t)n);
             pre += cc[i];
         }
-        if (tid == kTimeThreads - 1) coarse[kCoarse] = kBuckets;
+        if (tid == T - 1) coarse[ncoarse] = nbuckets;
     }
     __syncthreads();
     // the fine bucket of each of the thread's keys, two 13-bit ids per word,
@@ -351,10 +414,10 @@ __device__ bool bucket_sort(const double *keytab, uint16_t *perm, uint32_t *cnt,
     uint32_t fb[kTimeIPT / 2];
 #pragma unroll
     for (int i = 0; i < kTimeIPT; ++i) {
-        const int j = tid + i * kTimeThreads;
+        const int j = tid + i * T;
         uint32_t b = 0;
         if (j < n) {
-            b = fine_bucket(keytab[j], kmin, scale, coarse);
+            b = fine_bucket(keytab[j], kmin, scale, coarse, ncoarse);
             atomicAdd(&cnt[b >> 1], (b & 1) ? 0x10000u : 1u);
         }
         if (i & 1) fb[i / 2] |= b << 16;
@@ -392,7 +455,7 @@ __device__ bool bucket_sort(const double *keytab, uint16_t *perm, uint32_t *cnt,
     // scatter: afterwards cnt holds the end (= next start) of every bucket
 #pragma unroll
     for (int i = 0; i < kTimeIPT; ++i) {
-        const int j = tid + i * kTimeThreads;
+        const int j = tid + i * T;
         if (j < n) {
             const uint32_t b = (i & 1) ? (fb[i / 2] >> 16) : (fb[i / 2] & 0xFFFFu);
             const uint32_t old = atomicAdd(&cnt[b >> 1], (b & 1) ? 0x10000u : 1u);
@@ -426,35 +489,35 @@ __device__ bool bucket_sort(const double *keytab, uint16_t *perm, uint32_t *cnt,
 
 // Stable LSD radix sort (8 passes of 8 bits) of emitter indices by the
 // order-preserving 64-bit image of their keys; the fallback of bucket_sort.
-// Keys of positions >= n are +inf and stay at the end.
-__device__ void radix_sort(const double *keytab, uint16_t *perm, uint32_t *H, uint32_t *base) {
+// Positions from n on hold kPadKeyBits and stay at the end.
+__device__ void radix_sort(double *keytab, uint16_t *perm, uint32_t *H, uint32_t *base, int n, int ipt) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int S = 32 * kTimeIPT;
+    const int S = 32 * ipt, T = blockDim.x;
+    for (int m = n + tid; m < T * ipt; m += T) keytab[m] = __longlong_as_double(kPadKeyBits);
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint16_t idx[kTimeIPT];
-#pragma unroll
-    for (int i = 0; i < kTimeIPT; ++i) idx[i] = (uint16_t)(warp * S + i * 32 + lane);
+    for (int i = 0; i < ipt; ++i) idx[i] = (uint16_t)(warp * S + i * 32 + lane);
     __syncthreads();
     for (int pass = 0; pass < 8; ++pass) {
         const int shift = pass * 8;
         uint32_t *Hw = H + warp * 256;
         for (int k = lane; k < 256; k += 32) Hw[k] = 0;
         __syncwarp();
-        for (int i = 0; i < kTimeIPT; ++i) {
+        for (int i = 0; i < ipt; ++i) {
             const uint32_t dg = (uint32_t)(sortable(keytab[idx[i]]) >> shift) & 255u;
             const uint32_t peers = __match_any_sync(0xffffffffu, dg);
             if ((peers & lt_mask) == 0) Hw[dg] += __popc(peers);
             __syncwarp();
         }
         __syncthreads();
-        if (tid < 256) {
+        for (int k = tid; k < 256; k += T) {
             uint32_t run = 0;
-            for (int w = 0; w < kTimeWarps; ++w) {
-                const uint32_t h = H[w * 256 + tid];
-                H[w * 256 + tid] = run;
+            for (int w = 0; w < T / 32; ++w) {
+                const uint32_t h = H[w * 256 + k];
+                H[w * 256 + k] = run;
                 run += h;
             }
-            base[tid] = run;
+            base[k] = run;
         }
         __syncthreads();
         if (warp == 0) {
@@ -480,7 +543,7 @@ __device__ void radix_sort(const double *keytab, uint16_t *perm, uint32_t *H, ui
         __syncthreads();
         for (int k = lane; k < 256; k += 32) Hw[k] += base[k];
         __syncwarp();
-        for (int i = 0; i < kTimeIPT; ++i) {
+        for (int i = 0; i < ipt; ++i) {
             const uint32_t dg = (uint32_t)(sortable(keytab[idx[i]]) >> shift) & 255u;
             const uint32_t peers = __match_any_sync(0xffffffffu, dg);
             const uint32_t b0 = Hw[dg];
@@ -491,8 +554,7 @@ __device__ void radix_sort(const double *keytab, uint16_t *perm, uint32_t *H, ui
             perm[rank] = idx[i];
         }
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < kTimeIPT; ++i) idx[i] = perm[warp * S + i * 32 + lane];
+        for (int i = 0; i < ipt; ++i) idx[i] = perm[warp * S + i * 32 + lane];
         __syncthreads();
     }
 }
@@ -503,17 +565,17 @@ __device__ __forceinline__ bool before(double ka, int ja, double kb, int jb) {
     return ka < kb || (ka == kb && ja < jb);
 }
 
-// Insertion sort of positions [lo, hi) (hi - lo < kSlotGroup) of the
+// Insertion sort of positions [lo, hi) (hi - lo < 2 ipt) of the
 // position-ordered emitter indices P by (key, emitter index), keys from the
 // table by emitter.  P comes from the previous pixel's order, so the inner
 // loop rarely runs; (kprev, jprev) is the entry at position m - 1
 // throughout, and the next position's entry is loaded one step ahead (an
 // insertion only rewrites positions up to m).
-__device__ __forceinline__ void window_sort(const double *keytab, uint16_t *P, int lo, int hi) {
-    // slots of [lo, hi): contiguous except for one pad slot at the next
-    // multiple of kSlotGroup
-    const int off = lo / kSlotGroup, cut = (off + 1) * kSlotGroup;
-    auto sl = [&](int m) { return m + off + (m >= cut ? 1 : 0); };
+__device__ __forceinline__ void window_sort(const TimeShape &sh, const double *keytab, uint16_t *P, int lo, int hi) {
+    // slots of [lo, hi): contiguous except for the two pad slots at the next
+    // multiple of 2 ipt
+    const int grp = (int)__umulhi((uint32_t)lo, sh.inv_group), off = 2 * grp, cut = (grp + 1) * 2 * sh.ipt;
+    auto sl = [&](int m) { return m + off + (m >= cut ? 2 : 0); };
     int jprev = P[sl(lo)];
     double kprev = keytab[jprev];
     int v = lo + 1 < hi ? P[sl(lo + 1)] : 0;
@@ -541,6 +603,172 @@ __device__ __forceinline__ void window_sort(const double *keytab, uint16_t *P, i
     }
 }
 
+// One pixel's direction for the scan.
+struct TimePixel {
+    double k, inv_tau, dx, dy, dz, dn, q0, q1, q2;
+};
+// A run of positions as an affine map of the value X that enters it (decayed to
+// the run's first position): x_m = D_m X + B_m, and, with w_m = expm1(-2 gap/tau)
+// of the gap after m, S1 = sum w D^2, S2 = sum w D B, S3 = sum w |B|^2, so that
+// sum w_m |x_m|^2 = |X|^2 S1 + 2 Re(X conj(S2)) + S3 once X is known.
+struct RunSums {
+    double D = 1.0, Br = 0.0, Bi = 0.0, S1 = 0.0, S2r = 0.0, S2i = 0.0, S3 = 0.0;
+    // the gap after the last position, em = expm1(-gap/tau): expm1(-2 gap/tau) = em (2 + em)
+    __device__ __forceinline__ void interval(double em) {
+        const double w = em * (2.0 + em), wD = w * D;
+        S1 = fma(wD, D, S1);
+        S2r = fma(wD, Br, S2r);
+        S2i = fma(wD, Bi, S2i);
+        S3 = fma(w, fma(Br, Br, Bi * Bi), S3);
+    }
+    // decay over that gap and the next amplitude
+    __device__ __forceinline__ void enter(double em, double re, double im) {
+        const double dec = 1.0 + em;
+        D *= dec;
+        Br = fma(dec, Br, re);
+        Bi = fma(dec, Bi, im);
+    }
+};
+
+// Buffer of scan_run's stream: an emitter may stand this many places late.
+constexpr int kStream = 4;
+
+// Decaying scan of the positions [m0, m0 + cnt) of the position-ordered emitter
+// indices P.  The gaps at the run's two ends are the caller's (the neighbouring
+// threads' runs may still change).  STREAM: P holds the previous pixel's order;
+// it passes through a sorted buffer of kStream entries, P is rewritten with what
+// leaves the buffer, and bad is set when that is not the sorted order.
+//
+// Two positions at a time: their phases, sines and gap polynomials are
+// independent chains, and the rows of a pair are loaded a pair ahead and reduced
+// to its phases before the next ones are needed.
+template <bool NF, bool SCALE, bool DIGEST, bool STREAM>
+__device__ __forceinline__ RunSums scan_run(const TimePixel &px, const TimeShape &sh, const double *keytab, uint16_t *P,
+                                            const double4 *__restrict__ atoms4, int n, int m0, int cnt, uint64_t &h,
+                                            bool &bad) {
+    RunSums r;
+    h = 0;
+    if (cnt <= 0) return r;
+    uint32_t *Pw = reinterpret_cast<uint32_t *>(P) + slot(sh, m0) / 2;
+    uint64_t pw = DIGEST ? digest_pow(m0) : 0;
+    const double inf = __longlong_as_double(0x7FF0000000000000ll);
+    // entry e of the run in the old order; past its end an entry that sorts behind all others
+    auto entry = [&](int e, uint32_t w, double &t, int &j) {
+        j = e < cnt ? (int)((e & 1) ? w >> 16 : w & 0xFFFFu) : 0x10000 + e;
+        t = e < cnt ? keytab[j] : inf;
+    };
+    double b0, b1, b2, b3, x0, x1;  // STREAM: the buffer and the next two entries
+    int i0, i1, i2, i3, y0, y1;
+    uint32_t wn = 0;  // the pair of indices after those
+    if (STREAM) {
+        uint32_t w = Pw[0];
+        entry(0, w, b0, i0);
+        entry(1, w, b1, i1);
+        if (cnt > 2) w = Pw[1];
+        entry(2, w, b2, i2);
+        entry(3, w, b3, i3);
+        bad = !(before(b0, i0, b1, i1) && before(b1, i1, b2, i2) && before(b2, i2, b3, i3));
+        if (cnt > 4) w = Pw[2];
+        entry(4, w, x0, y0);
+        entry(5, w, x1, y1);
+        if (cnt > 6) wn = Pw[3];
+    } else if (cnt > 2) {
+        wn = Pw[1];
+    }
+    // the next pair in order: emitters ja, jb at times ta, tb
+    int ja, jb;
+    double ta, tb;
+    auto insert = [&](double x, int y, double &t, int &j) {
+        t = b0;
+        j = i0;
+        if (y > 0xFFFF || before(b3, i3, x, y)) {  // (the run's end always goes last)
+            b0 = b1; i0 = i1; b1 = b2; i1 = i2; b2 = b3; i2 = i3; b3 = x; i3 = y;
+        } else if (before(b2, i2, x, y)) {
+            b0 = b1; i0 = i1; b1 = b2; i1 = i2; b2 = x; i2 = y;
+        } else if (before(b1, i1, x, y)) {
+            b0 = b1; i0 = i1; b1 = x; i1 = y;
+        } else if (before(b0, i0, x, y)) {
+            b0 = x; i0 = y;
+        } else {  // later than the buffer allows (or a NaN key)
+            t = x;
+            j = y;
+            bad = true;
+        }
+    };
+    auto next_pair = [&](int i) {  // entries i, i+1 of the order
+        if (STREAM) {
+            if (before(b3, i3, x0, y0) && before(x0, y0, x1, y1)) {
+                ta = b0; ja = i0; tb = b1; jb = i1;
+                b0 = b2; i0 = i2; b1 = b3; i1 = i3; b2 = x0; i2 = y0; b3 = x1; i3 = y1;
+            } else {
+                insert(x0, y0, ta, ja);
+                insert(x1, y1, tb, jb);
+            }
+            const uint32_t w = wn;
+            if (i + 8 < cnt) wn = Pw[i / 2 + 4];
+            entry(i + 6, w, x0, y0);
+            entry(i + 7, w, x1, y1);
+            if (i < cnt) Pw[i / 2] = (uint32_t)ja | ((uint32_t)jb << 16);
+        } else {
+            const uint32_t w = wn;
+            if (i + 2 < cnt) wn = Pw[i / 2 + 1];
+            entry(i, w, ta, ja);
+            entry(i + 1, w, tb, jb);
+        }
+    };
+    auto row = [&](int j) { return ld_row(atoms4 + min(j, n - 1)); };
+    if (!STREAM) {
+        const uint32_t w = wn;
+        wn = Pw[0];
+        next_pair(0);
+        wn = w;
+    } else {
+        next_pair(0);
+    }
+    double t0 = ta, t1 = tb, em_in = 0.0, th0, th1, r0, r1;  // the pair's times, phases and distances
+    uint32_t pj = (uint32_t)ja | ((uint32_t)jb << 16);
+    phase_of<NF>(px.k, px.dx, px.dy, px.dz, px.dn, px.q0, px.q1, px.q2, row(ja), th0, r0);
+    phase_of<NF>(px.k, px.dx, px.dy, px.dz, px.dn, px.q0, px.q1, px.q2, row(jb), th1, r1);
+#pragma unroll 1
+    for (int i = 0; i < cnt; i += 2) {
+        if (DIGEST) {
+            h += (uint64_t)((pj & 0xFFFFu) + 1) * pw;
+            pw *= kDigestBase;
+            if (i + 1 < cnt) h += (uint64_t)((pj >> 16) + 1) * pw;
+            pw *= kDigestBase;
+        }
+        next_pair(i + 2);
+        if (DIGEST) pj = (uint32_t)ja | ((uint32_t)jb << 16);
+        const double4 ra = row(ja), rb = row(jb);
+        double re0, im0, re1, im1, em0, em1;
+        sincos_pair(th0, th1, im0, re0, im1, re1);
+        if (NF && SCALE) {
+            re0 = __ddiv_rn(re0, r0);
+            im0 = __ddiv_rn(im0, r0);
+            re1 = __ddiv_rn(re1, r1);
+            im1 = __ddiv_rn(im1, r1);
+        }
+        expm1_neg_pair(__dsub_rn(t1, t0) * px.inv_tau, i + 2 < cnt ? __dsub_rn(ta, t1) * px.inv_tau : 0.0, em0, em1);
+        if (i == 0) {
+            r.Br = re0;
+            r.Bi = im0;
+        } else {
+            r.enter(em_in, re0, im0);
+        }
+        if (i + 1 < cnt) {
+            r.interval(em0);
+            r.enter(em0, re1, im1);
+            if (i + 2 < cnt) r.interval(em1);
+        }
+        em_in = em1;
+        t0 = ta;
+        t1 = tb;
+        phase_of<NF>(px.k, px.dx, px.dy, px.dz, px.dn, px.q0, px.q1, px.q2, ra, th0, r0);
+        phase_of<NF>(px.k, px.dx, px.dy, px.dz, px.dn, px.q0, px.q1, px.q2, rb, th1, r1);
+    }
+    return r;
+}
+
 template <bool NF, bool SCALE, bool DIGEST>
 __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams g, const double *__restrict__ atoms,
                                                                 const double *__restrict__ times, int n, double c,
@@ -548,14 +776,14 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
                                                                 WsHeader *__restrict__ hdr, int order_pixel,
                                                                 int *__restrict__ order_out,
                                                                 double *__restrict__ keys_out,
-                                                                uint64_t *__restrict__ digest, int chunk) {
+                                                                uint64_t *__restrict__ digest, int chunk, const TimeShape sh) {
     extern __shared__ __align__(16) unsigned char smem[];
     double *keytab = reinterpret_cast<double *>(smem);
-    uint16_t *P = reinterpret_cast<uint16_t *>(smem + (size_t)kTimeMaxN * 8);
-    uint32_t *H = reinterpret_cast<uint32_t *>(smem + (size_t)kTimeMaxN * 8 + (size_t)kTimeSlots * 2);
-    uint32_t *base = H + kTimeWarps * 256;
-    double *scratch = reinterpret_cast<double *>(base + 256);  // 128 doubles
-    uint32_t *coarse = reinterpret_cast<uint32_t *>(scratch + 128);
+    const int T = blockDim.x, nwarps = T / 32, ipt = sh.ipt, cap = T * ipt;
+    uint16_t *P = reinterpret_cast<uint16_t *>(smem + (size_t)cap * 8);
+    uint32_t *H = reinterpret_cast<uint32_t *>(P + cap + T);
+    double *scratch = reinterpret_cast<double *>(H + nwarps * 256);  // 8 doubles per warp
+    uint32_t *coarse = reinterpret_cast<uint32_t *>(scratch + 8 * nwarps), *base = coarse;
     __shared__ uint64_t s_dig[kTimeWarps];
     __shared__ int s_pix, s_flag;
 
@@ -570,7 +798,7 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
     // CTA-uniform sort state: whether (K, P) hold the previous pixel's order,
     // and whether warm starts are still tried
     bool have = false;
-    int fails = 0;
+    int fails = 0, slips = 0;
     // order_pixel >= 0: process that one pixel only, record its sorted order
     // and write its intensity to out[0]
     int iter = 0;
@@ -595,43 +823,50 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
                 iy = (ix & 1) ? g.ny - 1 - r : r;
             }
             const int p = ix * g.ny + iy;
-            double dx, dy, dz;
+            TimePixel px;
+            px.k = g.k;
+            px.inv_tau = inv_tau;
+            double &dx = px.dx, &dy = px.dy, &dz = px.dz;
             pixel_time(g, ix, iy, dx, dy, dz);
             // time.py:89-91 (np.linalg.norm = sqrt((x*x + y*y) + z*z); q = det/d; q_z -= 1)
             const double dn =
                 __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
             const double q0 = __ddiv_rn(dx, dn), q1 = __ddiv_rn(dy, dn), q2 = __dsub_rn(__ddiv_rn(dz, dn), 1.0);
+            px.dn = dn;
+            px.q0 = q0;
+            px.q1 = q1;
+            px.q2 = q2;
 
-            // ---- keys: table by emitter index (coalesced), padding last ----
-            // (the rows of KB emitters per thread are loaded before any is used)
-            double kmin = __longlong_as_double(0x7FF0000000000000ll), kmax = -kmin;
+            // ---- keys: table by emitter index (coalesced) ----
+            // (the rows of KB emitters per thread are loaded before any is used; only
+            // the last batch checks for the end of the list)
             {
                 constexpr int KB = NF ? 4 : 8;
-#pragma unroll 1
-                for (int b = 0; b < kTimeIPT; b += KB) {
+                auto key_batch = [&](int j0, auto last) {
+                    constexpr bool kLast = decltype(last)::value;
                     double4 aa[KB];
                     double tt[KB];
 #pragma unroll
                     for (int u = 0; u < KB; ++u) {
-                        const int j = tid + (b + u) * kTimeThreads;
-                        aa[u] = j < n ? ld_row(atoms4 + j) : make_double4(0.0, 0.0, 0.0, 0.0);
-                        tt[u] = j < n ? times[j] : 0.0;
+                        const int j = kLast ? min(j0 + u * T, n - 1) : j0 + u * T;
+                        aa[u] = ld_row(atoms4 + j);
+                        tt[u] = times[j];
                     }
                     if (!NF) {
                         // far field without branches: the Markstein quotient of every
                         // row, and the IEEE division after the batch for a quotient out of
-                        // div_rn's range (a zero path difference, say); the padding keys
-                        // (a NaN) leave min and max alone
+                        // div_rn's range (a zero path difference, say; the range is tested
+                        // on the quotient's exponent)
                         double tq[KB];
-                        bool redo = false;
+                        uint32_t redo = 0;
 #pragma unroll
                         for (int u = 0; u < KB; ++u) {
                             const double sp = __fma_rn(q2, aa[u].z, __fma_rn(q1, aa[u].y, __dmul_rn(q0, aa[u].x)));
                             const double qa = __dmul_rn(-sp, ic);
                             tq[u] = __fma_rn(__fma_rn(-c, qa, -sp), ic, qa);
-                            redo |= tid + (b + u) * kTimeThreads < n && !(fabs(qa) >= 0x1p-960 && fabs(qa) <= 0x1p1000);
+                            redo = max(redo, ((uint32_t)__double2hiint(qa) & 0x7FFFFFFFu) - kDivLow);
                         }
-                        if (redo) {
+                        if (redo >= kDivSpan) {
 #pragma unroll
                             for (int u = 0; u < KB; ++u) {
                                 const double sp =
@@ -640,35 +875,55 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
                             }
                         }
 #pragma unroll
-                        for (int u = 0; u < KB; ++u) {
-                            const int j = tid + (b + u) * kTimeThreads;
-                            const double t = j < n ? __dadd_rn(tq[u], tt[u]) : __longlong_as_double(kPadKeyBits);
-                            kmin = fmin(kmin, t);
-                            kmax = fmax(kmax, t);
-                            keytab[j] = t;
-                        }
+                        for (int u = 0; u < KB; ++u)
+                            if (!kLast || j0 + u * T < n) keytab[j0 + u * T] = __dadd_rn(tq[u], tt[u]);
                     } else {
 #pragma unroll
                         for (int u = 0; u < KB; ++u) {
-                            const int j = tid + (b + u) * kTimeThreads;
-                            double t = __longlong_as_double(kPadKeyBits);
-                            if (j < n) {
-                                double s, dist;
-                                arrival<NF, SCALE>(g, dx, dy, dz, dn, q0, q1, q2, aa[u], tt[u], c, ic, t, s, dist);
-                                kmin = fmin(kmin, t);
-                                kmax = fmax(kmax, t);
-                            }
-                            keytab[j] = t;
+                            double t, s, dist;
+                            arrival<NF, SCALE>(g, dx, dy, dz, dn, q0, q1, q2, aa[u], tt[u], c, ic, t, s, dist);
+                            if (!kLast || j0 + u * T < n) keytab[j0 + u * T] = t;
                         }
                     }
-                }
+                };
+                int j = 0;
+#pragma unroll 1
+                for (; j + KB * T <= n; j += KB * T) key_batch(j + tid, std::false_type{});
+                if (j < n) key_batch(j + tid, std::true_type{});
             }
             __syncthreads();
 
-            // ---- sort: warm start from the previous pixel's order ----
-            bool sorted = false;
-            if (have && fails < kWarmMaxFails) {
-                // thread t's window: [40t, 40t+40) on even passes, [40t-20, 40t+20) on odd
+            // ---- warm start: the previous pixel's order, repaired while it is scanned ----
+            // First the few positions around every run's start, so that no emitter has
+            // to cross it later.  Then every thread streams its run through a sorted
+            // buffer of four and scans what leaves it: an emitter that is less than
+            // five places late in the old order comes out in its place; a thread whose
+            // stream was not sorted by that sorts its run as a window and scans it again.
+            // The order is exact when every run ends before the next begins; otherwise
+            // the window passes below repair it and all runs are scanned again.
+            const int m0 = tid * ipt, cnt = min(max(n - m0, 0), ipt);
+            RunSums run;
+            uint64_t h = 0;
+            bool sorted = false, scan = true;
+            if (have && slips < kWarmMaxFails && fails < kWarmMaxFails && ipt >= 2 * kStream) {
+                if (cnt > 0) window_sort(sh, keytab, P, max(m0 - kStream, 0), min(m0 + kStream, n));
+                __syncthreads();
+                bool bad = false;
+                run = scan_run<NF, SCALE, DIGEST, true>(px, sh, keytab, P, atoms4, n, m0, cnt, h, bad);
+                if (bad) window_sort(sh, keytab, P, m0, m0 + cnt);
+                const int nbad = __syncthreads_count(bad);
+                bool apart = true;
+                if (m0 > 0 && cnt > 0) {
+                    const int u = P[slot(sh, m0 - 1)], v = P[slot(sh, m0)];
+                    apart = before(keytab[u], u, keytab[v], v);
+                }
+                sorted = __syncthreads_and(apart);
+                scan = bad || !sorted;
+                slips = sorted && nbad <= T / 8 ? 0 : slips + 1;
+            }
+            // ---- warm start by windows ----
+            if (!sorted && have && fails < kWarmMaxFails) {
+                // thread t's window: [rt, rt+r) on even passes (r = ipt), [rt-r/2, rt+r/2) on odd
                 // ones (the last thread's odd window runs to the end).  After a pass every
                 // window is sorted, so a window of the other grid -- two sorted halves --
                 // is out of order only if the boundary at its middle is: a thread sorts its
@@ -677,16 +932,16 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
                 // window; together the threads check every boundary of the pass's grid.
                 bool dirty = true;
                 for (int pass = 0; pass < kWarmPasses; ++pass) {
-                    const int sh = (pass & 1) ? kTimeIPT / 2 : 0;
-                    const int lo = max(tid * kTimeIPT - sh, 0);
-                    const int hi = min(tid == kTimeThreads - 1 ? kTimeMaxN : (tid + 1) * kTimeIPT - sh, n);
+                    const int half = (pass & 1) ? ipt / 2 : 0;
+                    const int lo = max(tid * ipt - half, 0);
+                    const int hi = min(tid == T - 1 ? cap : (tid + 1) * ipt - half, n);
                     // (the previous pass's __syncthreads_or ordered its reads before these writes)
-                    if (dirty && lo < hi) window_sort(keytab, P, lo, hi);
+                    if (dirty && lo < hi) window_sort(sh, keytab, P, lo, hi);
                     __syncthreads();
-                    const int b = (pass & 1) ? (tid + 1) * kTimeIPT - sh : tid * kTimeIPT;
+                    const int b = (pass & 1) ? (tid + 1) * ipt - half : tid * ipt;
                     bool bad = false;
                     if (b >= 1 && b < n) {
-                        const int u = P[slot(b - 1)], v = P[slot(b)];
+                        const int u = P[slot(sh, b - 1)], v = P[slot(sh, b)];
                         bad = !before(keytab[u], u, keytab[v], v);
                     }
                     dirty = bad;
@@ -697,22 +952,22 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
                     if (pass == 0) {
                         // Between neighbouring pixels the few pairs still out of order sit
                         // at even boundaries and have moved by a position or two: first a
-                        // window of 2 kPatch positions around each such boundary.  Only
+                        // window of 2 patch positions around each such boundary.  Only
                         // the pairs at those windows' ends can then be out of order; where
                         // one is, the odd window around it (which holds the short one)
                         // takes over in the next pass.
-                        constexpr int kPatch = 8;
-                        const int plo = max(b - kPatch, 0), phi = min(b + kPatch, n);
-                        if (bad) window_sort(keytab, P, plo, phi);
+                        const int patch = min(8, ipt / 2);
+                        const int plo = max(b - patch, 0), phi = min(b + patch, n);
+                        if (bad) window_sort(sh, keytab, P, plo, phi);
                         __syncthreads();
                         bool pbad = false;
                         if (bad) {
                             if (plo >= 1) {
-                                const int u = P[slot(plo - 1)], v = P[slot(plo)];
+                                const int u = P[slot(sh, plo - 1)], v = P[slot(sh, plo)];
                                 pbad = !before(keytab[u], u, keytab[v], v);
                             }
                             if (phi < n) {
-                                const int u = P[slot(phi - 1)], v = P[slot(phi)];
+                                const int u = P[slot(sh, phi - 1)], v = P[slot(sh, phi)];
                                 pbad = pbad || !before(keytab[u], u, keytab[v], v);
                             }
                         }
@@ -729,97 +984,51 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
             if (!sorted) {
                 // ---- full sort ----
                 if (tid == 0) atomicAdd(&hdr->work_counter2, 1u);  // full sorts
-                block_minmax(kmin, kmax, scratch + 96);
-                if (!bucket_sort(keytab, P, reinterpret_cast<uint32_t *>(H), coarse, n, kmin, kmax, scratch,
-                                 &s_flag)) {
-                    radix_sort(keytab, P, H, base);
+                double kmin = __longlong_as_double(0x7FF0000000000000ll), kmax = -kmin;
+                for (int j = tid; j < n; j += T) {
+                    kmin = fmin(kmin, keytab[j]);
+                    kmax = fmax(kmax, keytab[j]);
                 }
+                block_minmax(kmin, kmax, scratch + 6 * nwarps);
+                if (!bucket_sort(keytab, P, H, coarse, n, kmin, kmax, scratch, &s_flag))
+                    radix_sort(keytab, P, H, base, n, ipt);
                 // P[m] (unpadded) = emitter at sorted position m: move to slots
+                uint32_t *P2 = reinterpret_cast<uint32_t *>(P);
                 uint32_t pk[kTimeIPT / 2];
-                const int m0 = tid * kTimeIPT;
 #pragma unroll
-                for (int i = 0; i < kTimeIPT / 2; ++i)
-                    pk[i] = (uint32_t)P[m0 + 2 * i] | ((uint32_t)P[m0 + 2 * i + 1] << 16);
+                for (int i = 0; i < kTimeIPT / 2; ++i) pk[i] = 2 * i < ipt ? P2[tid * (ipt / 2) + i] : 0u;
                 __syncthreads();
 #pragma unroll
-                for (int i = 0; i < kTimeIPT / 2; ++i) {
-                    P[slot(m0) + 2 * i] = (uint16_t)(pk[i] & 0xFFFFu);
-                    P[slot(m0) + 2 * i + 1] = (uint16_t)(pk[i] >> 16);
-                }
+                for (int i = 0; i < kTimeIPT / 2; ++i)
+                    if (2 * i < ipt) P2[slot(sh, tid * ipt) / 2 + i] = pk[i];
                 __syncthreads();
             }
             have = true;
-            // P[slot(m)]: emitter at sorted position m < n
+            // P[slot(sh, m)]: emitter at sorted position m < n
 
             if (order_pixel >= 0) {
-                for (int m = tid; m < n; m += kTimeThreads) {
-                    order_out[m] = P[slot(m)];
-                    keys_out[m] = keytab[P[slot(m)]];
+                for (int m = tid; m < n; m += T) {
+                    order_out[m] = P[slot(sh, m)];
+                    keys_out[m] = keytab[P[slot(sh, m)]];
                 }
             }
 
-            // ---- decaying scan over the sorted sequence, one pass ----
-            // Thread t owns positions [40t, 40t+40).  Inside its run
-            //   x_m = D_m X + B_m,  D_m = prod of the run's decays up to m,
-            // with X the value entering the run (known only after the block scan),
-            // so sum_m w_m |x_m|^2 = |X|^2 S1 + 2 Re(X conj(S2)) + S3 with
-            //   S1 = sum w D^2, S2 = sum w D B, S3 = sum w |B|^2
-            // and w_m = -tau/2 expm1(-2 (t_{m+1} - t_m)/tau), w_{n-1} = tau/2
-            // (the interval integral of time.py:36-45).  Each gap g enters twice:
-            // as the decay exp(-g/tau) = 1 + em of the later position and as the
-            // weight -tau/2 expm1(-2 g/tau) = -tau/2 em (2 + em) of the earlier one,
-            // with em = expm1(-g/tau): one polynomial per gap, no cancellation.
-            const int m0 = tid * kTimeIPT;
-            const uint16_t *Pr = P + slot(m0);  // the run's slots are contiguous
-            double Dm = 1.0, Br = 0.0, Bi = 0.0;
-            double S1 = 0.0, S2r = 0.0, S2i = 0.0, S3 = 0.0;
-            uint64_t h = 0, pw = DIGEST && m0 < n ? digest_pow(m0) : 0;
-            // the neighbours' keys travel in registers from one position to the
-            // next, and the emitter rows are loaded two positions ahead
-            int j_next = 0;
-            double t_next = 0.0, em_in = 0.0;
-            double4 a_next = make_double4(0.0, 0.0, 0.0, 0.0), a_next2 = a_next;
-            if (m0 < n) {
-                j_next = Pr[0];
-                t_next = keytab[j_next];
-                a_next = ld_row(atoms4 + j_next);
-                if (m0 + 1 < n) a_next2 = ld_row(atoms4 + Pr[1]);
-                if (m0 > 0) em_in = expm1_neg(__dsub_rn(t_next, keytab[P[slot(m0 - 1)]]) * inv_tau);
+            if (scan) {
+                bool unused = false;
+                run = scan_run<NF, SCALE, DIGEST, false>(px, sh, keytab, P, atoms4, n, m0, cnt, h, unused);
             }
-            for (int i = 0; i < kTimeIPT; ++i) {
-                const int m = m0 + i;
-                if (m >= n) break;
-                const double tj = t_next;
-                const double4 a = a_next;
-                a_next = a_next2;
-                if (DIGEST) {
-                    h += (uint64_t)(j_next + 1) * pw;
-                    pw *= kDigestBase;
-                }
-                if (m + 1 < n) {
-                    j_next = i + 1 < kTimeIPT ? Pr[i + 1] : P[slot(m + 1)];
-                    t_next = keytab[j_next];
-                }
-                if (i + 2 < kTimeIPT && m + 2 < n) a_next2 = ld_row(atoms4 + Pr[i + 2]);
-                double s, dist, re, im;
-                path_only<NF>(dx, dy, dz, dn, q0, q1, q2, a, s, dist);
-                amplitude<NF, SCALE>(g.k, s, a.w, dist, re, im);
-                const double dec = m == 0 ? 0.0 : 1.0 + em_in;
-                Dm *= dec;
-                Br = fma(dec, Br, re);
-                Bi = fma(dec, Bi, im);
-                double w = tau / 2;
-                if (m < n - 1) {
-                    em_in = expm1_neg(__dsub_rn(t_next, tj) * inv_tau);
-                    w = (-tau / 2) * (em_in * (2.0 + em_in));
-                }
-                const double wD = w * Dm;
-                S1 = fma(wD, Dm, S1);
-                S2r = fma(wD, Br, S2r);
-                S2i = fma(wD, Bi, S2i);
-                S3 = fma(w, fma(Br, Br, Bi * Bi), S3);
+            // the gaps at the run's ends (an infinite one before position 0 and after n-1)
+            double em_first = -1.0, em_last = -1.0;
+            if (cnt > 0) {
+                if (m0 > 0)
+                    em_first = expm1_neg(__dsub_rn(keytab[P[slot(sh, m0)]], keytab[P[slot(sh, m0 - 1)]]) * inv_tau);
+                if (m0 + cnt < n)
+                    em_last = expm1_neg(
+                        __dsub_rn(keytab[P[slot(sh, m0 + cnt)]], keytab[P[slot(sh, m0 + cnt - 1)]]) * inv_tau);
+                run.interval(em_last);
             }
-            const Affine agg = {Dm, Br, Bi};
+            const double dec0 = 1.0 + em_first;
+            const Affine agg = {dec0 * run.D, run.Br, run.Bi};
             // block exclusive scan of the run maps
             Affine incl = agg;
 #pragma unroll
@@ -847,9 +1056,11 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
             excl.bi = __shfl_up_sync(0xffffffffu, incl.bi, 1);
             if (lane == 0) excl = Affine{1.0, 0.0, 0.0};
             excl = compose(wpre, excl);
-            // X entering this thread's run = excl applied to x_{-1} = 0
-            const double Xr = excl.br, Xi = excl.bi;
-            double part = fma(fma(Xr, Xr, Xi * Xi), S1, fma(2.0, fma(Xr, S2r, Xi * S2i), S3));
+            // X entering this thread's run = excl applied to x_{-1} = 0, decayed to its
+            // first position
+            const double Xr = dec0 * excl.br, Xi = dec0 * excl.bi;
+            double part = (-tau / 2) *
+                          fma(fma(Xr, Xr, Xi * Xi), run.S1, fma(2.0, fma(Xr, run.S2r, Xi * run.S2i), run.S3));
             // block sum (and of the order digest)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -858,18 +1069,19 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
             }
             __syncthreads();
             if (lane == 0) {
-                scratch[64 + warp] = part;
+                scratch[4 * nwarps + warp] = part;
                 if (DIGEST) s_dig[warp] = h;
             }
             __syncthreads();
             if (tid == 0) {
                 double tot = 0.0;
                 uint64_t hh = 0;
-                for (int w = 0; w < kTimeWarps; ++w) {
-                    tot += scratch[64 + w];
+                for (int w = 0; w < nwarps; ++w) {
+                    tot += scratch[4 * nwarps + w];
                     if (DIGEST) hh += s_dig[w];
                 }
-                out[order_pixel >= 0 ? 0 : p] = tot;
+                // far field: every amplitude has the pixel's own distance
+                out[order_pixel >= 0 ? 0 : p] = !NF && SCALE ? tot / (dn * dn) : tot;
                 if (DIGEST && order_pixel < 0) digest[p] = hh;
             }
             // the next pixel's key pass overwrites the key table and P, which the scan reads
@@ -910,7 +1122,7 @@ __host__ __device__ __forceinline__ size_t large_slice_bytes(int64_t n) {
 
 // The two-level map of bucket_sort with nb fine buckets (nb >= 8192 here).
 __device__ __forceinline__ uint32_t fine_bucket_n(double t, double kmin, double scale, const uint32_t *coarse) {
-    return fine_bucket(t, kmin, scale, coarse);
+    return fine_bucket(t, kmin, scale, coarse, kCoarse);
 }
 
 // Sorted (key, emitter) records in rec: the scatter moves each record to its
@@ -931,7 +1143,7 @@ __device__ bool bucket_sort_large(const double *keys, SortRec *rec, uint32_t *cn
     if (tid == 0) *s_flag = 0;
     __syncthreads();
     for (int j = tid; j < n; j += kTimeThreads)
-        atomicAdd(&coarse[coarse_of(__dmul_rn(__dsub_rn(keys[j], kmin), scale))], 1u);
+        atomicAdd(&coarse[coarse_of(__dmul_rn(__dsub_rn(keys[j], kmin), scale), kCoarse)], 1u);
     __syncthreads();
     uint32_t *wsum = reinterpret_cast<uint32_t *>(scratch);
     {
@@ -1190,7 +1402,7 @@ __global__ void __launch_bounds__(kTimeThreads, 2) time_kernel_large(
             }
             double s, dist, re, im;
             path_only<NF>(dx, dy, dz, dn, q0, q1, q2, a, s, dist);
-            amplitude<NF, SCALE, false>(g.k, s, a.w, dist, re, im);
+            amplitude<NF, SCALE>(g.k, s, a.w, dist, re, im);
             const double dec = m == 0 ? 0.0 : exp(-__dsub_rn(tj, t_prev) * inv_tau);
             t_prev = tj;
             Dm *= dec;
@@ -1306,6 +1518,24 @@ static int large_ctas(const idiwf_geom *geom, int order_pixel) {
     return std::max(1, std::min(geom->nx * geom->ny, sms * std::max(occ, 1)));
 }
 
+// Threads of a pixel's CTA: 512 / threads pixels share an SM (the kernel's 128
+// registers allow 16 warps per SM at any split).  Few threads with long runs cost
+// least per pixel -- the fixed costs (barriers, block scan, run ends) are shared by
+// more positions and the CTAs of an SM are in different phases -- as long as the
+// tables of 512 / threads pixels fit in shared memory.  But a CTA's first pixel
+// pays a full sort, so every CTA gets at least two.  100 x 100 pixels, us, 512
+// threads against the choice: 500 emitters 400 / 121 (32 threads), 2,000 565 / 273
+// (64), 5,000 883 / 590 (128), 10,000 1251 / 1164 (256).  32 x 32 pixels, 1,000
+// emitters: 79 (32), 57 (128), 63 (160, the choice), 80 (512).
+static TimeShape choose_shape(int n, int npix, int sms) {
+    for (const int threads : {32, 64, 128, 160, 256}) {
+        const TimeShape s = time_shape(threads, n);
+        const int per_sm = kTimeThreads / threads;
+        if (s.ipt <= kTimeIPT && per_sm * (s.smem + kCtaShared) <= kSmShared && npix >= 2 * per_sm * sms) return s;
+    }
+    return time_shape(kTimeThreads, n);
+}
+
 static size_t time_ws_bytes(const idiwf_geom *geom, int64_t n, int order_pixel) {
     if (n <= kTimeMaxN) return kWsDataOffset;
     return kWsDataOffset + (size_t)large_ctas(geom, order_pixel) * large_slice_bytes(n);
@@ -1340,17 +1570,18 @@ static idiwf_status time_launch(const idiwf_geom *geom, const double *atoms, con
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fl, dim3(grid), dim3(kTimeThreads), args, kLargeSmem, stream));
         return IDIWF_OK;
     }
-    const bool dg = digest != nullptr;
-    void *fn = nf ? (sc ? time_kernel_ptr<true, true>(dg) : time_kernel_ptr<true, false>(dg))
-                  : (sc ? time_kernel_ptr<false, true>(dg) : time_kernel_ptr<false, false>(dg));
-    IDIWF_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTimeSmem));
-    // queue counter, error word, and the full-sort / given-up warm-start counts
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, 5 * sizeof(uint32_t), stream));
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int npix = geom->nx * geom->ny;
-    const int grid = order_pixel >= 0 ? 1 : std::min(npix, sms);
+    const TimeShape sh = choose_shape((int)n, npix, sms);
+    const bool dg = digest != nullptr;
+    void *fn = nf ? (sc ? time_kernel_ptr<true, true>(dg) : time_kernel_ptr<true, false>(dg))
+                  : (sc ? time_kernel_ptr<false, true>(dg) : time_kernel_ptr<false, false>(dg));
+    IDIWF_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTimeSmemMax));
+    // queue counter, error word, and the full-sort / given-up warm-start counts
+    IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, 5 * sizeof(uint32_t), stream));
+    const int grid = order_pixel >= 0 ? 1 : std::min(npix, sms * (kTimeThreads / sh.threads));
     // pixels per queue claim: an equal share of the detector per CTA, walked in
     // serpentine order (every pixel of a CTA but its first warm-starts from a
     // neighbour's order; the per-pixel cost hardly varies, so equal shares
@@ -1358,8 +1589,8 @@ static idiwf_status time_launch(const idiwf_geom *geom, const double *atoms, con
     int chunk = (npix + grid - 1) / grid;
     int ni = (int)n;
     void *args[] = {(void *)&g, &atoms, &times, &ni, &c, &tau, &out, &hdr, &order_pixel, &order_out, &keys_out,
-                    &digest, &chunk};
-    IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(kTimeThreads), args, kTimeSmem, stream));
+                    &digest, &chunk, (void *)&sh};
+    IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(sh.threads), args, sh.smem, stream));
     return IDIWF_OK;
 }
 
