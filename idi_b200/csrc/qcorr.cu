@@ -9,7 +9,7 @@
 // bin changes -- the radial reference kernel's accumulation, and for the 3d
 // one (which adds every pair to FP32 bins) far fewer atomics.
 //
-//  * qcorr_radial_kernel — CTA = (reference row, group of kRowsPerCta target
+//  * qcorr_radial_kernel — CTA = (reference row, group of target
 //    rows, up to two images and their mirror rows).  The reference row and each
 //    target row are staged in shared memory, q as float4 and the values of all
 //    images beside each other.  The bin round(sqrt(d2)) is re-derived
@@ -27,7 +27,7 @@
 
 namespace idiwf {
 
-constexpr int kRowsPerCta = 8;
+constexpr int kRowsPerCta = 8;  // target rows of a 3d correlator's CTA
 constexpr int kQcorrMaxSmemCols = 4096;
 
 // ---------------------------------------------------------------------------
@@ -46,7 +46,7 @@ constexpr int kQcorrMaxSmemCols = 4096;
 // the second walk's target is the first's next one, so each shared-memory load of a
 // target serves both (shared memory bounded the one-offset form: ten wavefronts per
 // pair and four values).  Targets are stored by column parity, which keeps the lanes, two
-// columns apart, on consecutive addresses.  2 x 512^2, 256 bins: 15.8 ms against 35.5 with
+// columns apart, on consecutive addresses.  2 x 512^2, 256 bins: 16.0 ms against 35.5 with
 // one walk per image, row pair and offset.  What bounds it now is the bin changes: a lane
 // changes bins every 10 to 50 pairs, a warp at every other pair.
 constexpr int kRadialImages = 2;
@@ -101,7 +101,7 @@ __device__ __forceinline__ RadialPoint<V> radial_point(const float4 *__restrict_
 
 template <int NB, bool MIR>
 __device__ __forceinline__ void radial_walks(const float4 *__restrict__ q, const float *__restrict__ images, int nr,
-                                             int nc, int qmax, int refr, float4 *sref, float4 *stgt,
+                                             int nc, int qmax, int rows, int refr, float4 *sref, float4 *stgt,
                                              float *vref, float *vtgt, double *hist, const float *bound) {
     constexpr int V = NB * (MIR ? 2 : 1);
     const int tid = threadIdx.x;
@@ -117,9 +117,9 @@ __device__ __forceinline__ void radial_walks(const float4 *__restrict__ q, const
             if (MIR) vref[c * V + NB + k] = row_mirrors ? images[k * npix + (int64_t)(nr - refr) * nc + c] : 0.0f;
         }
     }
-    // column offsets o and o + 1; tc = refc + offset in [0, nc)
-    const int o = 2 * tid - qmax;
-    const bool active[2] = {o <= qmax, o + 1 <= qmax};
+    // column offsets o and o + 1 of -most..most; tc = refc + offset in [0, nc)
+    const int most = min(qmax, nc - 1), o = 2 * tid - most;
+    const bool active[2] = {o <= most, o + 1 <= most};
     int c0[2], c1[2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
@@ -127,8 +127,8 @@ __device__ __forceinline__ void radial_walks(const float4 *__restrict__ q, const
         c1[w] = active[w] ? max(min(nc, nc - (o + w)), c0[w]) : c0[w];
     }
     const int both0 = max(c0[0], c0[1]), both1 = min(c1[0], c1[1]);
-    const int dr0 = blockIdx.y * kRowsPerCta;
-    for (int dr = dr0; dr < min(dr0 + kRowsPerCta, qmax); ++dr) {
+    const int dr0 = blockIdx.y * rows;
+    for (int dr = dr0; dr < min(dr0 + rows, qmax); ++dr) {
         const int tr = refr + dr;
         if (tr >= nr) break;
         // the mirror pair of rows (nr - tr, nr - refr): the smaller reference row walks for both
@@ -151,7 +151,7 @@ __device__ __forceinline__ void radial_walks(const float4 *__restrict__ q, const
         for (int w = 0; w < 2; ++w) {
 #pragma unroll
             for (int k = 0; k < V; ++k) wk[w].val[k] = 0.0f;
-            wk[w].dqold = (2 * tid + w) / 2;  // the reference's initial run bin (receives an empty run)
+            wk[w].dqold = tid;  // any bin (receives an empty run), another for every thread
             wk[w].dq = qmax + 1;
             wk[w].lo = 1.0f;  // empty: the first pair derives its bin
             wk[w].hi = 0.0f;
@@ -212,12 +212,12 @@ __device__ __forceinline__ void radial_walks(const float4 *__restrict__ q, const
     }
 }
 
-// CTA = (reference row, kRowsPerCta target rows, NB images); mirror: flag 0 says that the
+// CTA = (reference row, `rows` target rows, NB images); mirror: flag 0 says that the
 // rows mirror (nullptr: not looked at, the rows would not fit in shared memory).
 template <int NB, int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) qcorr_radial_kernel(const float4 *__restrict__ q,
                                                             const float *__restrict__ images, int nr, int nc,
-                                                            int qmax, double *__restrict__ out,
+                                                            int qmax, int rows, double *__restrict__ out,
                                                             const uint32_t *__restrict__ mirror) {
     extern __shared__ __align__(16) unsigned char qsm[];
     const bool mir = mirror && *mirror == 0u;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) qcorr_radial_kernel(const flo
     const int refr = blockIdx.x;
     const int tid = threadIdx.x;
     // rows past the detector, or (mirrored) walked by their mirror rows: nothing to do
-    const int dr0 = blockIdx.y * kRowsPerCta;
+    const int dr0 = blockIdx.y * rows;
     if (refr + dr0 >= nr || (mir && refr > 0 && 2 * refr + dr0 > nr)) return;
     for (int i = tid; i < NB * (qmax + 1); i += blockDim.x) hist[i] = 0.0;
     // bound[k]: smallest float d2 >= 0 with rint(sqrt(d2)) >= k, k = 0..qmax+1,
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) qcorr_radial_kernel(const flo
         }
         bound[k] = b;
     }
-    if (mir) radial_walks<NB, true>(q, images, nr, nc, qmax, refr, sref, stgt, vref, vtgt, hist, bound);
-    else radial_walks<NB, false>(q, images, nr, nc, qmax, refr, sref, stgt, vref, vtgt, hist, bound);
+    if (mir) radial_walks<NB, true>(q, images, nr, nc, qmax, rows, refr, sref, stgt, vref, vtgt, hist, bound);
+    else radial_walks<NB, false>(q, images, nr, nc, qmax, rows, refr, sref, stgt, vref, vtgt, hist, bound);
     __syncthreads();
     for (int k = 0; k < NB; ++k)
         for (int i = tid; i < qmax; i += blockDim.x)
@@ -388,7 +388,8 @@ extern "C" idiwf_status idiwf_qcorr_radial(const float *q, const float *images, 
     if (reinterpret_cast<uintptr_t>(q) & 15) return set_error(IDIWF_ERR_INVALID_ARGUMENT, "q must be 16-byte aligned");
     if (!workspace || workspace_bytes < 256) return set_error(IDIWF_ERR_WORKSPACE, "workspace too small");
     IDIWF_CUDA_CHECK(cudaMemsetAsync(out, 0, sizeof(double) * (size_t)n_images * qmax, stream));
-    const int threads = (qmax + 1 + 31) / 32 * 32;  // two of the 2 qmax + 1 column offsets each
+    // two of the 2 min(qmax, nc - 1) + 1 column offsets each
+    const int threads = (std::min(qmax, nc - 1) + 1 + 31) / 32 * 32;
     const float4 *q4 = reinterpret_cast<const float4 *>(q);
     // as many images per walk, and the mirror rows, as 200 KB of shared memory hold (every
     // detector up to 2048 columns takes 2 images and the mirror rows)
@@ -404,19 +405,28 @@ extern "C" idiwf_status idiwf_qcorr_radial(const float *q, const float *images, 
         qcorr_mirror_kernel<<<blocks, 256, 0, stream>>>(q4, nr, nc, flag);
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
-    const dim3 grid(nr, (qmax + kRowsPerCta - 1) / kRowsPerCta);
+    // Target rows per CTA: two where that leaves a dozen waves of CTAs (row pairs, half of
+    // them walked by their mirror pairs), else one, so that small detectors fill the chip.
+    // us with 1, 2 and 8 rows: 2 images of 99 x 64, 103 bins 108, 122, 225; 2 of 72 x 287,
+    // 112 bins 226, 285, 621; 3 of 249 x 360, 167 bins 3970, 3998, 4652; 2 of 400 x 400, 256
+    // bins 8533, 8350, 8633.
+    const int64_t in_reach = std::min(qmax, nr);
+    const int64_t row_pairs = in_reach * nr - in_reach * (in_reach - 1) / 2;
+    int rows = row_pairs >= 4 * 12 * 4 * (int64_t)qcorr_sms() ? 2 : 1;
+    const dim3 grid(nr, ((int)in_reach + rows - 1) / rows);
     for (int b = 0; b < n_images;) {
         const int n = std::min(nb, n_images - b);
         // blocks of up to 288 threads (up to 287 bins) fit four to an SM at 56 registers: bin
         // changes stall a warp for long, so more warps pay although a few values spill (2 x 512^2,
-        // 256 bins: 15.8 ms; 16.7 with three at 72 registers, 20.3 with two)
+        // 256 bins: 16.0 ms; 16.7 with three at 72 registers, 20.3 with two)
         void *fn = threads <= 288 ? (n == 2 ? (void *)qcorr_radial_kernel<2, 288, 4> : (void *)qcorr_radial_kernel<1, 288, 4>)
                                   : (n == 2 ? (void *)qcorr_radial_kernel<2, 512, 2> : (void *)qcorr_radial_kernel<1, 512, 2>);
         const size_t smem = radial_smem(nc, qmax, n, mirror);
-        IDIWF_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // (one limit for every call: calls from several threads do not lower it under one another)
+        IDIWF_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
         const float *im = images + (int64_t)b * nr * nc;
         double *o = out + (int64_t)b * qmax;
-        void *args[] = {&q4, &im, &nr, &nc, &qmax, &o, &flag};
+        void *args[] = {&q4, &im, &nr, &nc, &qmax, &rows, &o, &flag};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, grid, dim3(threads), args, smem, stream));
         b += n;
     }

@@ -20,6 +20,7 @@ from idi_b200.simulation import _core  # noqa: E402
     ((48, 35), 511, (None, None)),   # odd columns, more bins than the detector reaches
     ((40, 64), 300, (20.0, 11.0)),   # mirrored rows, columns off centre
     ((40, 64), 64, (19.5, None)),    # rows off centre
+    ((300, 12), 121, (None, None)),  # enough row pairs for two target rows per CTA, the last alone
 ])
 def test_radial_shared_walks_vs_oracle(images, shape, qmax, centre):
     """The runs are the reference's, so only the FP64 additions' order differs (1e-11)."""
