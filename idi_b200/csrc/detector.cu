@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(256) cs_gather_kernel(const T *__restrict__ co
     if (bad) record_error(err, kErrValue);
 }
 
-// Tiled gather: a CTA owns a kCsTR x kCsTC tile of output pixels, four per thread.  It
+// Tiled gather: a CTA owns a TR x kCsTC tile of output pixels, one per thread and 8 rows.  It
 // stages the counts of the tile and its w-pixel halo, numbers the region's photons
 // (exclusive scan), and takes them in chunks of `cap`: one thread per photon draws its
 // offsets, one per (photon, factor) computes the 2 (2w + 1) charge factors, and every
@@ -445,11 +445,11 @@ __global__ void __launch_bounds__(256) cs_gather_kernel(const T *__restrict__ co
 // tiles carry 13 % halo (8 x 32: 33 %), and 16 KB chunks let five CTAs share an SM whatever the
 // density.  8 x 1024^2, 1e5 photons each, s = 0.5: 0.24 ms, against 0.62 ms with 8 x 32 tiles,
 // 64 KB of factors and a look at every neighbour pixel.
-constexpr int kCsTR = 32, kCsTC = 32, kCsThreads = 256, kCsMaxW = 4;
+constexpr int kCsTC = 32, kCsThreads = 256, kCsMaxW = 4;
 constexpr size_t kCsChunkBytes = 16 * 1024;
 constexpr int kCsMaxPhotons = 1 << 24;  // a region with more takes cs_pixel
 
-template <typename T, bool INJ>
+template <typename T, bool INJ, int TR>
 __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restrict__ counts, const CsParams P,
                                                              const double *__restrict__ positions,
                                                              const double *__restrict__ scales,
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restr
     __shared__ int wsum[8];
     __shared__ int s_total;
     const int w = P.w, KW = 2 * w + 1;
-    const int RH = kCsTR + 2 * w, RW = kCsTC + 2 * w, RN = RH * RW;
+    const int RH = TR + 2 * w, RW = kCsTC + 2 * w, RN = RH * RW;
     double *fx = csm;
     double *fy = fx + (size_t)cap * KW;
     double *scl = fy + (size_t)cap * KW;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restr
     int *rs = rc + RN;  // RN + 1: the end
     const int64_t npix = (int64_t)P.nx * P.ny;
     const int b = blockIdx.z;
-    const int r0 = blockIdx.y * kCsTR, c0 = blockIdx.x * kCsTC;
+    const int r0 = blockIdx.y * TR, c0 = blockIdx.x * kCsTC;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     bool bad = false;
     for (int ri = tid; ri < RN; ri += kCsThreads) {
@@ -504,11 +504,11 @@ __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restr
     if (tid == kCsThreads - 1) s_total = rs[RN] = run;
     __syncthreads();
     const int total = s_total;
-    constexpr int kPer = kCsTR * kCsTC / kCsThreads;  // output pixels per thread, kCsTR / kPer rows apart
+    constexpr int kPer = TR * kCsTC / kCsThreads;  // output pixels per thread, TR / kPer rows apart
     const int tr = tid / kCsTC, col = c0 + tid % kCsTC;
     if (total >= kCsMaxPhotons) {  // uniform across the CTA
         for (int k = 0; k < kPer; ++k) {
-            const int r = r0 + tr + k * (kCsTR / kPer);
+            const int r = r0 + tr + k * (TR / kPer);
             if (r < P.nx && col < P.ny)
                 out[(int64_t)b * npix + (int64_t)r * P.ny + col] =
                     cs_pixel<T, INJ>(counts, P, positions, scales, start, b, r, col, bad);
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restr
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int r = r0 + tr + k * (kCsTR / kPer);
+            const int r = r0 + tr + k * (TR / kPer);
             if (r >= P.nx || col >= P.ny) continue;
             // the photons of a region row's columns [col - w, col + w] are numbered in one run
             // (a halo position off the detector holds none)
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kCsThreads, 5) cs_tile_kernel(const T *__restr
     }
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        const int r = r0 + tr + k * (kCsTR / kPer);
+        const int r = r0 + tr + k * (TR / kPer);
         if (r < P.nx && col < P.ny) out[(int64_t)b * npix + (int64_t)r * P.ny + col] = acc[k];
     }
     if (bad) record_error(err, kErrValue);
@@ -662,21 +662,34 @@ static idiwf_status photons_out(int32_t out_dtype, const void *probs, int32_t n_
     }
 }
 
+template <typename T, bool INJ, int TR>
+static void launch_cs_tiles(const T *counts, const CsParams &P, const double *positions, const double *scales,
+                            const int64_t *start, double *out, WsHeader *hdr, cudaStream_t stream) {
+    const int KW = 2 * P.w + 1;
+    const int RN = (TR + 2 * P.w) * (kCsTC + 2 * P.w);
+    const size_t per = (2 * (size_t)KW + 3) * sizeof(double) + 2 * sizeof(int);  // bytes of a photon
+    const int cap = (int)(kCsChunkBytes / per) / 2 * 2;
+    const size_t smem = (size_t)cap * per + (2 * (size_t)RN + 1) * sizeof(int);  // 29 KB at most
+    const dim3 grid((P.ny + kCsTC - 1) / kCsTC, (P.nx + TR - 1) / TR, P.n_images);
+    cs_tile_kernel<T, INJ, TR><<<grid, kCsThreads, smem, stream>>>(counts, P, positions, scales, start, out,
+                                                                   &hdr->error, cap);
+}
+
 template <typename T, bool INJ>
 static idiwf_status launch_cs_gather(const T *counts, const CsParams &P, const double *positions,
                                      const double *scales, const int64_t *start, double *out, WsHeader *hdr,
                                      int blocks, cudaStream_t stream) {
     if (P.w <= kCsMaxW && P.n_images <= 65535) {
-        const int KW = 2 * P.w + 1;
-        const int RN = (kCsTR + 2 * P.w) * (kCsTC + 2 * P.w);
-        const size_t per = (2 * (size_t)KW + 3) * sizeof(double) + 2 * sizeof(int);  // bytes of a photon
-        const int cap = (int)(kCsChunkBytes / per) / 2 * 2;
-        const size_t smem = (size_t)cap * per + (2 * (size_t)RN + 1) * sizeof(int);
-        IDIWF_CUDA_CHECK(cudaFuncSetAttribute(cs_tile_kernel<T, INJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-        const dim3 grid((P.ny + kCsTC - 1) / kCsTC, (P.nx + kCsTR - 1) / kCsTR, P.n_images);
-        cs_tile_kernel<T, INJ><<<grid, kCsThreads, smem, stream>>>(counts, P, positions, scales, start, out,
-                                                                   &hdr->error, cap);
+        // 32 rows from a full wave of tiles on (five to an SM), else 8: fewer tiles leave SMs
+        // without work, and a tile's photons are a serial chain of chunks.  Photon counts and
+        // charge sharing together, us, 8 / 32 rows: 1 x 73 x 140, 1.2e4 photons 143 / 223;
+        // 4 x 216 x 301, 4.6e4 202 / 216; 5 x 276 x 336, 5e3 132 / 131 (495 tiles); 7 x 745 x 534,
+        // 6e3 209 / 176.
+        const int64_t tiles = (int64_t)((P.ny + kCsTC - 1) / kCsTC) * ((P.nx + 31) / 32) * P.n_images;
+        if (tiles >= 5 * (int64_t)dev_sms())
+            launch_cs_tiles<T, INJ, 32>(counts, P, positions, scales, start, out, hdr, stream);
+        else
+            launch_cs_tiles<T, INJ, 8>(counts, P, positions, scales, start, out, hdr, stream);
     } else {
         cs_gather_kernel<T, INJ><<<blocks, 256, 0, stream>>>(counts, P, positions, scales, start, out, &hdr->error);
     }

@@ -23,3 +23,11 @@ def test_tiles_and_chunks_vs_oracle(shape, s, ns, mean):
     out = _core.chargesharing(torch.from_numpy(counts).cuda(), s, ns, key=(5, 6), stream=3).cpu().numpy()
     ref = np.stack([oracle.chargesharing(counts, s, ns, key=(5, 6), stream=3)[b] for b in range(2)])
     np.testing.assert_allclose(out, ref, rtol=1e-12, atol=1e-15)
+
+
+@pytest.mark.parametrize("s,ns,mean", [(0.5, 0.0, 0.05), (0.9, 0.2, 1.0)])
+def test_tall_tiles_vs_oracle(s, ns, mean):
+    """Enough 32 x 32 tiles for the tall form (a full wave of them), the last row of tiles one pixel high."""
+    counts = np.random.default_rng(17).poisson(mean, (2, 97, 3000)).astype(np.int32)
+    out = _core.chargesharing(torch.from_numpy(counts).cuda(), s, ns, key=(5, 6), stream=3).cpu().numpy()
+    np.testing.assert_allclose(out, oracle.chargesharing(counts, s, ns, key=(5, 6), stream=3), rtol=1e-12, atol=1e-15)
