@@ -168,7 +168,7 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     L.off_part = o;   o += align256((size_t)L.n_chunks * L.nrec * kBwdNAcc * 4);
     int64_t nmax = 0;
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
-    L.nodes = (double)nmax * (double)npix >= kNodeMinPairs && make_node_geom(make_geom(g)).ok;
+    L.nodes = (double)nmax * (double)npix >= kNodeMinPairsDiff && make_node_geom(make_geom(g)).ok;
     if (L.nodes) {
         L.entries = node_entries(npix);
         L.lx_bytes = (size_t)g->nx * node_cap(g->nx) * 8;
@@ -330,7 +330,7 @@ __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, co
         ai.n0 = ai.n1 = ai.cpx = ai.nchunks = ai.nblocks = ai.unit0 = ai.pad = 0;
         const double r = sqrt((double)__uint_as_float(r2)), pairs = (double)n * g.nx * g.ny;
         bool use = false;
-        if (nodes && n > 0 && (ai.path == kPathRuns || ai.path == kPathPixel) && pairs >= kNodeMinPairs &&
+        if (nodes && n > 0 && (ai.path == kPathRuns || ai.path == kPathPixel) && pairs >= kNodeMinPairsDiff &&
             node_reach(g, ng, r, false)) {
             double e[2];
 #pragma unroll

@@ -67,6 +67,7 @@ struct NodeGeom {
     double e[3][3];  // unit vectors of the detector axes and their normal
     double phi[2], t[2], s[2];
     double inv_d;
+    double min_pairs;  // fewest pairs of an image that may take nodes
     int32_t ok, ortho;  // ortho: the axes are orthonormal (cells need it)
 };
 
@@ -169,8 +170,11 @@ __device__ __forceinline__ void node_weights_row(double *__restrict__ L, int n, 
 }
 
 // Fewest pairs of an image for which nodes are considered: below it the three
-// further kernels cost more than the direct sum (split precision, FP64).
-constexpr double kNodeMinPairs = 8e6, kNodeMinPairs64 = 2e6;
+// further kernels cost more than the direct sum (split precision, FP64).  In
+// differentiation (split-precision complex128 fields, and the adjoint) the host's launches
+// set the pace of small images, and the direct kernels have fewer: a gradient step of
+// 26e6 pairs 0.67 ms direct, 0.69 over nodes, of 47e6 pairs 0.68 and 0.66.
+constexpr double kNodeMinPairs = 8e6, kNodeMinPairs64 = 2e6, kNodeMinPairsDiff = 3.2e7;
 
 // Floats as unsigned integers in their order (0 lies below them all).
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -268,7 +272,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         // (amplitudes whose fixed-point unit would leave FP32's exponents, infinite or NaN
         // ones take the direct kernels)
         if (bp.nodes && n > 0 && (direct == kPathRuns || direct == kPathPixel) &&
-            pairs >= (fine ? kNodeMinPairs64 : kNodeMinPairs) && node_reach(g, ng, r, fine) &&
+            pairs >= ng.min_pairs && node_reach(g, ng, r, fine) &&
             (amax == 0u || (amax >= __float_as_uint(0x1p-40f) && amax <= __float_as_uint(0x1p100f)))) {
             double lo[3], w[3];
 #pragma unroll

@@ -1,6 +1,8 @@
 """Band-limited evaluation (nodes and interpolation) of the split forward: against
 the cancellation-free FP64 oracle at the edges of its tiles and of its dispatch."""
 
+from functools import partial
+
 import numpy as np
 import pytest
 
@@ -18,6 +20,9 @@ from idi_b200.simulation import _core  # noqa: E402
 # term 5e-8; FP32 sums over 16 emitters 8.5e-8; interpolation below 1e-8.  In quadrature
 # 1.2e-7; the bound leaves a factor 2 for the pixels' uneven weights.
 FIELD_2NORM = 2.4e-7
+# Complex128 fields take the sums in FP64: turns in 2^-32, 4e-10 rms; polynomials 1.4e-9 at
+# most; interpolation below 1e-8.
+FINE_2NORM = 1.5e-8
 
 
 def _err(E, ref):
@@ -49,17 +54,45 @@ def test_forward_nodes_vs_oracle(ndet, n, r, tilt, settings):
     oflags = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
     ref = oracle.wavefield(oracle.geometry(ndet, 75.0, 1e5, K64, tilt, off), oflags, at, amp)
     for dt in (np.float32, np.float64):
-        E, pairs = _forward(at, [0, n], geom, amp.astype(dt))
+        E, pairs = _forward(at, [0, n], geom, amp.astype(dt), out=nat.OUT_C64)
         assert 0 < pairs < n * ndet[0] * ndet[1] / 4
         # float32 amplitudes are the kernel's own precision: compare with theirs
         assert _err(E[0], ref) < FIELD_2NORM + 4e-8, (dt, _err(E[0], ref))
+
+
+@pytest.mark.parametrize("ndet,n,r,tilt", [
+    ([64, 125], 4000, 0.01, (0, 0)),       # the smallest images that take nodes for complex128
+    ([65, 131], 4021, 0.008, (0.1, -0.05)),
+    ([300, 77], 1400, 0.012, (0, 0.2)),
+    ([1000, 24], 1391, 0.006, (0, 0)),
+])
+@pytest.mark.parametrize("settings", ["", "nf", "nf scale", "scale", "secondorder"])
+def test_forward_nodes_fp64_sums(ndet, n, r, tilt, settings):
+    g = rng(ndet[0] + n)
+    at = atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n))
+    amp = g.uniform(0.5, 1.5, n).astype(np.float32)
+    flags, _, _ = _core.parse_settings(settings)
+    off = (300.0, -200.0)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, tilt, off, flags)
+    oflags = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(oracle.geometry(ndet, 75.0, 1e5, K64, tilt, off), oflags, at, amp.astype(np.float64))
+    E, pairs = _forward(at, [0, n], geom, amp)
+    assert 0 < pairs < n * ndet[0] * ndet[1] / 4
+    E0 = E[0]
+    if "nf" in settings:  # moduli: the pixels' constant phases reach 2e8 rad, whose FP64 rounding is 2e-8
+        E0, ref = np.abs(E0), np.abs(ref)
+    # (the near field's 1/r factors are FP32, 6e-8 of the amplitude each)
+    assert _err(E0, ref) < FINE_2NORM + (6e-8 if settings == "nf scale" else 0), _err(E0, ref)
+    fewer = 31999999 // (ndet[0] * ndet[1])
+    _, pairs = _forward(at[:fewer], [0, fewer], geom, amp[:fewer])
+    assert pairs in (0, fewer * ndet[0] * ndet[1])
 
 
 def test_mixed_batch_is_the_same_image_by_image():
     """Images on nodes, direct ones, empty ones in one batch: each the same, bit for bit, as
     alone (the fixed-point sums do not depend on how the work is cut), in fields and intensities."""
     g = rng(4)
-    spec = [(3000, 0.01), (0, 0.01), (500, 0.4), (2500, 0.02), (700, 0.01), (20001, 0.004)]
+    spec = [(4000, 0.01), (0, 0.01), (500, 0.4), (3500, 0.02), (1700, 0.01), (700, 0.01), (20001, 0.004)]
     imgs = [atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n)) for n, r in spec]
     off = np.concatenate([[0], np.cumsum([n for n, _ in spec])])
     geom = _core.make_geom([96, 101], 75.0, 1e5, K64, flags=nat.NF)
@@ -94,6 +127,7 @@ def test_dispatch_limits():
     n = 3000
     at = atoms(sphere(g, n, 0.01), g.uniform(0, 2 * np.pi, n))
     geom = _core.make_geom([72, 64], 75.0, 1e5, K64, flags=nat.NF)
+    _forward = partial(globals()["_forward"], out=nat.OUT_C64)
     full = n * 72 * 64
     E, pairs = _forward(at, [0, n], geom, np.ones(n))
     assert 0 < pairs < full / 4
@@ -197,9 +231,9 @@ def _exact_nf(ndet, tilt, off, scale, at, amp, target=None):
 
 
 @pytest.mark.parametrize("ndet,n,r,tilt", [
-    ([64, 64], 2048, 0.01, (0, 0)),
-    ([65, 131], 1029, 0.008, (0.1, -0.05)),
-    ([300, 77], 517, 0.012, (0, 0.2)),
+    ([64, 125], 4000, 0.01, (0, 0)),  # the smallest images that take nodes in differentiation
+    ([65, 131], 4021, 0.008, (0.1, -0.05)),
+    ([300, 77], 1400, 0.012, (0, 0.2)),
 ])
 @pytest.mark.parametrize("settings", ["", "nf", "nf scale", "scale", "secondorder"])
 def test_adjoint_nodes_vs_oracle(ndet, n, r, tilt, settings):
