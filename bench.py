@@ -8,12 +8,15 @@ an fcc lattice (a = 0.36 nm) filling a 12 nm cube with 0.01 nm Gaussian
 jitter, uniform phases, 8.0 keV, 1024 x 1024 detector with 50 um pixels at
 0.2 m, 32 images with independent phase draws, near-field geometry, split
 precision.  Inputs are synthetic (seeded Philox).  One step = one batched
-forward of the 32 images (1.68e12 emitter-pixel pairs).
+forward of the 32 images (1.68e12 emitter-pixel pairs).  The rate counts the pairs of
+the sum that the fields are; the kernels sum the emitters on the nodes that a
+band-limited field needs and interpolate, and the line gives the emitter-node pairs
+that they evaluate beside it (roofline.evaluated_pairs_per_step).
 
 The JSON line carries the headline value (pairs/s with inputs resident in
 HBM), the end-to-end figure through the public API (host emitters in, host
 fields out), the forward+adjoint cost on the differentiation configuration,
-the all-FP64 comparator, split-vs-FP64 error statistics, the MUFU roofline
+the all-FP64 comparator, split-vs-FP64 error statistics, the FP64 roofline
 and the CPU baseline (the oracle's C restatement on the host cores).
 
 Multi-GPU (torchrun): images are independent, so every rank runs its own 32
@@ -210,13 +213,13 @@ def c2_oracle_windows(out, pos, ph, k, w=64, seed=9):
 
 
 def summarize_targets(line, t):
-    """The target figures (C2 rate, SFU fraction, split/FP64 speed-up and error,
+    """The target figures (C2 rate, FP64 fraction, split/FP64 speed-up and error,
     end-to-end rate, forward+adjoint ratio, batched rate and balance, time
     path) in one compact object, last on the line."""
     def r4(x):
         return None if x is None else float(f"{x:.4g}")
 
-    out = {"c2_pairs_per_s": r4(t["c2_pairs_per_s"]), "c2_sfu_frac": r4(t["c2_sfu_frac"])}
+    out = {"c2_pairs_per_s": r4(t["c2_pairs_per_s"]), "c2_fp64_frac": r4(t["c2_fp64_frac"])}
     fp64 = line.get("fp64", {}).get("value")
     if fp64:
         out["c2_split_over_fp64"] = r4(t["c2_pairs_per_s"] / fp64)
@@ -405,20 +408,17 @@ def main():
     value = pairs_per_step * world / (ms_per_step * 1e-3)
     kern_avg = sum(kern_ms) / len(kern_ms)
 
-    # MUFU roofline: the split kernel issues one sin and one cos per pair
-    mufu = _core.microbench("mufu_sincos", dev)
-    achieved_mufu = 2.0 * pairs_per_step / (kern_avg * 1e-3)
+    # What bounds the step now is the FP64 pipe: the field is band-limited over the detector, so
+    # each image's emitters are summed on nodes (cells of the object, each with its own small
+    # grid) and interpolated to the pixels.  19 FP64 operations per emitter and node (the
+    # phase 3, the angle 1, the near-field term 1, sine and cosine 12, the sums 2), counted in
+    # the source; the interpolation's are not counted.
+    evaluated = _core.evaluated_pairs(dev)
+    fp64_peak = 0.5 * _core.microbench("fp64_fma", dev)  # (2 flop an operation)
+    achieved = 19.0 * evaluated / (kern_avg * 1e-3)
     clocks = clk.summary()
-    traffic = None
-    try:  # DRAM bytes per launch from the committed ncu capture, scaled to this launch
-        with open(os.path.join(ROOT, "profiles", "fwd_split_traffic.json")) as f:
-            cap = json.load(f)
-        traffic = (cap["dram_bytes_read"] + cap["dram_bytes_write"]) * (N_IMG * N_EMIT) / (
-            cap["images"] * cap["emitters_per_image"])
-    except (OSError, KeyError, ValueError):
-        pass
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    nominal_mufu = sms * 16 * (clocks["sm_max_mhz"] or 1965.0) * 1e6
+    # bytes that a step cannot do without: the emitters' rows, read once, and the fields
+    traffic = float(N_IMG * N_EMIT * 32 + N_IMG * NDET * NDET * 16)
 
     line = {
         "metric": METRIC,
@@ -431,22 +431,25 @@ def main():
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "f64 phase / f32 sincos+sum",
+        "dtype": "f64 phases, sincos, sums and interpolation (f32 near-field term)",
         "data": "synthetic (seeded Philox)",
         "config": {"workload": WORKLOAD, "images": N_IMG, "emitters": N_EMIT, "detector": [NDET, NDET],
                    "settings": SETTINGS, "parallelism": f"images per rank, {world} rank(s)",
                    "l2": "flushed between steps (256 MiB write)", "kernel_shape": cfg},
-        # per step: prep_split_kernel, the pixel-run kernel, and the per-pixel and exact near-field
-        # kernels (both return at once on this workload)
-        "gpu_launches": 4 * args.steps,
+        # per step: extents and plan, cell counts, record prep, the three direct kernels (which
+        # return at once on this workload), and seven node kernels for each of six groups of
+        # images (clearing, sums, weights, two for the cells, two interpolations)
+        "gpu_launches": 48 * args.steps,
         "clocks": clocks,
-        "roofline": {"bound": "sfu", "achieved": achieved_mufu / 1e9, "peak": mufu / 1e9, "unit": "Gop/s (MUFU)",
-                     "frac": achieved_mufu / mufu, "frac_of_nominal": achieved_mufu / nominal_mufu,
-                     "peak_source": "measured: in-repo MUFU sin/cos microbenchmark (idiwf_microbench kind 0)",
-                     "ops_per_pair": 2, "kernel_ms": kern_avg, "traffic": traffic,
-                     "traffic_unit": "bytes per launch (ncu capture of 8 images, scaled by emitter records)"},
+        "roofline": {"bound": "fp64", "achieved": achieved / 1e9, "peak": fp64_peak / 1e9,
+                     "unit": "G FP64 operations/s (node sums)", "frac": achieved / fp64_peak,
+                     "peak_source": "measured: in-repo FP64 FMA microbenchmark",
+                     "ops_per_evaluated_pair": 19, "evaluated_pairs_per_step": evaluated,
+                     "pairs_per_evaluated_pair": pairs_per_step / max(evaluated, 1),
+                     "kernel_ms": kern_avg, "traffic": traffic,
+                     "traffic_unit": "bytes per step that the call cannot do without (emitter rows, complex128 fields)"},
     }
-    targets = {"c2_pairs_per_s": value, "c2_sfu_frac": achieved_mufu / mufu}
+    targets = {"c2_pairs_per_s": value, "c2_fp64_frac": achieved / fp64_peak}
     if not args.no_extras and rank == 0:
         line.update(extras(args, torch, dev, _core, nat, cuda, simobj, pos, ph, k, geom, atoms, offsets, cfg))
     if not args.no_cpu_baseline and rank == 0 and world == 1:
