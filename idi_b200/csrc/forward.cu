@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(256)
             if (amps) amp = amp_dtype == IDIWF_F32 ? (double)static_cast<const float *>(amps)[s]
                                                   : static_cast<const double *>(amps)[s];
             rec.ra[r] = amp;
-            if (plan) ex.add(ng, a, __double2float_ru(fabs(amp)));
+            // (a phase that is not finite goes the way of such an amplitude: the fixed-point
+            // sums would lose the NaN that the direct kernel returns)
+            if (plan) ex.add(ng, a, isfinite(a.w) ? __double2float_ru(fabs(amp)) : NAN);
         } else {
             rec.r64[r] = make_double4(0, 0, 0, 0);
             rec.ra[r] = 0.0;

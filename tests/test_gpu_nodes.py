@@ -184,6 +184,20 @@ def test_fp64_nodes_vs_oracle(ndet, n, r, tilt, settings):
     assert _core.evaluated_pairs() == 0
 
 
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_fp64_phase_not_finite(bad):
+    """An emitter whose phase is not finite makes its FP64 image NaN, and no other image."""
+    g = rng(11)
+    n = 1200
+    at = atoms(sphere(g, 2 * n, 0.01), g.uniform(0, 2 * np.pi, 2 * n))
+    at[n + 77, 3] = bad
+    geom = _core.make_geom([64, 64], 75.0, 1e5, K64)
+    E = _core.forward(torch.from_numpy(at).cuda(), [0, n, 2 * n], geom, nat.DOUBLE, nat.OUT_C128).cpu().numpy()
+    assert _core.evaluated_pairs() > 0
+    assert np.isfinite(E[0]).all()
+    assert np.isnan(E[1].real).all() and np.isnan(E[1].imag).all()
+
+
 # 2-norm of the gradients' errors.  The adjoint pairs carry the forward's 1.2e-7, their FP32
 # sums over at most 512 nodes 2.4e-8 sqrt(512 / 2) = 3.8e-7, and G = 4 (I - T) conj(E) about
 # three times the field's relative error; 7e-7 in quadrature, times 4 for what cancels in
