@@ -114,7 +114,7 @@ class _Workspaces:
 
     def __init__(self):
         self._bufs = {}
-        self._lock = threading.Lock()
+        self._lock = threading.RLock()  # (a collected plan drops its buffer, also from within get)
 
     def get(self, nbytes: int, device: torch.device, role: str = "main") -> torch.Tensor:
         key = (device.index if device.index is not None else torch.cuda.current_device(), role)

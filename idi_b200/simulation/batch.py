@@ -10,6 +10,7 @@ host->device copy plus one graph replay.
 
 from __future__ import annotations
 
+import weakref
 from typing import Optional, Sequence
 
 import numpy as np
@@ -52,6 +53,8 @@ class BatchPlan:
         self._use_graph = graph
         self._graph = None
         self._role = f"plan{id(self)}"
+        # a plan's workspace (up to half a gigabyte of node sums) goes with the plan
+        weakref.finalize(self, _core.WORKSPACES.drop, self.device, self._role).atexit = False
 
     def _launch(self):
         return _core.forward(self.atoms, self.offsets, self.geom, self.precision, self.out_kind,
@@ -99,6 +102,8 @@ class BatchPlan:
             self._graph.replay()
         else:
             self._launch()
+        # (the allocator may hand the workspace on only after this stream's work on it)
+        _core.WORKSPACES.get(0, self.device, self._role).record_stream(torch.cuda.current_stream(self.device))
         return self.out
 
     def cta_times(self) -> np.ndarray:

@@ -60,3 +60,27 @@ def test_more_images_than_one_launch():
     og = oracle.geometry([4, 4], 75.0, 1e5, K64)
     for b in (0, 511, 512, 599):
         assert np.abs(E[b] - oracle.wavefield(og, oracle.NF, imgs[b])).max() < 1e-12
+
+
+def test_plan_workspace_goes_with_the_plan():
+    """A plan that is dropped without close() gives its workspace back, also one made while
+    another is in use, and the other's results stay."""
+    import gc
+
+    geom = _core.make_geom([64, 64], 75.0, 1e5, K64, flags=nat.NF)
+    counts = [5000, 300]
+    imgs, _ = _batch(5, counts)
+    at = torch.from_numpy(np.concatenate(imgs)).cuda()
+    gc.collect()  # earlier plans
+    kept = BatchPlan(counts, geom, nat.SPLIT, nat.OUT_C64, autotune=False)
+    first = kept.run(at).clone()
+    before = set(_core.WORKSPACES._bufs)
+    for _ in range(3):
+        other = BatchPlan(counts, geom, nat.SPLIT, nat.OUT_C64, autotune=False)
+        assert torch.equal(other.run(at), first)
+        assert len(_core.WORKSPACES._bufs) == len(before) + 1
+        del other
+        gc.collect()
+        assert set(_core.WORKSPACES._bufs) == before
+    assert torch.equal(kept.run(at), first)
+    kept.close()
