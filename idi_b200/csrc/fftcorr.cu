@@ -561,7 +561,7 @@ __global__ void fc_twiddle_kernel(double2 *tw, int N) {
 // ---------------------------------------------------------------------------
 // General lengths: the reference pads each axis to fastlen(2 n) (factors 2,
 // 3, 5, 7, 11).  The same three kernels, with mixed-radix Stockham passes
-// (radix 8/4/2 and 3, 5, 7, 11), rows packed in pairs as x_a + i x_b for the
+// (radix 10/8/6/4/2 and 3, 5, 7, 11), rows packed in pairs as x_a + i x_b for the
 // row FFT, and the inverse along rows of length L1 = G1 through a complex
 // inverse of L1/2 values (the real parts only at frequencies 0 and L1/2, as
 // a c2r transform).  The output is the centre crop (i - n0) mod G0,
@@ -605,11 +605,26 @@ template <int R> __host__ __device__ constexpr int fcg_out(int q) { return (R & 
 
 // R-point DFT in registers, output q in v[fcg_out<R>(q)]; odd R by the
 // symmetric pairs x_k +- x_{R-k} (real and imaginary halves), R = 2^m by
-// dft_reg.
+// dft_reg, R = 2 B with odd B by the prime-factor map (Good 1958: inputs
+// B i + 2 j, outputs by their remainders modulo 2 and B; no twiddles).
 template <int R, bool INV, typename V> __device__ __forceinline__ void fcg_dft(V *v) {
     using T = decltype(v[0].x);
     if constexpr ((R & (R - 1)) == 0) {
         dft_reg<R, INV>(v);
+    } else if constexpr (R % 2 == 0) {
+        constexpr int B = R / 2;
+        static_assert(B % 2 == 1, "2 x odd");
+        V u[2][B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+            const V a = v[(2 * j) % R], b = v[(B + 2 * j) % R];
+            u[0][j] = cx_add(a, b);
+            u[1][j] = cx_sub(a, b);
+        }
+        fcg_dft<B, INV>(u[0]);
+        fcg_dft<B, INV>(u[1]);
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = u[q % 2][q % B];
     } else {
         constexpr int h = (R - 1) / 2, off = fcg_odd_off<R>();
         V a[h], b[h];
@@ -642,8 +657,7 @@ template <int R, bool INV, typename V> __device__ __forceinline__ void fcg_dft(V
     }
 }
 
-// Radices of one general length n (pass order: 11, 7, 5, 3, then 8s, then
-// the remaining 4 or 2).
+// Radices of one general length n, in pass order (fcg_radices).
 constexpr int kFcgMaxPasses = 14;
 struct FcgRad {
     int n, np;
@@ -676,6 +690,34 @@ struct FcgIdx {
     }
 };
 
+// v[r] *= exp(-/+ 2 pi i at r / ntab), r = 1..R-1, from the table's values for 1 and 4
+// (a power r by repeated products carries r times the table's rounding and r - 1 of its
+// own; from the two values no factor is a product of more than three).  The second load
+// takes 6 % (8 x 1000 x 1050 FP64), and the error against exact sums of whole numbers
+// falls from 3.3e-16 to 2.7e-16.
+template <int R, bool INV, typename V>
+__device__ __forceinline__ void fcg_twiddle(V *v, const double2 *__restrict__ tab, int at) {
+    using T = decltype(v[0].x);
+    double2 w[R < 4 ? 4 : R];
+    w[1] = __ldg(&tab[at]);
+    if (INV) w[1].y = -w[1].y;
+    w[2] = cx_mul(w[1], w[1]);
+    w[3] = cx_mul(w[2], w[1]);
+    if constexpr (R > 4) {
+        w[4] = __ldg(&tab[4 * at]);
+        if (INV) w[4].y = -w[4].y;
+#pragma unroll
+        for (int r = 5; r < R; ++r) w[r] = cx_mul(w[r < 8 ? 4 : r - 4], w[r < 8 ? r - 4 : 4]);
+    }
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+        V q;
+        q.x = (T)w[r].x;
+        q.y = (T)w[r].y;
+        v[r] = cx_mul(v[r], q);
+    }
+}
+
 // Out-of-place Stockham pass of radix R (in -> out), one butterfly of R
 // values in registers per loop iteration.
 template <typename V, int R, bool INV>
@@ -691,11 +733,7 @@ __device__ __forceinline__ void fcg_pass(const V *in, V *out, int stride, int n,
         V v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = in[fcg_slot<V>(q, j + r * nb, stride)];
-        if (Ns > 1) {
-            double2 w = __ldg(&tab[k * tstep]);
-            if (INV) w.y = -w.y;
-            twiddle_powers<R>(v, w);
-        }
+        if (Ns > 1) fcg_twiddle<R, INV>(v, tab, k * tstep);
         fcg_dft<R, INV>(v);
         const int base = (j - k) * R + k;
 #pragma unroll
@@ -703,37 +741,66 @@ __device__ __forceinline__ void fcg_pass(const V *in, V *out, int stride, int n,
     }
 }
 
-// The FFT of `count` sequences of length rad.n: the values from `ld` (or
-// already in A) go through the passes between buffers A and B; returns the
-// buffer holding the result.
-template <typename V, bool INV, class Ld>
-__device__ __forceinline__ V *fcg_fft(V *A, V *B, int stride, const FcgRad &rad, int count,
-                                      const double2 *__restrict__ tab, int ntab, const Ld &ld, bool from_loader) {
-    const int n = rad.n;
-    if (from_loader) {
-        FcgIdx it(threadIdx.x, blockDim.x, n);
-        for (int idx = threadIdx.x; idx < count * n; idx += blockDim.x, it.next())
-            A[fcg_slot<V>(it.a, it.b, stride)] = ld(it.a, it.b);
-        __syncthreads();
+// First pass (Ns = 1, no twiddles) on the values of `ld`, R of them in flight
+// per thread: a copy of the block's values into shared memory, with its
+// barrier, is saved.  The kernels are bound by the latency of these trips (two blocks
+// of 256 threads per SM): 8 x 1000 x 1050 FP64 1.15 -> 0.99 ms with the first passes so
+// and radices 10 and 6, 8 x 1000^2 0.96 -> 0.80, FP32 0.61 -> 0.52.  QFAST: neighbouring threads take neighbouring sequences.
+template <typename V, int R, bool INV, bool QFAST, class Ld>
+__device__ __forceinline__ void fcg_first(V *out, int stride, int n, int count, const Ld &ld) {
+    const int nb = n / R, total = count * nb;
+    FcgIdx it(threadIdx.x, blockDim.x, QFAST ? count : nb);
+    for (int g = threadIdx.x; g < total; g += blockDim.x, it.next()) {
+        const int q = QFAST ? it.b : it.a, j = QFAST ? it.a : it.b;
+        V v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = ld(q, j + r * nb);
+        fcg_dft<R, INV>(v);
+#pragma unroll
+        for (int r = 0; r < R; ++r) out[fcg_slot<V>(q, j * R + r, stride)] = v[fcg_out<R>(r)];
     }
+}
+
+// fn(integral constant R) for the radix R of a pass.
+template <class F> __device__ __forceinline__ void fcg_radix(int R, const F &fn) {
+    switch (R) {
+        case 1: fn(std::integral_constant<int, 1>{}); break;
+        case 2: fn(std::integral_constant<int, 2>{}); break;
+        case 3: fn(std::integral_constant<int, 3>{}); break;
+        case 4: fn(std::integral_constant<int, 4>{}); break;
+        case 5: fn(std::integral_constant<int, 5>{}); break;
+        case 6: fn(std::integral_constant<int, 6>{}); break;
+        case 7: fn(std::integral_constant<int, 7>{}); break;
+        case 8: fn(std::integral_constant<int, 8>{}); break;
+        case 10: fn(std::integral_constant<int, 10>{}); break;
+        default: fn(std::integral_constant<int, 11>{}); break;
+    }
+}
+
+// The FFT of `count` sequences of length rad.n: the first pass takes the values
+// from `ld` and writes A (LOADER; `ld` may read B), or finds them in A; the
+// others go to and fro between the buffers A and B.  Returns the buffer holding
+// the result.
+template <typename V, bool INV, bool LOADER, bool QFAST = false, class Ld>
+__device__ __forceinline__ V *fcg_fft(V *A, V *B, int stride, const FcgRad &rad, int count,
+                                      const double2 *__restrict__ tab, int ntab, const Ld &ld) {
+    const int n = rad.n;
     V *in = A, *out = B;
-    int Ns = 1;
-    for (int p = 0; p < rad.np; ++p) {
-        const int R = rad.r[p];
-        switch (R) {
-            case 2: fcg_pass<V, 2, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            case 3: fcg_pass<V, 3, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            case 4: fcg_pass<V, 4, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            case 5: fcg_pass<V, 5, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            case 7: fcg_pass<V, 7, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            case 8: fcg_pass<V, 8, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-            default: fcg_pass<V, 11, INV>(in, out, stride, n, count, Ns, tab, ntab); break;
-        }
+    int Ns = 1, p = 0;
+    if constexpr (LOADER) {
+        fcg_radix(rad.r[0], [&](auto R) { fcg_first<V, R.value, INV, QFAST>(A, stride, n, count, ld); });
+        __syncthreads();
+        Ns = rad.r[0];
+        p = 1;
+    }
+    for (; p < rad.np; ++p) {
+        const int radix = rad.r[p];
+        fcg_radix(radix, [&](auto R) { fcg_pass<V, R.value, INV>(in, out, stride, n, count, Ns, tab, ntab); });
         __syncthreads();
         V *t = in;
         in = out;
         out = t;
-        Ns *= R;
+        Ns *= radix;
     }
     return in;
 }
@@ -764,7 +831,7 @@ __global__ void __launch_bounds__(512) fcg_blue_filter_kernel(const double2 *__r
         if (m < 0) return make_double2(0.0, 0.0);
         return make_double2(c[m].x, -c[m].y);
     };
-    const double2 *F = fcg_fft<double2, false>(S, S + stride, stride, radM, 1, twM, M, ld, true);
+    const double2 *F = fcg_fft<double2, false, true>(S, S + stride, stride, radM, 1, twM, M, ld);
     const double inv = 1.0 / (double)M;
     for (int i = threadIdx.x; i < M; i += blockDim.x) {
         const double2 v = F[fcg_slot<double2>(0, i, stride)];
@@ -802,7 +869,7 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_
         }
         return z;
     };
-    const V *Z = fcg_fft<V, false>(S, S + ppb * stride, stride, rad, ppb, twg1, G1, ld, true);
+    const V *Z = fcg_fft<V, false, true>(S, S + ppb * stride, stride, rad, ppb, twg1, G1, ld);
     // X_a[k] = (Z[k] + conj Z[-k]) / 2, X_b[k] = (Z[k] - conj Z[-k]) / (2i); pairs fastest
     FcgIdx it(threadIdx.x, blockDim.x, ppb);
     for (int idx = threadIdx.x; idx < m * ppb; idx += blockDim.x, it.next()) {
@@ -843,7 +910,7 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_cols(
         return z;
     };
     V *S2 = S + cpb * stride;
-    V *F = fcg_fft<V, false>(S, S2, stride, rad, cpb, twg0, G0, ldT, true);
+    V *F = fcg_fft<V, false, true>(S, S2, stride, rad, cpb, twg0, G0, ldT);
     const int npair = (cpb + 1) >> 1;
     auto ldP = [&](int q, int r) -> V {
         const V u = F[fcg_slot<V>(2 * q, r, stride)];
@@ -856,9 +923,8 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_cols(
         }
         return z;
     };
-    // the packed spectra load into the other buffer, then the passes run
-    // between it and F
-    const V *P = fcg_fft<V, true>(F == S ? S2 : S, F, stride, rad, npair, twg0, G0, ldP, true);
+    // the first pass takes the packed spectra from F into the other buffer
+    const V *P = fcg_fft<V, true, true>(F == S ? S2 : S, F, stride, rad, npair, twg0, G0, ldP);
     const T half = T(0.5) / (T)G0;
     FcgIdx it(threadIdx.x, blockDim.x, n0 + 1);
     for (int idx = threadIdx.x; idx < npair * (n0 + 1); idx += blockDim.x, it.next()) {
@@ -923,9 +989,8 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_
     };
     // Z[k] = (Y[k] + conj Y[Hp-k]) + i W^-k (Y[k] - conj Y[Hp-k]); rows fastest
     // (BLUE: times the chirp, zero-padded to M)
-    FcgIdx it(threadIdx.x, blockDim.x, rpb);
-    for (int idx = threadIdx.x; idx < rpb * NF; idx += blockDim.x, it.next()) {
-        const int k = it.a, rr = it.b, r = r0 + rr;
+    auto ldZ = [&](int rr, int k) -> V {
+        const int r = r0 + rr;
         V z = cx_zero<V>();
         if (r < rows && k < Hp) {
             V yk = spec(k, r), yc = cx_conj(spec(Hp - k, r));
@@ -943,21 +1008,20 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_
             z.y = e.y + wd.x;
             if constexpr (BLUE) z = cx_mul(z, cvt(__ldg(&chirp[k])));
         }
-        S[fcg_slot<V>(rr, k, stride)] = z;
-    }
-    __syncthreads();
+        return z;
+    };
     const V *Z;
     if constexpr (BLUE) {
-        V *F = fcg_fft<V, false>(S, S2, stride, rad, rpb, twm, NF, FcNoLoad<V>{}, false);
+        V *F = fcg_fft<V, false, true, true>(S, S2, stride, rad, rpb, twm, NF, ldZ);
         for (int idx = threadIdx.x; idx < rpb * NF; idx += blockDim.x) {
             const int rr = idx / NF, i = idx - rr * NF;
             V &v = F[fcg_slot<V>(rr, i, stride)];
             v = cx_mul(v, cvt(__ldg(&Bf[i])));
         }
         __syncthreads();
-        Z = fcg_fft<V, true>(F, F == S ? S2 : S, stride, rad, rpb, twm, NF, FcNoLoad<V>{}, false);
+        Z = fcg_fft<V, true, false>(F, F == S ? S2 : S, stride, rad, rpb, twm, NF, FcNoLoad<V>{});
     } else {
-        Z = fcg_fft<V, true>(S, S2, stride, rad, rpb, twl1, L1, FcNoLoad<V>{}, false);
+        Z = fcg_fft<V, true, true, true>(S, S2, stride, rad, rpb, twl1, L1, ldZ);
     }
     const T scale = T(1) / (T)L1;
     auto val = [&](int rr, int c) -> T {
@@ -1126,29 +1190,45 @@ static int fcg_fastlen(int x) {
         if (m == 1) return n;
     }
 }
-// Radices of n (11, 7, 5, 3, then 8s, then 4 or 2); false if n has another
-// prime factor or needs too many passes.
+// Radices of n; false if n has another prime factor.  Twos pair up with fives and
+// threes (radices 10 and 6) as far as that leaves fewer passes, and odd radices
+// come first: a first pass writes R apart.  A pass costs its barrier and its trip
+// through shared memory whatever its radix (2100 = 7 5 10 6 in four passes, not
+// 7 5 5 3 4 in five).
 static bool fcg_radices(int n, FcgRad &rad) {
     rad = FcgRad{};
     rad.n = n;
+    int e[12] = {};  // exponents of 2, 3, 5, 7, 11
     int m = n;
-    for (int f : {11, 7, 5, 3})
+    for (int f : {2, 3, 5, 7, 11})
         while (m % f == 0) {
-            if (rad.np == kFcgMaxPasses) return false;
-            rad.r[rad.np++] = f;
+            ++e[f];
             m /= f;
         }
-    while (m % 8 == 0 && m > 1) {
-        if (rad.np == kFcgMaxPasses) return false;
-        rad.r[rad.np++] = 8;
-        m /= 8;
-    }
-    if (m == 2 || m == 4) {
-        if (rad.np == kFcgMaxPasses) return false;
-        rad.r[rad.np++] = m;
-        m = 1;
-    }
-    return m == 1;
+    if (m != 1) return false;
+    // tens and sixes for the fewest passes, then the smallest sum of radices
+    int best = 1 << 30, t10 = 0, t6 = 0;
+    for (int t = 0; t <= std::min(e[2], e[5]); ++t)
+        for (int u = 0; u <= std::min(e[2] - t, e[3]); ++u) {
+            const int twos = e[2] - t - u, rest = twos % 3;
+            const int passes = e[5] + e[3] + (twos + 2) / 3;
+            const int sum = 5 * (e[5] + t) + 3 * (e[3] + u) + 8 * (twos / 3) + (rest ? 2 << (rest - 1) : 0);
+            if (passes * 1000 + sum < best) {
+                best = passes * 1000 + sum;
+                t10 = t;
+                t6 = u;
+            }
+        }
+    const int twos = e[2] - t10 - t6;
+    const int list[][2] = {{11, e[11]}, {7, e[7]},     {5, e[5] - t10},     {3, e[3] - t6},      {10, t10},
+                           {6, t6},     {8, twos / 3}, {4, twos % 3 == 2}, {2, twos % 3 == 1}};
+    for (const auto &l : list)
+        for (int i = 0; i < l[1]; ++i) {
+            if (rad.np == kFcgMaxPasses) return false;
+            rad.r[rad.np++] = l[0];
+        }
+    if (n == 1) rad.r[rad.np++] = 1;  // (one value: a pass that moves it)
+    return true;
 }
 // Threads of a general-path block holding `values` complex values in
 // `smem` bytes (every pass loops over its butterflies, so any count works):

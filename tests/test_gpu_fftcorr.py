@@ -231,3 +231,29 @@ def test_hand_fft_1d_odd_vs_cufft(n):
     assert torch.equal(torch.isnan(hn), torch.isnan(rn))
     ok = ~torch.isnan(rn)
     assert ((hn - rn).abs() * pairs)[ok].max().item() <= 2e-12 * ref.abs().max().item()
+
+
+# Four transforms of at most five passes, about six roundings a value and pass, all of one
+# sign: 120 x 2^-53 = 1.4e-14, and 120 x 2^-24 = 7e-6, of the result's norm.
+@pytest.mark.parametrize("shape", [
+    (2, 500, 30),    # G0 = 1000 = 10 10 10, two columns a block in FP64
+    (1, 512, 48),    # G0 = 1024: the longest that is paired
+    (2, 520, 33),    # 1050: one column a block, the power between the transforms kept in registers
+    (1, 605, 36),    # 1210 = 11 11 10
+    (1, 1029, 20),   # 2058 = 7 7 7 6
+    (1, 1080, 50),   # 2160 = 10 6 6 6: one column a block in FP32 too
+    (3, 4, 1050),    # L1 / 2 = 1050: two rows a block in FP64
+    (2, 3, 1100),    # three rows: blocks of two, one of them past the end
+    (1, 30, 3),      # G1 = 6
+])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_passes_against_whole_numbers(shape, dtype):
+    """Autocorrelations of whole numbers are whole numbers."""
+    g = torch.Generator().manual_seed(sum(shape))
+    x = torch.randint(0, 8, shape, generator=g)
+    n0, n1 = shape[-2:]
+    y = cusimple._hand_autocorr(x.to("cuda", dtype)).double().cpu()
+    z = np.fft.irfft2(np.abs(np.fft.rfft2(x.numpy().astype(np.float64), s=(2 * n0, 2 * n1))) ** 2, s=(2 * n0, 2 * n1))
+    z = torch.from_numpy(np.rint(np.fft.fftshift(z, axes=(-2, -1))))
+    assert y.shape == z.shape
+    assert float((y - z).norm() / z.norm()) < (1.4e-14 if dtype == torch.float64 else 7e-6)
