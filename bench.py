@@ -949,7 +949,7 @@ def qcorr_leg(torch, dev, args):
     msgc = timed(lambda: cusimple._crop(cusimple._autocorr(stack_g, 2, [2000, 2000]), 2, [1000, 1000]), reps=3)
     out["fft_corr_general"] = {"ms": msg, "images_per_s": 8 / (msg * 1e-3), "cufft_path_ms": msgc,
                                "workload": "cusimple.corr of 8 x 1000x1000 float64 (2000^2 transforms, radices "
-                                           "5, 8, 2), on the device; hand-written FFTs"}
+                                           "5, 10, 8), on the device; hand-written FFTs"}
     if not args.no_cpu_baseline:
         import oracle
 
