@@ -925,7 +925,7 @@ template <typename T>
 __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_cols(const typename Cx<T>::t *__restrict__ Tt, size_t t_img, int n0,
                                                 int ncols, int cpb, FcgRad rad, int stride,
                                                 const double2 *__restrict__ twg0, typename Cx<T>::t *__restrict__ C,
-                                                int cst, size_t c_img) {
+                                                size_t c_img) {
     using V = typename Cx<T>::t;
     extern __shared__ __align__(16) unsigned char fsm[];
     V *S = reinterpret_cast<V *>(fsm);
@@ -976,13 +976,13 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_cols(
             V c0;
             c0.x = (zp.x + zm.x) * half;
             c0.y = (zp.y + zm.y) * half;
-            C[(size_t)col * cst + r] = c0;
+            C[(size_t)col * (n0 + 1) + r] = c0;
         }
         if (2 * q + 1 < cpb && col + 1 < ncols) {
             V c1;
             c1.x = (zp.y - zm.y) * half;
             c1.y = -(zp.x - zm.x) * half;
-            C[(size_t)(col + 1) * cst + r] = c1;
+            C[(size_t)(col + 1) * (n0 + 1) + r] = c1;
         }
     }
 }
@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_cols(
 // BLUE: the inverse of Hp values by Bluestein's algorithm through FFTs of
 // length rad.n = M (chirp c, filter spectrum Bf); otherwise rad.n = Hp.
 template <typename T, bool ONED, bool BLUE>
-__global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_inv(const typename Cx<T>::t *__restrict__ C, int cst, size_t c_img, int n0,
+__global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_inv(const typename Cx<T>::t *__restrict__ C, size_t c_img, int n0,
                                                     int n1, int Hp, int rpb, FcgRad rad, int stride,
                                                     const double2 *__restrict__ twl1, const double2 *__restrict__ twm,
                                                     const double2 *__restrict__ chirp,
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(kFcgMaxThreads<T>, kFcgMinBlocks<T>) fcg_rows_
     V *S = reinterpret_cast<V *>(fsm);
     V *S2 = S + rpb * stride;
     const int L1 = 2 * Hp, r0 = blockIdx.x * rpb, W = 2 * n1, NF = rad.n;
-    const int rows = ONED ? n0 : n0 + 1;
+    const int rows = ONED ? n0 : n0 + 1, cst = ONED ? n0 : n0 + 1;
     C += (size_t)blockIdx.y * c_img;
     out += (size_t)blockIdx.y * (ONED ? n0 : 2 * n0) * W;
     auto spec = [&](int k, int r) -> V {
@@ -1291,7 +1291,6 @@ static int fcg_stride(int n, int lkc) { return n + ((n - 1) >> lkc) + 1; }
 struct FcgPlan {
     int n0, n1, G0, G1, L1, m, Hp;
     int ppb, cpb, rpb;  // row pairs (pass A), columns (B), rows (C) per block
-    int cst;            // stride of C's columns (of T's lines with oned)
     FcgRad radA, radB, radC;  // radC: Hp, or M with blue
     int thrA, thrB, thrC, strA, strB, strC;
     size_t vsz, t_img, c_img;
@@ -1334,13 +1333,10 @@ static bool fcg_plan(int64_t batch, int n0, int n1, int dtype, FcgPlan &p, bool 
     p.ppb = std::max(1, std::min(be / p.G1, (n0 + 1) / 2));
     p.cpb = std::max(1, std::min(be / p.G0, p.m));
     p.rpb = std::max(1, std::min(be / nC, oned ? n0 : n0 + 1));
-    // FP64: pass C reads two rows of every column, a whole 32-byte sector (and so up to 2304
+    // FP64: pass C reads two rows of every column, 32 bytes side by side (and so up to 2304
     // values a block, of which two fit an SM): 8 x 1000 x 1050 0.99 -> 0.93 ms; in FP32,
-    // three rows a block against four aligned ones, 0.52 and 0.53 ms
-    const int sec = p.vsz == 16 ? 2 : 1;
-    if (!oned && p.rpb == 1 && sec * nC <= be + be / 8) p.rpb = std::min(sec, n0 + 1);
-    else if (!oned && p.rpb > sec) p.rpb -= p.rpb % sec;
-    p.cst = oned ? n0 : (n0 + sec) / sec * sec;
+    // three rows a block against four, 0.52 and 0.53 ms
+    if (!oned && p.vsz == 16 && p.rpb == 1 && 2 * nC <= be + be / 8) p.rpb = std::min(2, n0 + 1);
     p.strA = fcg_stride(p.G1, lkc);
     p.strB = fcg_stride(p.G0, lkc);
     p.strC = fcg_stride(nC, lkc);
@@ -1349,7 +1345,7 @@ static bool fcg_plan(int64_t batch, int n0, int n1, int dtype, FcgPlan &p, bool 
     p.thrB = fcg_threads(p.cpb * p.G0, 2 * (size_t)p.cpb * p.strB * p.vsz, p.vsz);
     p.thrC = fcg_threads(p.rpb * nC, 2 * (size_t)p.rpb * p.strC * p.vsz, p.vsz);
     p.t_img = (size_t)p.m * n0;
-    p.c_img = oned ? 0 : (size_t)p.m * p.cst;
+    p.c_img = oned ? 0 : (size_t)p.m * (n0 + 1);
     p.twA_bytes = fc_align((size_t)p.G1 * sizeof(double2));
     p.twB_bytes = oned ? 0 : fc_align((size_t)p.G0 * sizeof(double2));
     p.twC_bytes = fc_align((size_t)p.L1 * sizeof(double2));
@@ -1419,13 +1415,13 @@ static idiwf_status fcg_run(const T *x, int64_t batch, const FcgPlan &p, const T
                                                                   twA, p.m, Tt, p.t_img);
         if (!p.oned)
             fcg_cols<T><<<dim3(blkB, g), p.thrB, smB, stream>>>(Tt, p.t_img, p.n0, p.m, p.cpb, p.radB, p.strB, twB,
-                                                                  C, p.cst, p.c_img);
+                                                                  C, p.c_img);
         IDIWF_CUDA_CHECK(cudaGetLastError());
         const V *Csrc = p.oned ? Tt : C;
         const size_t c_img = p.oned ? p.t_img : p.c_img;
         T *o = out + b0 * out_img;
         T thr = (T)threshold;
-        void *args[] = {(void *)&Csrc, (void *)&p.cst, (void *)&c_img, (void *)&p.n0, (void *)&p.n1, (void *)&p.Hp, (void *)&p.rpb,
+        void *args[] = {(void *)&Csrc, (void *)&c_img, (void *)&p.n0, (void *)&p.n1, (void *)&p.Hp, (void *)&p.rpb,
                         (void *)&p.radC, (void *)&p.strC, (void *)&twC, (void *)&twM, (void *)&chirp, (void *)&Bf,
                         (void *)&norm, (void *)&mode, (void *)&thr, (void *)&o};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(kC, dim3(blkC, g), dim3(p.thrC), args, smC, stream));
