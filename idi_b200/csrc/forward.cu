@@ -2311,7 +2311,8 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                 for (int i = 0; i < bp.n_images; ++i) nbig = std::max(nbig, bp.img[i].n);
                 node_extents_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, ext, hdr, g,
                                                                ng, nl.caps, plan);
-                cell_count_kernel<<<dim3((nbig + kCellSort - 1) / kCellSort, bp.n_images), 256, 0, stream>>>(
+                // (a launch of empty images has no emitters to sort)
+                cell_count_kernel<<<dim3(std::max(1, (nbig + kCellSort - 1) / kCellSort), bp.n_images), 256, 0, stream>>>(
                     bp, b->atoms, ng, plan, cs);
                 prep_split_kernel<false><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                     max_abs, split_recs(ws, nrec), hdr, g, ng, ext,

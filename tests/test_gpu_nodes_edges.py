@@ -1,0 +1,37 @@
+"""Band-limited evaluation at its edges: batches over several launches, images beside
+others, differentiation outputs of cut objects, large counts, tuning, large detectors."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from helpers import K64, atoms, rng, sphere  # noqa: E402
+from idi_b200 import _native as nat  # noqa: E402
+from idi_b200.simulation import _core  # noqa: E402
+
+
+def _image(g, n, r):
+    return atoms(sphere(g, n, r), g.uniform(0, 2 * np.pi, n))
+
+
+def _forward(at, off, geom, out, precision=nat.SPLIT, **kw):
+    t = torch.from_numpy(np.ascontiguousarray(at)).cuda()
+    E = _core.forward(t, off, geom, precision, out, **kw).cpu().numpy()
+    _core.workspace_error()
+    return E
+
+
+@pytest.mark.parametrize("n_images", [513, 520])
+def test_a_launch_of_empty_images(n_images):
+    """Of more than 512 images, one large enough for cells and a last launch without emitters."""
+    g = rng(20)
+    at = _image(g, 6000, 0.01)
+    geom = _core.make_geom([64, 64], 75.0, 1e5, K64)
+    off = np.full(n_images + 1, len(at), np.int64)
+    off[0] = 0
+    E = _forward(at, off, geom, nat.OUT_C64)
+    assert np.all(E[1:] == 0)
+    assert np.array_equal(E[0], _forward(at, [0, len(at)], geom, nat.OUT_C64)[0])
