@@ -627,7 +627,9 @@ def qcorr_radial(q: torch.Tensor, images: torch.Tensor, qmax: int) -> torch.Tens
     B, nr, nc = images.shape
     dev = images.device
     out = torch.empty((B, int(qmax)), dtype=torch.float64, device=dev)
-    ws = WORKSPACES.get(lib.idiwf_qcorr_workspace_size(nr, nc), dev, "qcorr")
+    # a workspace of the call's own, from its stream's pool: the kernels keep in it whether the
+    # rows of q mirror, and calls on other streams may run at the same time
+    ws = torch.empty(lib.idiwf_qcorr_workspace_size(nr, nc), dtype=torch.uint8, device=dev)
     nat.check(lib.idiwf_qcorr_radial(ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(images.data_ptr()), B, nr, nc,
                                      int(qmax), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(ws.data_ptr()),
                                      ws.numel(), _stream(dev)))

@@ -16,7 +16,8 @@
  *    optionally rotated by rot (idi/simulation/cpu.py:76-80).
  *  - Every device buffer is allocated by the caller.  Scratch space is a
  *    caller-provided workspace whose size the *_workspace_size functions report;
- *    no entry point allocates device or pinned memory.
+ *    no entry point allocates device or pinned memory.  A workspace serves one call
+ *    at a time: calls whose work may overlap on the GPU need workspaces of their own.
  *  - Work is enqueued on `stream` and is asynchronous: the compute entry points
  *    do not synchronise, so they can be captured in a CUDA graph.  The entry
  *    points that read results back (idiwf_tune, idiwf_forward_cta_times,
