@@ -141,7 +141,7 @@ __device__ __forceinline__ int64_t sort_block0(const BatchParams &bp, int img) {
 __global__ void __launch_bounds__(256)
     node_extents_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                         const void *__restrict__ amps, int amp_dtype, uint32_t *__restrict__ ext,
-                        WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, NodeCaps caps,
+                        WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng,
                         NodePlan *__restrict__ plan) {
     const int b = blockIdx.y;
     const ImageDesc d = bp.img[b];
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256)
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < d.n; j += (int64_t)gridDim.x * blockDim.x)
         ex.add(ng, reinterpret_cast<const double4 *>(atoms)[d.src + j], load_amp(amps, amp_dtype, d.src + j));
     ex.raise(ext, b);
-    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, caps, hdr, plan);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, hdr, plan);
 }
 
 // Emitters per cell of every sort block; an image's last block turns the counts into
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256)
     prep_split_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                       const void *__restrict__ amps, int amp_dtype, int w_mode, double max_abs, SplitRecs rec,
                       WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext,
-                      NodeCaps caps, NodePlan *__restrict__ plan, CellSort cs) {
+                      NodePlan *__restrict__ plan, CellSort cs) {
     const int b = blockIdx.y, tid = threadIdx.x;
     const ImageDesc d = bp.img[b];
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
@@ -304,13 +304,13 @@ __global__ void __launch_bounds__(256)
         return;
     }
     ex.raise(ext, b);
-    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, caps, hdr, plan);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, hdr, plan);
 }
 
 __global__ void __launch_bounds__(256)
     prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                        const void *__restrict__ amps, int amp_dtype, DoubleRecs rec, WsHeader *__restrict__ hdr,
-                       const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext, NodeCaps caps,
+                       const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext,
                        NodePlan *__restrict__ plan) {
     const int b = blockIdx.y;
     const ImageDesc d = bp.img[b];
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256)
     }
     if (!plan) return;
     ex.raise(ext, b);
-    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, true, caps, hdr, plan);
+    if (last_block(hdr)) plan_nodes(bp, g, ng, ext, true, hdr, plan);
 }
 
 // ---------------------------------------------------------------------------
@@ -2310,21 +2310,21 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                 int nbig = 0;
                 for (int i = 0; i < bp.n_images; ++i) nbig = std::max(nbig, bp.img[i].n);
                 node_extents_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, ext, hdr, g,
-                                                               ng, nl.caps, plan);
+                                                               ng, plan);
                 // (a launch of empty images has no emitters to sort)
                 cell_count_kernel<<<dim3(std::max(1, (nbig + kCellSort - 1) / kCellSort), bp.n_images), 256, 0, stream>>>(
                     bp, b->atoms, ng, plan, cs);
                 prep_split_kernel<false><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                     max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
-                                                                    nl.caps, plan, cs);
+                                                                    plan, cs);
             } else {
                 prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                    max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
-                                                                   nl.caps, plan, cs);
+                                                                   plan, cs);
             }
         } else {
             prep_double_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype,
-                                                          double_recs(ws, nrec), hdr, g, ng, ext, nl.caps, plan);
+                                                          double_recs(ws, nrec), hdr, g, ng, ext, plan);
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
@@ -2642,7 +2642,7 @@ extern "C" idiwf_status idiwf_forward_noalloc(const idiwf_geom *geom, const idiw
         const double max_abs = kMaxTurns / (3.0 * 2.0 * geom->k * kInvTwoPi);
         dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), bp.n_images);
         prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, batch->atoms, batch->amplitudes, batch->amp_dtype, w_mode,
-                                                           max_abs, rec, hdr, g, NodeGeom{}, nullptr, NodeCaps{},
+                                                           max_abs, rec, hdr, g, NodeGeom{}, nullptr,
                                                            nullptr, CellSort{});
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }

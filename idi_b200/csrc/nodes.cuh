@@ -60,6 +60,7 @@ constexpr int kCellMax = 512;        // cells per image
 constexpr int kCellNodes = 64;       // nodes per axis of a cell's grid
 constexpr int kCellMinEmitters = 4096;  // images below this are not cut
 constexpr int kCellSort = 1024;      // emitters per block of the sort
+constexpr int64_t kCellPixels = 1 << 18;  // most pixels that cells are interpolated to directly
 
 // Node geometry of a detector (host side, make_node_geom): Phi per unit of
 // emitter extent, curvature ratios, and the largest |d_hat . e| along each axis.
@@ -100,15 +101,24 @@ struct NodeCaps {
 __host__ __device__ inline int64_t node_entries(int64_t npix) { return npix / 4 + 4096; }
 __host__ __device__ inline int node_cap(int n) { return (n / 2 + 64 < kNodeMax ? n / 2 + 64 : kNodeMax) / 2 * 2; }
 
+// Limits of an image's cut, from its own emitter count (not from the others of its batch):
+// sums of its cells, and their values interpolated along y (16384 a cell on average: 128
+// columns of 128 nodes).
+constexpr int64_t kCellSums = 1 << 19, kCellValues = 3 * (1 << 20);
+__host__ __device__ inline int64_t cell_most(int64_t n) { return n / 64 < kCellMax ? n / 64 : kCellMax; }
+__host__ __device__ inline int64_t cell_values(int64_t n) {
+    return cell_most(n) * 16384 < kCellValues ? cell_most(n) * 16384 : kCellValues;
+}
+// Buffers that hold any cut of images of up to nmax emitters.
 __host__ __device__ inline NodeCaps node_caps(int64_t npix, int64_t nmax, bool cells) {
     NodeCaps c;
     c.v = node_entries(npix);
     c.f = c.y = 0;
     if (cells) {
-        const int64_t n = nmax / 64 < kCellMax ? nmax / 64 : kCellMax;
-        if (npix <= (1 << 18) && c.v < npix) c.v = npix;  // the pixels as the target
-        c.f = n * 2304 < (1 << 19) ? n * 2304 : (1 << 19);
-        c.y = n * 16384 < 3 * (1 << 20) ? n * 16384 : 3 * (1 << 20);
+        const int64_t f = cell_most(nmax) * kCellNodes * kCellNodes;
+        if (npix <= kCellPixels && c.v < npix) c.v = npix;  // the pixels as the target
+        c.f = f < kCellSums ? f : kCellSums;
+        c.y = cell_values(nmax);
     }
     return c;
 }
@@ -247,7 +257,7 @@ __device__ __forceinline__ double node_cost(double n, int nx, int ny, const Node
 // depends on the image and the geometry alone, as split_path's does.  fine: the FP64
 // kernel's images (their direct path counts as kPathPixel).
 __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, const NodeGeom &ng,
-                                  const uint32_t *ext, bool fine, NodeCaps caps, WsHeader *hdr, NodePlan *plan) {
+                                  const uint32_t *ext, bool fine, WsHeader *hdr, NodePlan *plan) {
     __shared__ long long s_work[kMaxImagesPerLaunch];
     __threadfence();
     const int npix = g.nx * g.ny, lane = threadIdx.x & 31;
@@ -313,7 +323,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
                 cut.c[2] = max(cut.c[2], 1);
                 const double nc = (double)cut.c[0] * cut.c[1] * cut.c[2];
                 double c = 1e30;
-                if (nc > 1.0 && nc <= kCellMax && nc * 64.0 <= n && (cut.pix ? (double)npix <= (double)caps.v : whole)) {
+                if (nc > 1.0 && nc <= (double)cell_most(n) && (cut.pix ? npix <= kCellPixels : whole)) {
                     cut.ncell = (int)nc;
                     double h[3];
 #pragma unroll
@@ -324,8 +334,8 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
                         h[k] = 0.5 * cut.size[k] * (1.0 + 1e-9);
                     }
                     node_grid(ng, r, sqrt(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]), h[0], h[1], fine, cut.g0, cut.g1);
-                    if (cut.g0 <= kCellNodes && cut.g1 <= kCellNodes && nc * cut.g0 * cut.g1 <= (double)caps.f &&
-                        nc * cut.n1 * cut.g0 <= (double)caps.y)
+                    if (cut.g0 <= kCellNodes && cut.g1 <= kCellNodes && nc * cut.g0 * cut.g1 <= (double)kCellSums &&
+                        nc * cut.n1 * cut.g0 <= (double)cell_values(n))
                         c = node_cost(n, g.nx, g.ny, cut, rate);
                 }
                 double least = c;

@@ -35,3 +35,27 @@ def test_a_launch_of_empty_images(n_images):
     E = _forward(at, off, geom, nat.OUT_C64)
     assert np.all(E[1:] == 0)
     assert np.array_equal(E[0], _forward(at, [0, len(at)], geom, nat.OUT_C64)[0])
+
+
+@pytest.mark.parametrize("ndet,spec", [
+    # (emitters, radius): in each, an image whose cut would be limited by buffers sized for
+    # it alone, beside a larger one
+    ([512, 512], [(5000, 0.015), (20000, 0.015)]),  # one grid alone, 72 cells beside
+    ([881, 941], [(8169, 0.0076), (20000, 0.01)]),  # to the image's nodes
+    ([170, 157], [(7418, 0.107), (100000, 0.1)]),   # direct alone, cells to the pixels beside
+])
+def test_cut_does_not_depend_on_the_batch(ndet, spec):
+    """An image of a batch takes the cut that it takes alone: the pairs formed add up, and the
+    float32 intensities are the same."""
+    g = rng(21)
+    imgs = [_image(g, n, r) for n, r in spec]
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, flags=nat.NF)
+    off = np.concatenate([[0], np.cumsum([n for n, _ in spec])])
+    E = _forward(np.concatenate(imgs), off, geom, nat.OUT_I32)
+    pairs = _core.evaluated_pairs()
+    for b, a in enumerate(imgs):
+        one = _forward(a, [0, len(a)], geom, nat.OUT_I32)[0]
+        pairs -= _core.evaluated_pairs()
+        # (another order of the cells' FP64 additions moves a float32 by at most an ulp)
+        np.testing.assert_allclose(one, E[b], rtol=1.2e-7, atol=0)
+    assert pairs == 0
