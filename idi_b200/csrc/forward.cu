@@ -1421,7 +1421,9 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_interp_kernel(const Geom
 // contiguous share of (image, target tile, cell), 32 x 32 targets each; the cells' tiles
 // are FP64 products (mma.m8n8k4, K in blocks of 16 by cp.async), turned by the
 // phase (FP64 turns, polynomial sine and cosine) and added in registers; a tile's total goes
-// to the fixed-point sums by atomics.
+// to the fixed-point sums by atomics.  How the shares cut a tile's cells depends on the batch, so
+// every cell's value is rounded to a grid (2^-50 of the largest possible sum) on which the
+// FP64 additions are exact in any order.
 constexpr int kExpTile = 32;
 struct ExpandSmem {
     double a[2][kExpTile * kGemmLd];
@@ -1481,6 +1483,8 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_expand_kernel(const Geom
         for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int b = 0; b < 4; ++b) tot[a][b][0] = tot[a][b][1] = 0.0;
+        // adding and taking it back rounds to multiples of 2^9 units (|sum| < 2^60 units)
+        const double grid = 0x1.8p61 / (double)ni.scale;
         const int steps = (c1 - c0) * nk;
         auto issue = [&](int st) {
             const int s = st & 1, cell = c0 + st / nk, k0 = st % nk * kGemmK;
@@ -1552,8 +1556,8 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_expand_kernel(const Geom
                     for (int e = 0; e < 2; ++e) {
                         const double c = flip_sign(e ? cs.y : cs.x, w[e]), s = flip_sign(e ? sn.y : sn.x, w[e]);
                         const double re = acc[a][b + e][0], im = acc[a][b + e][1];
-                        tot[a][b + e][0] += c * re - s * im;
-                        tot[a][b + e][1] += c * im + s * re;
+                        tot[a][b + e][0] += __dsub_rn(__dadd_rn(c * re - s * im, grid), grid);
+                        tot[a][b + e][1] += __dsub_rn(__dadd_rn(c * im + s * re, grid), grid);
                     }
                 }
         }

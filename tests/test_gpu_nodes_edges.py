@@ -59,3 +59,22 @@ def test_cut_does_not_depend_on_the_batch(ndet, spec):
         # (another order of the cells' FP64 additions moves a float32 by at most an ulp)
         np.testing.assert_allclose(one, E[b], rtol=1.2e-7, atol=0)
     assert pairs == 0
+
+
+@pytest.mark.parametrize("out", [nat.OUT_C128, nat.OUT_C64, nat.OUT_I64])
+@pytest.mark.parametrize("ndet,spec", [
+    ([512, 512], [(5000, 0.015), (20000, 0.015)]),
+    ([300, 301], [(4096, 0.02), (9000, 0.04), (12001, 0.01), (30000, 0.03)]),
+    ([64, 80], [(100000, 0.15), (5000, 0.01), (70001, 0.12)]),  # to the pixels and to nodes
+])
+def test_images_cut_into_cells_have_the_bits_they_have_alone(ndet, spec, out):
+    """The cells' sums are added on a grid on which FP64 additions are exact, so the bits do not
+    depend on how the batch's cells were shared out."""
+    g = rng(22)
+    imgs = [_image(g, n, r) for n, r in spec]
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, flags=nat.NF)
+    off = np.concatenate([[0], np.cumsum([n for n, _ in spec])])
+    E = _forward(np.concatenate(imgs), off, geom, out)
+    assert _core.evaluated_pairs() < off[-1] * ndet[0] * ndet[1] / 2
+    for b, a in enumerate(imgs):
+        assert np.array_equal(_forward(a, [0, len(a)], geom, out)[0], E[b]), b
