@@ -1420,8 +1420,9 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_interp_kernel(const Geom
 // theta = the phase of the cell's centre at the target point.  A CTA takes an equal,
 // contiguous share of (image, target tile, cell), 32 x 32 targets each; the cells' tiles
 // are FP64 products (mma.m8n8k4, K in blocks of 16 by cp.async), turned by the
-// phase (FP64 turns, polynomial sine and cosine) and added in registers; a tile's total goes
-// to the fixed-point sums by atomics.  How the shares cut a tile's cells depends on the batch, so
+// phase (FP64 turns, FP64 polynomials: every emitter of a cell shares the error of its turn, and
+// of a cell's emitters in phase that is far more than their sums' own) and added in registers; a
+// tile's total goes to the fixed-point sums by atomics.  How the shares cut a tile's cells depends on the batch, so
 // every cell's value is rounded to a grid (2^-50 of the largest possible sum) on which the
 // FP64 additions are exact in any order.
 constexpr int kExpTile = 32;
@@ -1540,25 +1541,18 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_expand_kernel(const Geom
 #pragma unroll
             for (int a = 0; a < 2; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; b += 2) {
-                    uint32_t w[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int at = (wr * 16 + a * 8 + (lane >> 2)) * (kExpTile + 1) + wc * 16 + (b + e) * 4 + (lane & 3);
-                        double t = __fma_rn(sm.nq[0][at], ctr[0], kTurnMagic + 0.25 + 0x1p-25);
-                        t = __fma_rn(sm.nq[1][at], ctr[1], t);
-                        t = __fma_rn(sm.nq[2][at], ctr[2], t);
-                        w[e] = (uint32_t)__double2loint(t);
-                    }
-                    float2 sn, cs;
-                    sincospi2(half_turns2(w[0], w[1]), sn, cs);
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const double c = flip_sign(e ? cs.y : cs.x, w[e]), s = flip_sign(e ? sn.y : sn.x, w[e]);
-                        const double re = acc[a][b + e][0], im = acc[a][b + e][1];
-                        tot[a][b + e][0] += __dsub_rn(__dadd_rn(c * re - s * im, grid), grid);
-                        tot[a][b + e][1] += __dsub_rn(__dadd_rn(c * im + s * re, grid), grid);
-                    }
+                for (int b = 0; b < 4; ++b) {
+                    const int at = (wr * 16 + a * 8 + (lane >> 2)) * (kExpTile + 1) + wc * 16 + b * 4 + (lane & 3);
+                    double t = __fma_rn(sm.nq[0][at], ctr[0], kTurnMagic + 0.25 + 0x1p-25);
+                    t = __fma_rn(sm.nq[1][at], ctr[1], t);
+                    t = __fma_rn(sm.nq[2][at], ctr[2], t);
+                    const uint32_t w = (uint32_t)__double2loint(t);
+                    double sn, cs;
+                    sincospi64(half_turn64(w), sn, cs);
+                    const double c = flip_sign64(cs, w), s = flip_sign64(sn, w);
+                    const double re = acc[a][b][0], im = acc[a][b][1];
+                    tot[a][b][0] += __dsub_rn(__dadd_rn(c * re - s * im, grid), grid);
+                    tot[a][b][1] += __dsub_rn(__dadd_rn(c * im + s * re, grid), grid);
                 }
         }
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(nb.v + lo * nb.caps.v);

@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
 
+import oracle  # noqa: E402
 from helpers import K64, atoms, rng, sphere  # noqa: E402
 from idi_b200 import _native as nat  # noqa: E402
 from idi_b200.simulation import _core  # noqa: E402
@@ -78,3 +79,56 @@ def test_images_cut_into_cells_have_the_bits_they_have_alone(ndet, spec, out):
     assert _core.evaluated_pairs() < off[-1] * ndet[0] * ndet[1] / 2
     for b, a in enumerate(imgs):
         assert np.array_equal(_forward(a, [0, len(a)], geom, out)[0], E[b]), b
+
+
+# Complex128 fields: turns in 2^-32, 4e-10 rms; polynomials 1.4e-9 at most, FP64 sums, for the
+# emitters and for their cells' turns; interpolation below 1e-8 (twice for cells).
+FINE_2NORM = 1.5e-8
+
+
+@pytest.mark.parametrize("ndet,n,r,flat", [
+    ([64, 80], 100000, 0.15, 1.0),    # cells straight to the pixels
+    ([200, 333], 9001, 0.03, 1.0),    # to the image's nodes
+    ([300, 500], 60000, 0.02, 0.01),  # one layer of cells
+])
+@pytest.mark.parametrize("settings", ["", "nf", "nf scale"])
+def test_complex128_fields_of_cut_objects(ndet, n, r, flat, settings):
+    g = rng(n)
+    at = atoms(sphere(g, n, r) * [1, 1, flat] + [0.01, -0.02, 0.005], g.uniform(0, 2 * np.pi, n))
+    amp = g.uniform(0.5, 1.5, n).astype(np.float32)
+    flags, _, _ = _core.parse_settings(settings)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64, (0.1, -0.2), flags=flags)
+    E = _forward(at, [0, n], geom, nat.OUT_C128, amplitudes=torch.from_numpy(amp).cuda())[0]
+    assert _core.evaluated_pairs() < n * ndet[0] * ndet[1] / 2
+    of = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(oracle.geometry(ndet, 75.0, 1e5, K64, (0.1, -0.2)), of, at, amp.astype(np.float64))
+    if "nf" in settings:  # moduli: the pixels' constant phases reach 2e8 rad, whose FP64 rounding is 2e-8
+        E, ref = np.abs(E), np.abs(ref)
+    err = np.linalg.norm(E - ref) / np.linalg.norm(ref)
+    assert err < FINE_2NORM + (6e-8 if settings == "nf scale" else 0), err  # (FP32 1/r factors)
+
+
+@pytest.mark.parametrize("out", [nat.OUT_C128, nat.OUT_C64])
+@pytest.mark.parametrize("n,lattice", [(2500, False), (20000, False), (50000, True)])
+def test_emitters_in_phase(n, lattice, out):
+    """A bright peak over dark pixels: an error shared by emitters in phase, or spread by the
+    interpolation from the peak, must not reach the dark pixels.  The direct kernels are the
+    measure, in the dark (below three times the field of random phases) and over all."""
+    g = rng(n)
+    if lattice:
+        m = np.stack(np.meshgrid(*[np.arange(40)] * 3, indexing="ij"), -1).reshape(-1, 3)
+        pos = np.concatenate([m + o for o in ([0, 0, 0], [.5, .5, 0], [.5, 0, .5], [0, .5, .5])]) * 0.00036
+        pos = pos[g.choice(len(pos), n, replace=False)] - pos.mean(0)
+    else:
+        pos = sphere(g, n, 0.01)
+    at = atoms(pos, np.zeros(n))
+    ndet = [120, 121]
+    geom = _core.make_geom(ndet, 170.0, 1e5, K64)
+    ref = oracle.wavefield(oracle.geometry(ndet, 170.0, 1e5, K64), 0, at)
+    E = _forward(at, [0, n], geom, out)[0]
+    assert 0 < _core.evaluated_pairs() < n * ndet[0] * ndet[1] / 2
+    D = _forward(at, [0, n], geom, out, config={"pixel_groups": -1})[0]
+    dark = np.abs(ref) < 3 * np.sqrt(n)
+    assert np.abs(ref).max() > 30 * np.sqrt(n) and dark.sum() > 1000
+    for part in (dark, np.ones_like(dark)):
+        assert np.linalg.norm((E - ref)[part]) <= np.linalg.norm((D - ref)[part])
