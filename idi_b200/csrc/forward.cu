@@ -895,6 +895,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
 struct NodeBuffers {
     double2 *v, *f, *y;  // [image of the group][entries]
     NodeCaps caps;
+    int two_words;       // FP64: f holds the second words of v
     double *lx, *ly;     // [image of the group][nx or ny][n0 or n1]
     double *sx, *sy;     // [image of the group][n0 or n1][g0 or g1]
     double2 *w;          // [image of the group][ny][n0]
@@ -1223,6 +1224,15 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
 // Four images of 2,000 emitters on 256^2 pixels (76^2 nodes): whole call 0.31 ms against
 // 2.87 ms, error against extended references 2.7e-15 against 1e-14 (sums without Kahan
 // steps, but a twelfth of the pairs and exact totals).
+//
+// One 64-bit word counts in 2^-58 to 2^-59 of n max|a|, too coarse for FP64 where n is
+// large (1.3e-13 of the field of 1e6 emitters, the direct kernel 6e-15).  A second word takes
+// what the first leaves.
+__device__ __forceinline__ void add_two_words(double x, long long &hi, long long &lo) {
+    const double h = rint(x);
+    hi += __double2ll_rn(h);
+    lo += __double2ll_rn((x - h) * (1.0 / kLowUnit));
+}
 template <bool ACC, bool SCALE, bool SECOND>
 __global__ void __launch_bounds__(kNodeThreads)
     node_sum64_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, DoubleRecs rec,
@@ -1297,9 +1307,9 @@ __global__ void __launch_bounds__(kNodeThreads)
             qz[i] = -kTwoPi * q.nqz;
             c2[i] = 0.5 * g.k * q.invD;
         }
-        long long sre[PPT], sim[PPT];
+        long long sre[PPT], sim[PPT], lre[PPT], lim[PPT];
 #pragma unroll
-        for (int i = 0; i < PPT; ++i) sre[i] = sim[i] = 0;
+        for (int i = 0; i < PPT; ++i) sre[i] = sim[i] = lre[i] = lim[i] = 0;
         for (int t = 0; t < nt; ++t) {
             const uint32_t slot = consumed & 1;
             if (!mbar_wait_bounded(&bar[slot], (consumed >> 1) & 1)) {
@@ -1338,8 +1348,8 @@ __global__ void __launch_bounds__(kNodeThreads)
             }
 #pragma unroll
             for (int i = 0; i < PPT; ++i) {
-                sre[i] += __double2ll_rn(re[i] * (double)ni.scale);
-                sim[i] += __double2ll_rn(im[i] * (double)ni.scale);
+                add_two_words(re[i] * (double)ni.scale, sre[i], lre[i]);
+                add_two_words(im[i] * (double)ni.scale, sim[i], lim[i]);
             }
             ++consumed;
             __syncthreads();
@@ -1354,12 +1364,15 @@ __global__ void __launch_bounds__(kNodeThreads)
             if (tid == 0 && t + 2 < nt) issue(t + 2);
         }
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(nb.v + (img - img0) * nb.caps.v);
+        unsigned long long *low = reinterpret_cast<unsigned long long *>(nb.f + (img - img0) * nb.caps.f);
 #pragma unroll
         for (int i = 0; i < PPT; ++i) {
             const int m = m0 + i * kNodeThreads;
             if (m < nodes) {
                 atomicAdd(dst + 2 * m, (unsigned long long)sre[i]);
                 atomicAdd(dst + 2 * m + 1, (unsigned long long)sim[i]);
+                atomicAdd(low + 2 * m, (unsigned long long)lre[i]);
+                atomicAdd(low + 2 * m + 1, (unsigned long long)lim[i]);
             }
         }
     }
@@ -1370,7 +1383,7 @@ __global__ void __launch_bounds__(kNodeThreads)
 __global__ void __launch_bounds__(256) node_zero_kernel(const NodePlan *__restrict__ plan, NodeBuffers nb, int img0) {
     const NodeImage &ni = plan->img[img0 + blockIdx.y];
     if (ni.path != kPathNodes) return;
-    const int64_t nv = (int64_t)ni.n0 * ni.n1, nf = ni.ncell > 1 ? (int64_t)ni.ncell * ni.g0 * ni.g1 : 0;
+    const int64_t nv = (int64_t)ni.n0 * ni.n1, nf = nb.two_words ? nv : (ni.ncell > 1 ? (int64_t)ni.ncell * ni.g0 * ni.g1 : 0);
     double2 *v = nb.v + blockIdx.y * nb.caps.v, *f = nb.f + blockIdx.y * nb.caps.f;
     for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv + nf; i += gridDim.x * blockDim.x)
         (i < nv ? v[i] : f[i - nv]) = make_double2(0.0, 0.0);
@@ -1409,8 +1422,8 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_interp_kernel(const Geom
     for (int t = blockIdx.x; t < tm * tn * ni.ncell; t += gridDim.x) {
         const int cell = t / (tm * tn), u = t - cell * (tm * tn);
         double2 *Y = nb.y + blockIdx.y * nb.caps.y + (int64_t)cell * ni.n1 * ni.g0;
-        interp_tile<true>(*reinterpret_cast<GemmSmem *>(smem), S,
-                          nb.f + blockIdx.y * nb.caps.f + (int64_t)cell * ni.g0 * ni.g1, ni.n1, ni.g0, ni.g1,
+        interp_tile<1>(*reinterpret_cast<GemmSmem *>(smem), S,
+                          nb.f + blockIdx.y * nb.caps.f + (int64_t)cell * ni.g0 * ni.g1, nullptr, ni.n1, ni.g0, ni.g1,
                           u % tm * kGemmM, u / tm * kGemmN, unit,
                           [&](int B, int a, double re, double im) { Y[(size_t)B * ni.g0 + a] = make_double2(re, im); });
     }
@@ -1570,6 +1583,7 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_expand_kernel(const Geom
     }
 }
 
+template <int WORDS>
 __global__ void __launch_bounds__(kGemmThreads, 4) node_interp_y_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
                                                                      NodeBuffers nb, int img0) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1581,7 +1595,7 @@ __global__ void __launch_bounds__(kGemmThreads, 4) node_interp_y_kernel(const Ge
     double2 *W = nb.w + blockIdx.y * nb.w_stride;
     const int tm = (g.ny + kGemmM - 1) / kGemmM, tn = (ni.n0 + kGemmN - 1) / kGemmN;
     for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
-        interp_tile<true>(*reinterpret_cast<GemmSmem *>(smem), L, V, g.ny, ni.n0, ni.n1, t % tm * kGemmM,
+        interp_tile<WORDS>(*reinterpret_cast<GemmSmem *>(smem), L, V, nb.f + blockIdx.y * nb.caps.f, g.ny, ni.n0, ni.n1, t % tm * kGemmM,
                           t / tm * kGemmN, unit,
                           [&](int j, int a, double re, double im) { W[(size_t)j * ni.n0 + a] = make_double2(re, im); });
 }
@@ -1606,7 +1620,7 @@ __global__ void __launch_bounds__(kGemmThreads, 4) node_interp_x_kernel(const Ge
     const double2 *W = nb.w + blockIdx.y * nb.w_stride;
     const int tm = (g.nx + kGemmM - 1) / kGemmM, tn = (g.ny + kGemmN - 1) / kGemmN;
     for (int t = blockIdx.x; t < tm * tn; t += gridDim.x)
-        interp_tile<false>(*reinterpret_cast<GemmSmem *>(smem), L, W, g.nx, g.ny, ni.n0, t % tm * kGemmM, t / tm * kGemmN,
+        interp_tile<0>(*reinterpret_cast<GemmSmem *>(smem), L, W, nullptr, g.nx, g.ny, ni.n0, t % tm * kGemmM, t / tm * kGemmN,
                            1.0, [&](int i, int j, double re, double im) {
                                finish_pixel_at<NF, SCALE>(g, i, j, re, im, out, out_kind, obase + i * g.ny + j);
                            });
@@ -2021,7 +2035,7 @@ static int64_t total_records(const idiwf_batch *b, int te, int nodes) {
 constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
 struct NodeLayout {
     size_t ext, counts, first, tot, v, f, y, lx, ly, sx, sy, w, total;  // offsets from the region's start (the plan)
-    int group;
+    int group, two_words;
     NodeCaps caps;
     NodeBuffers at(char *base, const idiwf_geom *g) const {
         NodeBuffers nb;
@@ -2029,6 +2043,7 @@ struct NodeLayout {
         nb.f = reinterpret_cast<double2 *>(base + f);
         nb.y = reinterpret_cast<double2 *>(base + y);
         nb.caps = caps;
+        nb.two_words = two_words;
         nb.lx = reinterpret_cast<double *>(base + lx);
         nb.ly = reinterpret_cast<double *>(base + ly);
         nb.sx = reinterpret_cast<double *>(base + sx);
@@ -2046,8 +2061,9 @@ struct NodeLayout {
                         reinterpret_cast<int *>(base + tot)};
     }
 };
-static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int nodes) {
+static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int precision, int nodes) {
     NodeLayout L;
+    L.two_words = precision != IDIWF_SPLIT;
     const bool cells = nodes > 1;
     const int imgs = std::min(b->n_images, kMaxImagesPerLaunch);
     int64_t nmax = 0, nlaunch = 0;  // largest image, largest number of emitters of a launch
@@ -2057,6 +2073,7 @@ static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int nod
             nlaunch = std::max(nlaunch, b->offsets[std::min(i + kMaxImagesPerLaunch, b->n_images)] - b->offsets[i]);
     }
     L.caps = node_caps((int64_t)g->nx * g->ny, nmax, cells);
+    if (L.two_words) L.caps.f = L.caps.v;
     const size_t v = (size_t)L.caps.v * 16, f = (size_t)L.caps.f * 16, y = (size_t)L.caps.y * 16,
                  lx = (size_t)g->nx * node_cap(g->nx) * 8, ly = (size_t)g->ny * node_cap(g->ny) * 8,
                  sx = cells ? (size_t)std::max(g->nx, node_cap(g->nx)) * kCellNodes * 8 : 0,
@@ -2094,7 +2111,7 @@ static size_t forward_ws_bytes(const idiwf_geom *g, const idiwf_batch *b, int pr
     const int nodes = nodes_possible(g, b, precision, IDIWF_OUT_C64, s);  // the output with the most images on nodes
     const int64_t nrec = std::max<int64_t>(total_records(b, s.te, nodes), 1);
     return node_region_offset(g, b, precision, nrec, choose_ksplit(g, b)) +
-           (nodes ? node_layout(g, b, nodes).total : 0);
+           (nodes ? node_layout(g, b, precision, nodes).total : 0);
 }
 
 // Dynamic shared memory of a forward kernel: two stages of emitter records,
@@ -2207,7 +2224,8 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
                 : (so ? (void *)node_sum64_kernel<false, false, true> : (void *)node_sum64_kernel<false, false, false>);
     void *fx = nf ? (void *)node_interp_x_kernel<true, false>
                   : (sc ? (void *)node_interp_x_kernel<false, true> : (void *)node_interp_x_kernel<false, false>);
-    idiwf_status st = ensure_smem((void *)node_interp_y_kernel, sizeof(GemmSmem));
+    void *fy = dbl ? (void *)node_interp_y_kernel<2> : (void *)node_interp_y_kernel<1>;
+    idiwf_status st = ensure_smem(fy, sizeof(GemmSmem));
     if (st == IDIWF_OK) st = ensure_smem(fx, sizeof(GemmSmem));
     if (st == IDIWF_OK) st = ensure_smem((void *)cell_interp_kernel, sizeof(GemmSmem));
     if (st == IDIWF_OK) st = ensure_smem((void *)cell_expand_kernel, sizeof(ExpandSmem));
@@ -2229,8 +2247,9 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
             cell_interp_kernel<<<dim3(4 * per, n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
             cell_expand_kernel<<<egrid, kGemmThreads, sizeof(ExpandSmem), stream>>>(g, ng, plan, nb, i0, i1);
         }
-        node_interp_y_kernel<<<dim3(std::min(ty, 64), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
         IDIWF_CUDA_CHECK(cudaGetLastError());
+        void *ay[] = {(void *)&g, &plan, (void *)&nb, &i0};
+        IDIWF_CUDA_CHECK(cudaLaunchKernel(fy, dim3(std::min(ty, 64), n), dim3(kGemmThreads), ay, sizeof(GemmSmem), stream));
         void *ax[] = {(void *)&g, &plan, (void *)&nb, &i0, &out, &out_kind};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fx, dim3(std::min(tx, 4096), n), dim3(kGemmThreads), ax, sizeof(GemmSmem), stream));
     }
@@ -2278,7 +2297,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                       (size_t)i0 * npix * (out_kind == IDIWF_OUT_C128 ? 16 : (out_kind == IDIWF_OUT_I32 ? 4 : 8));
 
     // prep
-    const NodeLayout nl = bp.nodes ? node_layout(geom, b, bp.nodes) : NodeLayout{};
+    const NodeLayout nl = bp.nodes ? node_layout(geom, b, precision, bp.nodes) : NodeLayout{};
     char *node_base = static_cast<char *>(ws) + (bp.nodes ? node_region_offset(geom, b, precision, nrec, ksplit) : 0);
     NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
     NodeGeom ng = make_node_geom(g);

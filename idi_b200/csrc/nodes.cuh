@@ -90,8 +90,12 @@ struct NodePlan {
     int64_t pad;
     NodeImage img[kMaxImagesPerLaunch];
 };
+// Second words of the FP64 kernel's node sums: units of the first word's unit.  A block of
+// emitters adds at most half a unit of the first, 2^37 of the second, and an image has at
+// most 2^24 blocks.
+constexpr double kLowUnit = 0x1p-38;
 // What the buffers of an image hold: sums on the target grid, sums of the cells, and the
-// cells' sums interpolated along one axis.
+// cells' sums interpolated along one axis (FP64: f holds the second words of v).
 struct NodeCaps {
     int64_t v, f, y;
 };
@@ -485,11 +489,13 @@ union GemmSmem {
     double2 y[kGemmM * (kGemmN + 1)];  // the finished tile, for stores along rows
 };
 
-// One tile at (i0, j0); `store(i, j, re, im)` receives every element inside M x N.  FIXED: X
-// holds fixed-point sums (two 64-bit integers, value / unit).
-template <bool FIXED, class Store>
+// One tile at (i0, j0); `store(i, j, re, im)` receives every element inside M x N.  WORDS: X
+// holds fixed-point sums (two 64-bit integers, value / unit) of one word or, the second in
+// `low` (kLowUnit of the first's units), of two.
+template <int WORDS, class Store>
 __device__ __forceinline__ void interp_tile(GemmSmem &sm, const double *__restrict__ L, const double2 *__restrict__ X,
-                                            int M, int N, int K, int i0, int j0, double unit, const Store &store) {
+                                            const double2 *__restrict__ low, int M, int N, int K, int i0, int j0,
+                                            double unit, const Store &store) {
     const int tid = threadIdx.x, lane = tid & 31, wr = (tid >> 5) >> 1, wc = (tid >> 5) & 1;
     double acc[4][4][2];
 #pragma unroll
@@ -509,10 +515,18 @@ __device__ __forceinline__ void interp_tile(GemmSmem &sm, const double *__restri
         for (int q = 0; q < kGemmN * kGemmK / kGemmThreads; ++q) {
             const int c = tid + q * kGemmThreads, r = c / kGemmK, k = c % kGemmK;
             const bool ok = j0 + r < N && k0 + k < K;
-            if (FIXED) {
+            if (WORDS) {
                 longlong2 v = make_longlong2(0, 0);
                 if (ok) v = reinterpret_cast<const longlong2 *>(X)[(size_t)(j0 + r) * K + k0 + k];
-                sm.b[s][r * kGemmLd + k] = make_double2((double)v.x * unit, (double)v.y * unit);
+                double2 x = make_double2((double)v.x, (double)v.y);
+                if (WORDS == 2) {
+                    // (the first word's part below FP64's 53 bits joins the second)
+                    longlong2 w = make_longlong2(0, 0);
+                    if (ok) w = reinterpret_cast<const longlong2 *>(low)[(size_t)(j0 + r) * K + k0 + k];
+                    x.x += (double)(v.x - (long long)x.x) + (double)w.x * kLowUnit;
+                    x.y += (double)(v.y - (long long)x.y) + (double)w.y * kLowUnit;
+                }
+                sm.b[s][r * kGemmLd + k] = make_double2(x.x * unit, x.y * unit);
             } else {
                 cp_async16(&sm.b[s][r * kGemmLd + k], X + (ok ? (size_t)(j0 + r) * K + k0 + k : 0), ok);
             }

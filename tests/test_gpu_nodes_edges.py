@@ -132,3 +132,40 @@ def test_emitters_in_phase(n, lattice, out):
     assert np.abs(ref).max() > 30 * np.sqrt(n) and dark.sum() > 1000
     for part in (dark, np.ones_like(dark)):
         assert np.linalg.norm((E - ref)[part]) <= np.linalg.norm((D - ref)[part])
+
+
+def _far_field_extended(at, ndet, pixelsize, detz, sel):
+    """The far field at the pixels `sel`, phases and sums in extended precision."""
+    ld = np.longdouble
+    x = ((sel // ndet[1] - ndet[0] / 2) * pixelsize).astype(ld)
+    y = ((sel % ndet[1] - ndet[1] / 2) * pixelsize).astype(ld)
+    D = np.sqrt(x * x + y * y + ld(detz) ** 2)
+    a, k = at.astype(ld), ld(K64)
+    turn = 2 * (ld(np.pi) + ld(1.2246467991473532e-16))
+    E = np.empty(len(sel), complex)
+    for i in range(len(sel)):
+        q = [x[i] / D[i], y[i] / D[i], -(x[i] ** 2 + y[i] ** 2) / (D[i] * (D[i] + ld(detz)))]
+        ph = a[:, 3] - k * (a[:, 0] * q[0] + a[:, 1] * q[1] + a[:, 2] * q[2])
+        ph = ph - turn * np.rint(ph / turn)
+        p = ph.astype(np.float64)
+        d = (ph - p).astype(np.float64)  # cos(p + d) = cos p - d sin p
+        c, s = np.cos(p), np.sin(p)
+        E[i] = complex(np.sum((c - s * d).astype(ld)), np.sum((s + c * d).astype(ld)))
+    return E
+
+
+@pytest.mark.parametrize("n", [2000, 100_000, 1_000_000])
+def test_fp64_totals_at_large_counts(n):
+    """FP64 on nodes is no further from extended precision than the direct FP64 kernel, whatever
+    the number of emitters."""
+    g = rng(n)
+    at, ndet = _image(g, n, 0.004), [64, 65]
+    sel = g.choice(ndet[0] * ndet[1], 24, replace=False)
+    ref = _far_field_extended(at, ndet, 75.0, 1e5, sel)
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64)
+    errs = []
+    for config in (None, {"pixel_groups": -1}):
+        E = _forward(at, [0, n], geom, nat.OUT_C128, nat.DOUBLE, config=config)[0].ravel()[sel]
+        assert (0 < _core.evaluated_pairs() < n * 4160 / 4) == (config is None)
+        errs.append(np.linalg.norm(E - ref) / np.linalg.norm(ref))
+    assert errs[0] <= errs[1], errs
