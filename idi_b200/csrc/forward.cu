@@ -1812,6 +1812,7 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
 struct LaunchShape {
     int threads, ppt, te, ctas_per_sm;
     int groups = 1;  // split: pixel runs with a base phase where bounded
+    bool direct_only = false;  // (the tuner:) without the images on nodes
 };
 
 static int sm_count() {
@@ -2387,7 +2388,8 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                                                                             out_chunk, out_kind, plan);
             IDIWF_CUDA_CHECK(cudaGetLastError());
         }
-        if (plan) return launch_nodes(geom, g, ng, bp, &rec, nullptr, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
+        if (plan && !s.direct_only)
+            return launch_nodes(geom, g, ng, bp, &rec, nullptr, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     } else {
         DoubleRecs rec = double_recs(ws, nrec);
         void *args[] = {&bp, (void *)&g, &rec, &out_chunk, &out_kind, &hdr, &cta_ns, &plan};
@@ -2397,7 +2399,8 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
         idiwf_status st = grid_for(fn, smem, grid);
         if (st != IDIWF_OK) return st;
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(s.threads), args, smem, stream));
-        if (plan) return launch_nodes(geom, g, ng, bp, nullptr, &rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
+        if (plan && !s.direct_only)
+            return launch_nodes(geom, g, ng, bp, nullptr, &rec, plan, nl, node_base, hdr, cta_ns, out_chunk, out_kind, stream);
     }
     return IDIWF_OK;
 }
@@ -2479,6 +2482,20 @@ extern "C" idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *ba
     if ((st = validate_batch(batch)) != IDIWF_OK) return st;
     if (precision != IDIWF_SPLIT && precision != IDIWF_DOUBLE)
         return set_error(IDIWF_ERR_INVALID_ARGUMENT, "precision must be IDIWF_SPLIT or IDIWF_DOUBLE");
+    // The shape is the direct kernels': images on nodes do not run them, and their own kernels'
+    // time would drown the differences.  So the direct images alone are timed, and a batch
+    // without any keeps the default shape and leaves the cache to others' tuning.
+    LaunchShape best_s = default_shape(precision);
+    bool tune = true;
+    if (nodes_possible(geom, batch, precision, out_kind, best_s)) {
+        best_s.direct_only = true;
+        if ((st = forward_impl(geom, batch, precision, out_kind, out, workspace, workspace_bytes, best_s, stream)) != IDIWF_OK)
+            return st;
+        WsHeader h;
+        IDIWF_CUDA_CHECK(cudaMemcpyAsync(&h, workspace, sizeof(h), cudaMemcpyDeviceToHost, stream));
+        IDIWF_CUDA_CHECK(cudaStreamSynchronize(stream));
+        tune = h.direct > 0;
+    }
     std::vector<LaunchShape> cands;
     if (precision == IDIWF_SPLIT) {
         // CTAs per SM: as many as fit.  The persistent queue balances any grid,
@@ -2505,8 +2522,9 @@ extern "C" idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *ba
     IDIWF_CUDA_CHECK(cudaEventCreate(&e0));
     IDIWF_CUDA_CHECK(cudaEventCreate(&e1));
     float best_ms = 1e30f;
-    LaunchShape best_s = default_shape(precision);
-    for (const LaunchShape &s : cands) {
+    for (LaunchShape &s : cands) {
+        if (!tune) break;
+        s.direct_only = true;
         if (forward_ws_bytes(geom, batch, precision, s) > workspace_bytes) continue;
         {  // more CTAs per SM than fit would only repeat a smaller candidate
             void *fn = kernel_for(precision, s.ppt, geom->flags, false);
@@ -2536,7 +2554,11 @@ extern "C" idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *ba
     cudaEventDestroy(e1);
     if (st != IDIWF_OK) return st;
     IDIWF_CUDA_CHECK(cudaGetLastError());
-    {
+    best_s.direct_only = false;
+    // the batch's result, every image's
+    if ((st = forward_impl(geom, batch, precision, out_kind, out, workspace, workspace_bytes, best_s, stream)) != IDIWF_OK)
+        return st;
+    if (tune) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_cache[TuneKey{precision, geom->flags, geom->nx, geom->ny, n_bucket(batch)}] = best_s;
     }

@@ -43,7 +43,8 @@ struct WsHeader {
     uint32_t work_counter3; // third work queue (split forward: exact near-field kernel; time path:
                             // warm-started sorts given up)
     uint32_t ticket;        // finished blocks of the split forward's prep kernel
-    uint32_t pad32[2];
+    uint32_t direct;        // images that the node plan left to the direct kernels
+    uint32_t pad32;
     unsigned long long pairs;  // emitter-pixel (or emitter-node) pairs the split forward evaluates
     uint64_t pad[27];
 };

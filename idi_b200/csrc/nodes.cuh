@@ -381,6 +381,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         }
         if (lane == 0) {
             atomicAdd(&hdr->pairs, pr);
+            if (n > 0 && ni.path != kPathNodes) atomicAdd(&hdr->direct, 1u);
             s_work[i] = work;
             plan->img[i] = ni;
         }

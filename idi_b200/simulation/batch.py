@@ -2,10 +2,10 @@
 
 A :class:`BatchPlan` fixes the batch structure (emitters per image), the
 detector geometry and the precision.  It owns static device buffers for the
-emitters, amplitudes and output, autotunes the forward kernel shape on the
-first batch, and captures the whole forward (workspace reset, record prep,
-persistent direct-sum kernel) in one CUDA graph, so each later batch is a
-host->device copy plus one graph replay.
+emitters, amplitudes and output, autotunes the direct kernels' shape on the
+first batch (where an image takes them), and captures the whole forward
+(workspace reset, node plan, record prep, direct-sum and node kernels) in one
+CUDA graph, so each later batch is a host->device copy plus one graph replay.
 """
 
 from __future__ import annotations

@@ -553,10 +553,12 @@ idiwf_status idiwf_welford_update(const float *x, float *mean, float *nvar, int6
 /* ------------------------------------------------------------------------ */
 
 /*
- * Autotune the forward kernel shape for this geometry/batch/precision: times
- * each candidate idiwf_config on a subsample of the work with CUDA events and
- * caches the fastest under a key of (precision, flags, nx, ny, emitter-count
- * bucket).  Later idiwf_forward calls with cfg == NULL use the cached shape.
+ * Autotune the direct forward kernels' shape for this geometry/batch/precision:
+ * times each candidate idiwf_config with CUDA events on the images that are not
+ * evaluated on nodes and caches the fastest under a key of (precision, flags, nx,
+ * ny, emitter-count bucket).  Later idiwf_forward calls with cfg == NULL use the
+ * cached shape.  A batch whose images are all on nodes keeps the default shape,
+ * and nothing is cached.  `out` receives the batch's result, as idiwf_forward's.
  * Synchronises `stream`.  Writes the chosen shape to *best when non-NULL.
  */
 idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *batch, int32_t precision,

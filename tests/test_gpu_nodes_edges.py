@@ -169,3 +169,34 @@ def test_fp64_totals_at_large_counts(n):
         assert (0 < _core.evaluated_pairs() < n * 4160 / 4) == (config is None)
         errs.append(np.linalg.norm(E - ref) / np.linalg.norm(ref))
     assert errs[0] <= errs[1], errs
+
+
+@pytest.mark.parametrize("precision,out", [(nat.SPLIT, nat.OUT_C64), (nat.DOUBLE, nat.OUT_C128)])
+def test_tuning_times_the_direct_images_alone(precision, out):
+    """A batch all on nodes keeps the default shape, and tuning on it does not change the shape
+    that direct images of the same detector and counts run with; a batch with a direct image
+    is tuned on that."""
+    g = rng(23)
+    n, ndet = 4000, [144, 148]
+    geom = _core.make_geom(ndet, 75.0, 1e5, K64)
+    wide = np.concatenate([_image(g, n, 0.8) for _ in range(8)])
+    off = np.arange(9) * n
+    _forward(wide, off, geom, out, precision)
+    assert _core.evaluated_pairs() == 8 * n * ndet[0] * ndet[1]  # direct
+    ctas = _core.cta_times().size
+    dense = torch.from_numpy(np.concatenate([_image(g, n, 0.01) for _ in range(8)])).cuda()
+    default = ({"threads": 256, "pixels_per_thread": 4, "emitters_per_tile": 512, "ctas_per_sm": 3, "pixel_groups": 1}
+               if precision == nat.SPLIT else
+               {"threads": 128, "pixels_per_thread": 2, "emitters_per_tile": 128, "ctas_per_sm": 2, "pixel_groups": 1})
+    for _ in range(3):
+        assert _core.tune(dense, off, geom, precision, out) == default
+    _forward(wide, off, geom, out, precision)
+    assert _core.cta_times().size == ctas
+    mixed = torch.cat([dense[:n], torch.from_numpy(wide[:7 * n]).cuda()])
+    other = _core.make_geom(ndet, 75.0, 1.01e5, K64, flags=nat.SECONDORDER)  # (a key of its own: the choice is kept)
+    best = _core.tune(mixed, off, other, precision, out)
+    assert best["threads"] in (128, 256) and best["pixels_per_thread"] in (1, 2, 4, 8)
+    assert _core.evaluated_pairs() > 0  # (the tuner's last run is a whole call)
+    E = _forward(mixed.cpu().numpy(), off, other, out, precision)
+    F = _forward(mixed.cpu().numpy(), off, other, out, precision, config=best)
+    assert np.array_equal(E, F)
