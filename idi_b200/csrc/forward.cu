@@ -2558,6 +2558,7 @@ extern "C" idiwf_status idiwf_tune(const idiwf_geom *geom, const idiwf_batch *ba
     // the batch's result, every image's
     if ((st = forward_impl(geom, batch, precision, out_kind, out, workspace, workspace_bytes, best_s, stream)) != IDIWF_OK)
         return st;
+    IDIWF_CUDA_CHECK(cudaStreamSynchronize(stream));
     if (tune) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_cache[TuneKey{precision, geom->flags, geom->nx, geom->ny, n_bucket(batch)}] = best_s;
