@@ -95,7 +95,6 @@ constexpr int kAdjEmitters = 4;
 constexpr int kAdjBlock = kNodeThreads * kAdjEmitters;
 constexpr int kAdjTile = 64;
 constexpr int kAdjChunk = 512;
-constexpr size_t kAdjGroupBytes = (size_t)512 << 20;
 
 struct AdjImage {
     int32_t path, n0, n1;
@@ -169,13 +168,14 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     int64_t nmax = 0;
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
     L.nodes = (double)nmax * (double)npix >= kNodeMinPairsDiff && make_node_geom(make_geom(g)).ok;
+    L.entries = node_entries(g->nx, g->ny);
+    L.lx_bytes = (size_t)g->nx * node_cap(g->nx) * 8;
+    L.ly_bytes = (size_t)g->ny * node_cap(g->ny) * 8;
+    L.t_bytes = (size_t)g->ny * node_cap(g->nx) * 16;
+    const size_t per = L.lx_bytes + L.ly_bytes + L.t_bytes + (size_t)L.entries * 80;
+    L.nodes = L.nodes && node_buffers_fit(g->nx, g->ny, per);
     if (L.nodes) {
-        L.entries = node_entries(npix);
-        L.lx_bytes = (size_t)g->nx * node_cap(g->nx) * 8;
-        L.ly_bytes = (size_t)g->ny * node_cap(g->ny) * 8;
-        L.t_bytes = (size_t)g->ny * node_cap(g->nx) * 16;
-        const size_t per = L.lx_bytes + L.ly_bytes + L.t_bytes + (size_t)L.entries * 80;
-        L.group = (int)std::max<size_t>(1, std::min<size_t>(b->n_images, kAdjGroupBytes / per));
+        L.group = (int)std::max<size_t>(1, std::min<size_t>(b->n_images, kNodeGroupBytes / per));
         L.off_plan = o; o += align256(sizeof(AdjPlan));
         L.off_lx = o;   o += align256(L.group * L.lx_bytes);
         L.off_ly = o;   o += align256(L.group * L.ly_bytes);
@@ -344,7 +344,7 @@ __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, co
             t.g0 = ai.n0 = t.n0;
             t.g1 = ai.n1 = t.n1;
             use = t.n0 <= node_cap(g.nx) && t.n1 <= node_cap(g.ny) &&
-                  (double)t.n0 * t.n1 <= (double)node_entries((int64_t)g.nx * g.ny) &&
+                  (double)t.n0 * t.n1 <= (double)node_entries(g.nx, g.ny) &&
                   node_cost(n, g.nx, g.ny, t, 6.5e11) < pairs / 1.05e12;
         }
         if (use) {

@@ -2007,6 +2007,26 @@ static size_t partials_bytes(const idiwf_geom *g, const idiwf_batch *b, int kspl
 static double node_min_pairs(int precision, int out_kind) {
     return precision != IDIWF_SPLIT ? kNodeMinPairs64 : (out_kind == IDIWF_OUT_C128 ? kNodeMinPairsDiff : kNodeMinPairs);
 }
+// Bytes of the node buffers of one image of up to nmax emitters.
+struct NodeBytes {
+    NodeCaps caps;
+    size_t v, f, y, lx, ly, sx, sy, w;
+    size_t all() const { return v + f + y + lx + ly + sx + sy + w; }
+};
+static NodeBytes node_bytes(const idiwf_geom *g, int64_t nmax, int precision, bool cells) {
+    NodeBytes b;
+    b.caps = node_caps(g->nx, g->ny, nmax, cells);
+    if (precision != IDIWF_SPLIT) b.caps.f = b.caps.v;  // the sums' second words
+    b.v = (size_t)b.caps.v * 16;
+    b.f = (size_t)b.caps.f * 16;
+    b.y = (size_t)b.caps.y * 16;
+    b.lx = (size_t)g->nx * node_cap(g->nx) * 8;
+    b.ly = (size_t)g->ny * node_cap(g->ny) * 8;
+    b.sx = cells ? (size_t)std::max(g->nx, node_cap(g->nx)) * kCellNodes * 8 : 0;
+    b.sy = cells ? (size_t)std::max(g->ny, node_cap(g->ny)) * kCellNodes * 8 : 0;
+    b.w = (size_t)g->ny * node_cap(g->nx) * 16;
+    return b;
+}
 static int nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precision, int out_kind, const LaunchShape &s) {
     const bool split = precision == IDIWF_SPLIT;
     if (!s.groups || (!split && (g->flags & IDIWF_NF) && !(g->flags & IDIWF_ACCURATE))) return 0;
@@ -2014,7 +2034,7 @@ static int nodes_possible(const idiwf_geom *g, const idiwf_batch *b, int precisi
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
     if ((double)nmax * g->nx * g->ny < node_min_pairs(precision, out_kind)) return 0;
     const NodeGeom ng = make_node_geom(make_geom(g));
-    if (!ng.ok) return 0;
+    if (!ng.ok || !node_buffers_fit(g->nx, g->ny, node_bytes(g, INT32_MAX, precision, split && ng.ortho).all())) return 0;
     return split && nmax >= kCellMinEmitters && ng.ortho ? 2 : 1;
 }
 
@@ -2033,7 +2053,6 @@ static int64_t total_records(const idiwf_batch *b, int te, int nodes) {
 
 // Node part of the workspace: the plan, the emitters' sort, and buffers for groups of
 // images that together stay within kNodeGroupBytes.
-constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
 struct NodeLayout {
     size_t ext, counts, first, tot, v, f, y, lx, ly, sx, sy, w, total;  // offsets from the region's start (the plan)
     int group, two_words;
@@ -2073,14 +2092,9 @@ static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int pre
         if (i % kMaxImagesPerLaunch == 0)
             nlaunch = std::max(nlaunch, b->offsets[std::min(i + kMaxImagesPerLaunch, b->n_images)] - b->offsets[i]);
     }
-    L.caps = node_caps((int64_t)g->nx * g->ny, nmax, cells);
-    if (L.two_words) L.caps.f = L.caps.v;
-    const size_t v = (size_t)L.caps.v * 16, f = (size_t)L.caps.f * 16, y = (size_t)L.caps.y * 16,
-                 lx = (size_t)g->nx * node_cap(g->nx) * 8, ly = (size_t)g->ny * node_cap(g->ny) * 8,
-                 sx = cells ? (size_t)std::max(g->nx, node_cap(g->nx)) * kCellNodes * 8 : 0,
-                 sy = cells ? (size_t)std::max(g->ny, node_cap(g->ny)) * kCellNodes * 8 : 0,
-                 w = (size_t)g->ny * node_cap(g->nx) * 16;
-    L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / (v + f + y + lx + ly + sx + sy + w)));
+    const NodeBytes nb = node_bytes(g, nmax, precision, cells);
+    L.caps = nb.caps;
+    L.group = (int)std::max<size_t>(1, std::min<size_t>(imgs, kNodeGroupBytes / nb.all()));
     size_t o = align256(sizeof(NodePlan));
     const auto take = [&](size_t bytes) {
         const size_t at = o;
@@ -2091,14 +2105,14 @@ static NodeLayout node_layout(const idiwf_geom *g, const idiwf_batch *b, int pre
     L.counts = take(cells ? (size_t)(nlaunch / kCellSort + imgs + 1) * kCellMax * 4 : 0);
     L.first = take(cells ? (size_t)imgs * (kCellMax + 1) * 4 : 0);
     L.tot = take(cells ? (size_t)imgs * kCellMax * 4 : 0);
-    L.v = take(L.group * v);
-    L.f = take(L.group * f);
-    L.y = take(L.group * y);
-    L.lx = take(L.group * lx);
-    L.ly = take(L.group * ly);
-    L.sx = take(L.group * sx);
-    L.sy = take(L.group * sy);
-    L.w = take(L.group * w);
+    L.v = take(L.group * nb.v);
+    L.f = take(L.group * nb.f);
+    L.y = take(L.group * nb.y);
+    L.lx = take(L.group * nb.lx);
+    L.ly = take(L.group * nb.ly);
+    L.sx = take(L.group * nb.sx);
+    L.sy = take(L.group * nb.sy);
+    L.w = take(L.group * nb.w);
     L.total = o;
     return L;
 }

@@ -100,10 +100,21 @@ struct NodeCaps {
     int64_t v, f, y;
 };
 
-// Node sums of an image (16 bytes each), and the node limits along each axis that
-// the weight and intermediate arrays hold.
-__host__ __device__ inline int64_t node_entries(int64_t npix) { return npix / 4 + 4096; }
+// Node limits along each axis that the weight and intermediate arrays hold, and node sums of
+// an image (16 bytes each).
 __host__ __device__ inline int node_cap(int n) { return (n / 2 + 64 < kNodeMax ? n / 2 + 64 : kNodeMax) / 2 * 2; }
+__host__ __device__ inline int64_t node_entries(int nx, int ny) {
+    const int64_t part = (int64_t)nx * ny / 4 + 4096, most = (int64_t)node_cap(nx) * node_cap(ny);
+    return part < most ? part : most;
+}
+// Node buffers of a group of images, and of one image: no more than 512 MB, or than the
+// detector's smallest output (4 bytes a pixel); a detector whose images need more (a strip of
+// very many columns, say) keeps the direct kernels.
+constexpr size_t kNodeGroupBytes = (size_t)512 << 20;
+inline bool node_buffers_fit(int nx, int ny, size_t image_bytes) {
+    const size_t out = (size_t)nx * ny * 4;
+    return image_bytes <= (out > kNodeGroupBytes ? out : kNodeGroupBytes);
+}
 
 // Limits of an image's cut, from its own emitter count (not from the others of its batch):
 // sums of its cells, and their values interpolated along y (16384 a cell on average: 128
@@ -114,9 +125,10 @@ __host__ __device__ inline int64_t cell_values(int64_t n) {
     return cell_most(n) * 16384 < kCellValues ? cell_most(n) * 16384 : kCellValues;
 }
 // Buffers that hold any cut of images of up to nmax emitters.
-__host__ __device__ inline NodeCaps node_caps(int64_t npix, int64_t nmax, bool cells) {
+inline NodeCaps node_caps(int nx, int ny, int64_t nmax, bool cells) {
+    const int64_t npix = (int64_t)nx * ny;
     NodeCaps c;
-    c.v = node_entries(npix);
+    c.v = node_entries(nx, ny);
     c.f = c.y = 0;
     if (cells) {
         const int64_t f = cell_most(nmax) * kCellNodes * kCellNodes;
@@ -300,7 +312,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
             best.g0 = best.n0;
             best.g1 = best.n1;
             const bool whole = best.n0 <= node_cap(g.nx) && best.n1 <= node_cap(g.ny) &&
-                               (double)best.n0 * best.n1 <= (double)node_entries(npix);
+                               (double)best.n0 * best.n1 <= (double)node_entries(g.nx, g.ny);
             const double rate = fine ? 1.3e11 : 1.0e12;
             double cost = pairs / (fine ? 1.6e11 : (direct == kPathRuns ? 1.8e12 : 1.5e12));
             bool use = false;

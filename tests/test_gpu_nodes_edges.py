@@ -200,3 +200,18 @@ def test_tuning_times_the_direct_images_alone(precision, out):
     E = _forward(mixed.cpu().numpy(), off, other, out, precision)
     F = _forward(mixed.cpu().numpy(), off, other, out, precision, config=best)
     assert np.array_equal(E, F)
+
+
+def test_detectors_of_more_pixels_than_nodes_can_be():
+    """Buffers bounded by the nodes of an axis (1024) rather than by the pixels: fields and
+    gradients against the direct kernels'."""
+    g = rng(24)
+    n, ndet = 4500, [3000, 2900]
+    at = torch.from_numpy(_image(g, n, 0.004)).cuda()
+    geom = _core.make_geom(ndet, 75.0, 4e5, K64, flags=nat.NF)
+    E, D = (_core.forward(at, [0, n], geom, nat.SPLIT, nat.OUT_C128, config=c) for c in (None, {"pixel_groups": -1}))
+    assert float((E - D).norm() / D.norm()) < 1e-6  # the direct kernels' 2.7e-7 and this path's
+    gI = (E.real ** 2 + E.imag ** 2).contiguous()
+    ga, da = (_core.backward(at, [0, n], geom, E, gI, config=c)[0] for c in (None, {"pixel_groups": -1}))
+    _core.backward_workspace_error()
+    assert not torch.equal(ga, da) and float((ga - da).norm() / da.norm()) < 1e-5
