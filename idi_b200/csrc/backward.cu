@@ -78,6 +78,7 @@ static_assert(kBwdTP % kRun == 0 && kBwdChunk % kRun == 0, "tiles hold whole run
 struct BwdLayout {
     int npix_pad;          // pixels rounded up to the chunk size
     int n_chunks, chunk_px;
+    int part_chunks;       // chunks that the partial sums hold: n_chunks, or the nodes' where some image may take them
     int64_t nrec;          // emitter records (images padded to the emitter block)
     size_t off_p64, off_pf, off_pg, off_pd, off_rb64, off_rbf, off_px, off_rmax, off_erec64, off_erecf, off_part;
     // node part (nodes: some image may take it): the plan, and per group of images the
@@ -164,7 +165,6 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     L.off_rmax = o; o += align256((size_t)kMaxImagesPerLaunch * 4 * kNodeExt);
     L.off_erec64 = o; o += align256((size_t)L.nrec * 32);
     L.off_erecf = o;  o += align256((size_t)L.nrec * 16);
-    L.off_part = o;   o += align256((size_t)L.n_chunks * L.nrec * kBwdNAcc * 4);
     int64_t nmax = 0;
     for (int i = 0; i < b->n_images; ++i) nmax = std::max(nmax, b->offsets[i + 1] - b->offsets[i]);
     L.nodes = (double)nmax * (double)npix >= kNodeMinPairsDiff && make_node_geom(make_geom(g)).ok;
@@ -174,6 +174,9 @@ static BwdLayout bwd_layout(const idiwf_geom *g, const idiwf_batch *b) {
     L.t_bytes = (size_t)g->ny * node_cap(g->nx) * 16;
     const size_t per = L.lx_bytes + L.ly_bytes + L.t_bytes + (size_t)L.entries * 80;
     L.nodes = L.nodes && node_buffers_fit(g->nx, g->ny, per);
+    // (npix / 2048 + 8: an image's nodes in chunks of kAdjChunk, however few its detector's own)
+    L.part_chunks = L.nodes ? std::max(L.n_chunks, (int)((L.entries + kAdjChunk - 1) / kAdjChunk)) : L.n_chunks;
+    L.off_part = o;   o += align256((size_t)L.part_chunks * L.nrec * kBwdNAcc * 4);
     if (L.nodes) {
         L.group = (int)std::max<size_t>(1, std::min<size_t>(b->n_images, kNodeGroupBytes / per));
         L.off_plan = o; o += align256(sizeof(AdjPlan));
@@ -316,9 +319,9 @@ __global__ void bwd_pixel_g_kernel(const GeomParams g, const double2 *__restrict
 
 // Plan of one call, by one block: every image's path, and for those on nodes their grid and
 // chunks.  The chunks make about 2400 units of a single image, as far as the partial-sum
-// buffer (max_chunks) reaches.
+// buffer (part_chunks) reaches.
 __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, const NodeGeom &ng, const uint32_t *ext,
-                                    int nodes, int max_chunks, AdjPlan *plan) {
+                                    int nodes, int part_chunks, AdjPlan *plan) {
     __shared__ int s_units[kMaxImagesPerLaunch];
     __threadfence();
     int direct = 0;
@@ -352,7 +355,7 @@ __device__ inline void plan_adjoint(const BwdParams &bp, const GeomParams &g, co
             const int m = ai.n0 * ai.n1;
             ai.nblocks = (n + kAdjBlock - 1) / kAdjBlock;
             const int want = max(1, min((m + kAdjTile - 1) / kAdjTile, (2400 + ai.nblocks - 1) / ai.nblocks));
-            const int cpx = max(min((m + want - 1) / want, kAdjChunk), (m + max_chunks - 1) / max_chunks);
+            const int cpx = max(min((m + want - 1) / want, kAdjChunk), (m + part_chunks - 1) / part_chunks);
             ai.cpx = (cpx + kAdjTile - 1) / kAdjTile * kAdjTile;
             ai.nchunks = (m + ai.cpx - 1) / ai.cpx;
         }
@@ -378,7 +381,7 @@ __global__ void __launch_bounds__(256)
     bwd_emitter_prep_kernel(const __grid_constant__ BwdParams bp, const double *__restrict__ atoms,
                             double4 *__restrict__ e64, float4 *__restrict__ ef, int w_mode,
                             uint32_t *__restrict__ rmax2, const GeomParams g, const NodeGeom ng, int nodes,
-                            int max_chunks, AdjPlan *__restrict__ plan, WsHeader *__restrict__ hdr) {
+                            int part_chunks, AdjPlan *__restrict__ plan, WsHeader *__restrict__ hdr) {
     const int b = blockIdx.y;
     NodeExtents ex;
     const BwdImage d = bp.img[b];
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(256)
         return;
     }
     ex.raise(rmax2, b);
-    if (last_block(hdr)) plan_adjoint(bp, g, ng, rmax2, nodes, max_chunks, plan);
+    if (last_block(hdr)) plan_adjoint(bp, g, ng, rmax2, nodes, part_chunks, plan);
 }
 
 __device__ __forceinline__ float2 g2(float a, float b) { return make_float2(a, b); }
@@ -1236,7 +1239,7 @@ extern "C" idiwf_status idiwf_backward(const idiwf_geom *geom, const idiwf_batch
         dim3 grid((unsigned)std::max(1, (max_blocks * eb + 255) / 256), batch->n_images);
         IDIWF_CUDA_CHECK(cudaMemsetAsync(rmax2, 0, sizeof(uint32_t) * kNodeExt * kMaxImagesPerLaunch, stream));
         bwd_emitter_prep_kernel<<<grid, 256, 0, stream>>>(bp, batch->atoms, e64, ef, w_mode, rmax2, g,
-                                                          make_node_geom(g), nodes, L.n_chunks, plan, hdr);
+                                                          make_node_geom(g), nodes, L.part_chunks, plan, hdr);
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
     bwd_pixel_geom_kernel<<<(L.npix_pad + pthreads - 1) / pthreads, pthreads, 0, stream>>>(

@@ -215,3 +215,55 @@ def test_detectors_of_more_pixels_than_nodes_can_be():
     ga, da = (_core.backward(at, [0, n], geom, E, gI, config=c)[0] for c in (None, {"pixel_groups": -1}))
     _core.backward_workspace_error()
     assert not torch.equal(ga, da) and float((ga - da).norm() / da.norm()) < 1e-5
+
+
+def _far_field_gradients(at, ndet, pixelsize, detz, g_intensity):
+    """E, and the gradients (atoms, amplitudes) of sum g_intensity |E|^2, by torch in FP64."""
+    dev = at.device
+    x = (torch.arange(ndet[0], device=dev, dtype=torch.float64) - ndet[0] / 2) * pixelsize
+    y = (torch.arange(ndet[1], device=dev, dtype=torch.float64) - ndet[1] / 2) * pixelsize
+    X, Y = (a.reshape(-1) for a in torch.meshgrid(x, y, indexing="ij"))
+    D = torch.sqrt(X * X + Y * Y + detz * detz)
+    q = K64 * torch.stack([X / D, Y / D, -(X * X + Y * Y) / (D * (D + detz))], 1)
+    E = torch.empty(len(q), dtype=torch.complex128, device=dev)
+    ga, gamp = torch.zeros_like(at), torch.zeros(len(at), dtype=torch.float64, device=dev)
+    for grad in (False, True):
+        for s in range(0, len(q), 256):
+            ph = at[:, 3][None] - q[s:s + 256] @ at[:, :3].T
+            e = torch.complex(torch.cos(ph), torch.sin(ph))
+            if not grad:
+                E[s:s + 256] = e.sum(1)
+                continue
+            z = (2 * g_intensity.reshape(-1)[s:s + 256] * E[s:s + 256].conj())[:, None] * e
+            gamp += z.real.sum(0)
+            ga[:, 3] -= z.imag.sum(0)
+            ga[:, :3] += z.imag.T @ q[s:s + 256]
+    return E.reshape(1, *ndet), ga, gamp
+
+
+# As tests/test_gpu_nodes.py: pairs 1.2e-7, FP32 sums over at most 512 nodes 3.8e-7, G about
+# three times the field's relative error; 7e-7 in quadrature, times 4 for what cancels.
+ADJOINT_2NORM = 3e-6
+
+
+@pytest.mark.parametrize("ndet,n,r,phases", [
+    ([100, 100], 60000, 0.03, 6.28),   # five chunks of 2048 pixels, 3,700 nodes
+    ([64, 64], 150000, 0.019, 6.28),    # two chunks, 2,100 nodes
+    ([64, 64], 150000, 0.019, 0.0),     # in phase
+    ([45, 91], 150000, 0.02, 6.28),
+])
+def test_adjoint_more_node_chunks_than_pixel_chunks(ndet, n, r, phases):
+    """Small detectors and many emitters: a chunk has at most 512 nodes, however few chunks the
+    pixels make."""
+    g = rng(ndet[0])
+    at = torch.from_numpy(atoms(sphere(g, n, r), g.uniform(0, 1, n) * phases)).cuda()
+    geom = _core.make_geom(ndet, 75.0 * 100 / max(ndet), 1e5, K64)
+    g_int = torch.from_numpy(g.normal(0, 1, [1] + ndet)).cuda()
+    E, ga, gamp = _far_field_gradients(at, ndet, 75.0 * 100 / max(ndet), 1e5, g_int)
+    out, out_amp = _core.backward(at, [0, n], geom, E, g_int)
+    direct, _ = _core.backward(at, [0, n], geom, E, g_int, config={"pixel_groups": -1})
+    _core.backward_workspace_error()
+    assert not torch.equal(out, direct)  # the node path was taken
+    for a, b in ((out[:, :3], ga[:, :3]), (out[:, 3], ga[:, 3]), (out_amp, gamp)):
+        err = float((a - b).norm() / b.norm())
+        assert err < ADJOINT_2NORM, err

@@ -52,3 +52,11 @@ def test_node_sums_are_bounded_by_the_nodes():
     a, b = _sizes(4096, 4096, [20000]), _sizes(8192, 8192, [20000])
     rows = 4 * 4096 * 1024 * 8 + 2 * 4096 * 64 * 8  # weights and columns, twice as many
     assert (b[0] - b[1]) - (a[0] - a[1]) <= rows + (1 << 20)
+
+
+@pytest.mark.parametrize("nx,ny,n", [(64, 64, 150000), (100, 100, 60000), (45, 91, 150000), (600, 700, 40000)])
+def test_partial_sums_hold_chunks_of_512_nodes(nx, ny, n):
+    """The adjoint's node chunks are at most 512 nodes (their sums stay in FP32) for as many nodes
+    as an image of the detector may have, 24 bytes per chunk and emitter."""
+    entries = min(nx * ny // 4 + 4096, (nx // 2 + 64) // 2 * 2 * ((ny // 2 + 64) // 2 * 2))
+    assert _sizes(nx, ny, [n])[2] >= 24 * n * -(-entries // 512)
