@@ -125,6 +125,14 @@ __device__ __forceinline__ void empty_record(const SplitRecs &rec, int64_t r) {
     rec.rC[r] = 0.0f;
 }
 
+// Clears the CTAs' busy times (first launch of a call), by all threads of a prep kernel: a
+// memset of its own costs 5 us of a small call.
+__device__ __forceinline__ void clear_times(uint64_t *__restrict__ cta_ns) {
+    if (!cta_ns) return;
+    const int threads = gridDim.x * gridDim.y * blockDim.x;
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < kMaxCtas; i += threads) cta_ns[i] = 0;
+}
+
 // Sort of the emitters by cell (images cut into cells): counts per block of kCellSort
 // emitters, their prefix over the blocks, the first record block (64 emitters) of every
 // cell, and the cells' totals.
@@ -234,8 +242,9 @@ __global__ void __launch_bounds__(256)
     prep_split_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                       const void *__restrict__ amps, int amp_dtype, int w_mode, double max_abs, SplitRecs rec,
                       WsHeader *__restrict__ hdr, const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext,
-                      NodePlan *__restrict__ plan, CellSort cs) {
+                      NodePlan *__restrict__ plan, CellSort cs, uint64_t *__restrict__ cta_ns) {
     const int b = blockIdx.y, tid = threadIdx.x;
+    clear_times(cta_ns);
     const ImageDesc d = bp.img[b];
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
     uint32_t *err = &hdr->error;
@@ -311,8 +320,9 @@ __global__ void __launch_bounds__(256)
     prep_double_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms,
                        const void *__restrict__ amps, int amp_dtype, DoubleRecs rec, WsHeader *__restrict__ hdr,
                        const GeomParams g, const NodeGeom ng, uint32_t *__restrict__ ext,
-                       NodePlan *__restrict__ plan) {
+                       NodePlan *__restrict__ plan, uint64_t *__restrict__ cta_ns) {
     const int b = blockIdx.y;
+    clear_times(cta_ns);
     const ImageDesc d = bp.img[b];
     NodeExtents ex;
     const int64_t nrec = (int64_t)d.ntiles * bp.te;
@@ -808,7 +818,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
 
@@ -857,7 +867,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
             }
         return;
     }
-    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
 }
 
 // ---------------------------------------------------------------------------
@@ -982,7 +992,7 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     int64_t pos = wend * blockIdx.x / gridDim.x;
@@ -1213,7 +1223,7 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
                 atomicAdd(dst + 2 * (m0 + i) + 1, (unsigned long long)sim[i]);
             }
     }
-    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
 }
 
 // Node sums in FP64 (IDIWF_DOUBLE in the far field, and in the near field with
@@ -1255,7 +1265,7 @@ __global__ void __launch_bounds__(kNodeThreads)
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     int64_t pos = wend * blockIdx.x / gridDim.x;
@@ -1376,7 +1386,7 @@ __global__ void __launch_bounds__(kNodeThreads)
             }
         }
     }
-    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
 }
 
 // Zeroes the sums that the group's images use.
@@ -1656,7 +1666,7 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = gridDim.x;
+        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     const int npix = g.nx * g.ny;
@@ -1802,7 +1812,7 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
             }
         return;
     }
-    if (tid == 0) cta_ns[blockIdx.x] = globaltimer_ns() - t_start;
+    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
 }
 
 // ---------------------------------------------------------------------------
@@ -2317,8 +2327,8 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
     NodePlan *plan = bp.nodes ? reinterpret_cast<NodePlan *>(node_base) : nullptr;
     NodeGeom ng = make_node_geom(g);
     ng.min_pairs = node_min_pairs(precision, out_kind);
-    // the header's counters and ticket; its error word and pair count add up over a
-    // call's launches, so only the first launch clears all of it
+    // the header's counters and ticket; its error word and pair count and the CTAs' busy times
+    // add up over a call's kernels, so only the first launch clears all of it
     if (i0 == 0) {
         IDIWF_CUDA_CHECK(cudaMemsetAsync(hdr, 0, offsetof(WsHeader, pad), stream));
     } else {
@@ -2329,7 +2339,10 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
         IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
     uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
     if (plan) IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, (size_t)kMaxImagesPerLaunch * 4 * kNodeExt, stream));
-    if (max_tiles > 0 || plan) {  // (the prep kernel also writes the plan)
+    uint64_t *clear_ns = i0 == 0 ? cta_ns : nullptr;
+    if (max_tiles == 0 && !plan) {
+        if (clear_ns) IDIWF_CUDA_CHECK(cudaMemsetAsync(clear_ns, 0, sizeof(uint64_t) * kMaxCtas, stream));
+    } else {  // (the prep kernel also writes the plan)
         dim3 pgrid((unsigned)std::max<int64_t>(std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), 1),
                    bp.n_images);
         if (precision == IDIWF_SPLIT) {
@@ -2348,15 +2361,15 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
                     bp, b->atoms, ng, plan, cs);
                 prep_split_kernel<false><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                     max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
-                                                                    plan, cs);
+                                                                    plan, cs, clear_ns);
             } else {
                 prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                    max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
-                                                                   plan, cs);
+                                                                   plan, cs, clear_ns);
             }
         } else {
             prep_double_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype,
-                                                          double_recs(ws, nrec), hdr, g, ng, ext, plan);
+                                                          double_recs(ws, nrec), hdr, g, ng, ext, plan, clear_ns);
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
     }
@@ -2689,7 +2702,7 @@ extern "C" idiwf_status idiwf_forward_noalloc(const idiwf_geom *geom, const idiw
 
     // every call starts from zero work counters and a zero error word; the
     // records are rewritten in full by the prep kernel
-    IDIWF_CUDA_CHECK(cudaMemsetAsync(ws, 0, 6 * sizeof(uint32_t), stream));  // counters 1-3, error word, n_ctas
+    IDIWF_CUDA_CHECK(cudaMemsetAsync(ws, 0, offsetof(WsHeader, pad), stream));
     IDIWF_CUDA_CHECK(cudaMemsetAsync(rec.rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
     if (max_tiles > 0) {
         const int w_mode = (geom->flags & IDIWF_NF) ? 1 : ((geom->flags & IDIWF_SECONDORDER) ? 2 : 0);
@@ -2697,8 +2710,10 @@ extern "C" idiwf_status idiwf_forward_noalloc(const idiwf_geom *geom, const idiw
         dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)max_tiles * s.te + 255) / 256, 1024), bp.n_images);
         prep_split_kernel<true><<<pgrid, 256, 0, stream>>>(bp, batch->atoms, batch->amplitudes, batch->amp_dtype, w_mode,
                                                            max_abs, rec, hdr, g, NodeGeom{}, nullptr,
-                                                           nullptr, CellSort{});
+                                                           nullptr, CellSort{}, cta_ns);
         IDIWF_CUDA_CHECK(cudaGetLastError());
+    } else {
+        IDIWF_CUDA_CHECK(cudaMemsetAsync(cta_ns, 0, sizeof(uint64_t) * kMaxCtas, stream));
     }
     double2 *no_partials = nullptr;  // bp.ksplit == 0: the kernels write the outputs themselves
     NodePlan *no_plan = nullptr;         // every image takes its direct path

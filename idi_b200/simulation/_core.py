@@ -304,7 +304,7 @@ def tune(atoms, offsets, geom, precision=nat.SPLIT, out_kind=nat.OUT_I32, amplit
 
 
 def cta_times(device=None, role="main") -> np.ndarray:
-    """Per-CTA busy time (ns) of the last forward launch on ``device``."""
+    """Per-CTA busy time (ns) of the last forward call on ``device``, over its kernels that form sums."""
     lib = nat.load()
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     ws = WORKSPACES.get(256, dev, role)

@@ -107,7 +107,7 @@ class BatchPlan:
         return self.out
 
     def cta_times(self) -> np.ndarray:
-        """Per-CTA busy time (ns) of the last launch (synchronises)."""
+        """Per-CTA busy time (ns) of the last run, over its kernels that form sums (synchronises)."""
         return _core.cta_times(self.device, role=self._role)
 
     def check(self):

@@ -146,9 +146,11 @@ idiwf_status idiwf_forward(const idiwf_geom *geom, const idiwf_batch *batch, int
                            int32_t out_kind, void *out, void *workspace, size_t workspace_bytes,
                            const idiwf_config *cfg, cudaStream_t stream);
 
-/* Per-CTA busy time of the last forward launch that used `workspace`
- * (nanoseconds, DEVICE->host copy + stream sync).  Fills up to `cap` entries,
- * returns the count in *n.  Used to report load imbalance. */
+/* Per-CTA busy time of the last forward call that used `workspace`, added up over
+ * its kernels that form sums (direct kernels, and the node sums of every group of
+ * images; nanoseconds, DEVICE->host copy + stream sync).  Fills up to `cap`
+ * entries, returns the count (the largest kernel's CTAs) in *n.  Used to report load
+ * imbalance; kernels of different grids share the first entries. */
 idiwf_status idiwf_forward_cta_times(const void *workspace, uint64_t *host_ns, int32_t cap,
                                      int32_t *n, cudaStream_t stream);
 

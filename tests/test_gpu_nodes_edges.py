@@ -267,3 +267,17 @@ def test_adjoint_more_node_chunks_than_pixel_chunks(ndet, n, r, phases):
     for a, b in ((out[:, :3], ga[:, :3]), (out[:, 3], ga[:, 3]), (out_amp, gamp)):
         err = float((a - b).norm() / b.norm())
         assert err < ADJOINT_2NORM, err
+
+
+def test_cta_times_add_up_over_the_groups():
+    """A large image in the first group of node buffers, small ones in the next: the busy time
+    is the call's, not the last group's."""
+    g = rng(25)
+    counts = [100_000] + [400] * 59
+    at = np.concatenate([_image(g, c, 0.01) for c in counts])
+    geom = _core.make_geom([600, 700], 75.0, 1e5, K64)
+    _forward(at[:counts[0]], [0, counts[0]], geom, nat.OUT_C64)
+    alone = _core.cta_times().astype(float)
+    _forward(at, np.concatenate([[0], np.cumsum(counts)]), geom, nat.OUT_C64)
+    busy = _core.cta_times().astype(float)
+    assert busy.sum() > 0.8 * alone.sum() and busy.size == alone.size
