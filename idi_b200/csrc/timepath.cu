@@ -805,12 +805,14 @@ __global__ void __launch_bounds__(kTimeThreads, 1) time_kernel(const GeomParams 
     for (;;) {
         __syncthreads();
         if (tid == 0)
-            s_pix = order_pixel >= 0 ? (iter == 0 ? 0 : npix) : (int)atomicAdd(&hdr->work_counter, (unsigned)chunk);
+            // (unsigned: every CTA's last claim goes past the end, up to twice npix < 2^31)
+            s_pix = order_pixel >= 0 ? (iter == 0 ? 0 : npix)
+                                     : (int)min(atomicAdd(&hdr->work_counter, (unsigned)chunk), (unsigned)npix);
         __syncthreads();
         ++iter;
         const int c0 = s_pix;
         if (c0 >= npix) break;
-        const int c1 = order_pixel >= 0 ? c0 + 1 : min(c0 + chunk, npix);
+        const int c1 = order_pixel >= 0 ? c0 + 1 : c0 + min(chunk, npix - c0);
         for (int pl = c0; pl < c1; ++pl) {
             int ix, iy;
             if (order_pixel >= 0) {
@@ -1341,7 +1343,8 @@ __global__ void __launch_bounds__(kTimeThreads, 2) time_kernel_large(
     for (;;) {
         __syncthreads();
         if (tid == 0)
-            s_pix = order_pixel >= 0 ? (iter == 0 ? order_pixel : npix) : (int)atomicAdd(&hdr->work_counter, 1u);
+            s_pix = order_pixel >= 0 ? (iter == 0 ? order_pixel : npix)
+                                     : (int)min(atomicAdd(&hdr->work_counter, 1u), (unsigned)npix);
         __syncthreads();
         ++iter;
         const int p = s_pix;
@@ -1586,7 +1589,7 @@ static idiwf_status time_launch(const idiwf_geom *geom, const double *atoms, con
     // serpentine order (every pixel of a CTA but its first warm-starts from a
     // neighbour's order; the per-pixel cost hardly varies, so equal shares
     // balance)
-    int chunk = (npix + grid - 1) / grid;
+    int chunk = (int)(((int64_t)npix + grid - 1) / grid);
     int ni = (int)n;
     void *args[] = {(void *)&g, &atoms, &times, &ni, &c, &tau, &out, &hdr, &order_pixel, &order_out, &keys_out,
                     &digest, &chunk, (void *)&sh};
