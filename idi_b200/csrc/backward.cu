@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(256)
         if ((threadIdx.x & 31) == 0 && r2max) atomicMax(&rmax2[b], r2max);
         return;
     }
-    ex.raise(rmax2, b);
+    ex.raise(rmax2, b, 1, kMaxImagesPerLaunch);
     if (last_block(hdr)) plan_adjoint(bp, g, ng, rmax2, nodes, part_chunks, plan);
 }
 

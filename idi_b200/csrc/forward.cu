@@ -160,79 +160,6 @@ __global__ void __launch_bounds__(256)
     if (last_block(hdr)) plan_nodes(bp, g, ng, ext, false, hdr, plan);
 }
 
-// Emitters per cell of every sort block; an image's last block turns the counts into
-// offsets and lays the cells out, each on whole blocks of 64 records.
-__global__ void __launch_bounds__(256)
-    cell_count_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms, const NodeGeom ng,
-                      NodePlan *__restrict__ plan, CellSort cs) {
-    __shared__ int s_cnt[kCellMax], s_part[8];
-    __shared__ int s_last;
-    const int img = blockIdx.y, tid = threadIdx.x;
-    const NodeImage &pi = plan->img[img];
-    if (pi.path != kPathNodes || pi.ncell == 1) return;
-    const NodeImage ni = pi;
-    const ImageDesc d = bp.img[img];
-    const int nb = (d.n + kCellSort - 1) / kCellSort;
-    int *counts = cs.counts + sort_block0(bp, img) * kCellMax;
-    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-        for (int c = tid; c < ni.ncell; c += 256) s_cnt[c] = 0;
-        __syncthreads();
-        for (int j = b * kCellSort + tid; j < min((b + 1) * kCellSort, d.n); j += 256)
-            atomicAdd(&s_cnt[cell_of(ng, ni, reinterpret_cast<const double4 *>(atoms)[d.src + j])], 1);
-        __syncthreads();
-        for (int c = tid; c < ni.ncell; c += 256) counts[(int64_t)b * kCellMax + c] = s_cnt[c];
-        __syncthreads();
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&plan->img[img].ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    int blocks0 = 0;
-    for (int c0 = 0; c0 < ni.ncell; c0 += 256) {
-        const int c = c0 + tid;
-        int sum = 0;
-        if (c < ni.ncell) {
-            // 16 loads in flight at a time: the chain is the additions, not the memory
-            for (int b0 = 0; b0 < nb; b0 += 16) {
-                int v[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k)
-                    v[k] = b0 + k < nb ? __ldcg(counts + (int64_t)(b0 + k) * kCellMax + c) : 0;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (b0 + k < nb) counts[(int64_t)(b0 + k) * kCellMax + c] = sum;
-                    sum += v[k];
-                }
-            }
-            cs.total[img * kCellMax + c] = sum;
-        }
-        // exclusive scan of the cells' record blocks over the 256 threads
-        const int nblk = (sum + kNodeBlock - 1) / kNodeBlock;
-        int x = nblk;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((tid & 31) >= o) x += y;
-        }
-        if ((tid & 31) == 31) s_part[tid >> 5] = x;
-        __syncthreads();
-        int before = 0, all = 0;
-        for (int w = 0; w < 8; ++w) {
-            before += w < (tid >> 5) ? s_part[w] : 0;
-            all += s_part[w];
-        }
-        if (c < ni.ncell) cs.first[img * (kCellMax + 1) + c] = blocks0 + before + x - nblk;
-        blocks0 += all;
-        __syncthreads();
-    }
-    if (tid == 0) {
-        cs.first[img * (kCellMax + 1) + ni.ncell] = blocks0;
-        plan->img[img].nblk = blocks0;
-    }
-}
-
 // Records.  MAKE_PLAN: the launch has no cells, and where there is a plan it is made here
 // (extents on the way, by the block that finishes last); else the plan is given, and
 // images cut into cells are written in cell order (stable: the order of an emitter's
@@ -1389,33 +1316,108 @@ __global__ void __launch_bounds__(kNodeThreads)
     if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
 }
 
-// Zeroes the sums that the group's images use.
-__global__ void __launch_bounds__(256) node_zero_kernel(const NodePlan *__restrict__ plan, NodeBuffers nb, int img0) {
-    const NodeImage &ni = plan->img[img0 + blockIdx.y];
-    if (ni.path != kPathNodes) return;
-    const int64_t nv = (int64_t)ni.n0 * ni.n1, nf = nb.two_words ? nv : (ni.ncell > 1 ? (int64_t)ni.ncell * ni.g0 * ni.g1 : 0);
-    double2 *v = nb.v + blockIdx.y * nb.caps.v, *f = nb.f + blockIdx.y * nb.caps.f;
-    for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv + nf; i += gridDim.x * blockDim.x)
-        (i < nv ? v[i] : f[i - nv]) = make_double2(0.0, 0.0);
+// Emitters per cell of every sort block; an image's last block turns the counts into
+// offsets and lays the cells out, each on whole blocks of 64 records.
+__device__ __forceinline__ void count_cells(const BatchParams &bp, const double *__restrict__ atoms, const NodeGeom &ng,
+                                            NodePlan *__restrict__ plan, const CellSort &cs) {
+    __shared__ int s_cnt[kCellMax], s_part[8];
+    __shared__ int s_last;
+    const int img = blockIdx.y, tid = threadIdx.x;
+    const NodeImage &pi = plan->img[img];
+    if (pi.path != kPathNodes || pi.ncell == 1) return;
+    const NodeImage ni = pi;
+    const ImageDesc d = bp.img[img];
+    const int nb = (d.n + kCellSort - 1) / kCellSort;
+    int *counts = cs.counts + sort_block0(bp, img) * kCellMax;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        for (int c = tid; c < ni.ncell; c += 256) s_cnt[c] = 0;
+        __syncthreads();
+        for (int j = b * kCellSort + tid; j < min((b + 1) * kCellSort, d.n); j += 256)
+            atomicAdd(&s_cnt[cell_of(ng, ni, reinterpret_cast<const double4 *>(atoms)[d.src + j])], 1);
+        __syncthreads();
+        for (int c = tid; c < ni.ncell; c += 256) counts[(int64_t)b * kCellMax + c] = s_cnt[c];
+        __syncthreads();
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&plan->img[img].ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int blocks0 = 0;
+    for (int c0 = 0; c0 < ni.ncell; c0 += 256) {
+        const int c = c0 + tid;
+        int sum = 0;
+        if (c < ni.ncell) {
+            // 16 loads in flight at a time: the chain is the additions, not the memory
+            for (int b0 = 0; b0 < nb; b0 += 16) {
+                int v[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    v[k] = b0 + k < nb ? __ldcg(counts + (int64_t)(b0 + k) * kCellMax + c) : 0;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    if (b0 + k < nb) counts[(int64_t)(b0 + k) * kCellMax + c] = sum;
+                    sum += v[k];
+                }
+            }
+            cs.total[img * kCellMax + c] = sum;
+        }
+        // exclusive scan of the cells' record blocks over the 256 threads
+        const int nblk = (sum + kNodeBlock - 1) / kNodeBlock;
+        int x = nblk;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((tid & 31) >= o) x += y;
+        }
+        if ((tid & 31) == 31) s_part[tid >> 5] = x;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 8; ++w) {
+            before += w < (tid >> 5) ? s_part[w] : 0;
+            all += s_part[w];
+        }
+        if (c < ni.ncell) cs.first[img * (kCellMax + 1) + c] = blocks0 + before + x - nblk;
+        blocks0 += all;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        cs.first[img * (kCellMax + 1) + ni.ncell] = blocks0;
+        plan->img[img].nblk = blocks0;
+    }
 }
 
-// The interpolation weights.
-__global__ void __launch_bounds__(256) node_weights_kernel(const GeomParams g, const NodePlan *__restrict__ plan,
-                                                           NodeBuffers nb, int img0) {
-    const NodeImage ni = plan->img[img0 + blockIdx.y];
-    if (ni.path != kPathNodes) return;
-    const int lane = threadIdx.x & 31;
-    double *lx = nb.lx + blockIdx.y * nb.lx_stride, *ly = nb.ly + blockIdx.y * nb.ly_stride;
-    double *sx = nb.sx + blockIdx.y * nb.sx_stride, *sy = nb.sy + blockIdx.y * nb.sy_stride;
-    const int fine = ni.pix ? 0 : g.nx + g.ny, rows = fine + (ni.ncell > 1 ? ni.n0 + ni.n1 : 0);
-    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8) {
+// What a group's images need before their sums: zeros in the sums' buffers, the interpolation
+// weights, and (COUNT, with the first group and for all images) the emitters' counts per
+// cell.  One kernel: where no image takes nodes, every kernel that returns at once
+// costs 1.5 us in a graph and up to 4 us in a stream.
+template <bool COUNT>
+__global__ void __launch_bounds__(256)
+    node_setup_kernel(const __grid_constant__ BatchParams bp, const double *__restrict__ atoms, const GeomParams g,
+                      const NodeGeom ng, NodePlan *__restrict__ plan, CellSort cs, NodeBuffers nb, int img0, int nimg) {
+    const int at = blockIdx.y, tid = threadIdx.x;
+    if (plan->img[img0 + at].path != kPathNodes) return;
+    if (COUNT && plan->img[img0 + at].ncell > 1) count_cells(bp, atoms, ng, plan, cs);
+    if (at >= nimg) return;
+    const NodeImage &ni = plan->img[img0 + at];
+    const int n0 = ni.n0, n1 = ni.n1, g0 = ni.g0, g1 = ni.g1, ncell = ni.ncell, pix = ni.pix;
+    const int64_t nv = (int64_t)n0 * n1, nf = nb.two_words ? nv : (ncell > 1 ? (int64_t)ncell * g0 * g1 : 0);
+    double2 *v = nb.v + at * nb.caps.v, *f = nb.f + at * nb.caps.f;
+    for (int64_t i = blockIdx.x * blockDim.x + tid; i < nv + nf; i += gridDim.x * blockDim.x)
+        (i < nv ? v[i] : f[i - nv]) = make_double2(0.0, 0.0);
+    const int lane = tid & 31;
+    double *lx = nb.lx + at * nb.lx_stride, *ly = nb.ly + at * nb.ly_stride;
+    double *sx = nb.sx + at * nb.sx_stride, *sy = nb.sy + at * nb.sy_stride;
+    const int fine = pix ? 0 : g.nx + g.ny, rows = fine + (ncell > 1 ? n0 + n1 : 0);
+    for (int row = blockIdx.x * 8 + (tid >> 5); row < rows; row += gridDim.x * 8) {
         if (row < fine) {
-            if (row < g.nx) node_weights_row(lx, ni.n0, pixel_x(g.nx, row), row, lane);
-            else node_weights_row(ly, ni.n1, pixel_x(g.ny, row - g.nx), row - g.nx, lane);
+            if (row < g.nx) node_weights_row(lx, n0, pixel_x(g.nx, row), row, lane);
+            else node_weights_row(ly, n1, pixel_x(g.ny, row - g.nx), row - g.nx, lane);
         } else {
             const int i = row - fine;
-            if (i < ni.n0) node_weights_row(sx, ni.g0, ni.pix ? pixel_x(g.nx, i) : node_x(ni.n0, i), i, lane);
-            else node_weights_row(sy, ni.g1, ni.pix ? pixel_x(g.ny, i - ni.n0) : node_x(ni.n1, i - ni.n0), i - ni.n0, lane);
+            if (i < n0) node_weights_row(sx, g0, pix ? pixel_x(g.nx, i) : node_x(n0, i), i, lane);
+            else node_weights_row(sy, g1, pix ? pixel_x(g.ny, i - n0) : node_x(n1, i - n0), i - n0, lane);
         }
     }
 }
@@ -2234,10 +2236,28 @@ static void *node_sum_fn(bool nf, bool sc, bool so) {
               : (so ? (void *)node_sum_kernel<false, false, true, FINE> : (void *)node_sum_kernel<false, false, false, FINE>);
 }
 
+// Blocks per image of a group of n images: about two per SM in all.
+static int group_blocks(int n) { return std::max(1, (2 * sm_count() + n - 1) / n); }
+// The setup of images [img0, img0 + n), with the cells' counts of every image where count.
+static void launch_setup(const GeomParams &g, const NodeGeom &ng, const BatchParams &bp, const double *atoms, NodePlan *plan,
+                         const NodeLayout &nl, const NodeBuffers &nb, char *node_base, int img0, int n, bool count,
+                         cudaStream_t stream) {
+    const CellSort cs = nl.sort(node_base);
+    int blocks = std::max((g.nx + g.ny + 15) / 16, group_blocks(n));
+    if (count) {
+        int nbig = 0;
+        for (int i = 0; i < bp.n_images; ++i) nbig = std::max(nbig, bp.img[i].n);
+        blocks = std::max(blocks, (nbig + kCellSort - 1) / kCellSort);
+        node_setup_kernel<true><<<dim3(blocks, bp.n_images), 256, 0, stream>>>(bp, atoms, g, ng, plan, cs, nb, 0, n);
+    } else {
+        node_setup_kernel<false><<<dim3(blocks, n), 256, 0, stream>>>(bp, atoms, g, ng, plan, cs, nb, img0, n);
+    }
+}
+
 // Node sums and interpolation of the images on kPathNodes (each kernel returns at
 // once where there is none).
 static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, const NodeGeom &ng, const BatchParams &bp,
-                                 const SplitRecs *split, const DoubleRecs *dbl, const NodePlan *plan,
+                                 const SplitRecs *split, const DoubleRecs *dbl, NodePlan *plan,
                                  const NodeLayout &nl, char *node_base, WsHeader *hdr, uint64_t *cta_ns, void *out, int out_kind, cudaStream_t stream) {
     const bool nf = geom->flags & IDIWF_NF, sc = geom->flags & IDIWF_SCALE, so = geom->flags & IDIWF_SECONDORDER;
     const NodeBuffers nb = nl.at(node_base, geom);
@@ -2262,14 +2282,12 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
     for (int i0 = 0; i0 < bp.n_images; i0 += nl.group) {
         int i1 = std::min(i0 + nl.group, bp.n_images);
         const int n = i1 - i0;
-        // (about two blocks per SM over the group's images)
-        const int per = std::max(1, (2 * sm_count() + n - 1) / n);
-        node_zero_kernel<<<dim3(per, n), 256, 0, stream>>>(plan, nb, i0);
+        // (cells: the first group's setup came with the emitters' counts, before the records)
+        if (!cells || i0 > 0) launch_setup(g, ng, bp, nullptr, plan, nl, nb, node_base, i0, n, false, stream);
         void *as[] = {(void *)&bp, (void *)&g, dbl ? (void *)dbl : (void *)split, &plan, (void *)&nb, &first, &hdr, &cta_ns, &i0, &i1};
         IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), as, 0, stream));
-        node_weights_kernel<<<dim3((g.nx + g.ny + 15) / 16, n), 256, 0, stream>>>(g, plan, nb, i0);
         if (cells) {
-            cell_interp_kernel<<<dim3(4 * per, n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
+            cell_interp_kernel<<<dim3(4 * group_blocks(n), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
             cell_expand_kernel<<<egrid, kGemmThreads, sizeof(ExpandSmem), stream>>>(g, ng, plan, nb, i0, i1);
         }
         IDIWF_CUDA_CHECK(cudaGetLastError());
@@ -2338,7 +2356,7 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
     if (precision == IDIWF_SPLIT && !plan)
         IDIWF_CUDA_CHECK(cudaMemsetAsync(split_recs(ws, nrec).rmax2, 0, sizeof(uint32_t) * bp.n_images, stream));
     uint32_t *ext = reinterpret_cast<uint32_t *>(node_base + nl.ext);
-    if (plan) IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, (size_t)kMaxImagesPerLaunch * 4 * kNodeExt, stream));
+    if (plan) IDIWF_CUDA_CHECK(cudaMemsetAsync(ext, 0, (size_t)bp.n_images * 4 * kNodeExt, stream));
     uint64_t *clear_ns = i0 == 0 ? cta_ns : nullptr;
     if (max_tiles == 0 && !plan) {
         if (clear_ns) IDIWF_CUDA_CHECK(cudaMemsetAsync(clear_ns, 0, sizeof(uint64_t) * kMaxCtas, stream));
@@ -2352,13 +2370,10 @@ static idiwf_status launch_chunk(const idiwf_geom *geom, const idiwf_batch *b, i
             const CellSort cs = nl.sort(node_base);
             if (bp.nodes > 1) {
                 // extents and plan, the emitters' sort by cell, then the records
-                int nbig = 0;
-                for (int i = 0; i < bp.n_images; ++i) nbig = std::max(nbig, bp.img[i].n);
                 node_extents_kernel<<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, ext, hdr, g,
                                                                ng, plan);
-                // (a launch of empty images has no emitters to sort)
-                cell_count_kernel<<<dim3(std::max(1, (nbig + kCellSort - 1) / kCellSort), bp.n_images), 256, 0, stream>>>(
-                    bp, b->atoms, ng, plan, cs);
+                launch_setup(g, ng, bp, b->atoms, plan, nl, nl.at(node_base, geom), node_base, 0,
+                             std::min(nl.group, bp.n_images), true, stream);
                 prep_split_kernel<false><<<pgrid, 256, 0, stream>>>(bp, b->atoms, b->amplitudes, b->amp_dtype, w_mode,
                                                                     max_abs, split_recs(ws, nrec), hdr, g, ng, ext,
                                                                     plan, cs, clear_ns);

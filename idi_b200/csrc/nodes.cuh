@@ -212,8 +212,8 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 // Largest extents of an emitter for the plan: |r|^2 and |a| (float bits, rounded up), and
-// r . e and -r . e along the three axes (keys, rounded up), raised per warp into ext
-// (kMaxImagesPerLaunch of each).
+// r . e and -r . e along the three axes (keys, rounded up), raised per block into ext: extent
+// k of image b at b * sb + k * sk.
 constexpr int kNodeExt = 8;
 struct NodeExtents {
     uint32_t v[kNodeExt] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -228,7 +228,7 @@ struct NodeExtents {
         }
     }
     // (one atomic per block and extent: a warp's own would queue up on the image's words)
-    __device__ __forceinline__ void raise(uint32_t *ext, int b) const {
+    __device__ __forceinline__ void raise(uint32_t *ext, int b, int sb = kNodeExt, int sk = 1) const {
         __shared__ uint32_t s_max[kNodeExt];
         if (threadIdx.x < kNodeExt) s_max[threadIdx.x] = 0;
         __syncthreads();
@@ -239,7 +239,7 @@ struct NodeExtents {
         }
         __syncthreads();
         if (threadIdx.x < kNodeExt && s_max[threadIdx.x])
-            atomicMax(ext + threadIdx.x * kMaxImagesPerLaunch + b, s_max[threadIdx.x]);
+            atomicMax(ext + b * sb + threadIdx.x * sk, s_max[threadIdx.x]);
     }
 };
 // True in every thread of the grid's last block to get here (a ticket in the header);
@@ -280,7 +280,7 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
     for (int i = threadIdx.x >> 5; i < bp.n_images; i += blockDim.x >> 5) {
         uint32_t x[kNodeExt];
 #pragma unroll
-        for (int k = 0; k < kNodeExt; ++k) x[k] = __ldcg(ext + k * kMaxImagesPerLaunch + i);
+        for (int k = 0; k < kNodeExt; ++k) x[k] = __ldcg(ext + i * kNodeExt + k);
         const int n = bp.img[i].n;
         const uint32_t amax = x[1];
         NodeImage ni;
