@@ -133,6 +133,11 @@ __device__ __forceinline__ void clear_times(uint64_t *__restrict__ cta_ns) {
     for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < kMaxCtas; i += threads) cta_ns[i] = 0;
 }
 
+// The CTA's busy time joins the call's (an atomic without a result: nothing waits for it).
+__device__ __forceinline__ void add_busy(uint64_t *__restrict__ cta_ns, uint64_t ns) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(cta_ns) + blockIdx.x, (unsigned long long)ns);
+}
+
 // Sort of the emitters by cell (images cut into cells): counts per block of kCellSort
 // emitters, their prefix over the blocks, the first record block (64 emitters) of every
 // cell, and the cells' totals.
@@ -745,7 +750,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
+        if (blockIdx.x == 0) atomicMax(&hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
 
@@ -794,7 +799,7 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
             }
         return;
     }
-    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
+    if (tid == 0) add_busy(cta_ns, globaltimer_ns() - t_start);
 }
 
 // ---------------------------------------------------------------------------
@@ -919,7 +924,7 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
+        if (blockIdx.x == 0) atomicMax(&hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     int64_t pos = wend * blockIdx.x / gridDim.x;
@@ -1150,7 +1155,7 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
                 atomicAdd(dst + 2 * (m0 + i) + 1, (unsigned long long)sim[i]);
             }
     }
-    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
+    if (tid == 0) add_busy(cta_ns, globaltimer_ns() - t_start);
 }
 
 // Node sums in FP64 (IDIWF_DOUBLE in the far field, and in the near field with
@@ -1192,7 +1197,7 @@ __global__ void __launch_bounds__(kNodeThreads)
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
+        if (blockIdx.x == 0) atomicMax(&hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     int64_t pos = wend * blockIdx.x / gridDim.x;
@@ -1313,7 +1318,7 @@ __global__ void __launch_bounds__(kNodeThreads)
             }
         }
     }
-    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
+    if (tid == 0) add_busy(cta_ns, globaltimer_ns() - t_start);
 }
 
 // Emitters per cell of every sort block; an image's last block turns the counts into
@@ -1668,7 +1673,7 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
         mbar_init(&bar[1], 1);
         s_abort = 0;
         mbar_fence_init();
-        if (blockIdx.x == 0) hdr->n_ctas = max(hdr->n_ctas, gridDim.x);
+        if (blockIdx.x == 0) atomicMax(&hdr->n_ctas, gridDim.x);
     }
     __syncthreads();
     const int npix = g.nx * g.ny;
@@ -1814,7 +1819,7 @@ __global__ void __launch_bounds__(256) fwd_double_kernel(const __grid_constant__
             }
         return;
     }
-    if (tid == 0) cta_ns[blockIdx.x] += globaltimer_ns() - t_start;
+    if (tid == 0) add_busy(cta_ns, globaltimer_ns() - t_start);
 }
 
 // ---------------------------------------------------------------------------
