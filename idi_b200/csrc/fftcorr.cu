@@ -6,6 +6,7 @@
 // lines).  For larger shapes, the elementwise steps around cuFFT's transforms
 // -- the power spectrum in place, the fftshift + centre crop fused with the
 // normalisation -- and the correlator's running mean / variance.
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -1236,12 +1237,14 @@ static int fcg_fastlen(int x) {
     }
 }
 // Radices of n; false if n has another prime factor.  Twos pair up with fives and
-// threes (radices 10 and 6) as far as that leaves fewer passes, and odd radices
-// come first, the smallest before the others: a first pass writes R apart, and its loads
-// spread over more threads (7 before 5 took 0.883 ms for 8 x 1000 x 1050 FP64, 5 before 7
-// takes 0.851).  A pass costs its barrier and its trip through shared memory whatever
-// its radix (2100 = 5 7 10 6 in four passes, not 7 5 5 3 4 in five).
-static bool fcg_radices(int n, FcgRad &rad) {
+// threes (radices 10 and 6) as far as that leaves fewer passes: a pass costs its barrier
+// and its trip through shared memory whatever its radix (2100 = 5 7 10 6 in four passes,
+// not 7 5 5 3 4 in five).  Odd radices come first.  loader: the first pass loads from global
+// memory, R values a thread, and writes R apart, so the smallest spreads its loads over the
+// most threads (7 before 5 took 0.883 ms for 8 x 1000 x 1050 FP64, 5 before 7 takes 0.851).
+// Else (Bluestein's rows, copied with their zeros) the largest, since a first pass has no
+// twiddles (8 x 512 x 113 FP64 103 -> 100 us, 3 x 333 x 422 109.5 -> 107.6).
+static bool fcg_radices(int n, FcgRad &rad, bool loader = true) {
     rad = FcgRad{};
     rad.n = n;
     int e[12] = {};  // exponents of 2, 3, 5, 7, 11
@@ -1266,8 +1269,9 @@ static bool fcg_radices(int n, FcgRad &rad) {
             }
         }
     const int twos = e[2] - t10 - t6;
-    const int list[][2] = {{3, e[3] - t6}, {5, e[5] - t10}, {7, e[7]},          {11, e[11]},        {10, t10},
-                           {6, t6},        {8, twos / 3},   {4, twos % 3 == 2}, {2, twos % 3 == 1}};
+    int list[][2] = {{3, e[3] - t6}, {5, e[5] - t10}, {7, e[7]},          {11, e[11]},        {10, t10},
+                     {6, t6},        {8, twos / 3},   {4, twos % 3 == 2}, {2, twos % 3 == 1}};
+    if (!loader) std::reverse(&list[0], &list[4]);
     for (const auto &l : list)
         for (int i = 0; i < l[1]; ++i) {
             if (rad.np == kFcgMaxPasses) return false;
@@ -1321,7 +1325,7 @@ static bool fcg_plan(int64_t batch, int n0, int n1, int dtype, FcgPlan &p, bool 
         // the shortest smooth length: measured faster than longer lengths with
         // cheaper radices (2304 or 640 instead of 2079 or 605)
         p.M = fcg_fastlen(2 * p.Hp - 1);
-        if (p.M > kFcgMaxLen || !fcg_radices(p.M, p.radC)) return false;
+        if (p.M > kFcgMaxLen || !fcg_radices(p.M, p.radC, false)) return false;
     }
     const int nC = p.radC.n;  // values per row in pass C
     p.vsz = dtype == IDIWF_F64 ? 16 : 8;
