@@ -27,6 +27,14 @@
 //
 // The FP64 kernel's images take a finer grid, 5 + 9.6 Phi^(1/3) + 30 t, which holds the
 // interpolation to about 2e-15 per emitter, below the rounding of the phases (k r 1e-16).
+// A needle along the beam changes its phase as k r t^2 / 4 T_2(x) over the detector, with
+// coefficients J_m of that at twice the order: 2 (a + 5 + 9.6 a^(1/3)) nodes at least, a its size.
+//
+// An object of next to no phase (Phi below 0.1) still has the near field's amplitude
+// 1/|d - r|, whose Chebyshev coefficients fall by rho = e^asinh((1 - r/D) / t) a node, the
+// singularity being D - r off the detector: no fewer than 20 / ln rho nodes (1e-8 of its
+// variation) or, for FP64, 1 + 35 / ln rho.  FP64 images reach to r = D / 20 (kNodeMaxReach64);
+// split-precision ones of that amplitude stay far below it (kNfScaleRho2).
 #pragma once
 
 #include "idiwf_internal.cuh"
@@ -36,6 +44,7 @@ namespace idiwf {
 constexpr int kPathNodes = 4;        // split_path() continued: nodes and interpolation
 constexpr int kNodeMax = 1024;       // nodes per axis
 constexpr double kNodeMaxT = 0.6;
+constexpr double kNodeMaxReach64 = 0.05;
 constexpr int kNodeThreads = 128;    // node kernel: threads per CTA, nodes per thread, emitters per stage
 constexpr int kNodePPT = 2;
 constexpr int kNodeTile = kNodeThreads * kNodePPT;
@@ -67,6 +76,7 @@ constexpr int64_t kCellPixels = 1 << 18;  // most pixels that cells are interpol
 struct NodeGeom {
     double e[3][3];  // unit vectors of the detector axes and their normal
     double phi[2], t[2], s[2];
+    double least[2][2];  // fewest nodes of an axis (split precision, FP64)
     double inv_d;
     double min_pairs;  // fewest pairs of an image that may take nodes
     int32_t ok, ortho;  // ortho: the axes are orthonormal (cells need it)
@@ -144,15 +154,16 @@ NodeGeom make_node_geom(const GeomParams &g);
 #if defined(__CUDACC__)
 
 // Nodes along one axis (even, for the 16-byte copies of weight rows) for a phase
-// half-range phi; fine: the FP64 kernel's.
-__device__ __forceinline__ int node_count(double phi, double t, bool fine) {
-    const double n = fine ? phi + 5.0 + 9.6 * cbrt(phi) + 30.0 * t : phi + 3.7 + 6.33 * cbrt(phi) + 14.0 * t;
+// half-range phi and a curved part of up to curve T_2(x); fine: the FP64 kernel's.
+__device__ __forceinline__ int node_count(double phi, double curve, double t, const double least[2], bool fine) {
+    const double n = fine ? fmax(fmax(phi + 5.0 + 9.6 * cbrt(phi) + 30.0 * t, 2.0 * (curve + 5.0 + 9.6 * cbrt(curve))), least[1])
+                          : fmax(phi + 3.7 + 6.33 * cbrt(phi) + 14.0 * t, least[0]);
     return n < (double)(2 * kNodeMax) ? ((int)ceil(n) + 1) / 2 * 2 : 2 * kNodeMax;
 }
 
 // Whether an object reaching r from the origin may take nodes at all (a NaN may not).
 __device__ __forceinline__ bool node_reach(const GeomParams &g, const NodeGeom &ng, double r, bool fine) {
-    if (!ng.ok || !(r * ng.inv_d <= 0.25)) return false;
+    if (!ng.ok || !(r * ng.inv_d <= (fine ? kNodeMaxReach64 : 0.25))) return false;
     return fine || !(g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) || 0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra;
 }
 // Nodes along both axes for emitters within rho of a centre, |rho . e| <= ex, ey along the
@@ -162,8 +173,8 @@ __device__ __forceinline__ bool node_reach(const GeomParams &g, const NodeGeom &
 __device__ __forceinline__ void node_grid(const NodeGeom &ng, double r, double rho, double ex, double ey, bool fine,
                                           int &n0, int &n1) {
     const double more = 2.0 * r * r * ng.inv_d;
-    n0 = node_count(ng.phi[0] * (fmin(rho, ex + ng.s[0] * rho) + more), ng.t[0], fine);
-    n1 = node_count(ng.phi[1] * (fmin(rho, ey + ng.s[1] * rho) + more), ng.t[1], fine);
+    n0 = node_count(ng.phi[0] * (fmin(rho, ex + ng.s[0] * rho) + more), 0.25 * ng.phi[0] * rho * ng.t[0], ng.t[0], ng.least[0], fine);
+    n1 = node_count(ng.phi[1] * (fmin(rho, ey + ng.s[1] * rho) + more), 0.25 * ng.phi[1] * rho * ng.t[1], ng.t[1], ng.least[1], fine);
 }
 
 // Node m of n on [-1, 1], its barycentric weight, and the (fractional) pixel

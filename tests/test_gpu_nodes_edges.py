@@ -281,3 +281,26 @@ def test_cta_times_add_up_over_the_groups():
     _forward(at, np.concatenate([[0], np.cumsum(counts)]), geom, nat.OUT_C64)
     busy = _core.cta_times().astype(float)
     assert busy.sum() > 0.8 * alone.sum() and busy.size == alone.size
+
+
+@pytest.mark.parametrize("pixel,r,kr", [
+    (1875.0, 2e4, 0.02),  # an object a fifth of the way to the detector
+    (1875.0, 4e3, 0.02),
+    (160.0, 4e3, 0.1),
+    (160.0, 50.0, 0.1),
+])
+@pytest.mark.parametrize("settings", ["nf scale accurate", "nf accurate", "double scale"])
+def test_fp64_objects_of_next_to_no_phase(pixel, r, kr, settings):
+    """The grid follows the near field's amplitude 1/|d - r| where the phase asks for few nodes:
+    interpolation 2e-15, FP64 sums of emitters in phase and weights a few 1e-16 each."""
+    g = rng(26)
+    n, ndet = 600, [64, 64]
+    # at the end nearest the detector, where the amplitude is sharpest
+    at = atoms(sphere(g, n, 0.01 * r) + [0, 0, 0.99 * r], g.uniform(0, 0.1, n))
+    flags, prec, _ = _core.parse_settings(settings)
+    geom = _core.make_geom(ndet, pixel, 1e5, kr / r, flags=flags)
+    E = _forward(at, [0, n], geom, nat.OUT_C128, prec)[0]
+    of = oracle.flags_from_settings(settings) | (oracle.ACCURATE if "nf" in settings else 0)
+    ref = oracle.wavefield(oracle.geometry(ndet, pixel, 1e5, kr / r), of, at)
+    err = np.abs(E - ref).max() / np.abs(ref).max()
+    assert err < 5e-15, err
