@@ -105,7 +105,7 @@ struct AdjImage {
     int32_t pad;
 };
 struct AdjPlan {
-    int32_t total_units, n_direct, n_nodes, pad;
+    int32_t total_units, n_direct;
     AdjImage img[kMaxImagesPerLaunch];
     uint32_t counter[kMaxImagesPerLaunch];  // work queue of the group that starts at this image
 };

@@ -1178,7 +1178,7 @@ __device__ __forceinline__ void add_two_words(double x, long long &hi, long long
 template <bool ACC, bool SCALE, bool SECOND>
 __global__ void __launch_bounds__(kNodeThreads)
     node_sum64_kernel(const __grid_constant__ BatchParams bp, const GeomParams g, DoubleRecs rec,
-                      const NodePlan *__restrict__ plan, NodeBuffers nb, const int *__restrict__ first,
+                      const NodePlan *__restrict__ plan, NodeBuffers nb,
                       WsHeader *__restrict__ hdr, uint64_t *__restrict__ cta_ns, int img0, int img1) {
     constexpr int PPT = kNodePPT64;
     constexpr uint32_t kStage = kNodeBlock * kDoubleRecBytes;
@@ -2291,8 +2291,9 @@ static idiwf_status launch_nodes(const idiwf_geom *geom, const GeomParams &g, co
         const int n = i1 - i0;
         // (cells: the first group's setup came with the emitters' counts, before the records)
         if (!cells || i0 > 0) launch_setup(g, ng, bp, nullptr, plan, nl, nb, node_base, i0, n, false, stream);
-        void *as[] = {(void *)&bp, (void *)&g, dbl ? (void *)dbl : (void *)split, &plan, (void *)&nb, &first, &hdr, &cta_ns, &i0, &i1};
-        IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), as, 0, stream));
+        void *as[] = {(void *)&bp, (void *)&g, (void *)split, &plan, (void *)&nb, &first, &hdr, &cta_ns, &i0, &i1};
+        void *ad[] = {(void *)&bp, (void *)&g, (void *)dbl, &plan, (void *)&nb, &hdr, &cta_ns, &i0, &i1};
+        IDIWF_CUDA_CHECK(cudaLaunchKernel(fs, dim3(grid), dim3(kNodeThreads), dbl ? ad : as, 0, stream));
         if (cells) {
             cell_interp_kernel<<<dim3(4 * group_blocks(n), n), kGemmThreads, sizeof(GemmSmem), stream>>>(g, plan, nb, i0);
             cell_expand_kernel<<<egrid, kGemmThreads, sizeof(ExpandSmem), stream>>>(g, ng, plan, nb, i0, i1);

@@ -83,7 +83,6 @@ struct NodeGeom {
 };
 
 struct NodeImage {
-    int64_t w0;         // work (tiles x blocks of kNodeBlock emitters) of the images before it
     int32_t path;       // split path of the image
     int32_t n0, n1;     // target grid: nodes along x and y, or (pix) the pixels
     int32_t pix;
@@ -96,8 +95,6 @@ struct NodeImage {
     double lo[3], size[3], inv[3];  // cells: origin, edges, 1/edges
 };
 struct NodePlan {
-    int64_t total;      // work of all images
-    int64_t pad;
     NodeImage img[kMaxImagesPerLaunch];
 };
 // Second words of the FP64 kernel's node sums: units of the first word's unit.  A block of
@@ -279,13 +276,11 @@ __device__ __forceinline__ double node_cost(double n, int nx, int ny, const Node
     return t + 100.0 * npix * (1.0 / 1.2e13);
 }
 
-// Plan of one launch, by one block: every image's path, grids, fixed-point scale and
-// share of the work; one warp per image, whose lanes try the ways to cut it.  The choice
+// Plan of one launch, by one block: every image's path, grids and fixed-point scale; one warp per image, whose lanes try the ways to cut it.  The choice
 // depends on the image and the geometry alone, as split_path's does.  fine: the FP64
 // kernel's images (their direct path counts as kPathPixel).
 __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, const NodeGeom &ng,
                                   const uint32_t *ext, bool fine, WsHeader *hdr, NodePlan *plan) {
-    __shared__ long long s_work[kMaxImagesPerLaunch];
     __threadfence();
     const int npix = g.nx * g.ny, lane = threadIdx.x & 31;
     for (int i = threadIdx.x >> 5; i < bp.n_images; i += blockDim.x >> 5) {
@@ -296,7 +291,6 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         const uint32_t amax = x[1];
         NodeImage ni;
         ni.path = fine ? kPathPixel : split_path(g, x[0], bp.groups != 0, false);
-        ni.w0 = 0;
         ni.n0 = ni.n1 = ni.g0 = ni.g1 = ni.pix = ni.ntiles = ni.nblk = 0;
         ni.scale = 1.0f;
         ni.ncell = ni.c[0] = ni.c[1] = ni.c[2] = 1;
@@ -305,7 +299,6 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         const double pairs = (double)n * npix;
         const int direct = ni.path;
         unsigned long long pr = (unsigned long long)n * npix;
-        long long work = 0;
         // (amplitudes whose fixed-point unit would leave FP32's exponents, infinite or NaN
         // ones take the direct kernels)
         if (bp.nodes && n > 0 && (direct == kPathRuns || direct == kPathPixel) &&
@@ -394,7 +387,6 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
                 ni.ntiles = (m + tile - 1) / tile;
                 ni.nblk = (n + kNodeBlock - 1) / kNodeBlock;  // (the sort replaces it where there are cells)
                 pr = (unsigned long long)n * m;
-                work = (long long)ni.ntiles * ni.nblk;
                 // |sum| <= n max |a| [times the largest 1/|d - r| <= 4/(3 D)] < 2^e; three bits to
                 // spare for the interpolated cells' partial sums
                 double bound = (double)n * (double)__uint_as_float(amax);
@@ -405,18 +397,8 @@ __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, co
         if (lane == 0) {
             atomicAdd(&hdr->pairs, pr);
             if (n > 0 && ni.path != kPathNodes) atomicAdd(&hdr->direct, 1u);
-            s_work[i] = work;
             plan->img[i] = ni;
         }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long w = 0;
-        for (int i = 0; i < bp.n_images; ++i) {
-            plan->img[i].w0 = w;
-            w += s_work[i];
-        }
-        plan->total = w;
     }
 }
 
