@@ -126,6 +126,12 @@ class _Workspaces:
                 self._bufs[key] = buf
             return buf
 
+    def peek(self, device: torch.device, role: str) -> Optional[torch.Tensor]:
+        """The buffer of a role, if it has one."""
+        key = (device.index if device.index is not None else torch.cuda.current_device(), role)
+        with self._lock:
+            return self._bufs.get(key)
+
     def drop(self, device: torch.device, role: str):
         key = (device.index if device.index is not None else torch.cuda.current_device(), role)
         with self._lock:

@@ -52,6 +52,7 @@ class BatchPlan:
         self._autotune = autotune and config is None
         self._use_graph = graph
         self._graph = None
+        self._graph_ws = None  # weakly: the workspace that the graph was captured with
         self._role = f"plan{id(self)}"
         # a plan's workspace (up to half a gigabyte of node sums) goes with the plan
         weakref.finalize(self, _core.WORKSPACES.drop, self.device, self._role).atexit = False
@@ -84,6 +85,7 @@ class BatchPlan:
             with torch.cuda.graph(g, stream=s):
                 self._launch()
             self._graph = g
+            self._graph_ws = weakref.ref(_core.WORKSPACES.peek(self.device, self._role))
 
     def load(self, atoms=None, amplitudes=None):
         """Copy a new batch into the static buffers (stream-ordered)."""
@@ -97,13 +99,19 @@ class BatchPlan:
     def run(self, atoms=None, amplitudes=None) -> torch.Tensor:
         """Forward of the loaded (or given) batch; returns the static output tensor."""
         self.load(atoms, amplitudes)
+        if self._graph is not None:
+            ws = self._graph_ws()
+            if ws is None or ws is not _core.WORKSPACES.peek(self.device, self._role):
+                self._graph = None  # (the workspaces were released: its memory may be someone else's)
         self._prepare()
         if self._graph is not None:
             self._graph.replay()
         else:
             self._launch()
         # (the allocator may hand the workspace on only after this stream's work on it)
-        _core.WORKSPACES.get(0, self.device, self._role).record_stream(torch.cuda.current_stream(self.device))
+        ws = _core.WORKSPACES.peek(self.device, self._role)
+        if ws is not None:
+            ws.record_stream(torch.cuda.current_stream(self.device))
         return self.out
 
     def cta_times(self) -> np.ndarray:
