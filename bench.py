@@ -76,6 +76,9 @@ def phases(seed, n_img=N_IMG):
 # clocks
 # ---------------------------------------------------------------------------
 class ClockSampler:
+    """SM clock and throttle reasons every 20 ms; :meth:`summary` covers the samples between
+    :meth:`start` and :meth:`stop` (a timed region of a few ms: the first one after it)."""
+
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
               "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -83,25 +86,38 @@ class ClockSampler:
     def __init__(self, gpu_index):
         self.idx = gpu_index
         self.proc = None
-        self.lines = []
+        self.lines = []  # (arrival time, line)
+        self.span = (float("-inf"), float("inf"))
+        self._first = threading.Event()
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.idx), f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                 "-lms", "20"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self._t = threading.Thread(target=self._read, daemon=True)
             self._t.start()
+            self._first.wait(5)  # nvidia-smi takes longer to start than a few steps
         except (OSError, FileNotFoundError):
             self.proc = None
         return self
 
     def _read(self):
         for line in self.proc.stdout:
-            self.lines.append(line.strip())
+            self.lines.append((time.perf_counter(), line.strip()))
+            self._first.set()
+
+    def start(self):
+        self.span = (time.perf_counter(), float("inf"))
+
+    def stop(self):
+        self.span = (self.span[0], time.perf_counter())
 
     def __exit__(self, *exc):
         if self.proc is not None:
+            deadline = time.perf_counter() + 1
+            while not any(t >= self.span[0] for t, _ in self.lines) and time.perf_counter() < deadline:
+                time.sleep(0.005)
             self.proc.terminate()
             try:
                 self.proc.wait(timeout=5)
@@ -111,7 +127,8 @@ class ClockSampler:
     def summary(self):
         sm, mx, reasons = [], None, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ln in self.lines:
+        lines = [ln for t, ln in self.lines if self.span[0] <= t <= self.span[1]]
+        for ln in lines or [ln for t, ln in self.lines if t > self.span[1]][:1]:
             parts = [p.strip() for p in ln.split(",")]
             if len(parts) < 9:
                 continue
@@ -223,6 +240,7 @@ def summarize_targets(line, t):
     fp64 = line.get("fp64", {}).get("value")
     if fp64:
         out["c2_split_over_fp64"] = r4(t["c2_pairs_per_s"] / fp64)
+        out["c2_split_over_fp64_is"] = "split precision on nodes over the direct FP64 kernel"
     acc = line.get("accuracy_c2_vs_cpu_oracle")
     if acc:
         out["c2_err_vs_cpu_oracle"] = {"max_rel_masked": r4(acc["max_rel_masked"]),
@@ -383,13 +401,13 @@ def main():
     def step():
         _core.forward(atoms, offsets, geom, precision, nat.OUT_C128, out=out, config=cfg)
 
-    for _ in range(args.warmup):
-        flush.fill_(1)
-        step()
-    barrier(world)
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     with ClockSampler(local) as clk:
+        for _ in range(args.warmup):
+            flush.fill_(1)
+            step()
         barrier(world)
+        clk.start()
         t0 = torch.cuda.Event(enable_timing=True)
         t1 = torch.cuda.Event(enable_timing=True)
         t0.record()
@@ -400,6 +418,7 @@ def main():
             ev[i][1].record()
         t1.record()
         barrier(world)
+        clk.stop()
     total_ms = t0.elapsed_time(t1)
     kern_ms = [a.elapsed_time(b) for a, b in ev]
     total_ms = max_over_ranks(total_ms, world)
@@ -436,10 +455,10 @@ def main():
         "config": {"workload": WORKLOAD, "images": N_IMG, "emitters": N_EMIT, "detector": [NDET, NDET],
                    "settings": SETTINGS, "parallelism": f"images per rank, {world} rank(s)",
                    "l2": "flushed between steps (256 MiB write)", "kernel_shape": cfg},
-        # per step: extents and plan, cell counts, record prep, the three direct kernels (which
-        # return at once on this workload), and seven node kernels for each of six groups of
-        # images (clearing, sums, weights, two for the cells, two interpolations)
-        "gpu_launches": 48 * args.steps,
+        # per step: extents and plan, record prep, the three direct kernels (which return at once on
+        # this workload), and six node kernels for each of six groups of images (setup, sums,
+        # two for the cells, two interpolations)
+        "gpu_launches": 41 * args.steps,
         "clocks": clocks,
         "roofline": {"bound": "fp64", "achieved": achieved / 1e9, "peak": fp64_peak / 1e9,
                      "unit": "G FP64 operations/s (node sums)", "frac": achieved / fp64_peak,
@@ -621,7 +640,7 @@ def batched_leg(torch, dev, _core, nat):
     """256 images, emitter counts log-uniform in [1e3, 1e5], sphere radii
     uniform in [5, 25] nm, amplitudes uniform in [0.5, 1.5] (float32),
     512x512 @ 75 um, 0.1 m, 6.4 keV, near field, split precision: one
-    persistent launch per batch, captured in a CUDA graph, shape autotuned."""
+    call per batch, captured in a CUDA graph, the direct kernels' shape autotuned."""
     from idi_b200.simulation.batch import BatchPlan
 
     g = np.random.Generator(np.random.Philox(33))
