@@ -9,10 +9,10 @@
 // detector, and the pixels follow by polynomial interpolation, two real
 // contractions in FP64: E = L_x V L_y^T.  Measured on a B200, whole calls: two
 // images of 50,000 emitters on 1024^2 pixels (66^2 nodes) 0.69 ms against 57.9 ms by
-// the direct kernels, 0.39 ms with the emitters cut into cells (below); eight of 2,000 on
-// 256^2 0.25 against 0.80 ms; field error against FP64 1.0e-7 against 2.1e-7.  The adjoint runs the transpose: the
-// pixel weights are contracted onto the nodes, and the adjoint sum runs over
-// nodes in place of pixels.
+// the direct kernels, 0.35 ms with the emitters cut into cells (below); eight of 2,000 on
+// 256^2 0.22 against 0.80 ms; field error against FP64 9e-8 against 2.1e-7.  The adjoint
+// runs the transpose: the pixel weights are contracted onto the nodes, and the adjoint
+// sum runs over nodes in place of pixels.
 //
 // Nodes per axis.  For phi linear in u, exp(i Phi t) on t in [-1, 1] has
 // Chebyshev coefficients 2 J_m(Phi): beyond m = Phi they fall
@@ -63,8 +63,8 @@ constexpr double kNodeMaxExtra = 0.06;
 // up with the phases of their centres.  The plan weighs the cells' sums, which shrink
 // with the cell, against the interpolation, which grows with their number.  Measured, with
 // cells against without (whole calls): 24 images of 1,000 to 100,000 emitters on 512^2
-// pixels 3.1 against 11.7 ms; 300,000 emitters in a micrometre on 128^2 pixels, which
-// undersample it, 1.20 against 3.30 ms (direct).
+// pixels 3.3 to 3.9 ms by card against 11.7; 300,000 emitters in a micrometre on 128^2
+// pixels, which undersample it, 1.16 against 3.30 ms (direct).
 constexpr int kCellMax = 512;        // cells per image
 constexpr int kCellNodes = 64;       // nodes per axis of a cell's grid
 constexpr int kCellMinEmitters = 4096;  // images below this are not cut

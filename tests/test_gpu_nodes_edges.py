@@ -304,3 +304,28 @@ def test_fp64_objects_of_next_to_no_phase(pixel, r, kr, settings):
     ref = oracle.wavefield(oracle.geometry(ndet, pixel, 1e5, kr / r), of, at)
     err = np.abs(E - ref).max() / np.abs(ref).max()
     assert err < 5e-15, err
+
+
+@pytest.mark.parametrize("n,r,ndet", [(10000, 0.015, [256, 256]), (20000, 0.01, [200, 201])])
+def test_gradients_of_small_residuals_of_cut_objects(n, r, ndet):
+    """Residuals 1e-2 of the intensities: their error is the intensities' (1.5e-9 here) a hundred times
+    over, beside the adjoint's own, pairs 1.2e-7 and FP32 sums over 512 nodes 3.8e-7; 4.3e-7 in
+    quadrature."""
+    g = rng(n)
+    pos, ph = sphere(g, n, r), g.uniform(0, 2 * np.pi, n)
+    at = torch.from_numpy(atoms(pos, ph)).cuda()
+    near = torch.from_numpy(atoms(pos + g.normal(0, 3e-6, pos.shape), ph)).cuda()
+    pixel = 75.0 * 512 / max(ndet)
+    geom = _core.make_geom(ndet, pixel, 1e5, K64)
+    none = torch.zeros([1] + ndet, dtype=torch.float64, device="cuda")
+    exact = _far_field_gradients(at, ndet, pixel, 1e5, none)[0].abs().square()
+    target = _far_field_gradients(near, ndet, pixel, 1e5, none)[0].abs().square()
+    assert float((exact - target).norm() / exact.norm()) < 2e-2
+    ref = _far_field_gradients(at, ndet, pixel, 1e5, 2 * (exact - target))[1]
+    E = _core.forward(at, [0, n], geom, nat.SPLIT, nat.OUT_C128)
+    assert _core.evaluated_pairs() < n * ndet[0] * ndet[1] / 2
+    ga, _ = _core.backward(at, [0, n], geom, E, (2 * (E.real ** 2 + E.imag ** 2 - target)).contiguous())
+    _core.backward_workspace_error()
+    for k in (slice(0, 3), slice(3, 4)):
+        err = float((ga[:, k] - ref[:, k]).norm() / ref[:, k].norm())
+        assert err < 5e-7, err
