@@ -823,10 +823,10 @@ __global__ void __launch_bounds__(256, (PPT <= 4 ? (PATH == kPathRuns ? 3 : 2) :
 // FINE (complex128 fields, which differentiation reads): the residuals of a fit are
 // differences of nearly equal intensities, and where the direct kernels' rounding errors
 // average out over the pixels, a node's error reaches all of them.  So the sine, cosine
-// and sums are FP64 polynomials and FP64 additions (a block of 64 emitters each):
-// intensities to 1e-9 of 64-bit ones instead of 9e-8, and gradients of such residuals
-// to 1e-7 instead of 1e-6 (7e-6 on the direct path).  36 cycles of the FP64 pipe per
-// pair of a warp; 1.5 times the FP32 form's time (24 uneven images 4.7 ms against 3.1),
+// and sums are FP64 polynomials and FP64 additions (a block of 64 emitters each), and cells
+// are turned in FP64 as well: intensities to 1.2e-9 of 64-bit ones instead of 9e-8, and
+// gradients of residuals a hundredth of them to 1.9e-7 instead of 1e-6 (7e-6 on the direct
+// path).  36 cycles of the FP64 pipe per pair of a warp; 1.5 times the FP32 form's time,
 // which the other outputs keep; the fit of 10,000 emitters on 512^2 pixels 0.98 ms either
 // way.
 
@@ -1163,9 +1163,11 @@ __global__ void __launch_bounds__(kNodeThreads, 6)
 // near field's pixel constant; the plain near field keeps the direct kernel, whose
 // |d - r| - d_z rounding is no smooth function of the pixel.  Shares, blocks and
 // fixed-point totals as in node_sum_kernel; a block's 64 emitters are added in FP64.
-// Four images of 2,000 emitters on 256^2 pixels (76^2 nodes): whole call 0.31 ms against
+// Four images of 2,000 emitters on 256^2 pixels (70^2 nodes): whole call 0.29 ms against
 // 2.87 ms, error against extended references 2.7e-15 against 1e-14 (sums without Kahan
-// steps, but a twelfth of the pairs and exact totals).
+// steps, but a thirteenth of the pairs and exact totals); of 20,000 and 50,000 emitters in
+// phase 1.7e-15 and 1.4e-15 of the field, where the direct kernel's compensated sums hold
+// 1.2e-15 and 1.0e-15, and less in the dark beside the peak.
 //
 // One 64-bit word counts in 2^-58 to 2^-59 of n max|a|, too coarse for FP64 where n is
 // large (1.3e-13 of the field of 1e6 emitters, the direct kernel 6e-15).  A second word takes
@@ -1450,11 +1452,14 @@ __global__ void __launch_bounds__(kGemmThreads, 4) cell_interp_kernel(const Geom
 // theta = the phase of the cell's centre at the target point.  A CTA takes an equal,
 // contiguous share of (image, target tile, cell), 32 x 32 targets each; the cells' tiles
 // are FP64 products (mma.m8n8k4, K in blocks of 16 by cp.async), turned by the
-// phase (FP64 turns, FP64 polynomials: every emitter of a cell shares the error of its turn, and
-// of a cell's emitters in phase that is far more than their sums' own) and added in registers; a
-// tile's total goes to the fixed-point sums by atomics.  How the shares cut a tile's cells depends on the batch, so
-// every cell's value is rounded to a grid (2^-50 of the largest possible sum) on which the
-// FP64 additions are exact in any order.
+// phase and added in registers; a tile's total goes to the fixed-point sums by atomics.
+//
+// The turn takes FP64 polynomials: every emitter of a cell shares its error, which for emitters
+// in phase is far more than their sums' own (dark pixels beside the peak of 50,000 fcc
+// sites: 3.1e-7 with FP32 ones, 9e-8 with these, 2.2e-7 by the direct kernels; two such images
+// 0.360 and 0.364 ms).  How the shares cut a tile's cells depends on the batch, so every
+// cell's value is rounded to a grid (2^-50 of the largest possible sum) on which the FP64
+// additions are exact in any order.
 constexpr int kExpTile = 32;
 struct ExpandSmem {
     double a[2][kExpTile * kGemmLd];

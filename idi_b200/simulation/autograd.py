@@ -6,7 +6,9 @@
     loss.backward()        # pos.grad, phase.grad, amplitudes.grad
 
 Forward and adjoint both run the split-precision kernels (FP64 phase in
-turns, FP32 sincos and sums).  Device-side errors of both (a near-field
+turns).  Images large enough for it are formed on nodes, the field with FP64
+sines and sums (intensities to 1e-9) and the adjoint with FP32 ones (gradients to
+2e-7); smaller ones directly, with FP32 sincos and sums.  Device-side errors of both (a near-field
 geometry outside the split range, emitters out of range) raise at the end of
 the backward pass.  ``pos`` (N,3) and ``phase`` (N,) are float64
 CUDA tensors; ``amplitudes`` (N,) float32/float64 or None.  Several images

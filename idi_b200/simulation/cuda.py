@@ -240,8 +240,8 @@ def _nchunks(out_bytes, Nimg):
 
 def _prefault(a):
     """Touch one byte per 4 KiB page of a fresh host array, so that the page
-    faults happen now (while the GPU computes) and not in the copy of the
-    last chunk, which nothing overlaps."""
+    faults happen here (while the first chunk is computed and copied) and not
+    in the copy of the last chunk, which nothing overlaps."""
     flat = a.reshape(-1).view(np.uint8)
     flat[::4096] = 0
 
@@ -313,7 +313,7 @@ def _pipelined(Nimg, simobject, N, Ndet, chunk, dev, geom, precision, out_kind, 
                 h_out[slot][:nb].copy_(src, non_blocking=True)
             ev_copied[slot].record(copy)
             if i == 0 and result is not None and Nimg > nb:
-                _prefault(result)  # overlaps the first chunk's kernels
+                _prefault(result)  # overlaps the first chunk's kernels and copy
             if pending is not None:
                 _collect(*pending)
             pending = (slot, done, nb)
