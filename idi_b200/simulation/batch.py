@@ -85,7 +85,8 @@ class BatchPlan:
             with torch.cuda.graph(g, stream=s):
                 self._launch()
             self._graph = g
-            self._graph_ws = weakref.ref(_core.WORKSPACES.peek(self.device, self._role))
+            ws = _core.WORKSPACES.peek(self.device, self._role)
+            self._graph_ws = weakref.ref(ws) if ws is not None else lambda: None  # (released meanwhile)
 
     def load(self, atoms=None, amplitudes=None):
         """Copy a new batch into the static buffers (stream-ordered)."""
