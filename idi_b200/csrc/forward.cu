@@ -1906,7 +1906,7 @@ NodeGeom make_node_geom(const GeomParams &g) {
         n.phi[a] = g.k * half / g.dmin;
         n.t[a] = half / g.dmin;
         n.least[a][0] = n.t[a] > 0 ? 20.0 / std::asinh(1.0 / n.t[a]) : 0.0;
-        n.least[a][1] = n.t[a] > 0 ? 1.0 + 35.0 / std::asinh((1.0 - kNodeMaxReach64) / n.t[a]) : 0.0;
+        n.least[a][1] = n.t[a] > 0 ? 1.0 + 35.0 / std::asinh((1.0 - kNodeMaxReach) / n.t[a]) : 0.0;
         // |d . e| over the detector, over a lower bound of |d|
         const double de = far[a] * len[a] + far[1 - a] * std::fabs(dot(c[1 - a], n.e[a])) +
                           std::fabs(g.detz * dot(c[2], n.e[a]));

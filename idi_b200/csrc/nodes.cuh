@@ -33,7 +33,7 @@
 // An object of next to no phase (Phi below 0.1) still has the near field's amplitude
 // 1/|d - r|, whose Chebyshev coefficients fall by rho = e^asinh((1 - r/D) / t) a node, the
 // singularity being D - r off the detector: no fewer than 20 / ln rho nodes (1e-8 of its
-// variation) or, for FP64, 1 + 35 / ln rho.  FP64 images reach to r = D / 20 (kNodeMaxReach64);
+// variation) or, for FP64, 1 + 35 / ln rho.  FP64 images reach to r = D / 4 (kNodeMaxReach);
 // split-precision ones of that amplitude stay far below it (kNfScaleRho2).
 #pragma once
 
@@ -44,7 +44,7 @@ namespace idiwf {
 constexpr int kPathNodes = 4;        // split_path() continued: nodes and interpolation
 constexpr int kNodeMax = 1024;       // nodes per axis
 constexpr double kNodeMaxT = 0.6;
-constexpr double kNodeMaxReach64 = 0.05;
+constexpr double kNodeMaxReach = 0.25;  // largest |r| / D
 constexpr int kNodeThreads = 128;    // node kernel: threads per CTA, nodes per thread, emitters per stage
 constexpr int kNodePPT = 2;
 constexpr int kNodeTile = kNodeThreads * kNodePPT;
@@ -160,7 +160,7 @@ __device__ __forceinline__ int node_count(double phi, double curve, double t, co
 
 // Whether an object reaching r from the origin may take nodes at all (a NaN may not).
 __device__ __forceinline__ bool node_reach(const GeomParams &g, const NodeGeom &ng, double r, bool fine) {
-    if (!ng.ok || !(r * ng.inv_d <= (fine ? kNodeMaxReach64 : 0.25))) return false;
+    if (!ng.ok || !(r * ng.inv_d <= kNodeMaxReach)) return false;
     return fine || !(g.flags & (IDIWF_NF | IDIWF_SECONDORDER)) || 0.5 * g.k * r * r * ng.inv_d <= kNodeMaxExtra;
 }
 // Nodes along both axes for emitters within rho of a centre, |rho . e| <= ex, ey along the

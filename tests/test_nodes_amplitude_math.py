@@ -12,12 +12,12 @@ ld = np.longdouble
 
 def count(phi, curve, t, fine):
     n = (max(phi + 5.0 + 9.6 * np.cbrt(phi) + 30.0 * t, 2 * (curve + 5.0 + 9.6 * np.cbrt(curve)),
-             1.0 + 35.0 / np.arcsinh(0.95 / t)) if fine else
+             1.0 + 35.0 / np.arcsinh(0.75 / t)) if fine else
          max(phi + 3.7 + 6.33 * np.cbrt(phi) + 14.0 * t, 20.0 / np.arcsinh(1.0 / t)))
     return (int(np.ceil(n)) + 1) // 2 * 2
 
 
-@pytest.mark.parametrize("fine,reach", [(True, 0.05), (True, 1e-3), (False, 3e-4)])
+@pytest.mark.parametrize("fine,reach", [(True, 0.25), (True, 0.05), (True, 1e-3), (False, 3e-4)])
 @pytest.mark.parametrize("t", [0.005, 0.05, 0.2, 0.4, 0.6])
 @pytest.mark.parametrize("phi", [1e-4, 0.01, 0.1, 0.4, 2.0, 30.0])
 def test_amplitude_interpolation(fine, reach, t, phi):
