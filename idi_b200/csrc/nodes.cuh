@@ -276,9 +276,10 @@ __device__ __forceinline__ double node_cost(double n, int nx, int ny, const Node
     return t + 100.0 * npix * (1.0 / 1.2e13);
 }
 
-// Plan of one launch, by one block: every image's path, grids and fixed-point scale; one warp per image, whose lanes try the ways to cut it.  The choice
-// depends on the image and the geometry alone, as split_path's does.  fine: the FP64
-// kernel's images (their direct path counts as kPathPixel).
+// Plan of one launch, by one block: every image's path, grids and fixed-point scale; one warp
+// per image, whose lanes try the ways to cut it.  The choice depends on the image and the
+// geometry alone, as split_path's does.  fine: the FP64 kernel's images (their direct path
+// counts as kPathPixel).
 __device__ inline void plan_nodes(const BatchParams &bp, const GeomParams &g, const NodeGeom &ng,
                                   const uint32_t *ext, bool fine, WsHeader *hdr, NodePlan *plan) {
     __threadfence();
